@@ -76,6 +76,8 @@ class TraceRecord(C.Structure):
 UNIT_FN = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p)
 BATCH_FN = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p)
 
+ALLOC_FN = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_size_t)
+
 TP = C.POINTER(Tensor)
 
 # name -> (restype, argtypes); every symbol include/b200_fattn.h declares.
@@ -92,6 +94,7 @@ SYMBOLS = {
     "b200_fattn_plan": (C.c_int, _OP_ARGS + [C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "b200_fattn_workspace_bytes": (C.c_int, _OP_ARGS + [C.POINTER(C.c_size_t)]),
     "b200_fattn_launch": (C.c_int, _OP_ARGS + [C.c_void_p, C.c_size_t, C.c_void_p]),
+    "b200_fattn_launch_alloc": (C.c_int, _OP_ARGS + [ALLOC_FN, C.c_void_p, C.c_void_p]),
     "b200_fattn_forward_host": (C.c_int, _OP_ARGS),
     "b200_host_arena_release": (None, []),
     "b200_fattn_launch_static": (C.c_int, _OP_ARGS + [C.c_void_p]),

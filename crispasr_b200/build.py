@@ -1,4 +1,5 @@
-"""Builds libb200_fattn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Builds libb200_fattn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and _torch_op.so, the
+torch-facing call path over its C-ABI, with the host compiler."""
 from __future__ import annotations
 
 import hashlib
@@ -10,12 +11,14 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200_fattn.so")
+TORCH_OP = os.path.join(HERE, "_torch_op.so")
 STAMP = LIB + ".srchash"   # hash of the sources and flags the library next to it was built from
 SOURCES = ["fattn_api.cu", "fattn_mma.cu", "fattn_tc5.cu", "kv_slab.cu", "relpos_table.cu", "segment_sched.cpp", "slice_batch.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-fvisibility=hidden,-Wall", "--expt-relaxed-constexpr",
 ]
+TORCH_OP_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall"]
 
 
 def _nvcc() -> str:
@@ -36,7 +39,7 @@ def source_hash() -> str:
     for path in files:
         h.update(os.path.basename(path).encode() + b"\0")
         h.update(open(path, "rb").read())
-    h.update(" ".join(NVCC_FLAGS + SOURCES).encode())
+    h.update(" ".join(NVCC_FLAGS + SOURCES + TORCH_OP_FLAGS).encode())
     return h.hexdigest()
 
 
@@ -49,7 +52,21 @@ def built_hash() -> str | None:
 
 
 def needs_build() -> bool:
-    return built_hash() != source_hash()
+    return built_hash() != source_hash() or not os.path.exists(TORCH_OP)
+
+
+def _torch_op_command() -> list[str]:
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(shutil.which(_nvcc()) or _nvcc()))
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    return (["g++", *TORCH_OP_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            + [x for d in include for x in ("-isystem", d)] + [os.path.join(CSRC, "torch_op.cpp"), "-o", TORCH_OP]
+            + ["-L", HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN", "-L", os.path.join(root, "lib"),
+               "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -79,6 +96,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed")
     link = [_nvcc(), "-shared", "-o", LIB, *objs, "-lcudart", "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)
+    subprocess.run(_torch_op_command(), check=True)
     with open(STAMP, "w") as f:
         f.write(source_hash() + "\n")
     return LIB

@@ -682,6 +682,20 @@ B200_API int b200_fattn_launch(const b200_tensor* q, const b200_tensor* k, const
     return do_launch(plan, workspace, workspace_bytes, (cudaStream_t)cuda_stream);
 }
 
+B200_API int b200_fattn_launch_alloc(const b200_tensor* q, const b200_tensor* k, const b200_tensor* v,
+                                     const b200_tensor* mask, const b200_tensor* dst, const b200_fattn_params* params,
+                                     const b200_fattn_ext* ext, b200_alloc_fn alloc, void* user, void* cuda_stream) {
+    if (!alloc) return B200_E_NULL;
+    Plan plan;
+    int rc = make_plan(q, k, v, mask, dst, params, ext, false, &plan);
+    if (rc != B200_OK) return rc;
+    DeviceInfo di;
+    if ((rc = device_info(&di))) return rc;
+    void* ws = nullptr;
+    if (plan.ws_bytes && !(ws = alloc(user, plan.ws_bytes))) return B200_E_WORKSPACE;
+    return do_launch(plan, ws, plan.ws_bytes, (cudaStream_t)cuda_stream);
+}
+
 B200_API int b200_fattn_forward_host(const b200_tensor* q, const b200_tensor* k, const b200_tensor* v,
                                      const b200_tensor* mask, const b200_tensor* dst,
                                      const b200_fattn_params* params, const b200_fattn_ext* ext) {

@@ -101,40 +101,29 @@ def workspace_bytes(q, k, v, mask=None, **kw) -> int:
     return n.value
 
 
+_OP = None
+
+
+def _native():
+    """The torch-facing call path (csrc/torch_op.cpp); raises if it has not been built, there is no fallback."""
+    global _OP
+    if _OP is None:
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        _lib()
+        from . import _torch_op
+        _OP = _torch_op
+    return _OP
+
+
 def flash_attn_ext(q, k, v, mask=None, *, out=None, workspace=None, stream=None, **kw):
     """Device tensors in, device tensor out; asynchronous on `stream` (default: torch's current stream).
     `workspace` (uint8 device tensor) is allocated here when the launch needs one and none is given."""
-    import torch
-    if not q.is_cuda:
-        raise ValueError("flash_attn_ext takes CUDA tensors; use flash_attn_ext_host for host buffers")
-    dst = out if out is not None else _dst_like(q)
-    c = _make(q, k, v, mask, dst, kw, abi.from_torch)
-    L = _lib()
-    n = C.c_size_t(0)
-    rc = L.b200_fattn_workspace_bytes(*c.args(), C.byref(n))
-    if rc:
-        raise _err(rc, "b200_fattn_workspace_bytes")
-    ws_ptr, ws_len = None, 0
-    if n.value:
-        if workspace is None or workspace.numel() < n.value:
-            workspace = torch.empty(n.value, dtype=torch.uint8, device=q.device)
-        ws_ptr, ws_len = workspace.data_ptr(), workspace.numel()
-    st = stream if stream is not None else torch.cuda.current_stream(q.device).cuda_stream
-    with torch.cuda.device(q.device):
-        rc = L.b200_fattn_launch(*c.args(), ws_ptr, ws_len, st)
-    if rc:
-        raise _err(rc, "b200_fattn_launch")
-    return dst
+    return (_OP or _native()).launch(q, k, v, mask, out, workspace, stream, kw)
 
 
 def flash_attn_ext_host(q, k, v, mask=None, *, out=None, **kw):
     """Host (CPU, ideally pinned) tensors in, host tensor out: H2D, compute, D2H inside one C call."""
-    dst = out if out is not None else _dst_like(q)
-    c = _make(q, k, v, mask, dst, kw, abi.from_torch)
-    rc = _lib().b200_fattn_forward_host(*c.args())
-    if rc:
-        raise _err(rc, "b200_fattn_forward_host")
-    return dst
+    return (_OP or _native()).forward_host(q, k, v, mask, out if out is not None else _dst_like(q), kw)
 
 
 class KvCache:
@@ -171,14 +160,7 @@ class KvCache:
 
     def append(self, layer, k_new, v_new, pos=None, pos0=0, stream=None):
         """k_new/v_new: float32 CUDA tensors (n_streams, n_kv, n_new, hd)."""
-        import torch
-        tk, tv = abi.from_torch(k_new), abi.from_torch(v_new)
-        st = stream if stream is not None else torch.cuda.current_stream(k_new.device).cuda_stream
-        rc = _lib().b200_kv_append(self._h, layer, C.byref(tk), C.byref(tv),
-                                   pos.data_ptr() if pos is not None else None, int(pos0), st)
-        if rc:
-            raise _err(rc, "b200_kv_append")
-
+        (_OP or _native()).kv_append(self._h.value or 0, layer, k_new, v_new, pos, pos0, stream)
 
     def copy_stream(self, dst_stream, src_stream, n_rows, stream=None):
         """Fork a hypothesis: rows [0, n_rows) of every layer/head from one stream to another (kv_snapshot_pool)."""

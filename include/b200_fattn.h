@@ -202,6 +202,18 @@ B200_API int b200_fattn_launch(const b200_tensor* q, const b200_tensor* k, const
                                void* workspace, size_t workspace_bytes, void* cuda_stream);
 
 /*
+ * b200_fattn_launch_alloc — b200_fattn_workspace_bytes and b200_fattn_launch in one call, for hosts with a device
+ * allocator of their own: the operands are validated and planned once, and `alloc` (called at most once, on the calling
+ * thread) returns 256-byte aligned device memory of at least `bytes` that stays valid for the work enqueued on
+ * `cuda_stream`, or NULL (the call then returns B200_E_WORKSPACE and has enqueued nothing).
+ */
+typedef void* (*b200_alloc_fn)(void* user, size_t bytes);
+B200_API int b200_fattn_launch_alloc(const b200_tensor* q, const b200_tensor* k, const b200_tensor* v,
+                                     const b200_tensor* mask, const b200_tensor* dst,
+                                     const b200_fattn_params* params, const b200_fattn_ext* ext,
+                                     b200_alloc_fn alloc, void* user, void* cuda_stream);
+
+/*
  * b200_fattn_forward_host — the same operator for callers that hold HOST
  * buffers, i.e. the ggml_backend_tensor_set -> graph_compute -> tensor_get
  * round trip of src/voxtral.cpp:1196-1223 in one call.  All `data` pointers
