@@ -222,3 +222,34 @@ def test_batched_scheduler_over_two_gpus_equals_one(b200, orc):
         torch.cuda.synchronize(dev)
         assert torch.equal(out.cpu(), ref_dev[first:first + out.shape[0]].cpu())
     s.close()
+
+
+@pytest.mark.parametrize("type_", [abi.F16, abi.Q8_0])
+@pytest.mark.parametrize("hd", [32, 64, 96, 128])
+@pytest.mark.parametrize("n_new", [1, 3, 17, 65])
+def test_append_row_shapes(b200, orc, type_, hd, n_new):
+    """Rows of one to four Q8_0 blocks (even and odd block counts: aligned and straddling words), one to several CTAs per
+    head, token-major strided sources, sources that are only 8-byte aligned; every byte of the slab is compared, the rows
+    around the appended ones included."""
+    rng = np.random.default_rng(100 * hd + n_new)
+    S, Hkv, ctx, p0 = 2, 3, 96, 5
+    kv = b200.KvCache(type_, hd, Hkv, n_layers=1, max_ctx=ctx, n_streams=S)
+    new = rng.standard_normal((2, S, n_new, Hkv, hd)).astype(np.float32)
+    tk = torch.from_numpy(new[0]).cuda().permute(0, 2, 1, 3)
+    flat = torch.zeros(new[1].size + 2, dtype=torch.float32, device="cuda")
+    flat[2:] = torch.from_numpy(new[1]).cuda().reshape(-1)
+    tv = flat[2:].reshape(S, n_new, Hkv, hd).permute(0, 2, 1, 3)   # base 8 bytes off a 16-byte boundary
+    assert tv.data_ptr() % 16 == 8
+    pos = torch.tensor([p0, ctx - 2], dtype=torch.int32, device="cuda")   # stream 1: rows beyond the cache are dropped
+    kv.append(0, tk, tv, pos=pos)
+    torch.cuda.synchronize()
+    for t, x in zip(kv.view(0, ctx), new):
+        raw = _read_slab(t, t.nb[3] * S).reshape(S, Hkv, ctx, t.nb[1])
+        want = np.zeros_like(raw)
+        rows = x.transpose(0, 2, 1, 3)
+        enc = orc.quantize_q8_0(rows) if type_ == abi.Q8_0 else rows.astype(np.float16).view(np.uint8)
+        want[0, :, p0:p0 + n_new] = enc[0]
+        n1 = min(2, n_new)
+        want[1, :, ctx - 2:ctx - 2 + n1] = enc[1][:, :n1]
+        assert np.array_equal(raw, want)
+    kv.close()
