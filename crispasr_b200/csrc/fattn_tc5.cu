@@ -170,6 +170,16 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
         : "memory");
 }
+// One lane of a converged warp.  The issuing warps run their loops with all lanes and put only the tensor instructions
+// behind this: descriptors and TMEM addresses of a warp-uniform loop live in uniform registers, which is where
+// tcgen05.mma reads them.  Behind `if (lane == 0)` the compiler cannot know the loop to be uniform and moves every operand
+// over per instruction; the issue chain between P and the next score tile is what the softmax warps wait for (64 windows
+// of the large encoder 1139 -> 956 us by this alone).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -286,62 +296,13 @@ __device__ __forceinline__ float row_max64(const uint32_t (&sreg)[2][32], int co
     return max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]);
 }
 
-// 64 score columns -> 32 packed f16x2 probabilities exp2(s*c - m); updates the running raw maximum and the
-// row sum (f16x2 partial sums of four pairs, widened to fp32).
-template <bool MASKED>
-__device__ __forceinline__ void softmax64(const uint32_t (&sreg)[2][32], uint32_t (&preg)[32], float c, float m_use,
-                                          int col0, int n_valid, float& mx_io, float& lsum_io) {
-    // Per pair of columns: one three-input max, one packed FMA, two MUFU, one packed add, one f16x2 convert.
-    float mx[8];
-    uint64_t ls[4] = {0ull, 0ull, 0ull, 0ull};   // four packed pairs of fp32 partial sums
-    const uint64_t c2 = pack2(c, c), nm2 = pack2(-m_use, -m_use);
-#pragma unroll
-    for (int i = 0; i < 8; i++) mx[i] = -INFINITY;
-#pragma unroll
-    for (int q2 = 0; q2 < 2; q2++) {
-        if (MASKED && col0 + q2 * 32 >= n_valid) {   // a 32-column chunk beyond the last key: P = 0 without the exponentials
-#pragma unroll
-            for (int i = 0; i < 16; i++) preg[q2 * 16 + i] = 0u;
-            continue;
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-            float s0 = __uint_as_float(sreg[q2][i]), s1 = __uint_as_float(sreg[q2][i + 1]);
-            if (MASKED) {
-                if (col0 + q2 * 32 + i >= n_valid) s0 = -INFINITY;
-                if (col0 + q2 * 32 + i + 1 >= n_valid) s1 = -INFINITY;
-            }
-            mx[(i >> 1) & 7] = max3(mx[(i >> 1) & 7], s0, s1);
-            float t0, t1;
-            unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
-            const float p0 = ex2(t0), p1 = ex2(t1);
-            ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
-            preg[q2 * 16 + (i >> 1)] = cvt_f16x2(p0, p1);
-        }
-    }
-    mx_io = max3(mx_io, max3(fmaxf(mx[0], mx[1]), mx[2], mx[3]), max3(fmaxf(mx[4], mx[5]), mx[6], mx[7]));
-    float l0, l1;
-    unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), l0, l1);
-    lsum_io += l0 + l1;
-}
-
-// One 32-column chunk of the same arithmetic with the accumulators kept by the caller (mx[8], ls[4] live across the
-// four chunks of a tile): lets the TMEM load of a later chunk run under the exponentials of an earlier one.
-template <bool MASKED>
-__device__ __forceinline__ void softmax32(const uint32_t (&sreg)[32], uint32_t* preg16, uint64_t c2, uint64_t nm2, int col0, int n_valid,
-                                          float (&mx)[8], uint64_t (&ls)[4]) {
-    if (MASKED && col0 >= n_valid) {
-#pragma unroll
-        for (int i = 0; i < 16; i++) preg16[i] = 0u;
-        return;
-    }
+// 32 score columns -> 16 packed f16x2 probabilities exp2(s*c - m).  Per pair of columns: one three-input maximum, one packed
+// FMA, two ex2, one packed add, one f16x2 convert.  The accumulators are kept by the caller (mx[8], ls[4] live across the
+// four chunks of a tile), which lets the TMEM load of a later chunk run under the exponentials of an earlier one.
+__device__ __forceinline__ void softmax32(const uint32_t (&sreg)[32], uint32_t* preg16, uint64_t c2, uint64_t nm2, float (&mx)[8], uint64_t (&ls)[4]) {
 #pragma unroll
     for (int i = 0; i < 32; i += 2) {
-        float s0 = __uint_as_float(sreg[i]), s1 = __uint_as_float(sreg[i + 1]);
-        if (MASKED) {
-            if (col0 + i >= n_valid) s0 = -INFINITY;
-            if (col0 + i + 1 >= n_valid) s1 = -INFINITY;
-        }
+        const float s0 = __uint_as_float(sreg[i]), s1 = __uint_as_float(sreg[i + 1]);
         mx[(i >> 1) & 7] = max3(mx[(i >> 1) & 7], s0, s1);
         float t0, t1;
         unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
@@ -531,18 +492,10 @@ __device__ __forceinline__ void store_o_rows_coalesced(float* stage, int lane, f
     }
 }
 
-// EARLY (head_dim 64 without explicit mask; A/B variants, both measured slower than EARLY = 0 and opt-in):
-//   1  a softmax thread pulls its whole 128-column score row into registers at the start of a tile and says so
-//      (s_read); the MMA thread issues S[j+1] right then instead of after P[j], so the next score tile is computed
-//      under the exponentials of the current one.  With 168 registers per thread the row spills: 0.6x.
-//   2  the score columns are released after the SECOND 64-column half is in registers (no extra registers); a half
-//      that outgrew the reference maximum is redone from registers and the other half's probabilities are scaled.
-//      The score MMAs and the P.V MMAs are issued from two warps on two schedulers, each refilling the K (V) slots
-//      its own MMAs free.  Tile period of a traced CTA about equal to EARLY = 0; whole launches 0.79x.
 // QMODE / OTMA: how the query tile comes in and the output tile goes out (see q_tma below).  Template parameters, not
 // run-time flags: every path compiled into one kernel costs the others (the raw F32 form behind a flag took 5 % off the
 // F16-Q encoder launches and 9 % off the T = 407 prefill).
-template <int HD, int NSTG, bool HASMASK, int EARLY = 0, int QMODE = 0, bool OTMA = false>
+template <int HD, int NSTG, bool HASMASK, int QMODE = 0, bool OTMA = false>
 __global__ void __launch_bounds__(kThreadsTc5, 2)
 fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQ,
@@ -563,8 +516,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     const uint32_t sBar = sV + NSTG * TILE_BYTES;  // 8-byte slots
     const uint32_t bar_k_full = sBar, bar_k_empty = sBar + 8 * NSTG, bar_v_full = sBar + 16 * NSTG,
                    bar_v_empty = sBar + 24 * NSTG, bar_s_full = sBar + 32 * NSTG, bar_p_ready = bar_s_full + 8,
-                   bar_o_done = bar_s_full + 16, bar_pv_done = bar_s_full + 24, bar_s_read = bar_s_full + 32,
-                   bar_s_drain = bar_s_full + 40, bar_q_full = bar_s_full + 48, bar_q_conv = bar_s_full + 56;
+                   bar_o_done = bar_s_full + 16, bar_pv_done = bar_s_full + 24, bar_q_full = bar_s_full + 32, bar_q_conv = bar_s_full + 40;
     uint8_t* misc = smem_gen + (1 + 2 * NSTG) * TILE_BYTES + 32 * NSTG + 64;
     // q_tma: 0 = the softmax warps load and convert the Q tile; 1 = F16 rows by one tensor copy into the operand tile;
     // 2 = F32 rows by tensor copies into stages that are not needed yet, converted from there by the softmax warps.
@@ -573,7 +525,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     // loop issues at a few tens of clocks per instruction (T = 407 GQA prefill with an F32 Q: 4807 -> 5034 streams/s).
     // head_dim 64 (the raw tile in the two V stages) measured 1459 against 1481 segments/s for the register pass on the
     // encoder and is not launched.
-    constexpr bool RAW_OK = QMODE == 2 && EARLY == 0 && ((HD == 64 && NSTG == 2) || (HD == 128 && NSTG == 1));
+    constexpr bool RAW_OK = QMODE == 2 && ((HD == 64 && NSTG == 2) || (HD == 128 && NSTG == 1));
     static_assert(QMODE != 2 || RAW_OK, "the raw form needs stages to park the tile in");
     constexpr int RAW_OFF = HD == 64 ? (1 + NSTG) * TILE_BYTES : TILE_BYTES;   // V stages / K stage onwards
     constexpr bool q_raw = RAW_OK;
@@ -636,8 +588,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         mbar_init(bar_p_ready, 4);   // one arrival per softmax warp
         mbar_init(bar_o_done, 1);
         mbar_init(bar_pv_done, 1);
-        mbar_init(bar_s_read, 4);    // one arrival per softmax warp
-        mbar_init(bar_s_drain, 1);
         mbar_init(bar_q_full, 1);
         mbar_init(bar_q_conv, 4);    // one arrival per softmax warp
         *s_abort = 0;
@@ -695,7 +645,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *s_tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
     if (tid == 0) TC5_TRACE(2, 60, 1);
     const uint32_t tmem_S = tmem_base;            // cols [0,128)
     const uint32_t tmem_P = SEP_P ? tmem_base + kTile + HD : tmem_base;  // f16x2: cols [192,256) (hd 64) or aliasing S [0,64)
@@ -723,7 +673,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         }
     }
 
-    if (EARLY != 2 && warp == 4) {
+    if (warp == 4) {
         // ================= TMA producer =================
         if (lane == 0) {
             bool ok = true;
@@ -775,35 +725,16 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                     for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_v_full + 8 * (j % NSTG), (j / NSTG) & 1); ++it) __nanosleep(256);
             }
         }
-    } else if (EARLY == 2 && warp == 4) {
-        // ================= K loader + score-MMA issuer (half-tile release variant) =================
-        // An issuing thread costs the other warps of its scheduler issue slots (60-80 clk per tcgen05 instruction), and
-        // a tile ends when the slowest softmax warp is done: the two products are issued from two schedulers, and each
-        // issuer refills the operand slots its own MMAs free (their completion lies a tile back: no real wait).
-        if (lane == 0) {
-            const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16);
+    } else if (warp == 5) {
+        // ================= MMA issuer =================
+        // Order: S[0]; then per tile j: (barriers of tile j+1 are awaited while the softmax of tile j runs)
+        // wait P[j] -> PV[j] -> S[j+1], back to back, so the softmax threads of the next tile wake as early
+        // as the tensor pipe allows.  S[j+1] overwrites the columns P[j] lives in; tcgen05.mma executes in
+        // issue order, so PV[j] has consumed P[j] before S[j+1] writes.
+        {
+            const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), v_lo = smem_desc_lo(sV, kPanelBytes);
             constexpr uint32_t desc_hi = smem_desc_hi(1024);
-            bool ok = true;
-            int issued_k = min(NSTG, n_tiles);
-            for (int j = 0; j < n_tiles && ok; j++) {   // S[j]
-                const int slot = j % NSTG, use = j / NSTG;
-                // K[j+1] goes into the slot S[j-1] read (NSTG = 2); the softmax warps are already working on that product
-                const int jn = j + NSTG - 1;
-                if (j > 0 && jn < n_tiles) {
-                    const int ns = jn % NSTG, nu = jn / NSTG;
-                    ok = mbar_wait(bar_k_empty + 8 * ns, (nu - 1) & 1, s_abort);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(bar_k_full + 8 * ns, TILE_BYTES);
-#pragma unroll
-                    for (int p = 0; p < PANELS; p++)
-                        tma_load_4d(sK + ns * TILE_BYTES + p * kPanelBytes, &tmK, bar_k_full + 8 * ns, p * 64, jn * kTile, hk, bk);
-                    issued_k = jn + 1;
-                }
-                ok = mbar_wait(bar_k_full + 8 * slot, use & 1, s_abort);
-                if (ok && j > 0) ok = mbar_wait(bar_s_read, (j - 1) & 1, s_abort);   // every softmax warp holds S[j-1] in registers
-                if (!ok) break;
-                if (j > 0) TC5_TRACE(1, j - 1, 0);
-                tc_fence_after();
+            auto issue_s = [&](int slot) {
                 const uint32_t kd = k_lo + slot * (TILE_BYTES >> 4);
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ks++) {
@@ -811,151 +742,60 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                     mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(kd + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
                 }
                 tc_commit(bar_s_full);
-                tc_commit(bar_k_empty + 8 * slot);
-                if (j > 0) TC5_TRACE(1, j - 1, 1);
-            }
-            if (!ok) {   // no score MMA and no K copy of this CTA may still be running when the CTA ends
-                tc_commit(bar_s_drain);
-                for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_s_drain, 0); ++it) __nanosleep(256);
-                for (int j = max(0, issued_k - NSTG); j < issued_k; j++)
-                    for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_k_full + 8 * (j % NSTG), (j / NSTG) & 1); ++it) __nanosleep(256);
-            }
-        }
-    } else if (EARLY == 2 && warp == 5) {
-        // ================= V loader + P.V-MMA issuer (half-tile release variant) =================
-        if (lane == 0) {
-            const uint32_t v_lo = smem_desc_lo(sV, kPanelBytes);
-            constexpr uint32_t desc_hi = smem_desc_hi(1024);
-            bool ok = true;
-            int issued_v = min(NSTG, n_tiles);
-            for (int j = 0; j < n_tiles && ok; j++) {
-                const int slot = j % NSTG, use = j / NSTG;
-                // V[j+1] goes into the slot P.V[j-1] read; that product was issued a tile ago
-                const int jn = j + NSTG - 1;
-                if (j > 0 && jn < n_tiles) {
-                    const int ns = jn % NSTG, nu = jn / NSTG;
-                    ok = mbar_wait(bar_v_empty + 8 * ns, (nu - 1) & 1, s_abort);
-                    if (!ok) break;
-                    mbar_arrive_expect_tx(bar_v_full + 8 * ns, TILE_BYTES);
-#pragma unroll
-                    for (int p = 0; p < PANELS; p++)
-                        tma_load_4d(sV + ns * TILE_BYTES + p * kPanelBytes, &tmV, bar_v_full + 8 * ns, p * 64, jn * kTile, hk, bk);
-                    issued_v = jn + 1;
-                }
-                ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
-                TC5_TRACE(1, j, 2);
-                if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
-                if (!ok) break;
-                TC5_TRACE(1, j, 3);
-                tc_fence_after();
-                const uint32_t vd = v_lo + slot * (TILE_BYTES >> 4);
-                mma_ts(tmem_O, tmem_P, desc64(vd, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
-#pragma unroll
-                for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(vd + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
-                tc_commit(bar_v_empty + 8 * slot);
-                tc_commit(bar_pv_done);
-                if (j + 1 == n_tiles) tc_commit(bar_o_done);
-                TC5_TRACE(1, j, 4);
-            }
-            if (!ok) {
-                tc_commit(bar_o_done);
-                for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
-                for (int j = max(0, issued_v - NSTG); j < issued_v; j++)
-                    for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_v_full + 8 * (j % NSTG), (j / NSTG) & 1); ++it) __nanosleep(256);
-            }
-        }
-    } else if (warp == 5) {
-        // ================= MMA issuer =================
-        // Order: S[0]; then per tile j: (barriers of tile j+1 are awaited while the softmax of tile j runs)
-        // wait P[j] -> PV[j] -> S[j+1], back to back, so the softmax threads of the next tile wake as early
-        // as the tensor pipe allows.  S[j+1] overwrites the columns P[j] lives in; tcgen05.mma executes in
-        // issue order, so PV[j] has consumed P[j] before S[j+1] writes.
-        if (lane == 0) {
-            const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), v_lo = smem_desc_lo(sV, kPanelBytes);
-            constexpr uint32_t desc_hi = smem_desc_hi(1024);
+            };
             bool ok = mbar_wait(bar_k_full, 0, s_abort);
             if (ok && q_tma) ok = mbar_wait(q_raw ? bar_q_conv : bar_q_full, 0, s_abort);
             if (ok) {
                 TC5_TRACE(1, 0, 0);
                 tc_fence_after();
-#pragma unroll
-                for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t off = (ks >> 2) * kPanelBytes + (ks & 3) * 32;
-                    mma_ss(tmem_S, smem_desc(sQ + off, 16, 1024), smem_desc(sK + off, 16, 1024), IDESC_S, ks > 0 ? 1u : 0u);
+                if (elect_one()) {
+                    issue_s(0);
+                    tc_commit(bar_k_empty);
                 }
-                tc_commit(bar_s_full);
-                tc_commit(bar_k_empty);
+                __syncwarp();
                 TC5_TRACE(1, 0, 1);
             }
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int slot = j % NSTG, use = j / NSTG;
                 const int nslot = (j + 1) % NSTG, nuse = (j + 1) / NSTG;
                 const bool more = j + 1 < n_tiles;
-                if (EARLY) {
-                    // the score columns are free once all four softmax warps hold tile j in registers
-                    if (more) ok = mbar_wait(bar_k_full + 8 * nslot, nuse & 1, s_abort);
-                    if (ok) ok = mbar_wait(bar_s_read, j & 1, s_abort);
-                    if (!ok) break;
-                    if (j > 0) TC5_TRACE(1, j, 0);
-                    if (more) {
-                        tc_fence_after();
-                        const uint32_t kd = k_lo + nslot * (TILE_BYTES >> 4);
-#pragma unroll
-                        for (int ks = 0; ks < HD / 16; ks++) {
-                            const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                            mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(kd + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
-                        }
-                        tc_commit(bar_s_full);
-                        tc_commit(bar_k_empty + 8 * nslot);
-                    }
-                    if (j > 0) TC5_TRACE(1, j, 1);
-                    ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
-                } else {
-                    ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
-                    if (ok && more) ok = mbar_wait(bar_k_full + 8 * nslot, nuse & 1, s_abort);
-                }
+                ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
+                if (ok && more) ok = mbar_wait(bar_k_full + 8 * nslot, nuse & 1, s_abort);
                 if (!ok) break;
                 TC5_TRACE(1, j, 2);
                 ok = mbar_wait(bar_p_ready, j & 1, s_abort);
                 if (!ok) break;
                 TC5_TRACE(1, j, 3);
                 tc_fence_after();
-                // Descriptors differ only in the low word (address in 16-byte units): one add per MMA.  The issuing
-                // thread's latency, about 50 clocks per MMA and 100 per commit, is what the softmax threads wait for.
-                auto issue_next_s = [&]() {
-                    const uint32_t kd = k_lo + nslot * (TILE_BYTES >> 4);
+                if (elect_one()) {
+                    // with P in its own columns the next S goes first: the softmax threads wake after 4 MMAs, not 12
+                    if (SEP_P && more) issue_s(nslot);
+                    const uint32_t vd = v_lo + slot * (TILE_BYTES >> 4);
+                    mma_ts(tmem_O, tmem_P, desc64(vd, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
 #pragma unroll
-                    for (int ks = 0; ks < HD / 16; ks++) {
-                        const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                        mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(kd + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
+                    for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(vd + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
+                    if (SEP_P) {
+                        if (more) tc_commit(bar_k_empty + 8 * nslot);   // after the P.V MMAs: off the softmax threads' critical path
+                        tc_commit(bar_v_empty + 8 * slot);
+                        tc_commit(bar_pv_done);
+                    } else {
+                        tc_commit(bar_v_empty + 8 * slot);
+                        if (more) {
+                            issue_s(nslot);
+                            tc_commit(bar_k_empty + 8 * nslot);
+                        }
                     }
-                    tc_commit(bar_s_full);
-                };
-                // with P in its own columns the next S goes first: the softmax threads wake after 4 MMAs, not 12
-                if (SEP_P && more && !EARLY) issue_next_s();
-                const uint32_t vd = v_lo + slot * (TILE_BYTES >> 4);
-                mma_ts(tmem_O, tmem_P, desc64(vd, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
-#pragma unroll
-                for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(vd + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
-                if (SEP_P) {
-                    if (more && !EARLY) tc_commit(bar_k_empty + 8 * nslot);   // after the P.V MMAs: off the softmax threads' critical path
-                    tc_commit(bar_v_empty + 8 * slot);
-                    tc_commit(bar_pv_done);
-                } else {
-                    tc_commit(bar_v_empty + 8 * slot);
-                    if (more) {
-                        issue_next_s();
-                        tc_commit(bar_k_empty + 8 * nslot);
-                    }
+                    if (!more) tc_commit(bar_o_done);
                 }
-                if (!more) tc_commit(bar_o_done);
+                __syncwarp();
                 TC5_TRACE(1, j, 4);
             }
-            if (!ok) {
+            if (!ok && lane == 0) {
                 // make sure no MMA of this CTA is still running before TMEM is released
                 tc_commit(bar_o_done);
                 for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
             }
+            __syncwarp();
         }
     } else {
         // ================= softmax / correction / epilogue =================
@@ -975,209 +815,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                                             (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3
                                       : nullptr;
         const float c_exp = HASMASK ? 1.0f : c;   // with a mask the scores are moved to the log2 domain by apply_mask64
-        if constexpr (EARLY == 1) {
-            const uint64_t c2 = pack2(c, c);
-            for (int j = 0; j < n_tiles; j++) {
-                ok = mbar_wait(bar_s_full, j & 1, s_abort);
-                if (!ok) break;
-                if (tid == 0) TC5_TRACE(0, j, 0);
-                tc_fence_after();
-                uint32_t s[4][32];
-#pragma unroll
-                for (int q4 = 0; q4 < 4; q4++) tmem_ld32(tmem_S + lane_base + q4 * 32, s[q4]);
-                tmem_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_s_read);   // the tile is in registers: its columns may be overwritten
-                if (tid == 0) TC5_TRACE(0, j, 3);
-                const int n_valid = kend - j * kTile;     // columns >= n_valid of this row are masked
-                const bool full = __all_sync(0xffffffffu, n_valid >= kTile);
-                if (j == 0) {
-                    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float x0 = (i < n_valid) ? __uint_as_float(s[0][i]) : -INFINITY;
-                        const float x1 = (i + 1 < n_valid) ? __uint_as_float(s[0][i + 1]) : -INFINITY;
-                        m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], x0, x1);
-                    }
-                    m_ref = max3(fmaxf(m4[0], m4[1]), m4[2], m4[3]) * c;
-                }
-                float lsum = 0.0f;
-                bool pv_waited = false;
-                for (int attempt = 0; attempt < 2; attempt++) {
-                    const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
-                    const uint64_t nm2 = pack2(-m_use, -m_use);
-                    uint64_t ls[4] = {0ull, 0ull, 0ull, 0ull};
-                    float mx[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) mx[i] = -INFINITY;
-#pragma unroll
-                    for (int q4 = 0; q4 < 4; q4++) {
-                        uint32_t preg[16];
-                        if (full) {
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const float s0 = __uint_as_float(s[q4][i]), s1 = __uint_as_float(s[q4][i + 1]);
-                                mx[(i >> 1) & 7] = max3(mx[(i >> 1) & 7], s0, s1);
-                                float t0, t1;
-                                unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
-                                const float p0 = ex2(t0), p1 = ex2(t1);
-                                ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
-                                preg[i >> 1] = cvt_f16x2(p0, p1);
-                            }
-                        } else if (q4 * 32 >= n_valid) {
-#pragma unroll
-                            for (int i = 0; i < 16; i++) preg[i] = 0u;
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                float s0 = __uint_as_float(s[q4][i]), s1 = __uint_as_float(s[q4][i + 1]);
-                                if (q4 * 32 + i >= n_valid) s0 = -INFINITY;
-                                if (q4 * 32 + i + 1 >= n_valid) s1 = -INFINITY;
-                                mx[(i >> 1) & 7] = max3(mx[(i >> 1) & 7], s0, s1);
-                                float t0, t1;
-                                unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
-                                const float p0 = ex2(t0), p1 = ex2(t1);   // -inf -> 0
-                                ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
-                                preg[i >> 1] = cvt_f16x2(p0, p1);
-                            }
-                        }
-                        if (q4 == 0 && j > 0 && !pv_waited) {
-                            // the first 32 probabilities are in registers: only now must P[j-1] have been consumed
-                            ok = mbar_wait(bar_pv_done, (j - 1) & 1, s_abort);
-                            tc_fence_after();
-                            pv_waited = true;
-                        }
-                        tmem_st16(tmem_P + lane_base + q4 * 16, preg);
-                    }
-                    if (!ok) break;
-                    {
-                        float l0, l1;
-                        unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), l0, l1);
-                        lsum = l0 + l1;
-                    }
-                    const float m_tile = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7])) * c;
-                    if (!__any_sync(0xffffffffu, m_tile > m_ref + kRescaleThreshold)) break;
-                    // some row of this warp outgrew its reference maximum: rescale O and l (O is at rest: pv_done was
-                    // awaited above), then redo P from the registers
-                    const float m_new = fmaxf(m_ref, m_tile);
-                    const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
-                    l_run *= alpha;
-                    if (j > 0) {
-                        tmem_wait_st();
-#pragma unroll
-                        for (int q4 = 0; q4 < HD / 32; q4++) {
-                            uint32_t oreg[32];
-                            tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-                            tmem_st32(tmem_O + lane_base + q4 * 32, oreg);
-                        }
-                    }
-                    m_ref = m_new;
-                }
-                if (!ok) break;
-                l_run += lsum;
-                if (tid == 0) TC5_TRACE(0, j, 1);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_p_ready);
-                if (tid == 0) TC5_TRACE(0, j, 2);
-            }
-        } else if constexpr (EARLY == 2) {
-            // Half-tile release: the score columns are handed back (s_read) as soon as the second 64-column half is in
-            // registers, so the tensor pipe computes S[j+1] under the exponentials of that half and the next tile's
-            // scores are waiting when this loop comes round.  Nothing is read from the score columns afterwards: a
-            // half that outgrew the reference maximum is redone from the registers it still sits in, and when that
-            // is the second half the first half's probabilities (finite: they passed their own check) are scaled.
-            for (int j = 0; j < n_tiles; j++) {
-                ok = mbar_wait(bar_s_full, j & 1, s_abort);
-                if (!ok) break;
-                if (tid == 0) TC5_TRACE(0, j, 0);
-                tc_fence_after();
-                const int n_valid = kend - j * kTile;  // columns >= n_valid of this row are masked
-                const bool full_tile = __all_sync(0xffffffffu, n_valid >= kTile);
-                uint32_t preg[2][32];
-                float lsum = 0.0f;
-                bool pv_waited = false;
-#pragma unroll
-                for (int hh = 0; hh < 2; hh++) {
-                    uint32_t sreg[2][32];
-                    tmem_ld32(tmem_S + lane_base + hh * 64, sreg[0]);
-                    tmem_ld32(tmem_S + lane_base + hh * 64 + 32, sreg[1]);
-                    tmem_wait_ld();
-                    if (hh == 1) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_s_read);
-                        if (lane == 0) TC5_TRACE(2, j, 2 + warp);
-                    }
-                    if (tid == 0) TC5_TRACE(0, j, 3 + 2 * hh);
-                    if (HASMASK) apply_mask64(sreg, mrow + (int64_t)(j * kTile + hh * 64) * 2, a.Lk - (j * kTile + hh * 64), c);
-                    if (j == 0 && hh == 0) m_ref = row_max64(sreg, 0, full_tile ? 2 * kTile : n_valid) * c_exp;
-                    for (int attempt = 0; attempt < 2; attempt++) {
-                        const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
-                        float mx = -INFINITY, ls = 0.0f;
-                        if (full_tile) softmax64<false>(sreg, preg[hh], c_exp, m_use, 0, 0, mx, ls);
-                        else softmax64<true>(sreg, preg[hh], c_exp, m_use, hh * 64, n_valid, mx, ls);
-                        const float m_tile = mx * c_exp;
-                        if (attempt == 1 || !__any_sync(0xffffffffu, m_tile > m_ref + kRescaleThreshold)) {
-                            lsum += ls;
-                            break;
-                        }
-                        if (j > 0 && !pv_waited) {  // O must be at rest: P.V of the previous tile has completed
-                            ok = mbar_wait(bar_pv_done, (j - 1) & 1, s_abort);
-                            if (!ok) break;
-                            tc_fence_after();
-                            pv_waited = true;
-                        }
-                        const float m_new = fmaxf(m_ref, m_tile);
-                        const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
-                        l_run *= alpha;
-                        lsum *= alpha;
-                        if (hh == 1) {
-                            const __half2 a2 = __float2half2_rn(alpha);
-#pragma unroll
-                            for (int i = 0; i < 32; i++) {
-                                const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&preg[0][i]), a2);
-                                preg[0][i] = *reinterpret_cast<const uint32_t*>(&v);
-                            }
-                        }
-                        if (j > 0) {
-#pragma unroll
-                            for (int q4 = 0; q4 < HD / 32; q4++) {
-                                uint32_t oreg[32];
-                                tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                                tmem_wait_ld();
-#pragma unroll
-                                for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-                                tmem_st32(tmem_O + lane_base + q4 * 32, oreg);
-                            }
-                        }
-                        m_ref = m_new;
-                    }
-                    if (!ok) break;
-                    if (tid == 0) TC5_TRACE(0, j, 4 + 2 * hh);
-                }
-                if (!ok) break;
-                l_run += lsum;
-                if (j > 0 && !pv_waited) {  // P[j-1] must have been consumed before P[j] overwrites it
-                    ok = mbar_wait(bar_pv_done, (j - 1) & 1, s_abort);
-                    if (!ok) break;
-                    tc_fence_after();
-                }
-                if (tid == 0) TC5_TRACE(0, j, 1);
-                tmem_st32(tmem_P + lane_base, preg[0]);
-                tmem_st32(tmem_P + lane_base + 32, preg[1]);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_p_ready);
-                if (tid == 0) TC5_TRACE(0, j, 2);
-            }
-        } else
         for (int j = 0; j < n_tiles; j++) {
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
@@ -1247,7 +884,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                             for (int i = 0; i < 32; i++)
                                 if (col0 + i >= n_valid) sx[i] = 0xFF800000u;
                         }
-                        softmax32<false>(sx, p16, c2, nm2, 0, 0, mx8, ls4);
+                        softmax32(sx, p16, c2, nm2, mx8, ls4);
                     };
                     tmem_ld32(tmem_S + lane_base, sA);
                     tmem_ld32(tmem_S + lane_base + 32, sB);
@@ -1274,15 +911,10 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                     if (SEP_P && hh == 1 && j > 0 && !pv_waited && !pv_probe) pv_probe = mbar_test(bar_pv_done, (j - 1) & 1);
                     tmem_wait_ld();
                     if (tid == 0) TC5_TRACE(0, j, 3 + 2 * hh);
-                    if constexpr (HASMASK) {
-                        uint4 mv[8];
-                        load_mask64(mv, mrow + (int64_t)(j * kTile + hh * 64) * 2, a.Lk - (j * kTile + hh * 64));
-                        if (full_tile) softmax64_masked<false>(sreg, mv, preg[hh], c, m_use, 0, 0, mx, lsum);
-                        else softmax64_masked<true>(sreg, mv, preg[hh], c, m_use, hh * 64, n_valid, mx, lsum);
-                    } else {
-                        if (full_tile) softmax64<false>(sreg, preg[hh], c_exp, m_use, 0, 0, mx, lsum);
-                        else softmax64<true>(sreg, preg[hh], c_exp, m_use, hh * 64, n_valid, mx, lsum);
-                    }
+                    uint4 mv[8];
+                    load_mask64(mv, mrow + (int64_t)(j * kTile + hh * 64) * 2, a.Lk - (j * kTile + hh * 64));
+                    if (full_tile) softmax64_masked<false>(sreg, mv, preg[hh], c, m_use, 0, 0, mx, lsum);
+                    else softmax64_masked<true>(sreg, mv, preg[hh], c, m_use, hh * 64, n_valid, mx, lsum);
                     if (tid == 0) TC5_TRACE(0, j, 4 + 2 * hh);
                 }
                 if (tid == 0 && attempt == 1) TC5_TRACE(0, j, 7);
@@ -1527,7 +1159,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *s_tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
     const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + 128, tmem_X = tmem_base + 256;
 
     if (warp == 8) {
@@ -1552,17 +1184,20 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         }
     } else if (warp == 9) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
             // X[j] = Q_v . [ring slot 0 | ring slot 1]^T as ONE N=256 MMA per k-step (A is fetched once instead of
             // twice).  Slot 0 holds half-block j for even j and half-block j+1 for odd j, so for odd j the two
             // 128-column halves of X come out swapped; the softmax threads account for that in their column base.
+            const uint32_t q_lo = smem_desc_lo(sQ, 16), qv_lo = smem_desc_lo(sQv, 16), k_lo = smem_desc_lo(sK, 16), r_lo = smem_desc_lo(sR, 16),
+                           v_lo = smem_desc_lo(sV, kPanelBytes);
+            constexpr uint32_t desc_hi = smem_desc_hi(1024);
             auto issue_x = [&](int j) {
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ks++) {
                     // per panel: rows 0..127 of the B operand are slot 0, rows 128..255 slot 1 (contiguous 32 KB)
-                    const uint32_t off = (ks >> 2) * kPanelBytes + (ks & 3) * 32;
-                    const uint32_t roff = (ks >> 2) * 2 * kPanelBytes + (ks & 3) * 32;
-                    mma_ss(tmem_X, smem_desc(sQv + off, 16, 1024), smem_desc(sR + roff, 16, 1024), IDESC_X, ks > 0 ? 1u : 0u);
+                    const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
+                    const uint32_t roff16 = (uint32_t)(((ks >> 2) * 2 * kPanelBytes + (ks & 3) * 32) >> 4);
+                    mma_ss(tmem_X, desc64(qv_lo + off16, desc_hi), desc64(r_lo + roff16, desc_hi), IDESC_X, ks > 0 ? 1u : 0u);
                 }
                 tc_commit(bar_x_full);
                 tc_commit(bar_r_empty + 8 * (j & 1));
@@ -1570,8 +1205,8 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             auto issue_s = [&]() {
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t off = (ks >> 2) * kPanelBytes + (ks & 3) * 32;
-                    mma_ss(tmem_S, smem_desc(sQ + off, 16, 1024), smem_desc(sK + off, 16, 1024), IDESC_S, ks > 0 ? 1u : 0u);
+                    const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
+                    mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(k_lo + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
                 }
                 tc_commit(bar_s_full);
                 tc_commit(bar_k_empty);
@@ -1580,8 +1215,11 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                       mbar_wait(bar_k_full, 0, s_abort);
             if (ok) {
                 tc_fence_after();
-                issue_x(0);
-                issue_s();
+                if (elect_one()) {
+                    issue_x(0);
+                    issue_s();
+                }
+                __syncwarp();
             }
             for (int j = 0; j < n_tiles && ok; j++) {
                 const bool more = j + 1 < n_tiles;
@@ -1592,7 +1230,8 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                     if (!ok) break;
                     TC5_TRACE(1, j, 0);
                     tc_fence_after();
-                    issue_x(j + 1);
+                    if (elect_one()) issue_x(j + 1);
+                    __syncwarp();
                     TC5_TRACE(1, j, 1);
                 }
                 ok = mbar_wait(bar_v_full, j & 1, s_abort);
@@ -1601,19 +1240,23 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 if (!ok) break;
                 TC5_TRACE(1, j, 2);
                 tc_fence_after();
+                if (elect_one()) {
+                    mma_ts(tmem_O, tmem_P, desc64(v_lo, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
 #pragma unroll
-                for (int ks = 0; ks < kTile / 16; ks++)
-                    mma_ts(tmem_O, tmem_P + ks * 8, smem_desc(sV + ks * 2048, kPanelBytes, 1024), IDESC_PV,
-                           (j > 0 || ks > 0) ? 1u : 0u);
-                tc_commit(bar_v_empty);
-                if (more) issue_s();
-                else tc_commit(bar_o_done);
+                    for (int ks = 1; ks < kTile / 16; ks++)
+                        mma_ts(tmem_O, tmem_P + ks * 8, desc64(v_lo + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
+                    tc_commit(bar_v_empty);
+                    if (more) issue_s();
+                    else tc_commit(bar_o_done);
+                }
+                __syncwarp();
                 TC5_TRACE(1, j, 3);
             }
-            if (!ok) {
+            if (!ok && lane == 0) {
                 tc_commit(bar_o_done);
                 for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
             }
+            __syncwarp();
         }
     } else {
         // ================= softmax / bias / epilogue: thread (r, ch) owns columns [64ch, 64ch+64) of row r ========
@@ -1842,13 +1485,13 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// K/V as a rank-4 F16 tensor [hd, Lk, Hkv, Bk] with the caller's byte strides; box = 64 x 128 x 1 x 1.
-bool encode_kv_map(CUtensorMap* m, const View& v, int hd, int Lk, int Hkv, int Bk) {
+// K/V as a rank-4 F16 tensor [hd, Lk, Hkv, Bk] with the caller's byte strides; box = 64 columns x `keys` rows x 1 x 1.
+bool encode_kv_map(CUtensorMap* m, const View& v, int hd, int Lk, int Hkv, int Bk, int keys = kTile) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)hd, (cuuint64_t)Lk, (cuuint64_t)Hkv, (cuuint64_t)Bk};
     const cuuint64_t strides[3] = {(cuuint64_t)v.nb1, (cuuint64_t)v.nb2, (cuuint64_t)v.nb3};
-    const cuuint32_t box[4] = {64, (cuuint32_t)kTile, 1, 1};
+    const cuuint32_t box[4] = {64, (cuuint32_t)keys, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<uint8_t*>(v.p), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1949,109 +1592,7 @@ cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStrea
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-#include "fattn_tc5_pair.cuh"
-#include "fattn_tc5_split.cuh"
-
-// B200_PREFILL_SPLIT=1 selects the split-row kernel (eight softmax warps, scores released at once) for head_dim 64
-// without explicit mask.
-bool split_enabled() {
-    static const bool on = [] {
-        const char* e = getenv("B200_PREFILL_SPLIT");
-        return e && e[0] == '1';
-    }();
-    return on;
-}
-
-bool split_supported(const FattnArgs& a) { return split_enabled() && a.hd == 64 && !a.has_mask && !a.relpos; }
-
-int launch_split(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
-    CUtensorMap tmK, tmV;
-    if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq)) {
-        snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V");
-        return B200_E_CUDA;
-    }
-    const size_t smem = 1024 + (size_t)5 * kPanelBytes + 64 + 72 + 8 + 2048 + 16;
-    dim3 grid((a.Tq * a.gqa + kTile - 1) / kTile, a.Hkv, a.B);
-    auto kern = fattn_prefill_tc5_split_kernel;
-    static bool smem_set[64] = {false};
-    cudaError_t e = set_smem_once(kern, smem, smem_set);
-    if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsSplit, smem, st, a, tmK, tmV);
-    if (e != cudaSuccess) {
-        snprintf(errbuf, errlen, "tcgen05 split-row prefill launch: %s", cudaGetErrorString(e));
-        return B200_E_CUDA;
-    }
-    return B200_OK;
-}
-
-// The paired-tile persistent kernel takes head_dim 64 without explicit mask and without causal bound.
-// B200_PREFILL_PAIR=1 selects it (the one-tile kernel is the default); B200_PREFILL_POLY=n (2..16) moves every n-th pair of
-// exponentials of the paired kernel to the FMA pipe (0 = none).
-int pair_mode() {
-    static const int mode = [] {
-        const char* e = getenv("B200_PREFILL_PAIR");
-        if (!(e && e[0] == '1')) return -1;   // opt-in while it measures slower than the one-tile kernel
-        const char* p = getenv("B200_PREFILL_POLY");
-        const int n = p ? atoi(p) : 0;
-        return (n == 2 || n == 3 || n == 4 || n == 8) ? n : 0;
-    }();
-    return mode;
-}
-
-bool pair_supported(const FattnArgs& a) {
-    return pair_mode() >= 0 && a.hd == 64 && !a.has_mask && !a.causal && !a.relpos;
-}
-
-int launch_pair(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
-    CUtensorMap tmK, tmV;
-    if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq)) {
-        snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V");
-        return B200_E_CUDA;
-    }
-    const int n_pairs = (a.Tq * a.gqa + 2 * kTile - 1) / (2 * kTile);
-    const int64_t n_items64 = (int64_t)n_pairs * a.Hkv * a.B;
-    if (n_items64 > INT32_MAX) return B200_E_LIMIT;
-    const int n_items = (int)n_items64;
-    static const int chunk_env = [] {   // B200_PAIR_CHUNK=n: items per CTA (default 4)
-        const char* e = getenv("B200_PAIR_CHUNK");
-        const int n = e ? atoi(e) : 0;
-        return n >= 1 && n <= 1024 ? n : 4;
-    }();
-    const int chunk = chunk_env;
-    static const int stagger = [] {   // B200_PAIR_STAGGER=clocks: delay of slot 1's first tile (default 1200)
-        const char* e = getenv("B200_PAIR_STAGGER");
-        const int n = e ? atoi(e) : -1;
-        return n >= 0 && n <= 100000 ? n : 1200;
-    }();
-    dim3 grid((n_items + chunk - 1) / chunk);
-    cudaError_t e;
-    auto go = [&](auto kern) {
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, kPairSmem, smem_set);
-        if (e == cudaSuccess) e = launch_pdl(kern, grid, kPairThreads, kPairSmem, st, a, tmK, tmV, n_pairs, n_items, chunk, stagger);
-    };
-    switch (pair_mode()) {
-        case 2: go(fattn_prefill_tc5_pair_kernel<2>); break;
-        case 3: go(fattn_prefill_tc5_pair_kernel<3>); break;
-        case 4: go(fattn_prefill_tc5_pair_kernel<4>); break;
-        case 8: go(fattn_prefill_tc5_pair_kernel<8>); break;
-        default: go(fattn_prefill_tc5_pair_kernel<0>); break;
-    }
-    if (e != cudaSuccess) {
-        snprintf(errbuf, errlen, "tcgen05 paired prefill launch: %s", cudaGetErrorString(e));
-        return B200_E_CUDA;
-    }
-    return B200_OK;
-}
-
-// B200_PREFILL_EARLY=1 or 2 selects an early-score order in the one-tile head_dim 64 kernel (A/B runs; off by default).
-int early_scores_mode() {
-    static const int mode = [] {
-        const char* e = getenv("B200_PREFILL_EARLY");   // 0 (default), 1 or 2: see the kernel's EARLY parameter
-        const int v = e ? atoi(e) : 0;
-        return (v == 1 || v == 2) ? v : 0;
-    }();
-    return mode;
-}
+#include "fattn_tc5_h64.cuh"
 
 // One instantiation per kernel: its own "shared-memory attribute raised" flags per device.
 template <auto Kern, typename... Args>
@@ -2060,6 +1601,39 @@ cudaError_t launch_inst(dim3 grid, size_t smem, cudaStream_t st, Args... args) {
     cudaError_t e = set_smem_once(Kern, smem, smem_set);
     if (e == cudaSuccess) e = launch_pdl(Kern, grid, kThreadsTc5, smem, st, args...);
     return e;
+}
+
+// Whether the query rows / the output rows of a launch can travel as boxes of [columns, heads of the group, tokens]: the
+// rows of a warp (32 packed rows) are then whole tokens.
+bool gqa_box(const FattnArgs& a) { return a.gqa >= 1 && a.gqa <= 32 && 32 % a.gqa == 0; }
+bool q_box_ok(const FattnArgs& a) {
+    return a.q.vec16 && gqa_box(a) && !a.bias_u && a.q.nb1 % 16 == 0 && a.q.nb2 % 16 == 0 && a.q.nb3 % 16 == 0 && a.q.nb1 > 0 && a.q.nb2 > 0 &&
+           a.q.nb3 > 0;
+}
+
+int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
+    CUtensorMap tmK, tmV;
+    if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys)) {
+        snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V");
+        return B200_E_CUDA;
+    }
+    CUtensorMap tmQ = tmK, tmO = tmK;
+    const bool q_tma = a.q.type == B200_TYPE_F16 && q_box_ok(a) && encode_q_map(&tmQ, a);
+    const bool o_tma = gqa_box(a) && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);
+    dim3 grid((a.Tq * a.gqa + kTile - 1) / kTile, a.Hkv, a.B);
+    auto go = [&](auto kern, bool (&smem_set)[64]) {
+        cudaError_t e = set_smem_once(kern, kH64Smem, smem_set);
+        if (e == cudaSuccess) e = launch_pdl(kern, grid, kH64Threads, kH64Smem, st, a, tmK, tmV, tmQ, tmO);
+        return e;
+    };
+    static bool set[4][64] = {};
+    const cudaError_t e = q_tma ? (o_tma ? go(fattn_prefill_tc5_h64_kernel<true, true>, set[0]) : go(fattn_prefill_tc5_h64_kernel<true, false>, set[1]))
+                                : (o_tma ? go(fattn_prefill_tc5_h64_kernel<false, true>, set[2]) : go(fattn_prefill_tc5_h64_kernel<false, false>, set[3]));
+    if (e != cudaSuccess) {
+        snprintf(errbuf, errlen, "tcgen05 prefill launch: %s", cudaGetErrorString(e));
+        return B200_E_CUDA;
+    }
+    return B200_OK;
 }
 
 template <int HD, int NSTG>
@@ -2072,31 +1646,13 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     }
     constexpr int TILE_BYTES = kPanelBytes * (HD / 64);
     const size_t smem = 1024 + (size_t)(1 + 2 * NSTG) * TILE_BYTES + 32 * NSTG + 64 + 8;
-    // F16 query rows, 16-byte aligned: the Q tile is one tensor copy (B200_PREFILL_QTMA=0: through registers)
-    static const bool q_tma_on = [] {
-        const char* e = getenv("B200_PREFILL_QTMA");
-        return !(e && e[0] == '0');
-    }();
     constexpr bool RAW_INST = HD == 128 && NSTG == 1;   // the raw F32 form exists (and pays) at head_dim 128 only
     CUtensorMap tmQ = tmK;
     int q_tma = 0;
-    const bool gqa_box = a.gqa >= 1 && a.gqa <= 32 && 32 % a.gqa == 0;   // a warp's 32 packed rows are whole tokens
-    const bool early = HD == 64 && !a.has_mask && early_scores_mode() != 0;   // the A/B variants move their tiles through the threads
-    if (q_tma_on && !early && a.q.type == B200_TYPE_F16 && a.q.vec16 && gqa_box && !a.bias_u &&
-        a.q.nb1 % 16 == 0 && a.q.nb2 % 16 == 0 && a.q.nb3 % 16 == 0 && a.q.nb1 > 0 && a.q.nb2 > 0 && a.q.nb3 > 0)
-        q_tma = encode_q_map(&tmQ, a) ? 1 : 0;
-    else if (q_tma_on && RAW_INST && a.q.type == B200_TYPE_F32 && a.q.vec16 && gqa_box && !a.bias_u &&
-             early_scores_mode() == 0 && a.q.nb1 % 16 == 0 && a.q.nb2 % 16 == 0 && a.q.nb3 % 16 == 0 && a.q.nb1 > 0 && a.q.nb2 > 0 &&
-             a.q.nb3 > 0)
-        q_tma = encode_q_map(&tmQ, a) ? 2 : 0;   // F32 rows: raw tile into stages not needed yet, converted from shared memory
-    // a warp's rows of the output are a box of dst, written by tensor stores (B200_PREFILL_OTMA=0: by the threads)
-    static const bool o_tma_on = [] {
-        const char* e = getenv("B200_PREFILL_OTMA");
-        return !(e && e[0] == '0');
-    }();
+    if (a.q.type == B200_TYPE_F16 && q_box_ok(a)) q_tma = encode_q_map(&tmQ, a) ? 1 : 0;
+    else if (RAW_INST && a.q.type == B200_TYPE_F32 && q_box_ok(a)) q_tma = encode_q_map(&tmQ, a) ? 2 : 0;   // F32 rows: raw tile into stages not needed yet, converted from shared memory
     CUtensorMap tmO = tmK;
-    int o_tma = 0;
-    if (o_tma_on && !early && gqa_box && (uintptr_t)a.dst % 16 == 0) o_tma = encode_o_map(&tmO, a) ? 1 : 0;
+    const bool o_tma = gqa_box(a) && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);   // a warp's rows of the output are a box of dst
     cudaError_t e;
     dim3 grid((a.Tq * a.gqa + kTile - 1) / kTile, a.Hkv, a.B);   // packed (query, group head) rows per KV head
     // launch_inst is instantiated per kernel (the kernels share one function-pointer type, so a generic lambda would
@@ -2104,18 +1660,15 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     auto args = [&](auto launch) { e = launch(grid, smem, st, a, tmK, tmV, tmQ, tmO); };
     constexpr int QRAW = RAW_INST ? 2 : 0;
 #define B200_GO(...) args(launch_inst<fattn_prefill_tc5_kernel<__VA_ARGS__>, FattnArgs, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap>)
-    if (HD == 64 && !a.has_mask && early_scores_mode() == 2) {
-        B200_GO(HD, NSTG, false, HD == 64 ? 2 : 0);
-    } else if (HD == 64 && !a.has_mask && early_scores_mode() == 1) {
-        B200_GO(HD, NSTG, false, HD == 64 ? 1 : 0);
-    } else if (a.has_mask) {
-        if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, true, 0, QRAW, true); else B200_GO(HD, NSTG, true, 0, QRAW, false); }
-        else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, true, 0, 1, true); else B200_GO(HD, NSTG, true, 0, 1, false); }
-        else { if (o_tma) B200_GO(HD, NSTG, true, 0, 0, true); else B200_GO(HD, NSTG, true, 0, 0, false); }
-    } else {
-        if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, false, 0, QRAW, true); else B200_GO(HD, NSTG, false, 0, QRAW, false); }
-        else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, false, 0, 1, true); else B200_GO(HD, NSTG, false, 0, 1, false); }
-        else { if (o_tma) B200_GO(HD, NSTG, false, 0, 0, true); else B200_GO(HD, NSTG, false, 0, 0, false); }
+    // head_dim 64 comes here with an explicit mask only
+    if (a.has_mask) {
+        if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, true, QRAW, true); else B200_GO(HD, NSTG, true, QRAW, false); }
+        else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, true, 1, true); else B200_GO(HD, NSTG, true, 1, false); }
+        else { if (o_tma) B200_GO(HD, NSTG, true, 0, true); else B200_GO(HD, NSTG, true, 0, false); }
+    } else if constexpr (HD == 128) {
+        if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, false, QRAW, true); else B200_GO(HD, NSTG, false, QRAW, false); }
+        else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, false, 1, true); else B200_GO(HD, NSTG, false, 1, false); }
+        else { if (o_tma) B200_GO(HD, NSTG, false, 0, true); else B200_GO(HD, NSTG, false, 0, false); }
     }
 #undef B200_GO
     if (e != cudaSuccess) {
@@ -2147,8 +1700,7 @@ bool tc5_supported(const FattnArgs& a) {
 
 int launch_prefill_tc5(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
     if (a.relpos) return launch_relpos(a, st, errbuf, errlen);
-    if (pair_supported(a)) return launch_pair(a, st, errbuf, errlen);
-    if (split_supported(a)) return launch_split(a, st, errbuf, errlen);
+    if (a.hd == 64 && !a.has_mask) return launch_h64(a, st, errbuf, errlen);
     if (a.hd == 64) return launch_t<64, 2>(a, st, errbuf, errlen);
     return launch_t<128, 1>(a, st, errbuf, errlen);
 }

@@ -1,0 +1,357 @@
+// fattn_tc5_h64.cuh — head_dim 64 prefill without an explicit mask: four CTAs per SM, 64 keys per step.
+//
+// The exponential unit bounds this path (16 ex2 per clock and SM: 1024 clk per 128 x 128 scores, against 512 clk of
+// tensor work at head_dim 64), so the layout serves one aim: that on every scheduler some softmax warp always has
+// exponentials to issue.  Between two score tiles a softmax warp waits for its own chain (P stored -> barrier -> the
+// issuing thread -> 8 MMAs -> barrier -> TMEM load, about 1 k clk); with two CTAs per SM and 128-key tiles the unit idled
+// 35-50 % of the time.  A 64-key tile needs 64 + 64 TMEM columns (P takes the score columns it came from), 48 KB of shared
+// memory and 96 registers for 160 threads: four CTAs fit, and a chain of one is covered by 3 x 512 clk of exponentials of
+// the other three.  The price is a score product with N = 64, whose A operand (the query tile) is read from shared memory
+// twice as often: 384 instead of 256 clk per 128 x 128 scores, still below the exponentials.
+//
+//   warps 0-3  softmax / epilogue: thread r owns query row r (TMEM lane r)
+//   warp  4    TMEM allocation; its lane 0 issues all tensor copies and all MMAs
+//   TMEM       [0,64) S, P as f16x2 in [0,32); [64,128) O
+// Per step j the issuing thread waits for P[j] (which also says that S[j] and, through the order of the tensor pipe,
+// P[j-1].V[j-1] are complete), issues P[j].V[j] and S[j+1], then refills the K slot of S[j] and the V slot of step j - 1:
+// no "slot empty" barriers exist.
+//
+// 64 windows of the large encoder (T = 1500): 1277 -> 917 us (577 -> 804 TFLOP/s, 0.56 of the sustained GEMM rate), at the
+// 1000 W limit (1.65 GHz; 1.9 GHz before): 1.2 k clk per 128 x 128 scores.
+constexpr int kH64Keys = 64;
+constexpr int kH64Threads = 160;
+constexpr int kH64KvBytes = kH64Keys * 128;   // one K or V tile
+constexpr size_t kH64Smem = 1024 + (size_t)kPanelBytes + 4 * kH64KvBytes + 8 * 8 + 16;
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// 2^t of a pair on the FMA pipe, t <= 14: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds and leaves n in the low
+// bits), a degree-4 minimax polynomial of 2^f (computed here by weighted least squares; relative error 2.6e-6, a hundredth
+// of the rounding of P to f16), the exponent added as an integer.  t below -126 gives 2^-126: 0 as f16.
+__device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p1) {
+    t0 = fmaxf(t0, -126.0f), t1 = fmaxf(t1, -126.0f);
+    const uint64_t magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f), neg1 = pack2(-1.0f, -1.0f);
+    const uint64_t x = pack2(t0, t1), r = add2(x, magic), n = add2(r, nmagic), f = fma2(n, neg1, x);
+    const float C0 = 0.9999992847442627f, C1 = 0.6931217908859253f, C2 = 0.240247443318367f, C3 = 0.05591785907745361f, C4 = 0.009570102207362652f;
+    uint64_t p = fma2(f, pack2(C4, C4), pack2(C3, C3));
+    p = fma2(p, f, pack2(C2, C2));
+    p = fma2(p, f, pack2(C1, C1));
+    p = fma2(p, f, pack2(C0, C0));
+    float a, b, ra, rb;
+    unpack2(p, a, b);
+    unpack2(r, ra, rb);
+    p0 = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
+    p1 = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
+}
+// Every eighth pair of exponentials goes to the FMA pipe: 64 windows of the large encoder 925 -> 917 us, 8 windows 132 ->
+// 127 us; every fourth pair costs more issue slots (and power) than the unit's time it frees (990 us).
+constexpr int kH64PolyEvery = 8;
+
+// QTMA: F16 query rows arrive by one tensor copy (else the softmax warps load and convert them); OTMA: the output leaves by
+// tensor stores (else by the threads).
+template <bool QTMA, bool OTMA>
+__global__ void __launch_bounds__(kH64Threads, 4)
+fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmO) {
+    constexpr int HD = 64;
+    constexpr uint32_t IDESC_S = idesc_f16(kH64Keys, false), IDESC_PV = idesc_f16(HD, true);
+    extern __shared__ uint8_t smem_dyn[];
+    const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    uint8_t* smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));
+    const uint32_t sQ = smem_base, sK = sQ + kPanelBytes, sV = sK + 2 * kH64KvBytes, sBar = sV + 2 * kH64KvBytes;
+    const uint32_t bar_k = sBar, bar_v = sBar + 16, bar_s_full = sBar + 32, bar_p_ready = sBar + 40, bar_o_done = sBar + 48, bar_q = sBar + 56;
+    uint8_t* misc = smem_gen + kPanelBytes + 4 * kH64KvBytes + 64;
+    volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // launched with programmatic stream serialisation
+    // tile order and GQA packing as in fattn_prefill_tc5_kernel
+    int q0 = blockIdx.x * kTile, hk = blockIdx.y, b = blockIdx.z;
+    if (a.causal) {
+        const int lin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), hb = gridDim.y * gridDim.z;
+        q0 = (gridDim.x - 1 - lin / hb) * kTile;
+        hk = (lin % hb) % gridDim.y, b = (lin % hb) / gridDim.y;
+    }
+    const int bk = b / a.bq;
+    const int rows_total = a.Tq * a.gqa;
+    const int tq_b = q_rows_of(a, b);
+    const int rows_live = tq_b * a.gqa;
+    int len_b = a.Lk;
+    if (a.kv_len) {
+        const int v = a.kv_len[b];
+        len_b = v < 0 ? 0 : (v > a.Lk ? a.Lk : v);
+    }
+    const int n_past = n_past_of(a, len_b, tq_b);
+    int kmax = q0 < rows_live ? len_b : 0;
+    if (a.causal) kmax = min(kmax, n_past + min((q0 + kTile - 1) / a.gqa + 1, tq_b));
+    const int n_tiles = kmax > 0 ? (kmax + kH64Keys - 1) / kH64Keys : 0;
+    if (n_tiles == 0) {  // nothing to attend to: zeros
+        if (tid < kTile && q0 + tid < rows_total) {
+            const int iq = (q0 + tid) / a.gqa, h = hk * a.gqa + (q0 + tid) % a.gqa;
+            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD);
+#pragma unroll
+            for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        return;
+    }
+
+    auto load_k = [&](int j) {
+        const uint32_t bar = bar_k + 8 * (j & 1);
+        mbar_arrive_expect_tx(bar, kH64KvBytes);
+        tma_load_4d(sK + (j & 1) * kH64KvBytes, &tmK, bar, 0, j * kH64Keys, hk, bk);
+    };
+    auto load_v = [&](int j) {
+        const uint32_t bar = bar_v + 8 * (j & 1);
+        mbar_arrive_expect_tx(bar, kH64KvBytes);
+        tma_load_4d(sV + (j & 1) * kH64KvBytes, &tmV, bar, 0, j * kH64Keys, hk, bk);
+    };
+    if (warp == 4) {
+        if (lane == 0) {
+            for (int i = 0; i < 8; i++) mbar_init(sBar + 8 * i, sBar + 8 * i == bar_p_ready ? 4 : 1);   // P: one arrival per softmax warp
+            *s_abort = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            if (QTMA) {
+                mbar_arrive_expect_tx(bar_q, kPanelBytes);
+                tma_load_4d(sQ, &tmQ, bar_q, 0, hk * a.gqa, q0 / a.gqa, b);
+            }
+            load_k(0);
+            load_v(0);
+            if (n_tiles > 1) load_k(1);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(s_tmem_base))),
+                     "r"(128u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else if (!QTMA) {
+        const int iq = (q0 + tid) / a.gqa, h = hk * a.gqa + (q0 + tid) % a.gqa;
+        const uint8_t* rowp = a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)h * a.q.nb2 + (int64_t)b * a.q.nb3;
+        if (a.q.type == B200_TYPE_F32 && a.q.vec16) load_q_rows_f32_coalesced<HD>(smem_gen, warp, lane, q0 + tid < rows_total ? rowp : nullptr);
+        else if (a.q.type == B200_TYPE_F16 && a.q.vec16) load_q_rows_f16_coalesced<HD>(smem_gen, warp, lane, q0 + tid < rows_total ? rowp : nullptr);
+        else load_q_row<HD>(smem_gen, tid, rowp, a.q.type, a.q.vec16 != 0, q0 + tid < rows_total);
+        fence_proxy_async();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
+    const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + 64;
+
+    if (warp == 4) {
+        // ================= copies and MMAs =================
+        {
+            const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), v_lo = smem_desc_lo(sV, kPanelBytes);
+            constexpr uint32_t desc_hi = smem_desc_hi(1024);
+            auto issue_s = [&](int j) {
+                const uint32_t kd = k_lo + (j & 1) * (kH64KvBytes >> 4);
+#pragma unroll
+                for (int ks = 0; ks < HD / 16; ks++)
+                    mma_ss(tmem_S, desc64(q_lo + ks * 2, desc_hi), desc64(kd + ks * 2, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
+                tc_commit(bar_s_full);
+            };
+            int k_issued = min(2, n_tiles), v_issued = 1;
+            bool ok = (!QTMA || mbar_wait(bar_q, 0, s_abort)) && mbar_wait(bar_k, 0, s_abort);
+            if (ok) {
+                tc_fence_after();
+                if (elect_one()) {
+                    issue_s(0);
+                    if (n_tiles > 1) load_v(1);
+                }
+                v_issued = min(2, n_tiles);
+            }
+            for (int j = 0; j < n_tiles && ok; j++) {
+                const bool more = j + 1 < n_tiles;
+                ok = mbar_wait(bar_v + 8 * (j & 1), (j >> 1) & 1, s_abort);
+                if (ok && more) ok = mbar_wait(bar_k + 8 * ((j + 1) & 1), ((j + 1) >> 1) & 1, s_abort);
+                if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t vd = v_lo + (j & 1) * (kH64KvBytes >> 4);
+                if (elect_one()) {
+                    mma_ts(tmem_O, tmem_P, desc64(vd, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
+#pragma unroll
+                    for (int ks = 1; ks < kH64Keys / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(vd + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
+                    if (more) issue_s(j + 1);
+                    else tc_commit(bar_o_done);
+                    if (j > 0 && more) load_v(j + 1);       // the slot of P[j-1].V[j-1]
+                    if (j + 2 < n_tiles) load_k(j + 2);   // the slot of S[j]
+                }
+                __syncwarp();
+                if (j > 0 && more) v_issued = j + 2;
+                if (j + 2 < n_tiles) k_issued = j + 3;
+            }
+            if (!ok && lane == 0) {
+                // no MMA and no copy of this CTA may still be running when its memory is released
+                tc_commit(bar_o_done);
+                for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
+                if (QTMA)
+                    for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_q, 0); ++it) __nanosleep(256);
+                for (int j = max(0, k_issued - 2); j < k_issued; j++)
+                    for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_k + 8 * (j & 1), (j >> 1) & 1); ++it) __nanosleep(256);
+                for (int j = max(0, v_issued - 2); j < v_issued; j++)
+                    for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_v + 8 * (j & 1), (j >> 1) & 1); ++it) __nanosleep(256);
+            }
+            __syncwarp();
+        }
+    } else {
+        // ================= softmax / epilogue =================
+        const int r = tid;
+        const bool row_live = q0 + r < rows_live;
+        const int iq_dst = (q0 + r) / a.gqa, h = hk * a.gqa + (q0 + r) % a.gqa;
+        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+        const float c = a.scale * kLog2e;
+        int kend = len_b;
+        if (a.causal) kend = min(kend, n_past + (row_live ? iq_dst : a.Tq) + 1);
+        float m_ref = -INFINITY, l_run = 0.0f;
+        const uint64_t c2 = pack2(c, c);
+        bool ok = true;
+        for (int j = 0; j < n_tiles; j++) {
+            ok = mbar_wait(bar_s_full, j & 1, s_abort);
+            if (!ok) break;
+            tc_fence_after();
+            const int n_valid = kend - j * kH64Keys;   // columns >= n_valid of this row are masked
+            const bool full_tile = __all_sync(0xffffffffu, n_valid >= kH64Keys);
+            if (j == 0) {   // a first reference maximum: that of the row's first 16 scores (the lazy check below corrects it)
+                uint32_t s0[16];
+                tmem_ld16(tmem_S + lane_base, s0);
+                tmem_wait_ld();
+                float mx = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < 16; i++) mx = fmaxf(mx, i < n_valid ? __uint_as_float(s0[i]) : -INFINITY);
+                m_ref = mx * c;
+            }
+            uint32_t preg[32];
+            float lsum = 0.0f;
+            // P = exp2(S*c - m_ref) against a reference maximum that need not be the maximum: what has to hold is that P
+            // stays inside f16, and the tile's row sum (needed anyway) bounds every P of the row.  No running maximum is
+            // kept - one instruction in six of this loop; only a row whose sum passes 2^12 has its tile's maximum taken,
+            // O and l rescaled and P redone (947 -> 925 us at 64 windows).
+            for (int attempt = 0; attempt < 2; attempt++) {
+                const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                uint64_t ls2[2] = {0ull, 0ull};
+                const uint64_t nm2 = pack2(-m_use, -m_use);
+                uint32_t sA[16], sB[16];
+                auto chunk = [&](uint32_t (&sx)[16], uint32_t* p8, int col0) {
+                    if (!full_tile) {
+                        if (__all_sync(0xffffffffu, col0 >= n_valid)) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) p8[i] = 0u;
+                            return;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; i++)
+                            if (col0 + i >= n_valid) sx[i] = 0xFF800000u;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const float s0 = __uint_as_float(sx[i]), s1 = __uint_as_float(sx[i + 1]);
+                        float t0, t1;
+                        unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
+                        float p0, p1;
+                        if ((i >> 1) % kH64PolyEvery == kH64PolyEvery - 1) poly_ex2(t0, t1, p0, p1);
+                        else p0 = ex2(t0), p1 = ex2(t1);
+                        ls2[(i >> 1) & 1] = add2(ls2[(i >> 1) & 1], pack2(p0, p1));
+                        p8[i >> 1] = cvt_f16x2(p0, p1);
+                    }
+                };
+                // rolling 16-column chunks: the TMEM load of chunk k+2 runs under the exponentials of chunk k+1
+                tmem_ld16(tmem_S + lane_base, sA);
+                tmem_ld16(tmem_S + lane_base + 16, sB);
+                tmem_wait_ld();
+                chunk(sA, preg, 0);
+                tmem_ld16(tmem_S + lane_base + 32, sA);
+                chunk(sB, preg + 8, 16);
+                tmem_wait_ld();
+                tmem_ld16(tmem_S + lane_base + 48, sB);
+                chunk(sA, preg + 16, 32);
+                tmem_wait_ld();
+                chunk(sB, preg + 24, 48);
+                float l0, l1;
+                unpack2(add2(ls2[0], ls2[1]), l0, l1);
+                lsum = l0 + l1;
+                if (!__any_sync(0xffffffffu, lsum > 4096.0f || (m_ref == -INFINITY && lsum > 0.0f))) break;
+                // O is at rest: the commit behind S[j] covers P[j-1].V[j-1]
+                float mx = -INFINITY;
+#pragma unroll
+                for (int q4 = 0; q4 < 4; q4++) {
+                    tmem_ld16(tmem_S + lane_base + q4 * 16, sA);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; i++) mx = fmaxf(mx, q4 * 16 + i < n_valid ? __uint_as_float(sA[i]) : -INFINITY);
+                }
+                const float m_new = fmaxf(m_ref, mx * c);
+                const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
+                l_run *= alpha;
+                if (j > 0) {
+#pragma unroll
+                    for (int q4 = 0; q4 < HD / 16; q4++) {
+                        uint32_t oreg[16];
+                        tmem_ld16(tmem_O + lane_base + q4 * 16, oreg);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
+                        tmem_st16(tmem_O + lane_base + q4 * 16, oreg);
+                    }
+                }
+                m_ref = m_new;
+            }
+            l_run += lsum;
+            tmem_st32(tmem_P + lane_base, preg);   // over the score columns: this warp has read its lanes of them
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_p_ready);
+        }
+        if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
+        if (ok) {
+            tc_fence_after();
+            // rows beyond the live ones are written as literal zeros, rows outside the tensor not at all; the K/V slots are
+            // free once the last MMA has completed: they stage O
+            const float inv = row_live && l_run > 0.0f ? 1.0f / l_run : 0.0f;
+            float* stage = reinterpret_cast<float*>(smem_gen + kPanelBytes) + warp * 32 * HD;
+#pragma unroll
+            for (int q4 = 0; q4 < HD / 32; q4++) {
+                uint32_t oreg[32];
+                tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 o = row_live ? make_float4(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv,
+                                                            __uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv)
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                    // OTMA: panels of 32 columns in the copy's own swizzle; else whole rows, chunks swizzled by the row
+                    if (OTMA) *reinterpret_cast<float4*>(stage + q4 * 32 * 32 + lane * 32 + (((i >> 2) ^ (lane & 7)) << 2)) = o;
+                    else *reinterpret_cast<float4*>(stage + lane * HD + ((((q4 * 32 + i) >> 2) ^ (lane & 7)) << 2)) = o;
+                }
+            }
+            if (OTMA) {
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0 && q0 + warp * 32 < rows_total) {
+#pragma unroll
+                    for (int q4 = 0; q4 < HD / 32; q4++)
+                        tma_store_4d(&tmO, smem_u32(stage + q4 * 32 * 32), q4 * 32, hk * a.gqa, (q0 + warp * 32) / a.gqa, b);
+                    tma_store_commit_and_wait_read();
+                }
+            } else {
+                float* out = q0 + r < rows_total ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.H + h) * HD : nullptr;
+                store_o_rows_coalesced<HD>(stage, lane, out);
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 4) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(128u) : "memory");
+    }
+}
