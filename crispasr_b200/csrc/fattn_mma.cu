@@ -2053,39 +2053,117 @@ int launch_decode_t(const FattnArgs& a, cudaStream_t st) {
     }
 }
 
-// K or V of any supported type / stride -> contiguous F16 [hd, Lk, Hkv, Bk] (the operand form of the tcgen05 kernels).
-// blockIdx.y selects the tensor: K and V of one call are converted by one launch.
-__global__ void kv_to_f16_kernel(const View src0, uint8_t* dst0, const View src1, uint8_t* dst1, int hd, int Lk, int Hkv, int Bk) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the attention kernel may start its set-up
+// K or V of any supported type / stride -> contiguous F16 [hd, Lk, Hkv, Bk] (the operand form of the tcgen05 kernels);
+// blockIdx.y selects the tensor: K and V of one call are converted by one launch.  hd is 64 or 128.
+// Bound by its bytes; the first form (a grid-stride loop over 8-element pieces with four 64-bit divisions each) was bound by
+// index arithmetic (F32 K/V of four Whisper windows, 92 MB: 18.2 us, now 13.5 against 14.3 of copy time; Q8_0 rows of a
+// T = 407 prefill, 20 MB: 9.3 -> 7.3 us, most of it start-up).  A CTA now owns rows of one (head, batch entry), a lane
+// 8 elements, the loads of four rows in flight.
+constexpr int kCastUnroll = 4;
+template <int TYPE, bool VEC16, int HD>
+__global__ void __launch_bounds__(256) kv_to_f16_kernel(const View src0, uint8_t* dst0, const View src1, uint8_t* dst1, int Lk, int Hkv, int chunks) {
+    // launched with programmatic stream serialisation: the attention kernel may start its set-up, and nothing is read
+    // before the previous kernel of the stream (a cache append) has completed
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int LPR = HD / 8, RPW = 32 / LPR;   // lanes per row, rows per warp instruction
     const View& src = blockIdx.y ? src1 : src0;
-    uint8_t* dst = blockIdx.y ? dst1 : dst0;
-    const int cpr = hd / 8;
-    const int64_t total = (int64_t)Bk * Hkv * Lk * cpr;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int ch = (int)(i % cpr);
-        const int64_t row = i / cpr;  // ((b*Hkv + h)*Lk + k)
-        const int k = (int)(row % Lk);
-        const int h = (int)((row / Lk) % Hkv);
-        const int b = (int)(row / ((int64_t)Lk * Hkv));
-        const uint8_t* rowp = src.p + (int64_t)k * src.nb1 + (int64_t)h * src.nb2 + (int64_t)b * src.nb3;
-        *reinterpret_cast<uint4*>(dst + (row * cpr + ch) * 16) = load8_as_half(rowp, src.type, ch * 8, hd, src.vec16 != 0);
+    const int hb = blockIdx.x / chunks, chunk = blockIdx.x - hb * chunks, b = hb / Hkv, h = hb - b * Hkv;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (lane % LPR) * 8;
+    const uint8_t* base = src.p + (int64_t)h * src.nb2 + (int64_t)b * src.nb3;
+    uint4* out = reinterpret_cast<uint4*>((blockIdx.y ? dst1 : dst0) + (int64_t)hb * Lk * HD * 2) + lane % LPR;
+    const int row0 = (chunk * 8 + warp) * RPW * kCastUnroll + lane / LPR;
+    if constexpr (TYPE == B200_TYPE_F32 && VEC16) {
+        float4 x[kCastUnroll][2];
+#pragma unroll
+        for (int u = 0; u < kCastUnroll; u++)
+            if (row0 + u * RPW < Lk) {
+                const float4* p = reinterpret_cast<const float4*>(base + (int64_t)(row0 + u * RPW) * src.nb1 + c * 4);
+                x[u][0] = __ldcs(p), x[u][1] = __ldcs(p + 1);
+            }
+#pragma unroll
+        for (int u = 0; u < kCastUnroll; u++)
+            if (row0 + u * RPW < Lk)
+                out[(int64_t)(row0 + u * RPW) * LPR] = make_uint4(pack_half2(x[u][0].x, x[u][0].y), pack_half2(x[u][0].z, x[u][0].w),
+                                                                  pack_half2(x[u][1].x, x[u][1].y), pack_half2(x[u][1].z, x[u][1].w));
+    } else if constexpr (TYPE == B200_TYPE_Q8_0 && VEC16) {   // rows on 4-byte boundaries (here: VEC16 stands for that)
+        // a lane's 8 quants start at byte 2 + 8i of their block: on a word boundary in odd blocks, two bytes off one in even
+        // blocks (34-byte blocks), where a third word and a shift by 16 bits make them up
+        const int blk = c >> 5, off = 34 * blk + (c & 31), odd = blk & 1;
+        uint32_t w[kCastUnroll][3];
+        uint16_t d[kCastUnroll];
+#pragma unroll
+        for (int u = 0; u < kCastUnroll; u++)
+            if (row0 + u * RPW < Lk) {
+                const uint8_t* rowp = base + (int64_t)(row0 + u * RPW) * src.nb1;
+                const uint32_t* p = reinterpret_cast<const uint32_t*>(rowp + off + 2 * odd);
+                w[u][0] = __ldg(p), w[u][1] = __ldg(p + 1);
+                w[u][2] = odd ? 0u : (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p + 2));
+                d[u] = __ldg(reinterpret_cast<const uint16_t*>(rowp + 34 * blk));
+            }
+        const uint32_t fs = odd ? 0u : 16u;
+        const __half2 bias = __float2half2_rn(1152.0f);
+#pragma unroll
+        for (int u = 0; u < kCastUnroll; u++)
+            if (row0 + u * RPW < Lk) {
+                const __half2 d2 = __half2half2(__ushort_as_half(d[u]));
+                uint32_t o[4];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t q = __funnelshift_r(w[u][k], w[u][k + 1], fs) ^ 0x80808080u;   // int8 -> biased uint8
+                    // halves 0x64xx = 1024 + xx; minus 1152 is the signed value exactly; times d rounds once
+                    const uint32_t h01 = __byte_perm(q, 0x64646464u, 0x4140), h23 = __byte_perm(q, 0x64646464u, 0x4342);
+                    const __half2 v01 = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&h01), bias), d2);
+                    const __half2 v23 = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&h23), bias), d2);
+                    o[2 * k] = *reinterpret_cast<const uint32_t*>(&v01), o[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&v23);
+                }
+                out[(int64_t)(row0 + u * RPW) * LPR] = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+    } else {   // unaligned rows
+#pragma unroll
+        for (int u = 0; u < kCastUnroll; u++)
+            if (row0 + u * RPW < Lk)
+                out[(int64_t)(row0 + u * RPW) * LPR] = load8_as_half(base + (int64_t)(row0 + u * RPW) * src.nb1, TYPE, c, HD, VEC16);
+    }
+}
+
+template <int TYPE, bool VEC16>
+cudaError_t launch_cast(const View& k, void* kdst, const View& v, void* vdst, int n, int hd, int Lk, int Hkv, int Bk, cudaStream_t st) {
+    const int rows = 8 * (256 / hd) * kCastUnroll, chunks = (Lk + rows - 1) / rows;   // rows per CTA
+    if ((int64_t)chunks * Hkv * Bk > INT32_MAX) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(chunks * Hkv * Bk), n);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return hd == 64 ? cudaLaunchKernelEx(&cfg, kv_to_f16_kernel<TYPE, VEC16, 64>, k, (uint8_t*)kdst, v, (uint8_t*)vdst, Lk, Hkv, chunks)
+                    : cudaLaunchKernelEx(&cfg, kv_to_f16_kernel<TYPE, VEC16, 128>, k, (uint8_t*)kdst, v, (uint8_t*)vdst, Lk, Hkv, chunks);
+}
+
+int launch_cast_any(const View& k, void* kdst, const View& v, void* vdst, int n, int hd, int Lk, int Hkv, int Bk, cudaStream_t st) {
+    auto words = [](const View& x) { return ((uintptr_t)x.p | (uintptr_t)x.nb1 | (uintptr_t)x.nb2 | (uintptr_t)x.nb3) % 4 == 0; };
+    switch (k.type) {   // K and V have one type
+        case B200_TYPE_F32: return (int)(k.vec16 && v.vec16 ? launch_cast<B200_TYPE_F32, true>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st)
+                                                            : launch_cast<B200_TYPE_F32, false>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st));
+        case B200_TYPE_Q8_0: return (int)(words(k) && words(v) ? launch_cast<B200_TYPE_Q8_0, true>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st)
+                                                               : launch_cast<B200_TYPE_Q8_0, false>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st));
+        default: return (int)(k.vec16 && v.vec16 ? launch_cast<B200_TYPE_F16, true>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st)
+                                                 : launch_cast<B200_TYPE_F16, false>(k, kdst, v, vdst, n, hd, Lk, Hkv, Bk, st));
     }
 }
 
 }  // namespace
 
 int launch_kv_to_f16(const View& src, void* dst, int hd, int Lk, int Hkv, int Bk, cudaStream_t st) {
-    const int64_t total = (int64_t)Bk * Hkv * Lk * (hd / 8);
-    const int blocks = (int)((total + 255) / 256 > 148 * 32 ? 148 * 32 : (total + 255) / 256);
-    kv_to_f16_kernel<<<dim3(blocks, 1), 256, 0, st>>>(src, (uint8_t*)dst, src, (uint8_t*)dst, hd, Lk, Hkv, Bk);
-    return (int)cudaGetLastError();
+    return launch_cast_any(src, dst, src, dst, 1, hd, Lk, Hkv, Bk, st);
 }
 
 int launch_kv_pair_to_f16(const View& k, void* kdst, const View& v, void* vdst, int hd, int Lk, int Hkv, int Bk, cudaStream_t st) {
-    const int64_t total = (int64_t)Bk * Hkv * Lk * (hd / 8);
-    const int blocks = (int)((total + 255) / 256 > 148 * 16 ? 148 * 16 : (total + 255) / 256);
-    kv_to_f16_kernel<<<dim3(blocks, 2), 256, 0, st>>>(k, (uint8_t*)kdst, v, (uint8_t*)vdst, hd, Lk, Hkv, Bk);
-    return (int)cudaGetLastError();
+    return launch_cast_any(k, kdst, v, vdst, 2, hd, Lk, Hkv, Bk, st);
 }
 
 int launch_tile_mma(const FattnArgs& a, cudaStream_t st) {

@@ -1037,6 +1037,81 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
 // MMA order: X[0] S[0] | per tile j: X[j+1] as soon as the softmax threads have drained X[j]; then, once
 // P[j] is in TMEM, PV[j] and S[j+1].
 // ------------------------------------------------------------------------------------------------------
+// 128-element query rows -> swizzled f16 operand tiles, 16 rows per warp, a warp instruction covers whole rows: lane l reads
+// float4 l of one F32 row, or 16 bytes l % 16 of two F16 rows; all loads in flight at once.  BIAS: two tiles from one read,
+// Q + bias_u and Q + bias_v, sums formed in fp32 and rounded once.  Rows at or beyond `rows` (of the tile) are zero.
+// (A thread per half row read 32 rows per instruction, 16 bytes each, and the biases element by element.)
+template <bool F16, bool BIAS>
+__device__ __forceinline__ void load_relpos_q(uint8_t* tile_u, uint8_t* tile_v, const uint8_t* base, int64_t nb1, int q0, int rows, const float* bias_u,
+                                              const float* bias_v, int warp, int lane) {
+    constexpr int N = F16 ? 8 : 4, RPI = F16 ? 2 : 1, K = 16 / RPI;   // elements per lane; rows per instruction; instructions
+    const int c = (F16 ? lane & 15 : lane) * N;
+    float bu[N], bv[N];
+    if (BIAS) {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(bias_u + c + i)), y = __ldg(reinterpret_cast<const float4*>(bias_v + c + i));
+            bu[i] = x.x, bu[i + 1] = x.y, bu[i + 2] = x.z, bu[i + 3] = x.w;
+            bv[i] = y.x, bv[i + 1] = y.y, bv[i + 2] = y.z, bv[i + 3] = y.w;
+        }
+    }
+    uint4 v[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int r = warp * 16 + k * RPI + (F16 ? lane >> 4 : 0);
+        v[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows) v[k] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)(q0 + r) * nb1 + c * (F16 ? 2 : 4)));
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int r = warp * 16 + k * RPI + (F16 ? lane >> 4 : 0);
+        const uint32_t off = (c >> 6) * kPanelBytes + r * 128 + ((((c & 63) >> 3) ^ (r & 7)) << 4) + (c & 4) * 2;
+        if (F16 && !BIAS) {
+            *reinterpret_cast<uint4*>(tile_u + off) = v[k];
+            continue;
+        }
+        float f[N];
+        const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (F16) {
+                const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+                f[(2 * i) % N] = p.x, f[(2 * i + 1) % N] = p.y;
+            } else {
+                f[i] = __uint_as_float(w[i]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < (BIAS ? 2 : 1); t++) {
+            uint32_t o[N / 2];
+#pragma unroll
+            for (int i = 0; i < N; i += 2) {
+                const float x = BIAS && r < rows ? __fadd_rn(f[i], t ? bv[i] : bu[i]) : f[i];
+                const float y = BIAS && r < rows ? __fadd_rn(f[i + 1], t ? bv[i + 1] : bu[i + 1]) : f[i + 1];
+                o[i >> 1] = pack_half2(x, y);
+            }
+            uint8_t* p = (t ? tile_v : tile_u) + off;
+            if constexpr (F16) *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2 % (N / 2)], o[3 % (N / 2)]);
+            else *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
+        }
+    }
+}
+
+// 32 bytes of one row per lane: whole sectors without a staging pass through shared memory (`wide`: 32-byte aligned rows).
+__device__ __forceinline__ void store8(float* p, const uint32_t* r, float f, bool wide) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]) * f;
+    if (wide) {
+        asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
+                     "f"(v[6]), "f"(v[7])
+                     : "memory");
+    } else {
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
 constexpr int kBncStride = 128;  // bytes per bounce row: a ring of 64 f16 values
 
 constexpr int kThreadsRelpos = 320;  // 8 softmax warps (two threads per query row), TMA warp, MMA warp
@@ -1069,6 +1144,21 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     const int q0 = blockIdx.x * kTile, h = blockIdx.y, b = blockIdx.z;
     const int hk = h / a.gqa, bk = b / a.bq;
     const int rb3 = a.r_ne3 > 1 ? b : 0;
+    if (tid == 8 * 32) {
+        for (int i = 0; i < 17; i++) {
+            const uint32_t bar = sBar + 8 * i;
+            mbar_init(bar, (bar == bar_x_free || bar == bar_p_ready) ? 8 : (bar >= bar_pair ? 64 : 1));   // 8 = one arrival per softmax warp
+        }
+        *s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
+    }
+    // launched with programmatic stream serialisation: nothing is read before the previous kernel has completed
+    if (tid == 0) TC5_TRACE(2, 60, 0);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid == 0) TC5_TRACE(2, 60, 1);
 
     int len_b = a.Lk;
     if (a.kv_len) {
@@ -1106,15 +1196,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
 
     // ---- set-up ----
     if (tid == 8 * 32) {
-        for (int i = 0; i < 17; i++) {
-            const uint32_t bar = sBar + 8 * i;
-            mbar_init(bar, (bar == bar_x_free || bar == bar_p_ready) ? 8 : (bar >= bar_pair ? 64 : 1));   // 8 = one arrival per softmax warp
-        }
-        *s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
         load_r(0);
         load_r(1);
         load_kv(0, false);
@@ -1127,39 +1208,45 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (warp < 8) {
-        // Q_u and Q_v tiles -> shared memory: thread (r, ch) converts and stores half of each row
-        const int r = tid & 127, ch = tid >> 7;
-        const int iq = q0 + r;
-#pragma unroll
-        for (int which = 0; which < 2; which++) {
-            const View& qv = which ? a.qv : a.q;
-            const uint8_t* rowp = qv.p + (int64_t)iq * qv.nb1 + (int64_t)h * qv.nb2 + (int64_t)b * qv.nb3;
-            const float* bias = which ? a.bias_v : a.bias_u;  // untied position biases folded into the load
-            uint4 v[HD / 16];
-            if (bias != nullptr) {
-#pragma unroll
+        // Q_u and Q_v tiles -> shared memory.  Aligned rows: warp w takes rows [16w, 16w + 16) whole (load_relpos_q); with
+        // the position biases folded in, one read of Q serves both tiles.  Otherwise thread (r, ch) moves half of row r.
+        const uint8_t* q_base = a.q.p + (int64_t)h * a.q.nb2 + (int64_t)b * a.q.nb3;
+        const uint8_t* qv_base = a.qv.p + (int64_t)h * a.qv.nb2 + (int64_t)b * a.qv.nb3;
+        const int rows = a.Tq - q0;
+        if (a.bias_u != nullptr && a.q.vec16 && ((reinterpret_cast<uintptr_t>(a.bias_u) | reinterpret_cast<uintptr_t>(a.bias_v)) & 15) == 0) {
+            if (a.q.type == B200_TYPE_F32) load_relpos_q<false, true>(smem_gen, smem_gen + TILE_BYTES, q_base, a.q.nb1, q0, rows, a.bias_u + h * HD, a.bias_v + h * HD, warp, lane);
+            else load_relpos_q<true, true>(smem_gen, smem_gen + TILE_BYTES, q_base, a.q.nb1, q0, rows, a.bias_u + h * HD, a.bias_v + h * HD, warp, lane);
+        } else if (a.bias_u == nullptr && a.q.vec16 && a.qv.vec16) {
+            if (a.q.type == B200_TYPE_F32) load_relpos_q<false, false>(smem_gen, nullptr, q_base, a.q.nb1, q0, rows, nullptr, nullptr, warp, lane);
+            else load_relpos_q<true, false>(smem_gen, nullptr, q_base, a.q.nb1, q0, rows, nullptr, nullptr, warp, lane);
+            if (a.qv.type == B200_TYPE_F32) load_relpos_q<false, false>(smem_gen + TILE_BYTES, nullptr, qv_base, a.qv.nb1, q0, rows, nullptr, nullptr, warp, lane);
+            else load_relpos_q<true, false>(smem_gen + TILE_BYTES, nullptr, qv_base, a.qv.nb1, q0, rows, nullptr, nullptr, warp, lane);
+        } else {
+            const int r = tid & 127, ch = tid >> 7;
+            const int iq = q0 + r;
+#pragma unroll 1
+            for (int which = 0; which < 2; which++) {
+                const View& qv = which ? a.qv : a.q;
+                const uint8_t* rowp = (which ? qv_base : q_base) + (int64_t)iq * qv.nb1;
+                const float* bias = which ? a.bias_v : a.bias_u;
+#pragma unroll 1
                 for (int c = 0; c < HD / 16; c++) {
-                    const int c0 = (ch * (HD / 16) + c) * 8;
-                    v[c] = (iq < a.Tq) ? load8_plus_bias_as_half(rowp, qv.type, c0, qv.vec16 != 0, bias + h * HD + c0)
-                                       : make_uint4(0u, 0u, 0u, 0u);
+                    const int cc = ch * (HD / 16) + c;
+                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                    if (iq < a.Tq) v = bias != nullptr ? load8_plus_bias_as_half(rowp, qv.type, cc * 8, qv.vec16 != 0, bias + h * HD + cc * 8)
+                                                       : q_chunk(rowp, qv.type, cc * 8, qv.vec16 != 0);
+                    *reinterpret_cast<uint4*>(smem_gen + which * TILE_BYTES + r * 128 + (cc >> 3) * kPanelBytes + (((cc & 7) ^ (r & 7)) << 4)) = v;
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < HD / 16; c++)
-                    v[c] = (iq < a.Tq) ? q_chunk(rowp, qv.type, (ch * (HD / 16) + c) * 8, qv.vec16 != 0) : make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int c = 0; c < HD / 16; c++) {
-                const int cc = ch * (HD / 16) + c;
-                *reinterpret_cast<uint4*>(smem_gen + which * TILE_BYTES + r * 128 + (cc >> 3) * kPanelBytes + (((cc & 7) ^ (r & 7)) << 4)) = v[c];
             }
         }
         fence_proxy_async();
+        if (tid == 0) TC5_TRACE(2, 60, 2);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
+    if (tid == 0) TC5_TRACE(2, 60, 3);
     const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + 128, tmem_X = tmem_base + 256;
 
     if (warp == 8) {
@@ -1434,30 +1521,31 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             if (tid == 0) TC5_TRACE(0, j, 4);
         }
         if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
+        if (tid == 0) TC5_TRACE(2, 60, 4);
         if (ok) {
             tc_fence_after();
             const float l_tot = l_run + exchange(l_run);   // a failed wait has set the abort flag: the host reports it
             const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
             float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD + ch * 64;
+            const bool wide = (reinterpret_cast<uintptr_t>(a.dst) & 31) == 0;
 #pragma unroll
             for (int q4 = 0; q4 < 2; q4++) {
                 uint32_t oreg[32];
                 tmem_ld32(tmem_O + lane_base + ch * 64 + q4 * 32, oreg);
                 tmem_wait_ld();
-                if (iq < tq_b) {
+                if (iq >= tq_b) {   // padding row of a batched launch: literal zeros
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(out + q4 * 32 + i) =
-                            make_float4(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv,
-                                        __uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv);
-                } else if (iq < a.Tq) {   // padding row of a batched launch: literal zeros
+                    for (int i = 0; i < 32; i++) oreg[i] = 0u;
+                }
+                if (iq < a.Tq) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(out + q4 * 32 + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i = 0; i < 32; i += 8) store8(out + q4 * 32 + i, oreg + i, inv, wide);
                 }
             }
         }
     }
 
+    if (tid == 0) TC5_TRACE(2, 60, 5);
     tc_fence_before();
     __syncthreads();
     if (warp == 9) {
@@ -1540,40 +1628,6 @@ bool encode_r_map(CUtensorMap* m, const FattnArgs& a) {
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
-    CUtensorMap tmK, tmV, tmR;
-    if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq) ||
-        !encode_r_map(&tmR, a)) {
-        snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V/R");
-        return B200_E_CUDA;
-    }
-    const size_t smem = 1024 + (size_t)6 * 2 * kPanelBytes + (size_t)2 * kTile * kBncStride + 136 + 8 + 2 * 128 * sizeof(float) + 16;
-    cudaError_t e;
-    dim3 grid((a.Tq + kTile - 1) / kTile, a.H, a.B);
-    if (a.has_mask) {
-        auto kern = fattn_prefill_tc5_relpos_kernel<true>;
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, smem, smem_set);
-        if (e == cudaSuccess) {
-            kern<<<grid, kThreadsRelpos, smem, st>>>(a, tmK, tmV, tmR);
-            e = cudaGetLastError();
-        }
-    } else {
-        auto kern = fattn_prefill_tc5_relpos_kernel<false>;
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, smem, smem_set);
-        if (e == cudaSuccess) {
-            kern<<<grid, kThreadsRelpos, smem, st>>>(a, tmK, tmV, tmR);
-            e = cudaGetLastError();
-        }
-    }
-    if (e != cudaSuccess) {
-        snprintf(errbuf, errlen, "tcgen05 rel-pos prefill launch: %s", cudaGetErrorString(e));
-        return B200_E_CUDA;
-    }
-    return B200_OK;
-}
-
 // Launch that may begin while the previous kernel of the stream drains, if that kernel allows it
 // (griddepcontrol.launch_dependents: the K/V conversion pre-pass does).  The kernels wait for the predecessor's
 // completion (griddepcontrol.wait) before they read anything it may have written.
@@ -1590,6 +1644,30 @@ cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStrea
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
+    CUtensorMap tmK, tmV, tmR;
+    if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq) ||
+        !encode_r_map(&tmR, a)) {
+        snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V/R");
+        return B200_E_CUDA;
+    }
+    const size_t smem = 1024 + (size_t)6 * 2 * kPanelBytes + (size_t)2 * kTile * kBncStride + 136 + 8 + 2 * 128 * sizeof(float) + 16;
+    cudaError_t e;
+    dim3 grid((a.Tq + kTile - 1) / kTile, a.H, a.B);
+    static bool set[2][64] = {};
+    auto go = [&](auto kern, bool (&smem_set)[64]) {
+        e = set_smem_once(kern, smem, smem_set);
+        if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsRelpos, smem, st, a, tmK, tmV, tmR);
+    };
+    if (a.has_mask) go(fattn_prefill_tc5_relpos_kernel<true>, set[0]);
+    else go(fattn_prefill_tc5_relpos_kernel<false>, set[1]);
+    if (e != cudaSuccess) {
+        snprintf(errbuf, errlen, "tcgen05 rel-pos prefill launch: %s", cudaGetErrorString(e));
+        return B200_E_CUDA;
+    }
+    return B200_OK;
 }
 
 #include "fattn_tc5_h64.cuh"
