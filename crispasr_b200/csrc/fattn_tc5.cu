@@ -195,6 +195,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -250,6 +258,25 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
+}
+
+// 2^t of a pair on the FMA pipe, t <= 14: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds and leaves n in the low
+// bits), a degree-4 minimax polynomial of 2^f (computed here by weighted least squares; relative error 2.6e-6, a hundredth
+// of the rounding of P to f16), the exponent added as an integer.  t below -126 gives 2^-126: 0 as f16.
+__device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p1) {
+    t0 = fmaxf(t0, -126.0f), t1 = fmaxf(t1, -126.0f);
+    const uint64_t magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f), neg1 = pack2(-1.0f, -1.0f);
+    const uint64_t x = pack2(t0, t1), r = add2(x, magic), n = add2(r, nmagic), f = fma2(n, neg1, x);
+    const float C0 = 0.9999992847442627f, C1 = 0.6931217908859253f, C2 = 0.240247443318367f, C3 = 0.05591785907745361f, C4 = 0.009570102207362652f;
+    uint64_t p = fma2(f, pack2(C4, C4), pack2(C3, C3));
+    p = fma2(p, f, pack2(C2, C2));
+    p = fma2(p, f, pack2(C1, C1));
+    p = fma2(p, f, pack2(C0, C0));
+    float a, b, ra, rb;
+    unpack2(p, a, b);
+    unpack2(r, ra, rb);
+    p0 = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
+    p1 = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
 }
 
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
@@ -1033,9 +1060,16 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
 // reference's rounding point), parks them in its own row of a shared-memory buffer and reads 64 of them
 // back from its row-dependent offset.  Only the thread itself touches its row: no barrier is involved.
 // Consecutive KV tiles share half of the band, so R arrives in 128-row half-blocks through a 2-slot ring
-// (half-block m = rows rb_0 + 128m ..; tile j uses half-blocks j and j+1).
-// MMA order: X[0] S[0] | per tile j: X[j+1] as soon as the softmax threads have drained X[j]; then, once
+// (half-block m = rows rb_0 + 128m ..; tile j uses half-blocks j and j+1), and so does X: the product of a half-block is
+// computed once, into the 128 columns that the half-block two before it leaves.
+// MMA order: X_0 X_1 S[0] | per tile j: X_(j+2) as soon as the softmax threads have drained tile j's columns; then, once
 // P[j] is in TMEM, PV[j] and S[j+1].
+//
+// What bounds it: the chain of one tile through the eight softmax warps (extraction of the bias 1.35 k clk, exponentials
+// 1.7 k, hand-offs 0.9 k = 4.0 k), against 1.5 k of MMA and 1.0 k of exponential unit; TMEM and shared memory are full,
+// there is no room for a second query tile.  2 recordings of 7500 frames: 985 -> 856 us (both products per band half, a
+// separate maximum pass, and the R copies queued behind the V copies cost the rest); 8 utterances of up to 138 frames 29 ->
+// 16 us, a mask over 3000 frames 209 -> 186 us (the query tile by whole rows: 7 k clk of a CTA's start).
 // ------------------------------------------------------------------------------------------------------
 // 128-element query rows -> swizzled f16 operand tiles, 16 rows per warp, a warp instruction covers whole rows: lane l reads
 // float4 l of one F32 row, or 16 bytes l % 16 of two F16 rows; all loads in flight at once.  BIAS: two tiles from one read,
@@ -1123,7 +1157,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     constexpr int HD = 128;
     constexpr int TILE_BYTES = 2 * kPanelBytes;  // 128 rows x 128 halves
     constexpr uint32_t IDESC_S = idesc_f16(kTile, false);
-    constexpr uint32_t IDESC_X = idesc_f16(2 * kTile, false);  // N = 256: the whole band in one instruction
     constexpr uint32_t IDESC_PV = idesc_f16(HD, true);
 
     extern __shared__ uint8_t smem_dyn[];
@@ -1253,11 +1286,16 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         // ================= TMA producer =================
         if (lane == 0) {
             bool ok = true;
+            // half-block m goes into the slot half-block m - 2 leaves when its product is complete
+            auto next_r = [&](int m) {
+                ok = mbar_wait(bar_r_empty + 8 * (m & 1), ((m >> 1) - 1) & 1, s_abort);
+                if (ok) load_r(m);
+                return ok;
+            };
+            if (n_tiles > 1) next_r(2);
             for (int j = 1; j < n_tiles && ok; j++) {
-                // half-block j+1 goes into the slot half-block j-1 leaves once X[j-1] has been computed
-                ok = mbar_wait(bar_r_empty + 8 * ((j + 1) & 1), (((j - 1) >> 1)) & 1, s_abort);
-                if (!ok) break;
-                load_r(j + 1);
+                // two tiles ahead: behind the copy of V[j - 1], which waits for a product of its own
+                if (j + 2 <= n_tiles && !next_r(j + 2)) break;
                 ok = mbar_wait(bar_k_empty, (j - 1) & 1, s_abort);
                 if (!ok) break;
                 load_kv(j, false);
@@ -1272,22 +1310,21 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     } else if (warp == 9) {
         // ================= MMA issuer =================
         {
-            // X[j] = Q_v . [ring slot 0 | ring slot 1]^T as ONE N=256 MMA per k-step (A is fetched once instead of
-            // twice).  Slot 0 holds half-block j for even j and half-block j+1 for odd j, so for odd j the two
-            // 128-column halves of X come out swapped; the softmax threads account for that in their column base.
+            // X_m = Q_v . R_m^T, the product of half-block m, lives in X columns [128 (m & 1), +128): tile j reads those of
+            // half-blocks j and j + 1, and only half-block j + 2 is new to tile j + 1.
             const uint32_t q_lo = smem_desc_lo(sQ, 16), qv_lo = smem_desc_lo(sQv, 16), k_lo = smem_desc_lo(sK, 16), r_lo = smem_desc_lo(sR, 16),
                            v_lo = smem_desc_lo(sV, kPanelBytes);
             constexpr uint32_t desc_hi = smem_desc_hi(1024);
-            auto issue_x = [&](int j) {
+            auto issue_x = [&](int m) {
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ks++) {
-                    // per panel: rows 0..127 of the B operand are slot 0, rows 128..255 slot 1 (contiguous 32 KB)
                     const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
                     const uint32_t roff16 = (uint32_t)(((ks >> 2) * 2 * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(tmem_X, desc64(qv_lo + off16, desc_hi), desc64(r_lo + roff16, desc_hi), IDESC_X, ks > 0 ? 1u : 0u);
+                    mma_ss(tmem_X + (m & 1) * kTile, desc64(qv_lo + off16, desc_hi), desc64(r_lo + (m & 1) * (kPanelBytes >> 4) + roff16, desc_hi), IDESC_S,
+                           ks > 0 ? 1u : 0u);
                 }
-                tc_commit(bar_x_full);
-                tc_commit(bar_r_empty + 8 * (j & 1));
+                if (m > 0) tc_commit(bar_x_full);   // (tile 0 needs half-blocks 0 and 1)
+                tc_commit(bar_r_empty + 8 * (m & 1));
             };
             auto issue_s = [&]() {
 #pragma unroll
@@ -1304,6 +1341,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 tc_fence_after();
                 if (elect_one()) {
                     issue_x(0);
+                    issue_x(1);
                     issue_s();
                 }
                 __syncwarp();
@@ -1311,13 +1349,13 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             for (int j = 0; j < n_tiles && ok; j++) {
                 const bool more = j + 1 < n_tiles;
                 if (more) {
-                    // X[j+1] needs half-block j+2 (slot j%2, its (j+2)/2-th use) and the X columns drained
+                    // half-block j+2 is in its slot, and the columns of half-block j have been read
                     ok = mbar_wait(bar_r_full + 8 * (j & 1), ((j + 2) >> 1) & 1, s_abort) &&
                          mbar_wait(bar_x_free, j & 1, s_abort);
                     if (!ok) break;
                     TC5_TRACE(1, j, 0);
                     tc_fence_after();
-                    if (elect_one()) issue_x(j + 1);
+                    if (elect_one()) issue_x(j + 2);
                     __syncwarp();
                     TC5_TRACE(1, j, 1);
                 }
@@ -1364,7 +1402,8 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         // loads of logical word (const - lane/2) by all 32 lanes, both hit 32 distinct banks (found by enumeration)
         const uint32_t rot = 4u * ((lane + 3u * (lane >> 3)) & 7u);
         const uint32_t x_col0 = 96 - 32 * (warp & 3) + 64 * ch;   // first X column this thread's warp can need
-        float m_ref = -INFINITY, l_run = 0.0f;
+        const uint64_t l2e2 = pack2(kLog2e, kLog2e), c2 = pack2(bscale * kLog2e, bscale * kLog2e);
+        float m_ref = -INFINITY, l_run = 0.0f, l_max = 0.0f;   // l_max: half-row sum that calls for a new reference
         bool ok = true;
         // Explicit F16 mask added on top of the bias (bucket padding of src/canary_ctc.cpp:370-382, the local-attention
         // window of src/core/fastconformer.h:887-895): this thread's row of [Lk, Tq, 1|H, 1|B];
@@ -1373,14 +1412,20 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                                             (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3
                                       : nullptr;
         // Publish a value, meet the partner warp at the pair barrier (bounded wait), read the partner's value.
-        // One slot per thread is enough: the partner's next write comes after its wait for the next S tile, which the
-        // tensor pipe only produces after the P*V product that needed this thread's later arrival on bar_p_ready.
-        auto exchange = [&](float mine) {
-            s_xchg[ch * 128 + r] = mine;
+        // One slot per thread is enough for the row sums: between two of them lies either an exchange of maxima or the wait
+        // for the next S tile, which the tensor pipe only produces after the P*V product that needed the partner's arrival
+        // on bar_p_ready (behind its read).  The maxima travel through the first word of the thread's own bounce ring, free
+        // between the extraction of the bias and the next tile; an exchange of sums always follows them.
+        auto exchange_at = [&](volatile float* mine, volatile float* theirs, float v) {
+            *mine = v;
             mbar_arrive(my_pair_bar);
             ok = mbar_wait(my_pair_bar, pair_phase, s_abort);
             pair_phase ^= 1;
-            return s_xchg[(ch ^ 1) * 128 + r];
+            return *theirs;
+        };
+        auto exchange = [&](float v) { return exchange_at(s_xchg + ch * 128 + r, s_xchg + (ch ^ 1) * 128 + r, v); };
+        auto exchange_max = [&](float v) {
+            return exchange_at(reinterpret_cast<volatile float*>(bnc_gen), reinterpret_cast<volatile float*>(smem_gen + (sBnc - smem_base) + (tid ^ 128) * kBncStride), v);
         };
         for (int j = 0; j < n_tiles; j++) {
             // ---- phase A: the 64 bias values of this half row, fp32 registers holding f16-rounded numbers ----
@@ -1388,7 +1433,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             if (!ok) break;
             if (tid == 0) TC5_TRACE(0, j, 0);
             tc_fence_after();
-            float u[2][32];
+            uint32_t bias2[32];   // the 64 bias values as packed pairs
             auto bounce_chunk = [&](const uint32_t (&xr)[32], int k) {
                 // scale*x rounded to f16 (the reference's cast of its mask), 32 values = 16 words, into ring half k&1
                 uint32_t w[16];
@@ -1409,20 +1454,17 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
 #pragma unroll
                 for (int p2 = 0; p2 < 16; p2++) {
                     const uint32_t next = *reinterpret_cast<const uint32_t*>(bnc_gen + ((((h0 >> 1) + p2 + 1 + rot) & 31) << 2));
-                    const uint32_t pk = __funnelshift_r(prev, next, fs);
-                    const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&pk));
-                    u[qq][2 * p2] = f2.x, u[qq][2 * p2 + 1] = f2.y;
+                    bias2[qq * 16 + p2] = __funnelshift_r(prev, next, fs);
                     prev = next;
                 }
             };
             {
-                const uint32_t xswap = (j & 1) ? 128u : 0u;  // odd tiles: the two 128-column halves of X are swapped
+                const uint32_t xswap = (j & 1) ? 128u : 0u;  // half-block j lives in columns 128 (j & 1) ..
                 uint32_t xa[3][32];
 #pragma unroll
                 for (int k = 0; k < 3; k++) tmem_ld32(tmem_X + lane_base + ((x_col0 + k * 32 + xswap) & 255u), xa[k]);
                 tmem_wait_ld();
-                // the X columns are free the moment every warp holds its 96 values in registers: X[j+1] is computed
-                // under the rest of this tile instead of after the extraction
+                // the columns of half-block j are free the moment every warp holds its 96 values in registers
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_x_free);
@@ -1433,87 +1475,116 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 read_quarter(1);
             }
             if (tid == 0) TC5_TRACE(0, j, 1);
-            uint4 mv[8];
-            if (HASMASK) load_mask64(mv, mrow + (int64_t)(j * kTile + ch * 64) * 2, a.Lk - (j * kTile + ch * 64));   // in flight during the wait for S
+            float u[HASMASK ? 64 : 1];   // with an explicit mask: bias + mask, in fp32
+            if constexpr (HASMASK) {
+                uint4 mv[8];
+                load_mask64(mv, mrow + (int64_t)(j * kTile + ch * 64) * 2, a.Lk - (j * kTile + ch * 64));
+#pragma unroll
+                for (int i = 0; i < 64; i += 2) {
+                    const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias2[i >> 1])), m2 = mask_pair(mv, i);
+                    u[i] = b2.x + m2.x, u[i + 1] = b2.y + m2.y;
+                }
+            }
 
-            // ---- phase B: u = S*scale + bias (natural units), row maximum ----
+            // ---- phase B: P = exp2(S*scale*log2(e) + bias*log2(e) - m_ref) ----
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
             if (tid == 0) TC5_TRACE(0, j, 2);
             tc_fence_after();
             const int n_valid = len_b - j * kTile;
             const bool full_tile = n_valid >= kTile;   // uniform over the CTA: only the last tile is partial
-            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            {
-                uint32_t sreg[2][32];
-                tmem_ld32(tmem_S + lane_base + ch * 64, sreg[0]);
-                tmem_ld32(tmem_S + lane_base + ch * 64 + 32, sreg[1]);
-                tmem_wait_ld();
+            // logits (log2 domain) of 16 columns, minus `m`
+            auto logits16 = [&](const uint32_t (&sx)[16], int q, uint64_t nm2, float (&x)[16]) {
 #pragma unroll
-                for (int q2 = 0; q2 < 2; q2++)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        float u0, u1;
-                        unpack2(fma2(pack2(__uint_as_float(sreg[q2][i]), __uint_as_float(sreg[q2][i + 1])), bscale2,
-                                     pack2(u[q2][i], u[q2][i + 1])), u0, u1);
-                        if (HASMASK) {
-                            const float2 m2 = mask_pair(mv, q2 * 32 + i);
-                            u0 += m2.x, u1 += m2.y;
-                        }
-                        if (!full_tile) {
-                            if (ch * 64 + q2 * 32 + i >= n_valid) u0 = -INFINITY;
-                            if (ch * 64 + q2 * 32 + i + 1 >= n_valid) u1 = -INFINITY;
-                        }
-                        u[q2][i] = u0, u[q2][i + 1] = u1;
-                        mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], u0, u1);
-                    }
-            }
-            if (tid == 0) TC5_TRACE(0, j, 3);
-            const float mx_half = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            // after this barrier both threads of the row have read their S columns: P stores may alias them
-            const float m_tile = fmaxf(mx_half, exchange(mx_half)) * kLog2e;
-            if (!ok) break;
-            // lazy rescale: O and l are only touched when a row outgrew its reference maximum by 2^8; both warps of a
-            // pair see the same row maxima and take the same branch
-            const bool grow = m_tile > m_ref + kRescaleThreshold;  // also true for -inf -> finite
-            if (__any_sync(0xffffffffu, grow)) {
-                const float m_new = fmaxf(m_ref, m_tile);
-                const float alpha = (m_ref == -INFINITY) ? 0.0f : ex2(m_ref - m_new);
-                l_run *= alpha;
-                if (j > 0) {
-#pragma unroll
-                    for (int q4 = 0; q4 < 2; q4++) {
-                        uint32_t oreg[32];
-                        tmem_ld32(tmem_O + lane_base + ch * 64 + q4 * 32, oreg);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-                        tmem_st32(tmem_O + lane_base + ch * 64 + q4 * 32, oreg);
+                for (int i = 0; i < 16; i += 2) {
+                    float2 b2;
+                    if constexpr (HASMASK) b2 = make_float2(u[q * 16 + i], u[q * 16 + i + 1]);
+                    else b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias2[q * 8 + (i >> 1)]));
+                    unpack2(fma2(pack2(__uint_as_float(sx[i]), __uint_as_float(sx[i + 1])), c2, fma2(pack2(b2.x, b2.y), l2e2, nm2)), x[i], x[i + 1]);
+                    if (!full_tile) {
+                        if (ch * 64 + q * 16 + i >= n_valid) x[i] = -INFINITY;
+                        if (ch * 64 + q * 16 + i + 1 >= n_valid) x[i + 1] = -INFINITY;
                     }
                 }
-                m_ref = m_new;
-            }
-            const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
-            // P = exp2(u*log2(e) - m_ref) from registers; masked columns hold -inf and give 0
-            uint64_t ls[4] = {0ull, 0ull, 0ull, 0ull};
-            const uint64_t l2e2 = pack2(kLog2e, kLog2e), nm2 = pack2(-m_use, -m_use);
+            };
+            // The reference need not be the maximum: P only has to stay inside f16, and the half-row sums (needed anyway)
+            // bound it.  The two threads of a row exchange them - the exchange also says that both have read their S columns,
+            // which the P stores overwrite - and only when one passes 2^12 (or in the first tile) is the row's maximum taken,
+            // O and l rescaled and P computed again.  Both warps of a pair see the same sums and take the same branch.
             uint32_t preg[32];
+            float lsum;
+            bool take_max = j == 0;
+#pragma unroll 1
+            for (;;) {
+                uint32_t sA[16], sB[16];
+                if (take_max) {
+                    float mx = -INFINITY;
+#pragma unroll 1
+                    for (int q = 0; q < 4; q++) {
+                        // (bias2 is indexed by a run-time q here: the four cases are spelled out)
+                        tmem_ld16(tmem_S + lane_base + ch * 64 + q * 16, sA);
+                        tmem_wait_ld();
+                        float x[16];
+                        if (q == 0) logits16(sA, 0, 0ull, x);
+                        else if (q == 1) logits16(sA, 1, 0ull, x);
+                        else if (q == 2) logits16(sA, 2, 0ull, x);
+                        else logits16(sA, 3, 0ull, x);
 #pragma unroll
-            for (int q2 = 0; q2 < 2; q2++)
+                        for (int i = 0; i < 16; i++) mx = fmaxf(mx, x[i]);
+                    }
+                    const float m_new = fmaxf(m_ref, fmaxf(mx, exchange_max(mx)));
+                    if (!ok) break;
+                    const float alpha = (m_ref == -INFINITY) ? 0.0f : ex2(m_ref - m_new);
+                    l_run *= alpha;
+                    if (j > 0) {
+#pragma unroll 1
+                        for (int q4 = 0; q4 < 4; q4++) {
+                            tmem_ld16(tmem_O + lane_base + ch * 64 + q4 * 16, sA);
+                            tmem_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    float t0, t1;
-                    unpack2(fma2(pack2(u[q2][i], u[q2][i + 1]), l2e2, nm2), t0, t1);
-                    const float p0 = ex2(t0), p1 = ex2(t1);
-                    ls[(i >> 1) & 3] = add2(ls[(i >> 1) & 3], pack2(p0, p1));
-                    preg[q2 * 16 + (i >> 1)] = cvt_f16x2(p0, p1);
+                            for (int i = 0; i < 16; i++) sA[i] = __float_as_uint(__uint_as_float(sA[i]) * alpha);
+                            tmem_st16(tmem_O + lane_base + ch * 64 + q4 * 16, sA);
+                        }
+                    }
+                    m_ref = m_new;
                 }
-            tmem_st32(tmem_P + lane_base + ch * 32, preg);
-            {
+                const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                const uint64_t nm2 = pack2(-m_use, -m_use);
+                uint64_t ls[2] = {0ull, 0ull};
+                auto chunk = [&](const uint32_t (&sx)[16], int q) {
+                    float x[16];
+                    logits16(sx, q, nm2, x);
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const float p0 = ex2(x[i]), p1 = ex2(x[i + 1]);
+                        ls[(i >> 1) & 1] = add2(ls[(i >> 1) & 1], pack2(p0, p1));
+                        preg[q * 8 + (i >> 1)] = cvt_f16x2(p0, p1);
+                    }
+                };
+                const uint32_t s_cols = tmem_S + lane_base + ch * 64;
+                tmem_ld16(s_cols, sA);
+                tmem_ld16(s_cols + 16, sB);
+                tmem_wait_ld();
+                chunk(sA, 0);
+                tmem_ld16(s_cols + 32, sA);
+                chunk(sB, 1);
+                tmem_wait_ld();
+                tmem_ld16(s_cols + 48, sB);
+                chunk(sA, 2);
+                tmem_wait_ld();
+                chunk(sB, 3);
                 float l0, l1;
-                unpack2(add2(add2(ls[0], ls[1]), add2(ls[2], ls[3])), l0, l1);
-                l_run += l0 + l1;
+                unpack2(add2(ls[0], ls[1]), l0, l1);
+                lsum = l0 + l1;
+                if (tid == 0) TC5_TRACE(0, j, 3);
+                const float other = exchange(lsum);
+                if (!ok || take_max || !__any_sync(0xffffffffu, fmaxf(lsum, other) > l_max)) break;
+                take_max = true;
             }
+            if (!ok) break;
+            l_max = m_ref == -INFINITY ? 0.0f : 4096.0f;
+            l_run += lsum;
+            tmem_st32(tmem_P + lane_base + ch * 32, preg);
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();

@@ -23,33 +23,6 @@ constexpr int kH64Threads = 160;
 constexpr int kH64KvBytes = kH64Keys * 128;   // one K or V tile
 constexpr size_t kH64Smem = 1024 + (size_t)kPanelBytes + 4 * kH64KvBytes + 8 * 8 + 16;
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-
-// 2^t of a pair on the FMA pipe, t <= 14: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds and leaves n in the low
-// bits), a degree-4 minimax polynomial of 2^f (computed here by weighted least squares; relative error 2.6e-6, a hundredth
-// of the rounding of P to f16), the exponent added as an integer.  t below -126 gives 2^-126: 0 as f16.
-__device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p1) {
-    t0 = fmaxf(t0, -126.0f), t1 = fmaxf(t1, -126.0f);
-    const uint64_t magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f), neg1 = pack2(-1.0f, -1.0f);
-    const uint64_t x = pack2(t0, t1), r = add2(x, magic), n = add2(r, nmagic), f = fma2(n, neg1, x);
-    const float C0 = 0.9999992847442627f, C1 = 0.6931217908859253f, C2 = 0.240247443318367f, C3 = 0.05591785907745361f, C4 = 0.009570102207362652f;
-    uint64_t p = fma2(f, pack2(C4, C4), pack2(C3, C3));
-    p = fma2(p, f, pack2(C2, C2));
-    p = fma2(p, f, pack2(C1, C1));
-    p = fma2(p, f, pack2(C0, C0));
-    float a, b, ra, rb;
-    unpack2(p, a, b);
-    unpack2(r, ra, rb);
-    p0 = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
-    p1 = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
-}
 // Every eighth pair of exponentials goes to the FMA pipe: 64 windows of the large encoder 925 -> 917 us, 8 windows 132 ->
 // 127 us; every fourth pair costs more issue slots (and power) than the unit's time it frees (990 us).
 constexpr int kH64PolyEvery = 8;
