@@ -39,6 +39,7 @@ struct FattnArgs {
     const float* bias_v;  // the same for the Q of the relative-position bias
     // split-KV
     int32_t n_splits;
+    int32_t wide;  // split-KV over a Q8_0 cache: eight warps per CTA instead of four
     float* ws_o;   // [B][Hkv][n_splits][16][hd]
     float* ws_ml;  // [B][Hkv][n_splits][16][2]
 };
@@ -130,7 +131,7 @@ int launch_kv_to_f16(const View& src, void* dst, int hd, int Lk, int Hkv, int Bk
 // K and V of one call in one launch.
 int launch_kv_pair_to_f16(const View& k, void* kdst, const View& v, void* vdst, int hd, int Lk, int Hkv, int Bk, cudaStream_t st);
 size_t decode_split_ws_bytes(int B, int Hkv, int n_splits, int hd);
-int decode_split_choose(const FattnArgs& a, int B, int sm_count);
+int decode_split_choose(FattnArgs& a, int B, int sm_count);
 void decode_split_force(int n_splits);  // 0 = automatic
 bool decode_cluster_merge_ok(const FattnArgs& a);
 // True when a launch with these arguments (n_splits set) merges its splits inside thread-block clusters: it then

@@ -518,6 +518,28 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
+// The first tiles of a decode CTA, asked for while the CTA waits for the previous kernel of the stream: a prefetch returns
+// nothing, and L2 is where that kernel's writes arrive too, so it needs no ordering.  The lengths and index lists that say
+// what to ask for may still change (they are read again after the wait); they are read past L1, which would keep the old
+// values.  Two tiles: the first copies after the wait then hit L2 (one segment of the large decoder 6.6 -> 6.2 us per
+// launch, four segments 9.2 -> 8.4, 16 segments 19.6 -> 19.0); eight tiles per CTA compete with the copies of the others
+// (32 segments +10 %).  Over a Q8_0 cache, whose copies a CTA starts with a few instructions, it measured nothing.
+constexpr int kPrefetchTiles = 2;
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ int32_t peek(const int32_t* p) {
+    int32_t v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+// Logical keys [lo, hi) of this CTA's first tiles, as far as they can be told before the wait.
+__device__ __forceinline__ void peek_range(const FattnArgs& a, int b, int split, int& lo, int& hi) {
+    const int cap = a.kv_index ? a.kv_index_stride : a.Lk;
+    const int len = a.kv_len ? min(max(peek(a.kv_len + b), 0), cap) : cap;
+    const int n_tiles = (len + kDecBN - 1) / kDecBN, tps = (n_tiles + a.n_splits - 1) / a.n_splits;
+    lo = split * tps * kDecBN;
+    hi = min(len, lo + min(tps, kPrefetchTiles) * kDecBN);
+}
+
 // Raw bytes of this warp's 16 Q8_0 rows [row0 + 16*warp, +16) of a 64-row K tile and V tile: two contiguous,
 // 16-byte aligned ranges of at most 16 * (HD/32*34) bytes, one bulk copy each, issued by lane 0.  Only the bytes of
 // rows below row_hi are requested (rounded up to 16: the same footprint as 16-byte chunk copies; the rest of the
@@ -641,7 +663,7 @@ __host__ __device__ constexpr size_t cluster_push_bytes(int hd, int rows) { retu
 // A CTA with two or three tiles shares its SM with few others, but at the usual 256-stream size three neighbours are
 // in their key loops and every dependent step of a tail waits for an issue slot, so the chain is kept short: no
 // separate pass for the common maximum, no index division per element.
-template <int HD>
+template <int HD, int NW = 4, int ROWS = kDecRows>
 __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float* slab, const float (*s_m)[kDecRows],
                                                  const float (*s_l)[kDecRows], uint8_t* recv, int R, int b, int hk, int split,
                                                  int tq_b, int tid) {
@@ -653,22 +675,22 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
     float2* recv_ml = reinterpret_cast<float2*>(recv_o + (R * G + 8));
     const int n_groups = R * G, slots = (n_groups + a.n_splits - 1) / a.n_splits;
     if (push) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster has started
-    for (int rr = warp; rr < R; rr += 4) {
-        const float m0 = s_m[0][rr], m1 = s_m[1][rr], m2 = s_m[2][rr], m3 = s_m[3][rr];
-        const float l0 = s_l[0][rr], l1 = s_l[1][rr], l2 = s_l[2][rr], l3 = s_l[3][rr];
-        const float M = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-        const float w0 = m0 == ninf ? 0.0f : fast_ex2(m0 - M), w1 = m1 == ninf ? 0.0f : fast_ex2(m1 - M);
-        const float w2 = m2 == ninf ? 0.0f : fast_ex2(m2 - M), w3 = m3 == ninf ? 0.0f : fast_ex2(m3 - M);
-        const float L = (w0 * l0 + w1 * l1) + (w2 * l2 + w3 * l3);
+    for (int rr = warp; rr < R; rr += NW) {
+        float m[NW], w[NW], M = ninf, L = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NW; i++) m[i] = s_m[i][rr], M = fmaxf(M, m[i]);
+#pragma unroll
+        for (int i = 0; i < NW; i++) {
+            w[i] = m[i] == ninf ? 0.0f : fast_ex2(m[i] - M);
+            L = fmaf(w[i], s_l[i][rr], L);
+        }
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (lane < G) {
-            const float4 x0 = *reinterpret_cast<const float4*>(slab + (0 * kDecRows + rr) * STRIDE + 4 * lane);
-            const float4 x1 = *reinterpret_cast<const float4*>(slab + (1 * kDecRows + rr) * STRIDE + 4 * lane);
-            const float4 x2 = *reinterpret_cast<const float4*>(slab + (2 * kDecRows + rr) * STRIDE + 4 * lane);
-            const float4 x3 = *reinterpret_cast<const float4*>(slab + (3 * kDecRows + rr) * STRIDE + 4 * lane);
-            // a warp that saw no live key holds zeros and weight 0
-            v.x = (w0 * x0.x + w1 * x1.x) + (w2 * x2.x + w3 * x3.x), v.y = (w0 * x0.y + w1 * x1.y) + (w2 * x2.y + w3 * x3.y);
-            v.z = (w0 * x0.z + w1 * x1.z) + (w2 * x2.z + w3 * x3.z), v.w = (w0 * x0.w + w1 * x1.w) + (w2 * x2.w + w3 * x3.w);
+#pragma unroll
+            for (int i = 0; i < NW; i++) {   // a warp that saw no live key holds zeros and weight 0
+                const float4 x = *reinterpret_cast<const float4*>(slab + (i * ROWS + rr) * STRIDE + 4 * lane);
+                v.x = fmaf(w[i], x.x, v.x), v.y = fmaf(w[i], x.y, v.y), v.z = fmaf(w[i], x.z, v.z), v.w = fmaf(w[i], x.w, v.w);
+            }
         }
         if (a.n_splits == 1) {
             int iq, hq;
@@ -700,7 +722,7 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
     if (push) {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-        for (int pos = tid; pos * a.n_splits + split < n_groups; pos += kThreads) {
+        for (int pos = tid; pos * a.n_splits + split < n_groups; pos += 32 * NW) {
             const int grp = pos * a.n_splits + split, rr = grp / G, cg = grp % G;
             float2 ml[8];
             float M = ninf;
@@ -772,6 +794,17 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         __syncwarp();
+    }
+    // (rows of head_dim 128 split over a cluster, ahead of which a cache append runs, measured 0.5 us slower with it)
+    if (MODE == kDecAsyncF16 && (HD <= 64 || a.n_splits == 1)) {
+        constexpr int LPR = HD * 2 / 128 > 0 ? HD * 2 / 128 : 1;   // 128-byte lines per row
+        int lo, hi;
+        peek_range(a, b, split, lo, hi);
+        for (int i = tid; i < (hi - lo) * LPR; i += kThreads) {
+            const int key = lo + i / LPR, row = IDX ? min(max(peek(index + key), 0), a.Lk - 1) : key;
+            prefetch_l2(kbase + (int64_t)row * a.k.nb1 + (i % LPR) * 128);
+            prefetch_l2(vbase + (int64_t)row * a.v.nb1 + (i % LPR) * 128);
+        }
     }
     // Launched with programmatic stream serialisation: everything above (kernel parameters, this CTA's own shared
     // memory) ran while the previous kernel of the stream drained; from here on that kernel has completed and flushed
@@ -1379,30 +1412,18 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
     return y;
 }
 
-__device__ __forceinline__ void mma16832_s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// S8: the score product runs on the int8 tensor path.  The K quants are the A operand as they lie in the cache (no
-// byte permutes, no bias, no conversion at all); the query row is split once per CTA into two int8 planes per
-// 32-element block, q = dq*(hi + lo/254) with hi = round(x/dq), lo = round((x - dq*hi)*254/dq), dq = max|x|/127, which
-// keeps an absolute error of dq/508 = 1.5e-5 of the block maximum per element (F16 itself resolves 4.9e-4 of a
-// value).  Per block two k32 MMAs give exact int32 dots, combined as 254*hi + lo, converted once and scaled by
-// fp32(d_k)*dq/254.  This empties the integer ALU pipe of the K side, which bounds the F16 form of this kernel.
-template <int HD, bool S8>
-__global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const FattnArgs a) {
+template <int HD, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(const FattnArgs a) {
     constexpr int NBLK = HD / 32, RB = NBLK * 34;
-    constexpr int RAW_BYTES = kDecBN * RB;   // one raw K or V tile
+    constexpr int KT = 16 * NW;              // keys per tile
+    constexpr int RAW_BYTES = KT * RB;       // one raw K or V tile
     constexpr int NS = kDecRegStages;
     constexpr float kGrow = 4.0f;            // lazy-rescale bound in log2 units: P <= 16
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    __half* sQ = reinterpret_cast<__half*>(smem_raw);                                  // [16][HD], 16-byte chunks swizzled
-    uint8_t* sRaw = smem_raw + kDecRows * HD * sizeof(__half);                          // NS stages of raw K | V
-    __shared__ float s_m[4][kDecRows], s_l[4][kDecRows];
-    __shared__ __align__(8) uint64_t s_bar[4][NS];                                      // one barrier per (warp, stage)
+    __half* sQ = reinterpret_cast<__half*>(smem_raw);                                  // [8][HD], 16-byte chunks swizzled
+    uint8_t* sRaw = smem_raw + 8 * HD * sizeof(__half);                          // NS stages of raw K | V
+    __shared__ float s_m[NW][kDecRows], s_l[NW][kDecRows];
+    __shared__ __align__(8) uint64_t s_bar[NW][NS];                                      // one barrier per (warp, stage)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
@@ -1433,8 +1454,18 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
     Q8T_TRACE(1);
     const int len_b = clamp_len(a, b);
     const int tq_b = q_rows_of(a, b);
+    // Q rows (tiny): the eight rows this kernel has, one 8-element chunk per thread; rows >= R are zero.  Requested together
+    // with the lengths, ahead of everything that waits for them.
+    static_assert(8 * (HD / 8) <= 32 * NW, "one chunk per thread");
+    const int q_row = tid / (HD / 8), q_ch = tid % (HD / 8);
+    uint4 q_val = make_uint4(0u, 0u, 0u, 0u);
+    if (q_row < R) {
+        int iq, hq;
+        row_to_query(a, hk, q_row, iq, hq);
+        q_val = load8_as_half(a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3, a.q.type, q_ch * 8, a.hd, a.q.vec16);
+    }
     const int kmax = tq_b > 0 ? len_b : 0;
-    const int n_tiles = (kmax + kDecBN - 1) / kDecBN;
+    const int n_tiles = (kmax + KT - 1) / KT;
     const int tps = (n_tiles + a.n_splits - 1) / a.n_splits;
     const int tile_lo = split * tps, tile_hi = min(n_tiles, tile_lo + tps);
     // lanes 2s (K) and 2s+1 (V) of a warp copy the raw bytes of the warp's 16 keys of tile `tile0 + s`; lane 2s also
@@ -1443,7 +1474,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
         const int s_ = lane >> 1, tile = tile0 + s_;
         if (s_ < n_stages && tile < tile_hi) {
             const int stage = (tile - tile_lo) % NS;
-            const int r0 = tile * kDecBN + 16 * warp;
+            const int r0 = tile * KT + 16 * warp;
             const int n = min(16, max(0, len_b - r0));
             const uint32_t bytes = (uint32_t)((n * RB + 15) / 16 * 16);
             const uint32_t bar = smem_u32(&s_bar[warp][stage]);
@@ -1457,79 +1488,25 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
     auto issue = [&](int tile) { issue_lanes(tile, 1); };
     issue_lanes(tile_lo, NS);
     Q8T_TRACE(2);
-    // Q rows (tiny): the eight rows this kernel has, one 8-element chunk per thread; rows >= R are zero.  A single
-    // new token per stream (the usual decode step) needs no division by the group size.
-    static_assert(8 * (HD / 8) <= kThreads, "one chunk per thread");
-    if (tid < 8 * (HD / 8)) {
-        const int rr = tid / (HD / 8), ch = tid % (HD / 8);
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (rr < R) {
-            int iq, hq;
-            row_to_query(a, hk, rr, iq, hq);
-            val = load8_as_half(a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3,
-                                a.q.type, ch * 8, a.hd, a.q.vec16);
-        }
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (rr * (HD / 8) + swz<HD>(rr, ch)) * 16) = val;
-    }
+    if (tid < 8 * (HD / 8)) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (q_row * (HD / 8) + swz<HD>(q_row, q_ch)) * 16) = q_val;
     __syncthreads();
-    // S8: the two int8 planes and the block scales of the 8 query rows, built once by 8 * NBLK threads in shared memory
-    // behind the f16 rows (the raw stages are not touched: their copies are already in flight)
-    // (rows 8..15 of the f16 Q tile do not exist in this kernel: the planes take their 16 * HD bytes; the block scales
-    // borrow the first 8 * NBLK floats of s_l, which is not used before the epilogue - four CTAs per SM leave no room
-    // for more static shared memory)
-    int8_t* s_qhi = reinterpret_cast<int8_t*>(sQ) + 8 * HD * sizeof(__half);
-    int8_t* s_qlo = s_qhi + 8 * HD;
-    float* s_qd = &s_l[0][0];
-    if (S8) {
-        if (tid < 8 * NBLK) {
-            const int rr = tid / NBLK, blk = tid % NBLK;
-            float x[32];
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(sQ) + (rr * (HD / 8) + swz<HD>(rr, 4 * blk + c4)) * 16);
-                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&w4[i]));
-                    x[c4 * 8 + 2 * i] = f2.x, x[c4 * 8 + 2 * i + 1] = f2.y;
-                }
-            }
-            float amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 32; i++) amax = fmaxf(amax, fabsf(x[i]));
-            const float dq = amax / 127.0f, inv = dq > 0.0f ? 1.0f / dq : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 32; i++) {
-                const float hi = rintf(x[i] * inv);
-                const float lo = fminf(fmaxf(rintf((x[i] - dq * hi) * inv * 254.0f), -127.0f), 127.0f);
-                s_qhi[rr * HD + blk * 32 + i] = (int8_t)hi, s_qlo[rr * HD + blk * 32 + i] = (int8_t)lo;
-            }
-            s_qd[rr * NBLK + blk] = dq * (1.0f / 254.0f);
-        }
-        __syncthreads();
-    }
-    // Q as the B operand of S^T = K.Q^T: column n = query row g.  F16 form: per (block, k-step) the thread's four
+    float* s_qd = &s_l[0][0];   // the block sums of the query rows borrow s_l, free until the epilogue
+    // Q as the B operand of S^T = K.Q^T: column n = query row g.  Per (block, k-step) the thread's four
     // contraction indices are dims 32blk + 16ks + {4t..4t+3} (the same permutation the K bytes are read in): one 8-byte
-    // read.  S8 form: per block, k = 4t..4t+3 (b0) and 16+4t..16+4t+3 (b1) of both planes, no permutation.
+    // read.
     uint32_t qb[NBLK][2][2];
 #pragma unroll
     for (int blk = 0; blk < NBLK; blk++)
 #pragma unroll
         for (int ks = 0; ks < 2; ks++) {
-            if (S8) {
-                // ks = plane (0 = hi, 1 = lo); [.][0] = k 4t.., [.][1] = k 16+4t..
-                const int8_t* plane = (ks ? s_qlo : s_qhi) + g * HD;
-                qb[blk][ks][0] = *reinterpret_cast<const uint32_t*>(plane + blk * 32 + 4 * t);
-                qb[blk][ks][1] = *reinterpret_cast<const uint32_t*>(plane + blk * 32 + 16 + 4 * t);
-            } else {
+            {
                 const int ch = 4 * blk + 2 * ks + (t >> 1);
                 const uint2 w = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(sQ) + (g * (HD / 8) + swz<HD>(g, ch)) * 16 + (t & 1) * 8);
                 qb[blk][ks][0] = w.x, qb[blk][ks][1] = w.y;
             }
         }
-    // F16 form: -1152 * (sum of the query row's f16 values over a block); S8 form: the row's block scale dq / 254 -
-    // for this thread's accumulator columns (rows 2t, 2t+1)
-    if (!S8) {
+    // -1152 * (sum of the query row's f16 values over a block), for this thread's accumulator columns (rows 2t, 2t+1)
+    {
         // the 8 * NBLK block sums of the query rows, once per CTA: four threads per (row, block), one 16-byte chunk each
         // (s_l is free until the epilogue)
         const int pair = tid >> 2, c4 = tid & 3;
@@ -1567,7 +1544,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
 
     Q8T_TRACE(4);
     for (int tile = tile_lo; tile < tile_hi; tile++) {
-        const int k0 = tile * kDecBN;
+        const int k0 = tile * KT;
         const int stage = (tile - tile_lo) % NS;
         if (!mbar_wait_bounded(smem_u32(&s_bar[warp][stage]), (uint32_t)((tile - tile_lo) / NS) & 1u)) break;
         if (tile == tile_lo) Q8T_TRACE(5);
@@ -1583,32 +1560,6 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
         const bool live[2] = {all_live || g < rows_valid, all_live || g + 8 < rows_valid};
 #pragma unroll
         for (int blk = 0; blk < NBLK; blk++) {
-            if (S8) {
-                // the K bytes are the A operand as they lie: words at quants 4t..4t+3 and 16+4t.. of keys g and g+8
-                uint32_t af[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const uint8_t* bp = rowp[i & 1] + blk * 34 + 2 + 16 * (i >> 1) + 4 * t;
-                    if (blk & 1) {
-                        af[i] = *reinterpret_cast<const uint32_t*>(bp);
-                    } else {
-                        const uint16_t* hp = reinterpret_cast<const uint16_t*>(bp);
-                        af[i] = hp[0] | ((uint32_t)hp[1] << 16);
-                    }
-                }
-                int ahi[4] = {0, 0, 0, 0}, alo[4] = {0, 0, 0, 0};
-                mma16832_s8(ahi, af, qb[blk][0][0], qb[blk][0][1]);
-                mma16832_s8(alo, af, qb[blk][1][0], qb[blk][1][1]);
-                const uint16_t d0b = live[0] ? *reinterpret_cast<const uint16_t*>(rowp[0] + blk * 34) : (uint16_t)0;
-                const uint16_t d1b = live[1] ? *reinterpret_cast<const uint16_t*>(rowp[1] + blk * 34) : (uint16_t)0;
-                const float d0 = __half2float(__ushort_as_half(d0b)), d1 = __half2float(__ushort_as_half(d1b));
-                // exact integer dot of the block: 254 * hi + lo (|.| < 2^28), then one conversion and the two scales
-                st[0] = fmaf(d0 * negc[blk][0], (float)(ahi[0] * 254 + alo[0]), st[0]);
-                st[1] = fmaf(d0 * negc[blk][1], (float)(ahi[1] * 254 + alo[1]), st[1]);
-                st[2] = fmaf(d1 * negc[blk][0], (float)(ahi[2] * 254 + alo[2]), st[2]);
-                st[3] = fmaf(d1 * negc[blk][1], (float)(ahi[3] * 254 + alo[3]), st[3]);
-                continue;
-            }
             // the accumulators start at -1152 * sum_block(Q): the products of the biased halves land on the integer dot
             float acc[4] = {negc[blk][0], negc[blk][1], negc[blk][0], negc[blk][1]};
 #pragma unroll
@@ -1725,7 +1676,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // ---- merge the four warps' (m, l, O) in shared memory (same slabs as the kernel above) ----
     constexpr int SLAB_STRIDE = HD + 4;
-    float* slab = reinterpret_cast<float*>(smem_raw);   // [4][16][SLAB_STRIDE]
+    float* slab = reinterpret_cast<float*>(smem_raw);   // [NW][8][SLAB_STRIDE]
     float lq[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -1739,7 +1690,6 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
         s_m[warp][2 * t] = m_run[0], s_m[warp][2 * t + 1] = m_run[1];
         s_l[warp][2 * t] = lq[0], s_l[warp][2 * t + 1] = lq[1];
     }
-    if (lane < 8) s_m[warp][8 + lane] = ninf, s_l[warp][8 + lane] = 0.0f;   // rows 8..15 do not exist in this form
     __syncthreads();  // the warps' (m, l) are visible, and all warps are done with the raw stages (the merge slabs alias them)
     Q8T_TRACE(8);
     // Each warp parks its accumulators as they are (scaled to its OWN running maximum): a thread's accumulators of one
@@ -1750,14 +1700,14 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8t_kernel(const Fat
         if (2 * t + j >= R) continue;
 #pragma unroll
         for (int blk = 0; blk < NBLK; blk++)
-            *reinterpret_cast<float4*>(slab + (warp * kDecRows + 2 * t + j) * SLAB_STRIDE + 32 * blk + 4 * g) =
+            *reinterpret_cast<float4*>(slab + (warp * 8 + 2 * t + j) * SLAB_STRIDE + 32 * blk + 4 * g) =
                 make_float4(o[blk][0][j], o[blk][0][2 + j], o[blk][1][j], o[blk][1][2 + j]);
     }
     Q8T_TRACE(12);
     __syncthreads();
     Q8T_TRACE(9);
     Q8T_TRACE(13);
-    decode_write_out<HD>(a, slab, s_m, s_l, sRaw + NS * 2 * RAW_BYTES, R, b, hk, split, tq_b, tid);
+    decode_write_out<HD, NW, 8>(a, slab, s_m, s_l, sRaw + NS * 2 * RAW_BYTES, R, b, hk, split, tq_b, tid);
     Q8T_TRACE(10);
 }
 
@@ -1859,20 +1809,21 @@ bool cluster_merge_enabled() {
 
 bool use_cluster_merge(const FattnArgs& a) {
     // only while the whole grid is resident at once (2 to 4 CTAs on each of 148 SMs): with several waves the cluster
-    // barriers hold finished CTAs on their SMs and the form measured 10 % slower than the merge kernel
-    return decode_cluster_merge_ok(a) && a.n_splits > 1 && a.n_splits <= 8 &&
-           (long)a.n_splits * a.Hkv * a.B <= (long)decode_ctas_per_sm(a, true) * 148;
+    // barriers hold finished CTAs on their SMs and the form measured 10 % slower than the merge kernel.  Pairs at head_dim 64 over an F16
+    // cache hold little and save the merge kernel (32 segments of the large decoder 101.6 -> 97.5 us per layer).
+    return decode_cluster_merge_ok(a) && a.n_splits > 1 && a.n_splits <= 8 && ((a.n_splits == 2 && a.k.type == B200_TYPE_F16 && a.hd == 64) ||
+           (long)a.n_splits * a.Hkv * a.B <= (long)decode_ctas_per_sm(a, true) * 148);
 }
 
 template <typename Kern>
-void launch_split(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const FattnArgs& a) {
+void launch_split(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const FattnArgs& a, int threads = kThreads) {
     // Programmatic stream serialisation: the grid may become resident while the previous kernel of the stream drains
     // (its CTAs wait on the device before they touch memory), which hides the launch latency between the layers of a
     // decode step (+0.8 % on the 64-segment decode launches, +1 % at 32 streams).
     FattnArgs ac = a;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -1990,6 +1941,10 @@ int decode_mode(const FattnArgs& a, int hdp) {
     return kDecSync;
 }
 
+// The keys-on-M kernel: at most 8 query rows, plain form.
+bool q8t_form(const FattnArgs& a) { return !a.has_mask && a.softcap == 0.0f && !a.causal && a.Tq * a.gqa <= 8; }
+size_t q8t_smem(int hd, int nw) { return (size_t)8 * hd * sizeof(__half) + (size_t)kDecRegStages * 2 * 16 * nw * (hd / 32 * 34); }
+
 template <int HD>
 int launch_decode_q8reg(const FattnArgs& a, cudaStream_t st) {
     // a cluster launch carries the receive area of the merge behind the stages; the attribute is raised once, to that size
@@ -1998,30 +1953,16 @@ int launch_decode_q8reg(const FattnArgs& a, cudaStream_t st) {
     const size_t smem = smem_main + (use_cluster_merge(a) ? cluster_push_bytes(HD, a.Tq * a.gqa) : 0);
     dim3 grid(a.n_splits, a.Hkv, a.B);
     cudaError_t e;
-    // B200_DECODE_Q8T=0 keeps the rows-on-M register kernel, =1 (default) the keys-on-M kernel with F16 score MMAs, =2
-    // the keys-on-M kernel with int8 score MMAs (measured equal at 256 streams, 5 % slower at 8: its set-up; A/B runs)
-    static const int keys_on_m = [] {
-        const char* e = getenv("B200_DECODE_Q8T");
-        return (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 1;
-    }();
-    if (keys_on_m == 2 && !a.has_mask && a.softcap == 0.0f && !a.causal && a.Tq * a.gqa <= 8) {
-        auto kern = fattn_decode_q8t_kernel<HD, true>;
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, smem_attr, smem_set);
+    if (q8t_form(a)) {
+        auto go = [&](auto kern, int nw, bool (&smem_set)[64]) {
+            const size_t main = q8t_smem(HD, nw);
+            e = set_smem_once(kern, main + cluster_push_bytes(HD, 8), smem_set);
+            if (e == cudaSuccess) launch_split(kern, grid, main + (use_cluster_merge(a) ? cluster_push_bytes(HD, a.Tq * a.gqa) : 0), st, a, 32 * nw);
+        };
+        static bool set[2][64] = {};
+        if (a.wide) go(fattn_decode_q8t_kernel<HD, 8>, 8, set[0]);
+        else go(fattn_decode_q8t_kernel<HD, 4>, 4, set[1]);
         if (e != cudaSuccess) return (int)e;
-        launch_split(kern, grid, smem, st, a);
-    } else if (keys_on_m == 1 && !a.has_mask && a.softcap == 0.0f && !a.causal && a.Tq * a.gqa <= 8) {
-        auto kern = fattn_decode_q8t_kernel<HD, false>;
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, smem_attr, smem_set);
-        if (e != cudaSuccess) return (int)e;
-        launch_split(kern, grid, smem, st, a);
-    } else if (!a.has_mask && a.softcap == 0.0f && !a.causal && a.Tq * a.gqa <= 8) {
-        auto kern = fattn_decode_q8reg_kernel<HD, true, true>;
-        static bool smem_set[64] = {false};
-        e = set_smem_once(kern, smem_attr, smem_set);
-        if (e != cudaSuccess) return (int)e;
-        launch_split(kern, grid, smem, st, a);
     } else if (!a.has_mask && a.softcap == 0.0f && !a.causal) {
         auto kern = fattn_decode_q8reg_kernel<HD, true, false>;
         static bool smem_set[64] = {false};
@@ -2253,7 +2194,14 @@ int decode_ctas_per_sm(const FattnArgs& a, bool cluster) {
     const int hdp = a.hd <= 32 ? 32 : (a.hd <= 64 ? 64 : 128);
     size_t smem;
     switch (decode_mode(a, hdp)) {
-        case kDecRegQ8: smem = (size_t)kDecRows * hdp * 2 + (size_t)kDecRegStages * 2 * kDecBN * (hdp / 32 * 34); break;
+        case kDecRegQ8:
+            if (q8t_form(a)) {
+                smem = q8t_smem(hdp, a.wide ? 8 : 4) + (cluster ? cluster_push_bytes(hdp, a.Tq * a.gqa) : 0);
+                const int n = (int)((size_t)227 * 1024 / (smem + 1536 + 1024)), most = a.wide ? 2 : 4;
+                return n < 1 ? 1 : (n > most ? most : n);
+            }
+            smem = (size_t)kDecRows * hdp * 2 + (size_t)kDecRegStages * 2 * kDecBN * (hdp / 32 * 34);
+            break;
         case kDecAsyncF16: {
             const int ns = hdp >= 128 ? 3 : 4;
             smem = (size_t)(kDecRows + ns * 2 * kDecBN) * hdp * 2;
@@ -2277,7 +2225,8 @@ int decode_ctas_per_sm(const FattnArgs& a, bool cluster) {
 static std::atomic<int> g_forced_splits{0};
 void decode_split_force(int n_splits) { g_forced_splits.store(n_splits, std::memory_order_relaxed); }
 
-int decode_split_choose(const FattnArgs& a, int B, int sm_count) {
+int decode_split_choose(FattnArgs& a, int B, int sm_count) {
+    a.wide = 0;
     const int forced = g_forced_splits.load(std::memory_order_relaxed);
     static const int per_sm_env = [] {  // B200_DECODE_CTAS_PER_SM=1..16 overrides the resident-CTA estimate
         const char* e = getenv("B200_DECODE_CTAS_PER_SM");
@@ -2298,7 +2247,7 @@ int decode_split_choose(const FattnArgs& a, int B, int sm_count) {
         if ((tiles + tps - 1) / tps != n) continue;   // some split would get no tile
         const double w = units * n / cap;
         const double waves = w <= 4.0 ? ceil(w) : w + 0.5;
-        const bool cluster = cluster_ok && n > 1 && n <= 8 && units * n <= cap_cluster;
+        const bool cluster = cluster_ok && n > 1 && n <= 8 && (units * n <= cap_cluster || (n == 2 && a.k.type == B200_TYPE_F16 && a.hd == 64));
         double cost = waves * (tps + 1.5 + (n == 1 ? 0.0 : (cluster ? 0.5 : 1.0)));
         // the merge reads n partials per output row.  F16 kernel (100 KB CTAs, merge kernel launched under its tail):
         // merge kernel 0.8 + 0.2 n, cluster 1.0 + 0.1 n, fitted to one segment of Whisper cross-attention (24 tiles:
@@ -2309,6 +2258,11 @@ int decode_split_choose(const FattnArgs& a, int B, int sm_count) {
         if (n > 1) cost += cluster ? (f16 ? 1.0 : 0.0) + 0.1 * n : (f16 ? 0.8 : 3.0) + 0.2 * n;
         if (n == 1 || cost < best_cost - 1e-9) best = n, best_cost = cost;
     }
+    // Between the unit counts that clusters of two fill and those that fill the SMs by themselves, a four-warp CTA per unit
+    // leaves an SM with two CTAs, and a warp's chain through a tile (copy, dequantise, two products) sets the pace.  Eight
+    // warps per CTA split the keys once more without a merge outside the CTA: 32 streams x 8 KV heads, 535 keys, 16.5 ->
+    // 11.3 us per launch (two splits through the workspace: 13.7).
+    if (best == 1 && units <= 2.0 * sm_count && tiles > 2 && decode_mode(a, a.hd) == kDecRegQ8 && q8t_form(a)) a.wide = 1;
     return best;
 }
 

@@ -775,3 +775,27 @@ def test_launch_tracing_records_one_event_pair_per_launch(b200, orc):
     gpu_op(b200, qd, kd, kd, scale=0.1)
     n = C.c_int(5)
     assert L.b200_trace_read(None, 0, C.byref(n)) == 0 and n.value == 0
+
+
+@pytest.mark.parametrize("hd,Hkv,gqa", [(128, 8, 4), (128, 7, 1), (128, 8, 8)])
+@pytest.mark.parametrize("L", [130, 257, 400])
+def test_q8_0_decode_wide_ctas(b200, orc, hd, Hkv, gqa, L):
+    """Between the unit counts that clusters fill and those that fill the SMs one CTA of eight warps takes a (stream, KV
+    head) whole, in tiles of 128 keys: lengths around the edges of a tile and of a warp's 16 keys, an empty stream, one to
+    eight query rows per KV head."""
+    rng = np.random.default_rng(hd + L + gqa)
+    B = 34
+    q = randn_f16(rng, (B, Hkv * gqa, 1, hd))
+    k, v = (orc.quantize_q8_0(rng.standard_normal((B, Hkv, L, hd)).astype(np.float32)) for _ in "kv")
+    lens = rng.integers(1, L + 1, B).astype(np.int32)
+    edges = [0, 1, 15, 16, 17, 127, 128, 129, L]
+    lens[:len(edges)] = np.minimum(edges, L)
+    kw = dict(scale=hd ** -0.5, kv_type=abi.Q8_0, kv_len=lens)
+    ctx = -(-L // 32) * 32                       # rows per head as the slabs lay them out: 16-byte aligned heads
+    slabs = [np.zeros((B, Hkv, ctx, x.shape[-1]), np.uint8) for x in (k, v)]
+    for s, x in zip(slabs, (k, v)):
+        s[:, :, :L] = x
+    dk, dv = (cuda_view(s[:, :, :L], s) for s in slabs)
+    assert b200.plan(torch.from_numpy(q), dk, dv, scale=1.0, kv_type=abi.Q8_0) == (abi.KERNEL_DECODE_SPLIT, 1)
+    assert_close(gpu_op(b200, q, dk, dv, **kw), orc.flash_attn_ext(q, k, v, **kw), f"wide decode hd={hd} L={L}")
+    assert b200.lib().b200_device_status() == 0
