@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "fattn_tc5.cuh"
 
@@ -1702,19 +1703,26 @@ bool encode_r_map(CUtensorMap* m, const FattnArgs& a) {
 // Launch that may begin while the previous kernel of the stream drains, if that kernel allows it
 // (griddepcontrol.launch_dependents: the K/V conversion pre-pass does).  The kernels wait for the predecessor's
 // completion (griddepcontrol.wait) before they read anything it may have written.
+// `cluster` > 1: so many CTAs along x form a thread-block cluster.
 template <typename Kern, typename... Args>
-cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_pdl_cluster(Kern kern, dim3 grid, int cluster, int threads, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <typename Kern, typename... Args>
+cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    return launch_pdl_cluster(kern, grid, 1, threads, smem, st, args...);
 }
 
 int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
@@ -1760,6 +1768,26 @@ bool q_box_ok(const FattnArgs& a) {
            a.q.nb3 > 0;
 }
 
+// How many CTAs (a cluster of 1, 2, 4 or 8) share a query tile's `steps` key steps, for a launch of `tiles` query tiles on
+// 148 SMs with four places each.  A step takes 0.77 us in a CTA that has an SM to itself - its own hand-off chain - and
+// 0.92 / 1.2 / 1.48 us in one of two / three / four; sharing a tile costs 3 us (two cluster barriers, O through shared memory,
+// the merge).  One window of the base encoder (8 heads, 96 tiles of 24 steps): one CTA per tile 23.7 us, two 19.9, four
+// 16.9, eight (two waves) 22.1; 700 frames of 6 heads (36 tiles of 11) 13.2 / 11.8 / 10.5 / 11.5; 600 frames of 20 heads (100
+// tiles of 10) 12.0 / 13.3 / 13.3 / 19.7.
+int h64_splits(long tiles, int steps) {
+    constexpr double kStepUs[5] = {0.77, 0.77, 0.92, 1.2, 1.48};
+    int best = 1;
+    double best_cost = 0.0;
+    for (int n = 1; n <= 8; n *= 2) {
+        const long per_sm = (tiles * n + 147) / 148;
+        if (n > 1 && per_sm > 4) break;   // more than one wave
+        const double cost = (steps + n - 1) / n * kStepUs[per_sm < 4 ? per_sm : 4] + (n > 1 ? 2.9 + 0.2 * n : 0.0);
+        // (a clear gain only: where it is even, the result of an entry stays what it is inside a larger batch, bit for bit)
+        if (n == 1 || cost < 0.93 * best_cost) best = n, best_cost = cost;
+    }
+    return best;
+}
+
 int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
     CUtensorMap tmK, tmV;
     if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys)) {
@@ -1769,15 +1797,20 @@ int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen)
     CUtensorMap tmQ = tmK, tmO = tmK;
     const bool q_tma = a.q.type == B200_TYPE_F16 && q_box_ok(a) && encode_q_map(&tmQ, a);
     const bool o_tma = gqa_box(a) && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);
-    dim3 grid((a.Tq * a.gqa + kTile - 1) / kTile, a.Hkv, a.B);
+    FattnArgs as = a;
+    const int n_q = (a.Tq * a.gqa + kTile - 1) / kTile;
+    as.n_splits = h64_splits((long)n_q * a.Hkv * a.B, (a.Lk + kH64Keys - 1) / kH64Keys);
+    dim3 grid(n_q * as.n_splits, a.Hkv, a.B);
     auto go = [&](auto kern, bool (&smem_set)[64]) {
         cudaError_t e = set_smem_once(kern, kH64Smem, smem_set);
-        if (e == cudaSuccess) e = launch_pdl(kern, grid, kH64Threads, kH64Smem, st, a, tmK, tmV, tmQ, tmO);
+        if (e == cudaSuccess) e = launch_pdl_cluster(kern, grid, as.n_splits, kH64Threads, kH64Smem, st, as, tmK, tmV, tmQ, tmO);
         return e;
     };
-    static bool set[4][64] = {};
-    const cudaError_t e = q_tma ? (o_tma ? go(fattn_prefill_tc5_h64_kernel<true, true>, set[0]) : go(fattn_prefill_tc5_h64_kernel<true, false>, set[1]))
-                                : (o_tma ? go(fattn_prefill_tc5_h64_kernel<false, true>, set[2]) : go(fattn_prefill_tc5_h64_kernel<false, false>, set[3]));
+    static bool set[6][64] = {};
+    cudaError_t e;
+    if (as.n_splits > 1) e = q_tma ? go(fattn_prefill_tc5_h64_kernel<true, false, true>, set[4]) : go(fattn_prefill_tc5_h64_kernel<false, false, true>, set[5]);
+    else e = q_tma ? (o_tma ? go(fattn_prefill_tc5_h64_kernel<true, true>, set[0]) : go(fattn_prefill_tc5_h64_kernel<true, false>, set[1]))
+                   : (o_tma ? go(fattn_prefill_tc5_h64_kernel<false, true>, set[2]) : go(fattn_prefill_tc5_h64_kernel<false, false>, set[3]));
     if (e != cudaSuccess) {
         snprintf(errbuf, errlen, "tcgen05 prefill launch: %s", cudaGetErrorString(e));
         return B200_E_CUDA;

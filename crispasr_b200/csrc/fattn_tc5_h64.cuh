@@ -23,13 +23,32 @@ constexpr int kH64Threads = 160;
 constexpr int kH64KvBytes = kH64Keys * 128;   // one K or V tile
 constexpr size_t kH64Smem = 1024 + (size_t)kPanelBytes + 4 * kH64KvBytes + 8 * 8 + 16;
 
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, int rank) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    return remote;
+}
+__device__ __forceinline__ float4 ld_peer_v4(uint32_t p) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 ld_peer_v2(uint32_t p) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
+    return v;
+}
+
 // Every eighth pair of exponentials goes to the FMA pipe: 64 windows of the large encoder 925 -> 917 us, 8 windows 132 ->
 // 127 us; every fourth pair costs more issue slots (and power) than the unit's time it frees (990 us).
 constexpr int kH64PolyEvery = 8;
 
 // QTMA: F16 query rows arrive by one tensor copy (else the softmax warps load and convert them); OTMA: the output leaves by
-// tensor stores (else by the threads).
-template <bool QTMA, bool OTMA>
+// tensor stores (else by the threads).  SPLIT: the CTAs of a cluster share one query tile, each takes a range of its key
+// steps; at the end they leave their O rows and (m, l) in shared memory and each merges and writes a share of the rows.
+// For launches with fewer tiles than the SMs can run at full pace (h64_splits): a lone CTA per SM spends 0.75 us per step,
+// its own hand-off chain, which two CTAs per SM hide for each other and four CTAs fill.
+template <bool QTMA, bool OTMA, bool SPLIT = false>
 __global__ void __launch_bounds__(kH64Threads, 4)
 fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                              const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmO) {
@@ -47,8 +66,9 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // launched with programmatic stream serialisation
     // tile order and GQA packing as in fattn_prefill_tc5_kernel
-    int q0 = blockIdx.x * kTile, hk = blockIdx.y, b = blockIdx.z;
-    if (a.causal) {
+    const int n_split = SPLIT ? a.n_splits : 1, split = SPLIT ? (int)blockIdx.x % n_split : 0;
+    int q0 = ((int)blockIdx.x / n_split) * kTile, hk = blockIdx.y, b = blockIdx.z;
+    if (!SPLIT && a.causal) {
         const int lin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), hb = gridDim.y * gridDim.z;
         q0 = (gridDim.x - 1 - lin / hb) * kTile;
         hk = (lin % hb) % gridDim.y, b = (lin % hb) / gridDim.y;
@@ -65,9 +85,11 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     const int n_past = n_past_of(a, len_b, tq_b);
     int kmax = q0 < rows_live ? len_b : 0;
     if (a.causal) kmax = min(kmax, n_past + min((q0 + kTile - 1) / a.gqa + 1, tq_b));
-    const int n_tiles = kmax > 0 ? (kmax + kH64Keys - 1) / kH64Keys : 0;
-    if (n_tiles == 0) {  // nothing to attend to: zeros
-        if (tid < kTile && q0 + tid < rows_total) {
+    const int n_all = kmax > 0 ? (kmax + kH64Keys - 1) / kH64Keys : 0;
+    const int tps = (n_all + n_split - 1) / n_split, t0 = split * tps;   // this CTA's steps: [t0, t0 + n_tiles)
+    const int n_tiles = SPLIT ? max(0, min(n_all - t0, tps)) : n_all;
+    if (n_all == 0) {  // nothing to attend to: zeros
+        if (split == 0 && tid < kTile && q0 + tid < rows_total) {
             const int iq = (q0 + tid) / a.gqa, h = hk * a.gqa + (q0 + tid) % a.gqa;
             float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD);
 #pragma unroll
@@ -79,24 +101,26 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     auto load_k = [&](int j) {
         const uint32_t bar = bar_k + 8 * (j & 1);
         mbar_arrive_expect_tx(bar, kH64KvBytes);
-        tma_load_4d(sK + (j & 1) * kH64KvBytes, &tmK, bar, 0, j * kH64Keys, hk, bk);
+        tma_load_4d(sK + (j & 1) * kH64KvBytes, &tmK, bar, 0, (t0 + j) * kH64Keys, hk, bk);
     };
     auto load_v = [&](int j) {
         const uint32_t bar = bar_v + 8 * (j & 1);
         mbar_arrive_expect_tx(bar, kH64KvBytes);
-        tma_load_4d(sV + (j & 1) * kH64KvBytes, &tmV, bar, 0, j * kH64Keys, hk, bk);
+        tma_load_4d(sV + (j & 1) * kH64KvBytes, &tmV, bar, 0, (t0 + j) * kH64Keys, hk, bk);
     };
     if (warp == 4) {
         if (lane == 0) {
             for (int i = 0; i < 8; i++) mbar_init(sBar + 8 * i, sBar + 8 * i == bar_p_ready ? 4 : 1);   // P: one arrival per softmax warp
             *s_abort = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            if (QTMA) {
-                mbar_arrive_expect_tx(bar_q, kPanelBytes);
-                tma_load_4d(sQ, &tmQ, bar_q, 0, hk * a.gqa, q0 / a.gqa, b);
+            if (!SPLIT || n_tiles > 0) {
+                if (QTMA) {
+                    mbar_arrive_expect_tx(bar_q, kPanelBytes);
+                    tma_load_4d(sQ, &tmQ, bar_q, 0, hk * a.gqa, q0 / a.gqa, b);
+                }
+                load_k(0);
+                load_v(0);
             }
-            load_k(0);
-            load_v(0);
             if (n_tiles > 1) load_k(1);
         }
         __syncwarp();
@@ -131,8 +155,9 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                 tc_commit(bar_s_full);
             };
             int k_issued = min(2, n_tiles), v_issued = 1;
-            bool ok = (!QTMA || mbar_wait(bar_q, 0, s_abort)) && mbar_wait(bar_k, 0, s_abort);
-            if (ok) {
+            const bool any = !SPLIT || n_tiles > 0;   // a split beyond the last step has nothing to do
+            bool ok = !any || ((!QTMA || mbar_wait(bar_q, 0, s_abort)) && mbar_wait(bar_k, 0, s_abort));
+            if (ok && any) {
                 tc_fence_after();
                 if (elect_one()) {
                     issue_s(0);
@@ -190,7 +215,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
             tc_fence_after();
-            const int n_valid = kend - j * kH64Keys;   // columns >= n_valid of this row are masked
+            const int n_valid = kend - (t0 + j) * kH64Keys;   // columns >= n_valid of this row are masked
             const bool full_tile = __all_sync(0xffffffffu, n_valid >= kH64Keys);
             if (j == 0) {   // a first reference maximum: that of the row's first 16 scores (the lazy check below corrects it)
                 uint32_t s0[16];
@@ -283,8 +308,26 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
         }
-        if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
-        if (ok) {
+        if (ok && (!SPLIT || n_tiles > 0)) ok = mbar_wait(bar_o_done, 0, s_abort);
+        if constexpr (SPLIT) {
+            // O as it is (relative to this CTA's reference), whole rows, chunks swizzled by the row; (m, l) in the Q tile.  The
+            // K/V slots and the Q tile are free once the last MMA has completed.
+            tc_fence_after();
+            float* stage = reinterpret_cast<float*>(smem_gen + kPanelBytes) + r * HD;
+            const bool any = ok && n_tiles > 0;
+#pragma unroll 1
+            for (int q4 = 0; q4 < HD / 16; q4++) {
+                uint32_t x[16];
+                tmem_ld16(tmem_O + lane_base + q4 * 16, x);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; i += 4)
+                    *reinterpret_cast<float4*>(stage + ((((q4 * 16 + i) >> 2) ^ (lane & 7)) << 2)) =
+                        any ? make_float4(__uint_as_float(x[i]), __uint_as_float(x[i + 1]), __uint_as_float(x[i + 2]), __uint_as_float(x[i + 3]))
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            reinterpret_cast<float2*>(smem_gen)[r] = make_float2(any ? m_ref : -INFINITY, any ? l_run : 0.0f);
+        } else if (ok) {
             tc_fence_after();
             // rows beyond the live ones are written as literal zeros, rows outside the tensor not at all; the K/V slots are
             // free once the last MMA has completed: they stage O
@@ -321,6 +364,69 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
         }
     }
 
+    if constexpr (SPLIT) {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // Rows [split * 128 / n_split, ...) of every CTA of the cluster, 16 lanes per row, a float4 each.  All loads of a thread
+        // are in flight at once (a loop over the rows paid one round trip of 1 k clk each); peers' memory has been read when
+        // this CTA arrives at the second barrier, which it waits for behind its own stores.
+        auto merge = [&](auto ns_c) {
+            constexpr int NS = decltype(ns_c)::value, ROWS = 16 / NS;   // rows per thread
+            const int g4 = tid & 15;
+            float w[ROWS][NS], inv[ROWS];
+            {
+                float2 ml[ROWS][NS];
+#pragma unroll
+                for (int i = 0; i < ROWS; i++)
+#pragma unroll
+                    for (int s = 0; s < NS; s++) ml[i][s] = ld_peer_v2(peer_smem(smem_base + (split * (kTile / NS) + i * 8 + (tid >> 4)) * 8, s));
+#pragma unroll
+                for (int i = 0; i < ROWS; i++) {
+                    float M = -INFINITY, L = 0.0f;
+#pragma unroll
+                    for (int s = 0; s < NS; s++) M = fmaxf(M, ml[i][s].x);
+#pragma unroll
+                    for (int s = 0; s < NS; s++) {
+                        w[i][s] = ml[i][s].x == -INFINITY ? 0.0f : ex2(ml[i][s].x - M);
+                        L = fmaf(w[i][s], ml[i][s].y, L);
+                    }
+                    inv[i] = L > 0.0f ? 1.0f / L : 0.0f;
+                }
+            }
+            float4 x[ROWS][NS];
+#pragma unroll
+            for (int i = 0; i < ROWS; i++)
+#pragma unroll
+                for (int s = 0; s < NS; s++) {
+                    const int row = split * (kTile / NS) + i * 8 + (tid >> 4);
+                    x[i][s] = ld_peer_v4(peer_smem(smem_base + kPanelBytes + (row * HD + ((g4 ^ (row & 7)) << 2)) * 4, s));
+                }
+#pragma unroll
+            for (int i = 0; i < ROWS; i++) {
+                const int row = split * (kTile / NS) + i * 8 + (tid >> 4);
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int s = 0; s < NS; s++)
+                    o.x = fmaf(w[i][s], x[i][s].x, o.x), o.y = fmaf(w[i][s], x[i][s].y, o.y), o.z = fmaf(w[i][s], x[i][s].z, o.z),
+                    o.w = fmaf(w[i][s], x[i][s].w, o.w);
+                if (q0 + row < rows_total) {
+                    const int iq = (q0 + row) / a.gqa, h = hk * a.gqa + (q0 + row) % a.gqa;
+                    const bool live = q0 + row < rows_live;
+                    reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD)[g4] =
+                        live ? make_float4(o.x * inv[i], o.y * inv[i], o.z * inv[i], o.w * inv[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+        };
+        if (warp < 4) {
+            if (n_split == 2) merge(std::integral_constant<int, 2>{});
+            else if (n_split == 4) merge(std::integral_constant<int, 4>{});
+            else merge(std::integral_constant<int, 8>{});
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // peers may still read this CTA's rows
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 4) {

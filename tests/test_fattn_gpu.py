@@ -799,3 +799,32 @@ def test_q8_0_decode_wide_ctas(b200, orc, hd, Hkv, gqa, L):
     assert b200.plan(torch.from_numpy(q), dk, dv, scale=1.0, kv_type=abi.Q8_0) == (abi.KERNEL_DECODE_SPLIT, 1)
     assert_close(gpu_op(b200, q, dk, dv, **kw), orc.flash_attn_ext(q, k, v, **kw), f"wide decode hd={hd} L={L}")
     assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("T,H,gqa", [(700, 6, 1), (1000, 4, 2), (1473, 3, 1), (2050, 1, 1)])
+@pytest.mark.parametrize("form", ["plain", "causal", "lengths"])
+@pytest.mark.parametrize("q_f32", [False, True])
+def test_prefill_shared_query_tiles(b200, orc, T, H, gqa, form, q_f32):
+    """Few query tiles of head_dim 64 over many keys: the key steps of a tile are shared by the CTAs of a cluster (two to
+    eight).  Step counts that do not divide, tiles of which some CTAs see no key (causal, ragged lengths, an empty entry),
+    grouped heads, rows whose maximum moves far while the steps go by."""
+    rng = np.random.default_rng(T + H + q_f32)
+    B, Hkv = (2, H // gqa) if form == "lengths" else (1, H // gqa)
+    q, k, v = randn_f16(rng, (B, H, T, 64)), randn_f16(rng, (B, Hkv, T, 64)), randn_f16(rng, (B, Hkv, T, 64))
+    q[:, 0] *= 6.0
+    if q_f32:
+        q = q.astype(np.float32)
+    kw = dict(scale=0.125)
+    if form == "causal":
+        kw.update(causal=True, n_past=0)
+    if form == "lengths":
+        kw.update(kv_len=np.array([T, 70], np.int32), q_len=np.array([T - 1, 40], np.int32))
+    got = gpu_op(b200, q, k, v, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    q_len = kw.pop("q_len", None)
+    ref = orc.flash_attn_ext(q, k, v, **kw)
+    if q_len is not None:
+        for b, n in enumerate(q_len):
+            ref[b, n:] = 0.0
+    assert_close(got, ref, f"shared tiles T={T} H={H} gqa={gqa} {form}")
+    assert b200.lib().b200_device_status() == 0
