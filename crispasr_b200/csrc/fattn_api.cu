@@ -196,6 +196,7 @@ int make_plan(const b200_tensor* q, const b200_tensor* k, const b200_tensor* v, 
     a.k = make_view(k);
     a.v = make_view(v);
     a.dst = (float*)dst->data;
+    a.dst_heads = (int)H;
     a.hd = (int)hd, a.Tq = (int)Tq, a.H = (int)H, a.B = (int)B;
     a.Lk = (int)Lk, a.Hkv = (int)Hkv, a.gqa = (int)(H / Hkv), a.bq = (int)(B / Bk);
     a.relscale = p->scale;
@@ -401,20 +402,60 @@ int do_launch_untraced(Plan& plan, void* workspace, size_t ws_bytes, cudaStream_
 }
 
 // ---- per-thread staging arena of the host-buffer entry point ----
+constexpr int kMaxHostChunks = 16;
 struct Arena {
     uint8_t* base = nullptr;
     size_t cap = 0;
     int device = -1;
-    cudaStream_t stream = nullptr, stream2 = nullptr;
+    cudaStream_t in = nullptr, compute = nullptr, out = nullptr;   // uploads, kernels, downloads
+    cudaEvent_t arrived[kMaxHostChunks] = {}, computed[kMaxHostChunks] = {};
     ~Arena() { release(); }
+    // Streams and events of the current device; they stay with the thread.
+    cudaError_t open(int dev) {
+        if (device == dev) return cudaSuccess;
+        release();
+        device = dev;
+        cudaError_t e = cudaSuccess;
+        for (cudaStream_t* s : {&in, &compute, &out})
+            if (e == cudaSuccess) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+        for (int i = 0; i < kMaxHostChunks; i++) {
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&arrived[i], cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&computed[i], cudaEventDisableTiming);
+        }
+        if (e != cudaSuccess) release();
+        return e;
+    }
     void release() {
         if (base) cudaFree(base);
-        if (stream) cudaStreamDestroy(stream);
-        if (stream2) cudaStreamDestroy(stream2);
-        base = nullptr, cap = 0, stream = nullptr, stream2 = nullptr, device = -1;
+        for (cudaStream_t* s : {&in, &compute, &out}) {
+            if (*s) cudaStreamDestroy(*s);
+            *s = nullptr;
+        }
+        for (int i = 0; i < kMaxHostChunks; i++) {
+            if (arrived[i]) cudaEventDestroy(arrived[i]);
+            if (computed[i]) cudaEventDestroy(computed[i]);
+            arrived[i] = computed[i] = nullptr;
+        }
+        base = nullptr, cap = 0, device = -1;
     }
 };
 thread_local Arena g_arena;
+
+// The address at which kernels of the current device reach pinned host memory [p, p + bytes), or null.
+void* mapped_host(void* p, size_t bytes) {
+    cudaPointerAttributes at;
+    void* dev = nullptr;
+    for (size_t off : {(size_t)0, bytes - 1}) {
+        if (cudaPointerGetAttributes(&at, (uint8_t*)p + off) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+        if (off == 0) dev = at.devicePointer;
+        else if ((uint8_t*)at.devicePointer != (uint8_t*)dev + off) return nullptr;
+    }
+    return dev;
+}
 
 // Bytes spanned by a strided tensor (offset of the last element + one element/block).
 size_t span_bytes(const b200_tensor* t) {
@@ -722,152 +763,143 @@ B200_API int b200_fattn_forward_host(const b200_tensor* q, const b200_tensor* k,
     const size_t kvlen_off = (ext && ext->kv_len) ? bump((size_t)q->ne[3] * 4) : 0;
     const size_t qlen_off = (ext && ext->q_len) ? bump((size_t)q->ne[3] * 4) : 0;
     const size_t dst_bytes = (size_t)dst->ne[0] * dst->ne[1] * dst->ne[2] * dst->ne[3] * 4;
-    const size_t dst_off = bump(dst_bytes);
+    // A pinned result is written by the kernels themselves, row by row over the link: no copy is left behind the last kernel,
+    // and none shares the copy engines with the uploads (12 uploads and 4 downloads together took 1213 us, 896 and 590 alone).
+    float* const dst_host = (float*)mapped_host(dst->data, dst_bytes);
+    const size_t dst_off = dst_host ? 0 : bump(dst_bytes);
 
-    // Batch entries are independent, so the call is pipelined over chunks of the batch dimension on two
-    // streams: the H2D copy of chunk i+1 overlaps the kernel and the D2H copy of chunk i (separate copy
-    // engines).  Chunking needs the batch dimension outermost in every batched operand; otherwise one chunk.
-    const int64_t B = q->ne[3];
-    auto batch_outermost = [](const b200_tensor* t) {
+    // The call is pipelined over chunks - batch entries, or heads of one - that are independent: the upload of chunk i + 1
+    // overlaps the kernel and the write-back of chunk i, and what is left behind the last upload is one chunk's kernel.  A
+    // chunk more costs its three copies their start - 4 us each on an idle link, 22 us while results are written the other
+    // way - and shortens what is left behind by out / n: the best number goes with the root of the time that the result takes
+    // (4 / 2 / 2 / 1 chunks measured best for 31 / 7.7 / 8.6 / 3 MB).  Chunking needs the chunked dimensions outermost in the
+    // operands that have them.
+    const int64_t B = q->ne[3], Hkv = k->ne[2];
+    auto outermost = [](const b200_tensor* t, int dim) {   // slices along `dim` (and the dims behind it) do not interleave
         b200_tensor one = *t;
-        one.ne[3] = 1;
-        return t->ne[3] == 1 || t->nb[3] >= span_bytes(&one);
+        for (int d = dim; d < 4; d++) one.ne[d] = 1;
+        return t->ne[dim] == 1 || t->nb[dim] >= span_bytes(&one);
     };
-    bool chunkable = B >= 2 && k->ne[3] == B;
-    for (int i = 0; i < NIN && chunkable; i++)
-        if (in[i] && in[i]->ne[3] != 1 && (in[i]->ne[3] != B || !batch_outermost(in[i]))) chunkable = false;
-    static const int max_chunks = [] {  // B200_HOST_CHUNKS=1..16 overrides the default pipeline depth
+    bool by_batch = B >= 2 && k->ne[3] == B;
+    for (int i = 0; i < NIN && by_batch; i++)
+        if (in[i] && in[i]->ne[3] != 1 && (in[i]->ne[3] != B || !outermost(in[i], 3))) by_batch = false;
+    bool by_heads = dst_host != nullptr && (by_batch || B == 1) && (!mask || mask->ne[2] == 1) && !plan.args.relpos && plan.args.n2 == 0;
+    for (int i = 0; i < 3 && by_heads; i++) by_heads = outermost(in[i], 2);
+    static const int forced_chunks = [] {  // B200_HOST_CHUNKS=1..16 overrides the pipeline depth
         const char* e = getenv("B200_HOST_CHUNKS");
         const int n = e ? atoi(e) : 0;
-        return n >= 1 && n <= 16 ? n : 4;
+        return n >= 1 && n <= kMaxHostChunks ? n : 0;
     }();
-    const int n_chunks = chunkable ? (int)(B < max_chunks ? B : max_chunks) : 1;
-    // Workspace of one chunk: a smaller batch may be split over more KV ranges than the whole call would be,
-    // so the split-decode workspace is sized for the chunk batches, not taken from the full plan.
-    size_t ws_need = plan.ws_bytes;
-    if (plan.kernel == B200_KERNEL_DECODE_SPLIT) {
-        for (int c = 0; c < n_chunks; c++) {
-            const int64_t b0 = B * c / n_chunks;
-            const int nb = (int)(B * (c + 1) / n_chunks - b0);
-            // the split count depends on operand alignment: describe the operands where the chunk will find them
-            // (arena offsets behind a notional 1 MiB-aligned base), not where the host buffers are
-            FattnArgs ca = plan.args;
-            View* views[4] = {&ca.q, &ca.k, &ca.v, &ca.mask};
-            for (int i = 0; i < 4; i++) {
-                if (!in[i]) continue;
-                b200_tensor t = *in[i];
-                t.data = (void*)(uintptr_t)(((size_t)1 << 20) + off[i] +
-                                            (n_chunks > 1 && in[i]->ne[3] != 1 ? (size_t)b0 * in[i]->nb[3] : 0));
-                *views[i] = make_view(&t);
+    const double out_us = (double)dst_bytes / 52e3;
+    int want = forced_chunks ? forced_chunks : (dst_host ? (int)lround(sqrt(out_us / 45.0)) : 4);
+    want = want < 1 ? 1 : (want > kMaxHostChunks ? kMaxHostChunks : want);
+    const int n_batch = by_batch ? (int)(B < want ? B : want) : 1;
+    int n_heads = by_heads ? (want + n_batch - 1) / n_batch : 1;   // groups of KV heads per batch group
+    if (n_heads > Hkv) n_heads = (int)Hkv;
+    while (n_batch * n_heads > kMaxHostChunks) n_heads--;
+    const int n_chunks = n_batch * n_heads;
+
+    // The operands of chunk c as its launch sees them, in an arena at `base`; the plan of that launch.
+    b200_tensor ct[NIN];
+    auto chunk_plan = [&](int c, uint8_t* base, Plan* cplan) {
+        const int64_t b0 = B * (c / n_heads) / n_batch, nb = B * (c / n_heads + 1) / n_batch - b0;
+        const int64_t g0 = Hkv * (c % n_heads) / n_heads, ng = Hkv * (c % n_heads + 1) / n_heads - g0;
+        const int64_t gqa = q->ne[2] / Hkv;
+        for (int i = 0; i < NIN; i++) {
+            if (!in[i]) continue;
+            ct[i] = *in[i];
+            size_t o = off[i];
+            if (n_batch > 1 && in[i]->ne[3] != 1) ct[i].ne[3] = nb, o += (size_t)b0 * in[i]->nb[3];
+            if (n_heads > 1 && i < 3) {
+                ct[i].ne[2] = i == 0 ? ng * gqa : ng;
+                o += (size_t)(i == 0 ? g0 * gqa : g0) * in[i]->nb[2];
             }
-            const int ns = decode_split_choose(ca, nb, di.sm_count);
-            const size_t w = decode_split_ws_bytes(nb, plan.args.Hkv, ns, plan.args.hd);
-            if (w > ws_need) ws_need = w;
+            ct[i].data = base + o;
         }
+        b200_fattn_ext dext;
+        memset(&dext, 0, sizeof(dext));
+        if (ext) {
+            dext = *ext;
+            dext.q_v = ext->q_v ? &ct[4] : nullptr;
+            dext.r = ext->r ? &ct[5] : nullptr;
+            dext.pos_bias_u = ext->pos_bias_u ? &ct[6] : nullptr;
+            dext.pos_bias_v = ext->pos_bias_v ? &ct[7] : nullptr;
+            dext.kv_len = ext->kv_len ? (const int32_t*)(base + kvlen_off) + b0 : nullptr;
+            dext.q_len = ext->q_len ? (const int32_t*)(base + qlen_off) + b0 : nullptr;
+        }
+        b200_tensor cdst = *dst;
+        cdst.ne[3] = nb, cdst.ne[1] = ct[0].ne[2];
+        cdst.nb[2] = cdst.nb[1] * cdst.ne[1], cdst.nb[3] = cdst.nb[2] * cdst.ne[2];
+        cdst.data = dst_host ? (uint8_t*)dst_host : base + dst_off;   // (aligned like the result: rows are whole multiples of 16 bytes or unaligned alike)
+        const int rc = make_plan(&ct[0], &ct[1], &ct[2], mask ? &ct[3] : nullptr, &cdst, params, ext ? &dext : nullptr, false, cplan);
+        if (rc != B200_OK) return rc;
+        cplan->args.dst = (float*)((uint8_t*)cdst.data + (size_t)b0 * dst->nb[3] + (size_t)(g0 * gqa) * dst->nb[1]);
+        cplan->args.dst_heads = (int)q->ne[2];
+        cplan->args.dst_on_host = dst_host ? 1 : 0;
+        return (int)B200_OK;
+    };
+    // Workspace of the largest chunk, planned at a notional 1 MiB-aligned arena (the split count goes by operand alignment).
+    // The chunks' kernels follow one another on one stream and share it.
+    size_t ws_need = 0;
+    Plan cplan;
+    for (int c = 0; c < n_chunks; c++) {
+        if ((rc = chunk_plan(c, (uint8_t*)((size_t)1 << 20), &cplan))) return rc;
+        if (cplan.ws_bytes > ws_need) ws_need = cplan.ws_bytes;
     }
-    const size_t ws_each = (ws_need + 255) / 256 * 256;
-    const size_t ws_off = bump(2 * ws_each);  // one per stream in flight
+    const size_t ws_off = bump(ws_need);
 
     Arena& ar = g_arena;
     cudaError_t e;
-    if (ar.device != dev) ar.release();
-    if (!ar.stream) {
-        if ((e = cudaStreamCreateWithFlags(&ar.stream, cudaStreamNonBlocking)) != cudaSuccess)
-            return cuda_fail(e, "cudaStreamCreate");
-        ar.device = dev;
-    }
+    if ((e = ar.open(dev)) != cudaSuccess) return cuda_fail(e, "streams and events of the host entry point");
     if (ar.cap < total) {
         if (ar.base) cudaFree(ar.base);
         ar.base = nullptr, ar.cap = 0;
         if ((e = cudaMalloc((void**)&ar.base, total)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(arena)");
         ar.cap = total;
     }
-    if (!ar.stream2 && (e = cudaStreamCreateWithFlags(&ar.stream2, cudaStreamNonBlocking)) != cudaSuccess)
-        return cuda_fail(e, "cudaStreamCreate");
-
-    cudaStream_t streams[2] = {ar.stream, ar.stream2};
 
     // Everything below enqueues asynchronous work that reads and writes the caller's host buffers.  Whatever goes
-    // wrong, the call leaves through ONE exit that first waits for both streams, so the caller may free or reuse
-    // its buffers as soon as it has the return code, and the event is always destroyed.
-    b200_tensor dt[NIN];
-    cudaEvent_t shared_ready = nullptr;
+    // wrong, the call leaves through ONE exit that first waits for the streams, so the caller may free or reuse
+    // its buffers as soon as it has the return code.
     auto enqueue_all = [&]() -> int {
         cudaError_t e;
-        // operands without a batch dimension (ne[3] == 1) are copied once, ahead of everything, on stream 0
-        for (int i = 0; i < NIN; i++) {
-            if (!in[i]) continue;
-            dt[i] = *in[i];
-            dt[i].data = ar.base + off[i];
-            if (n_chunks == 1 || in[i]->ne[3] == 1) {
-                if ((e = cudaMemcpyAsync(dt[i].data, in[i]->data, span_bytes(in[i]), cudaMemcpyHostToDevice, streams[0])) !=
-                    cudaSuccess)
-                    return cuda_fail(e, "cudaMemcpyAsync(H2D)");
-            }
-        }
-        if (ext && ext->kv_len &&
-            (e = cudaMemcpyAsync(ar.base + kvlen_off, ext->kv_len, (size_t)B * 4, cudaMemcpyHostToDevice, streams[0])) !=
-                cudaSuccess)
-            return cuda_fail(e, "cudaMemcpyAsync(kv_len)");
-        if (ext && ext->q_len &&
-            (e = cudaMemcpyAsync(ar.base + qlen_off, ext->q_len, (size_t)B * 4, cudaMemcpyHostToDevice, streams[0])) !=
-                cudaSuccess)
-            return cuda_fail(e, "cudaMemcpyAsync(q_len)");
-        if (n_chunks > 1) {
-            if ((e = cudaEventCreateWithFlags(&shared_ready, cudaEventDisableTiming)) != cudaSuccess)
-                return cuda_fail(e, "cudaEventCreate");
-            if ((e = cudaEventRecord(shared_ready, streams[0])) != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
-            if ((e = cudaStreamWaitEvent(streams[1], shared_ready, 0)) != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
-        }
+        auto upload = [&](size_t o, const void* src, size_t n) { return cudaMemcpyAsync(ar.base + o, src, n, cudaMemcpyHostToDevice, ar.in); };
+        // operands that every chunk needs go first
+        for (int i = 0; i < NIN; i++)
+            if (in[i] && (n_chunks == 1 || (in[i]->ne[3] == 1 && !(n_heads > 1 && i < 3)) || (n_batch == 1 && i >= 3)))
+                if ((e = upload(off[i], in[i]->data, span_bytes(in[i]))) != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(H2D)");
+        if (ext && ext->kv_len && (e = upload(kvlen_off, ext->kv_len, (size_t)B * 4)) != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(kv_len)");
+        if (ext && ext->q_len && (e = upload(qlen_off, ext->q_len, (size_t)B * 4)) != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(q_len)");
         for (int c = 0; c < n_chunks; c++) {
-            const int64_t b0 = B * c / n_chunks, b1 = B * (c + 1) / n_chunks, nb = b1 - b0;
-            cudaStream_t st = streams[c & 1];
-            b200_tensor ct[NIN];
-            for (int i = 0; i < NIN; i++) {
-                if (!in[i]) continue;
-                ct[i] = dt[i];
-                if (n_chunks > 1 && in[i]->ne[3] != 1) {
-                    ct[i].data = (uint8_t*)dt[i].data + (size_t)b0 * in[i]->nb[3];
-                    ct[i].ne[3] = nb;
-                    b200_tensor hview = *in[i];
-                    hview.ne[3] = nb;
-                    if ((e = cudaMemcpyAsync(ct[i].data, (const uint8_t*)in[i]->data + (size_t)b0 * in[i]->nb[3], span_bytes(&hview),
-                                             cudaMemcpyHostToDevice, st)) != cudaSuccess)
-                        return cuda_fail(e, "cudaMemcpyAsync(H2D chunk)");
-                }
-            }
-            b200_fattn_ext dext;
-            memset(&dext, 0, sizeof(dext));
-            if (ext) {
-                dext = *ext;
-                dext.q_v = ext->q_v ? &ct[4] : nullptr;
-                dext.r = ext->r ? &ct[5] : nullptr;
-                dext.pos_bias_u = ext->pos_bias_u ? &ct[6] : nullptr;
-                dext.pos_bias_v = ext->pos_bias_v ? &ct[7] : nullptr;
-                dext.kv_len = ext->kv_len ? (const int32_t*)(ar.base + kvlen_off) + b0 : nullptr;
-                dext.q_len = ext->q_len ? (const int32_t*)(ar.base + qlen_off) + b0 : nullptr;
-            }
-            b200_tensor cdst = *dst;
-            cdst.ne[3] = nb;
-            cdst.data = ar.base + dst_off + (size_t)b0 * dst->nb[3];
             Plan cplan;
-            int rc_c = make_plan(&ct[0], &ct[1], &ct[2], mask ? &ct[3] : nullptr, &cdst, params, ext ? &dext : nullptr, false, &cplan);
+            const int rc_c = chunk_plan(c, ar.base, &cplan);
             if (rc_c != B200_OK) return rc_c;
-            if (cplan.ws_bytes > ws_each) return B200_E_WORKSPACE;
-            rc_c = do_launch(cplan, cplan.ws_bytes ? ar.base + ws_off + (size_t)(c & 1) * ws_each : nullptr, cplan.ws_bytes, st);
-            if (rc_c != B200_OK) return rc_c;
-            if ((e = cudaMemcpyAsync((uint8_t*)dst->data + (size_t)b0 * dst->nb[3], cdst.data, (size_t)nb * dst->nb[3],
-                                     cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+            if (cplan.ws_bytes > ws_need) return B200_E_WORKSPACE;
+            for (int i = 0; i < NIN && n_chunks > 1; i++) {
+                if (!in[i] || !((n_batch > 1 && in[i]->ne[3] != 1 && (i < 3 || c % n_heads == 0)) || (n_heads > 1 && i < 3))) continue;
+                const size_t o = (size_t)((uint8_t*)ct[i].data - ar.base);
+                if ((e = upload(o, (const uint8_t*)in[i]->data + (o - off[i]), span_bytes(&ct[i]))) != cudaSuccess)
+                    return cuda_fail(e, "cudaMemcpyAsync(H2D chunk)");
+            }
+            if ((e = cudaEventRecord(ar.arrived[c], ar.in)) != cudaSuccess || (e = cudaStreamWaitEvent(ar.compute, ar.arrived[c], 0)) != cudaSuccess)
+                return cuda_fail(e, "chunk event");
+            const int rc_l = do_launch(cplan, cplan.ws_bytes ? ar.base + ws_off : nullptr, cplan.ws_bytes, ar.compute);
+            if (rc_l != B200_OK) return rc_l;
+            if (dst_host) continue;
+            if ((e = cudaEventRecord(ar.computed[c], ar.compute)) != cudaSuccess || (e = cudaStreamWaitEvent(ar.out, ar.computed[c], 0)) != cudaSuccess)
+                return cuda_fail(e, "chunk event");
+            const int64_t b0 = B * c / n_batch, nb = B * (c + 1) / n_batch - b0;   // (heads are only chunked with a pinned result)
+            if ((e = cudaMemcpyAsync((uint8_t*)dst->data + (size_t)b0 * dst->nb[3], ar.base + dst_off + (size_t)b0 * dst->nb[3],
+                                     (size_t)nb * dst->nb[3], cudaMemcpyDeviceToHost, ar.out)) != cudaSuccess)
                 return cuda_fail(e, "cudaMemcpyAsync(D2H)");
         }
         return B200_OK;
     };
     const int rc_enqueue = enqueue_all();
-    const cudaError_t e0 = cudaStreamSynchronize(streams[0]), e1 = cudaStreamSynchronize(streams[1]);
-    if (shared_ready) cudaEventDestroy(shared_ready);
+    const cudaError_t done[3] = {cudaStreamSynchronize(ar.in), cudaStreamSynchronize(ar.compute), cudaStreamSynchronize(ar.out)};
     if (rc_enqueue != B200_OK) return rc_enqueue;
-    if (e0 != cudaSuccess) return cuda_fail(e0, "cudaStreamSynchronize");
-    if (e1 != cudaSuccess) return cuda_fail(e1, "cudaStreamSynchronize");
+    for (cudaError_t d : done)
+        if (d != cudaSuccess) return cuda_fail(d, "cudaStreamSynchronize");
     return B200_OK;
 }
 

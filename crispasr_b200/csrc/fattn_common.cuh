@@ -19,7 +19,9 @@ struct View {
 
 struct FattnArgs {
     View q, k, v, mask, qv, r;
-    float* dst;  // contiguous [hd, H, Tq, B]
+    float* dst;           // contiguous [hd, dst_heads, Tq, B], at the first of this launch's H heads
+    int32_t dst_heads;    // H, or more where a launch computes some of the heads
+    int32_t dst_on_host;  // pinned host memory: plain stores only
     int32_t hd, Tq, H, B;
     int32_t Lk, Hkv, gqa, bq;  // bq = B / Bk
     int32_t mask_ne2, mask_ne3, r_ne3, has_mask;

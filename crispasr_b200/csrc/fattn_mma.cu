@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kThreads) fattn_tile_mma_kernel(const FattnArg
     if (q0 >= tq_b) {
         for (int idx = tid; idx < BM * a.hd; idx += kThreads) {
             const int iq = q0 + idx / a.hd;
-            if (iq < a.Tq) a.dst[(((int64_t)b * a.Tq + iq) * a.H + h) * a.hd + idx % a.hd] = 0.0f;
+            if (iq < a.Tq) a.dst[(((int64_t)b * a.Tq + iq) * a.dst_heads + h) * a.hd + idx % a.hd] = 0.0f;
         }
         return;
     }
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kThreads) fattn_tile_mma_kernel(const FattnArg
     for (int rI = 0; rI < 2; rI++) {
         const int iq = q0 + warp * 16 + g + rI * 8;
         if (iq >= a.Tq) continue;
-        float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * a.hd;
+        float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * a.hd;
         const float inv = rI ? inv1 : inv0;
         const bool live = iq < tq_b;   // padding rows get literal zeros, whatever their Q rows held
 #pragma unroll
@@ -696,7 +696,7 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
             int iq, hq;
             row_to_query(a, hk, rr, iq, hq);
             const float inv = (L > 0.0f && iq < tq_b) ? 1.0f / L : 0.0f;
-            float* drow = a.dst + (((int64_t)b * a.Tq + iq) * a.H + hq) * a.hd;
+            float* drow = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + hq) * a.hd;
             if (lane < G) {
                 if (a.hd == HD) {
                     *reinterpret_cast<float4*>(drow + 4 * lane) = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
@@ -746,7 +746,7 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
             int iq, hq;
             row_to_query(a, hk, rr, iq, hq);
             const float inv = (L > 0.0f && iq < tq_b) ? 1.0f / L : 0.0f;
-            *reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + hq) * HD + 4 * cg) =
+            *reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + hq) * HD + 4 * cg) =
                 make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);   // the cluster form is offered for a.hd == HD only
         }
     }
@@ -1765,7 +1765,7 @@ __global__ void __launch_bounds__(kThreads) fattn_merge_kernel(const FattnArgs a
     }
     int iq, hq;
     row_to_query(a, hk, rr, iq, hq);
-    float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.H + hq) * a.hd;
+    float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + hq) * a.hd;
     const float inv = (L > 0.0f && iq < q_rows_of(a, b)) ? 1.0f / L : 0.0f;
 #pragma unroll
     for (int i = 0; i < HD / 32; i++) {

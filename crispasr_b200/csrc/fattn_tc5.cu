@@ -596,7 +596,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     if (n_tiles == 0) {  // nothing to attend to: zeros
         if (tid < kTile && q0 + tid < rows_total) {
             const int iq = (q0 + tid) / a.gqa, h = hk * a.gqa + (q0 + tid) % a.gqa;
-            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD);
+            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * HD);
 #pragma unroll
             for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -995,7 +995,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             // dead rows are written as literal zeros (whatever the padding row of Q held never reaches dst), rows
             // outside the tensor not at all.  The K/V stages are free once the last MMA has completed: they stage O.
             const float inv = row_live && l_run > 0.0f ? 1.0f / l_run : 0.0f;
-            float* out = (row_live || row_zero) ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.H + h) * HD : nullptr;
+            float* out = (row_live || row_zero) ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.dst_heads + h) * HD : nullptr;
             float* stage = reinterpret_cast<float*>(smem_gen + TILE_BYTES) + warp * 32 * HD;
             if (o_tma) {
                 // A warp's 32 packed rows x 32 columns are a box [32 columns, gqa heads, 32 / gqa tokens] of
@@ -1203,7 +1203,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     const int n_tiles = (len_b > 0 && q0 < tq_b) ? (len_b + kTile - 1) / kTile : 0;
     if (n_tiles == 0) {
         if (tid < kTile && q0 + tid < a.Tq) {
-            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + q0 + tid) * a.H + h) * HD);
+            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + q0 + tid) * a.dst_heads + h) * HD);
 #pragma unroll
             for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -1598,7 +1598,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             tc_fence_after();
             const float l_tot = l_run + exchange(l_run);   // a failed wait has set the abort flag: the host reports it
             const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-            float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD + ch * 64;
+            float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * HD + ch * 64;
             const bool wide = (reinterpret_cast<uintptr_t>(a.dst) & 31) == 0;
 #pragma unroll
             for (int q4 = 0; q4 < 2; q4++) {
@@ -1679,7 +1679,7 @@ bool encode_o_map(CUtensorMap* m, const FattnArgs& a) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)a.hd, (cuuint64_t)a.H, (cuuint64_t)a.Tq, (cuuint64_t)a.B};
-    const cuuint64_t strides[3] = {(cuuint64_t)a.hd * 4, (cuuint64_t)a.hd * 4 * a.H, (cuuint64_t)a.hd * 4 * a.H * a.Tq};
+    const cuuint64_t strides[3] = {(cuuint64_t)a.hd * 4, (cuuint64_t)a.hd * 4 * a.dst_heads, (cuuint64_t)a.hd * 4 * a.dst_heads * a.Tq};
     const cuuint32_t box[4] = {32, (cuuint32_t)a.gqa, (cuuint32_t)(32 / a.gqa), 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.dst, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1796,7 +1796,7 @@ int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen)
     }
     CUtensorMap tmQ = tmK, tmO = tmK;
     const bool q_tma = a.q.type == B200_TYPE_F16 && q_box_ok(a) && encode_q_map(&tmQ, a);
-    const bool o_tma = gqa_box(a) && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);
+    const bool o_tma = gqa_box(a) && !a.dst_on_host && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);
     FattnArgs as = a;
     const int n_q = (a.Tq * a.gqa + kTile - 1) / kTile;
     as.n_splits = h64_splits((long)n_q * a.Hkv * a.B, (a.Lk + kH64Keys - 1) / kH64Keys);
@@ -1834,7 +1834,7 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     if (a.q.type == B200_TYPE_F16 && q_box_ok(a)) q_tma = encode_q_map(&tmQ, a) ? 1 : 0;
     else if (RAW_INST && a.q.type == B200_TYPE_F32 && q_box_ok(a)) q_tma = encode_q_map(&tmQ, a) ? 2 : 0;   // F32 rows: raw tile into stages not needed yet, converted from shared memory
     CUtensorMap tmO = tmK;
-    const bool o_tma = gqa_box(a) && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);   // a warp's rows of the output are a box of dst
+    const bool o_tma = gqa_box(a) && !a.dst_on_host && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);   // a warp's rows of the output are a box of dst
     cudaError_t e;
     dim3 grid((a.Tq * a.gqa + kTile - 1) / kTile, a.Hkv, a.B);   // packed (query, group head) rows per KV head
     // launch_inst is instantiated per kernel (the kernels share one function-pointer type, so a generic lambda would

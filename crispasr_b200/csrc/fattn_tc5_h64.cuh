@@ -91,7 +91,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     if (n_all == 0) {  // nothing to attend to: zeros
         if (split == 0 && tid < kTile && q0 + tid < rows_total) {
             const int iq = (q0 + tid) / a.gqa, h = hk * a.gqa + (q0 + tid) % a.gqa;
-            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD);
+            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * HD);
 #pragma unroll
             for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -358,7 +358,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                     tma_store_commit_and_wait_read();
                 }
             } else {
-                float* out = q0 + r < rows_total ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.H + h) * HD : nullptr;
+                float* out = q0 + r < rows_total ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.dst_heads + h) * HD : nullptr;
                 store_o_rows_coalesced<HD>(stage, lane, out);
             }
         }
@@ -413,7 +413,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                 if (q0 + row < rows_total) {
                     const int iq = (q0 + row) / a.gqa, h = hk * a.gqa + (q0 + row) % a.gqa;
                     const bool live = q0 + row < rows_live;
-                    reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.H + h) * HD)[g4] =
+                    reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * HD)[g4] =
                         live ? make_float4(o.x * inv[i], o.y * inv[i], o.z * inv[i], o.w * inv[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }

@@ -828,3 +828,22 @@ def test_prefill_shared_query_tiles(b200, orc, T, H, gqa, form, q_f32):
             ref[b, n:] = 0.0
     assert_close(got, ref, f"shared tiles T={T} H={H} gqa={gqa} {form}")
     assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,Tq,Lk,hd", [(1, 20, 20, 1500, 1500, 64), (2, 16, 4, 1100, 1100, 128), (3, 8, 2, 300, 1300, 128), (2, 20, 20, 5, 1500, 64), (1, 6, 6, 650, 650, 80)])
+@pytest.mark.parametrize("q_f32", [False, True])
+def test_host_entry_point_pinned_result(b200, orc, B, H, Hkv, Tq, Lk, hd, q_f32):
+    """A pinned result is written by the kernels and lets the call run over chunks of heads: one to three entries, grouped
+    heads, each kernel family (head dims 64 and 128 on the tensor path, decode rows, a padded head dim), lengths per entry;
+    a pageable result of the same operands is staged and must agree."""
+    rng = np.random.default_rng(B * 1000 + H + hd)
+    q = randn_f16(rng, (B, H, Tq, hd))
+    k, v = (randn_f16(rng, (B, Hkv, Lk, hd)) for _ in "kv")
+    lens = np.array([Lk, 17, Lk - 1][:B], np.int32)
+    kw = dict(scale=hd ** -0.5, kv_len=torch.from_numpy(lens))
+    args = [torch.from_numpy(x.astype(np.float32) if q_f32 and i == 0 else x).pin_memory() for i, x in enumerate((q, k, v))]
+    out = torch.full((B, Tq, H, hd), float("nan"), dtype=torch.float32).pin_memory()
+    assert b200.flash_attn_ext_host(*args, out=out, **kw) is out
+    ref = orc.flash_attn_ext(q, k, v, scale=hd ** -0.5, kv_len=lens)
+    assert_close(out.numpy(), ref, "host entry point, pinned result")
+    assert_close(b200.flash_attn_ext_host(*args, **kw).numpy(), ref, "host entry point, pageable result")
