@@ -41,6 +41,7 @@ struct FattnArgs {
     const float* bias_v;  // the same for the Q of the relative-position bias
     // split-KV
     int32_t n_splits;
+    int32_t splits_mul;  // (x * splits_mul) >> 16 == x / n_splits for x < 4096 and up to eight splits
     int32_t wide;  // split-KV over a Q8_0 cache: eight warps per CTA instead of four
     float* ws_o;   // [B][Hkv][n_splits][16][hd]
     float* ws_ml;  // [B][Hkv][n_splits][16][2]

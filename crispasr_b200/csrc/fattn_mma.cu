@@ -437,48 +437,47 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// cp.async copy of rows [row0, row0+64) x HD halves into a swizzled fp16 tile; rows >= row_hi are zero-filled.
-// IDX: logical row `grow` lives in cache row index[grow] (clamped to the pool): the gather of ext->kv_index.
-template <int HD, bool IDX = false>
-__device__ __forceinline__ void issue_tile_f16(__half* sm, const uint8_t* base, int64_t nb1, int row0, int row_hi, int tid,
-                                               const int32_t* index = nullptr, int pool_rows = 0) {
-    constexpr int CPR = HD / 8;
-#pragma unroll
-    for (int it = 0; it < kDecBN * CPR / kThreads; it++) {
-        const int idx = tid + it * kThreads;
-        const int row = idx / CPR, ch = idx % CPR;
-        const int grow = row0 + row;
-        const bool valid = grow < row_hi;
-        int src = grow;
-        if (IDX && valid) src = min(max(__ldg(index + grow), 0), pool_rows - 1);
-        cp_async16(tile_addr<HD>(sm, row, ch), base + (valid ? (int64_t)src * nb1 + ch * 16 : 0), valid);
-    }
-}
-
-// The same copy for a gathered tile whose cache rows were looked up one tile ahead: `pre[it]` is the cache row of
-// this thread's it-th 16-byte piece (see load_tile_index), so the copies do not wait for the list.
+// The 16-byte pieces of a 64-row F16 tile that one thread copies: column chunk tid % (HD/8) of every kRows-th row from
+// tid / (HD/8) on.  The row step is a multiple of 8, so the place in the swizzled tile advances by a constant and the
+// source by one addition.  With a row, an index and a 64-bit product worked out per piece, issuing the first three tiles took
+// 2.1 k of the 9.7 k clk between the dependency wait and the end of a small CTA, and a good part of every tile after them.
 template <int HD>
-__device__ __forceinline__ void load_tile_index(int (&pre)[kDecBN * (HD / 8) / kThreads], const int32_t* index, int row0, int row_hi,
-                                                int tid) {
-    constexpr int CPR = HD / 8;
-#pragma unroll
-    for (int it = 0; it < kDecBN * CPR / kThreads; it++) {
-        const int grow = row0 + (tid + it * kThreads) / CPR;
-        pre[it] = grow < row_hi ? __ldg(index + grow) : 0;   // clamped where it is used: nothing here waits for the load
+struct TilePieces {
+    static constexpr int CPR = HD / 8, kRows = kThreads / CPR, N = kDecBN / kRows;   // pieces per thread
+    int row;        // first row
+    uint32_t dst;   // byte offset in the tile
+    __device__ __forceinline__ explicit TilePieces(int tid) {
+        row = tid / CPR;
+        dst = (uint32_t)((row * CPR + swz<HD>(row, tid % CPR)) * 16);
     }
-}
-template <int HD>
-__device__ __forceinline__ void issue_tile_f16_pre(__half* sm, const uint8_t* base, int64_t nb1, int row0, int row_hi, int tid,
-                                                   const int (&pre)[kDecBN * (HD / 8) / kThreads], int pool_rows) {
-    constexpr int CPR = HD / 8;
+    // rows [row0, row0 + 64) at `base` (which includes this thread's column); rows at or beyond row_hi are zero-filled
+    __device__ __forceinline__ void copy(uint32_t tile, const uint8_t* base, int64_t nb1, int row0, int row_hi) const {
+        const uint8_t* p = base + (int64_t)(row0 + row) * nb1;
+        const int left = row_hi - (row0 + row);
 #pragma unroll
-    for (int it = 0; it < kDecBN * CPR / kThreads; it++) {
-        const int idx = tid + it * kThreads;
-        const int row = idx / CPR, ch = idx % CPR;
-        const bool valid = row0 + row < row_hi;
-        cp_async16(tile_addr<HD>(sm, row, ch), base + (valid ? (int64_t)min(max(pre[it], 0), pool_rows - 1) * nb1 + ch * 16 : 0), valid);
+        for (int i = 0; i < N; i++) {
+            const bool valid = i * kRows < left;
+            cp_async16(tile + dst + i * kRows * CPR * 16, valid ? p : base, valid);
+            p += kRows * nb1;
+        }
     }
-}
+    // the same for gathered rows: idx[i] is the cache row of piece i
+    __device__ __forceinline__ void gather(uint32_t tile, const uint8_t* base, int64_t nb1, int row0, int row_hi, const int (&idx)[N], int pool_rows) const {
+        const int left = row_hi - (row0 + row);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const bool valid = i * kRows < left;
+            cp_async16(tile + dst + i * kRows * CPR * 16, base + (valid ? (int64_t)min(max(idx[i], 0), pool_rows - 1) * nb1 : 0), valid);
+        }
+    }
+    __device__ __forceinline__ void load_index(int (&idx)[N], const int32_t* index, int row0, int row_hi) const {
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int grow = row0 + row + i * kRows;
+            idx[i] = grow < row_hi ? __ldg(index + grow) : 0;   // clamped where it is used: nothing here waits for the load
+        }
+    }
+};
 
 // ---- bulk copies (one instruction per contiguous range) with a per-warp mbarrier per stage ----
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -531,11 +530,20 @@ __device__ __forceinline__ int32_t peek(const int32_t* p) {
     asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
+// x / n_splits: the cluster forms (at most eight splits) without a division.
+__device__ __forceinline__ int div_splits(const FattnArgs& a, int x) {
+    return a.n_splits == 1 ? x : (a.n_splits <= 8 && x < 4096 ? (x * a.splits_mul) >> 16 : x / a.n_splits);
+}
+// Eight consecutive floats, as two raw 16-byte pieces, rounded to fp16.
+__device__ __forceinline__ uint4 f32x8_to_half(const uint4& a, const uint4& b) {
+    return make_uint4(pack_half2(__uint_as_float(a.x), __uint_as_float(a.y)), pack_half2(__uint_as_float(a.z), __uint_as_float(a.w)),
+                      pack_half2(__uint_as_float(b.x), __uint_as_float(b.y)), pack_half2(__uint_as_float(b.z), __uint_as_float(b.w)));
+}
 // Logical keys [lo, hi) of this CTA's first tiles, as far as they can be told before the wait.
 __device__ __forceinline__ void peek_range(const FattnArgs& a, int b, int split, int& lo, int& hi) {
     const int cap = a.kv_index ? a.kv_index_stride : a.Lk;
     const int len = a.kv_len ? min(max(peek(a.kv_len + b), 0), cap) : cap;
-    const int n_tiles = (len + kDecBN - 1) / kDecBN, tps = (n_tiles + a.n_splits - 1) / a.n_splits;
+    const int n_tiles = (len + kDecBN - 1) / kDecBN, tps = div_splits(a, n_tiles + a.n_splits - 1);
     lo = split * tps * kDecBN;
     hi = min(len, lo + min(tps, kPrefetchTiles) * kDecBN);
 }
@@ -651,8 +659,8 @@ __host__ __device__ constexpr size_t cluster_push_bytes(int hd, int rows) { retu
 
 // Write-out shared by the split-KV decode kernels.  `slab` holds the four warps' partial O [4][16][HD + 4], each scaled
 // to its own warp's running maximum s_m[w][row] with row sum s_l[w][row]; the CTA has passed a barrier since they were
-// written.  One warp per live row, one 16-byte column group per lane, the log-sum-exp merge of the four partials on
-// the way; the result goes
+// written.  One 16-byte column group of the R live rows per thread, the log-sum-exp merge of the warps' partials on the way
+// (a warp per row left five rows of head_dim 64 to two passes of half a warp each); the result goes
 //   * n_splits == 1: to dst, divided by the row sum;
 //   * workspace form: to this split's [16][HD] partial and (M, L) pairs, for the merge kernel;
 //   * cluster form: the column groups of the R x HD result are dealt round-robin to the CTAs of the cluster; every CTA
@@ -668,55 +676,47 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
                                                  const float (*s_l)[kDecRows], uint8_t* recv, int R, int b, int hk, int split,
                                                  int tq_b, int tid) {
     constexpr int STRIDE = HD + 4, G = HD / 4;
-    const int warp = tid >> 5, lane = tid & 31;
     const float ninf = -INFINITY;
     const bool push = a.n_splits > 1 && a.cluster_merge;
     float4* recv_o = reinterpret_cast<float4*>(recv);
     float2* recv_ml = reinterpret_cast<float2*>(recv_o + (R * G + 8));
-    const int n_groups = R * G, slots = (n_groups + a.n_splits - 1) / a.n_splits;
+    const int n_groups = R * G, slots = div_splits(a, n_groups + a.n_splits - 1);
     if (push) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster has started
-    for (int rr = warp; rr < R; rr += NW) {
+    for (int grp = tid; grp < n_groups; grp += 32 * NW) {
+        const int rr = grp / G, cg = grp % G;
         float m[NW], w[NW], M = ninf, L = 0.0f;
+        float4 x[NW], v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int i = 0; i < NW; i++) m[i] = s_m[i][rr], M = fmaxf(M, m[i]);
+        for (int i = 0; i < NW; i++) m[i] = s_m[i][rr], x[i] = *reinterpret_cast<const float4*>(slab + (i * ROWS + rr) * STRIDE + 4 * cg);
 #pragma unroll
-        for (int i = 0; i < NW; i++) {
+        for (int i = 0; i < NW; i++) M = fmaxf(M, m[i]);
+#pragma unroll
+        for (int i = 0; i < NW; i++) {   // a warp that saw no live key holds zeros and weight 0
             w[i] = m[i] == ninf ? 0.0f : fast_ex2(m[i] - M);
             L = fmaf(w[i], s_l[i][rr], L);
-        }
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (lane < G) {
-#pragma unroll
-            for (int i = 0; i < NW; i++) {   // a warp that saw no live key holds zeros and weight 0
-                const float4 x = *reinterpret_cast<const float4*>(slab + (i * ROWS + rr) * STRIDE + 4 * lane);
-                v.x = fmaf(w[i], x.x, v.x), v.y = fmaf(w[i], x.y, v.y), v.z = fmaf(w[i], x.z, v.z), v.w = fmaf(w[i], x.w, v.w);
-            }
+            v.x = fmaf(w[i], x[i].x, v.x), v.y = fmaf(w[i], x[i].y, v.y), v.z = fmaf(w[i], x[i].z, v.z), v.w = fmaf(w[i], x[i].w, v.w);
         }
         if (a.n_splits == 1) {
             int iq, hq;
             row_to_query(a, hk, rr, iq, hq);
             const float inv = (L > 0.0f && iq < tq_b) ? 1.0f / L : 0.0f;
             float* drow = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + hq) * a.hd;
-            if (lane < G) {
-                if (a.hd == HD) {
-                    *reinterpret_cast<float4*>(drow + 4 * lane) = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
-                } else {   // a head dim padded up to HD: the row is a.hd floats long
-                    const float vv[4] = {v.x, v.y, v.z, v.w};
+            if (a.hd == HD) {
+                *reinterpret_cast<float4*>(drow + 4 * cg) = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+            } else {   // a head dim padded up to HD: the row is a.hd floats long
+                const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if (4 * lane + j < a.hd) drow[4 * lane + j] = vv[j] * inv;
-                }
+                for (int j = 0; j < 4; j++)
+                    if (4 * cg + j < a.hd) drow[4 * cg + j] = vv[j] * inv;
             }
         } else if (a.cluster_merge) {
-            if (lane < G) {
-                const int grp = rr * G + lane;   // owner grp % n_splits, its slot grp / n_splits
-                st_peer_v4(peer_addr(recv_o + split * slots + grp / a.n_splits, grp % a.n_splits), v);
-            }
-            if (lane < a.n_splits) st_peer_v2(peer_addr(recv_ml + split * kDecRows + rr, lane), M, L);
+            const int slot = (grp * a.splits_mul) >> 16, owner = grp - slot * a.n_splits;   // grp / n_splits, grp % n_splits
+            st_peer_v4(peer_addr(recv_o + split * slots + slot, owner), v);
+            if (cg < a.n_splits) st_peer_v2(peer_addr(recv_ml + split * kDecRows + rr, cg), M, L);
         } else {
             const int64_t unit = ((int64_t)b * a.Hkv + hk) * a.n_splits + split;
-            if (lane < G) *reinterpret_cast<float4*>(a.ws_o + unit * kDecRows * HD + rr * HD + 4 * lane) = v;   // live rows only: the merge kernel reads no others
-            if (lane == 0) a.ws_ml[(unit * kDecRows + rr) * 2] = M, a.ws_ml[(unit * kDecRows + rr) * 2 + 1] = L;
+            *reinterpret_cast<float4*>(a.ws_o + unit * kDecRows * HD + rr * HD + 4 * cg) = v;   // live rows only: the merge kernel reads no others
+            if (cg == 0) a.ws_ml[(unit * kDecRows + rr) * 2] = M, a.ws_ml[(unit * kDecRows + rr) * 2 + 1] = L;
         }
     }
     if (push) {
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
     const int n_past = n_past_of(a, len_b, tq_b);
     if (a.causal) kmax = min(kmax, n_past + tq_b);
     const int n_tiles = (kmax + kDecBN - 1) / kDecBN;
-    const int tps = (n_tiles + a.n_splits - 1) / a.n_splits;
+    const int tps = div_splits(a, n_tiles + a.n_splits - 1);
     const int tile_lo = split * tps, tile_hi = min(n_tiles, tile_lo + tps);
     // staged mask: the row of the mask this thread copies pieces of (the head and batch broadcasts are remainders by
     // run-time values: computed once, not per tile)
@@ -827,9 +827,37 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         row_to_query(a, hk, tid >> 3, iq, hq);
         mask_row = a.mask.p + (int64_t)iq * a.mask.nb1 + (int64_t)(hq % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3;
     }
-    int pre_rows[kDecBN * (HD / 8) / kThreads];   // gathered keys: this thread's cache rows of the next tile to be issued
-    if (IDX && tile_lo < tile_hi) load_tile_index<HD>(pre_rows, index, tile_lo * kDecBN, len_b, tid);
-    auto issue = [&](int tile) {
+    // Q rows (tiny): requested ahead of the copies, stored behind them; rows >= R are zero
+    constexpr int Q_PER = (kDecRows * (HD / 8) + kThreads - 1) / kThreads;
+    // (raw 16-byte pieces where the rows allow it: the conversion would wait for them ahead of the copies)
+    uint4 q_val[Q_PER], q_hi[Q_PER];
+    const bool q_f32 = a.q.type == B200_TYPE_F32 && a.q.vec16 && a.hd == HD;
+#pragma unroll
+    for (int i = 0; i < Q_PER; i++) {
+        const int idx = tid + i * kThreads, rr = idx / (HD / 8), ch = idx % (HD / 8);
+        q_val[i] = q_hi[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (rr < R) {
+            int iq, hq;
+            row_to_query(a, hk, rr, iq, hq);
+            const uint8_t* rowp = a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3;
+            if (q_f32) {
+                q_val[i] = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * ch);
+                q_hi[i] = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * ch + 1);
+            } else {
+                q_val[i] = load8_as_half(rowp, a.q.type, ch * 8, a.hd, a.q.vec16);
+            }
+        }
+    }
+    const TilePieces<HD> pieces(tid);
+    const uint8_t *kcol = kbase + tid % (HD / 8) * 16, *vcol = vbase + tid % (HD / 8) * 16;
+    // gathered keys: the cache rows of the first tiles, requested together, then of the next tile to be issued
+    int first_rows[IDX ? NS - 1 : 1][TilePieces<HD>::N], pre_rows[TilePieces<HD>::N];
+    if (IDX) {
+#pragma unroll
+        for (int s0 = 0; s0 < NS - 1; s0++) pieces.load_index(first_rows[s0], index, (tile_lo + s0) * kDecBN, min(len_b, tile_hi * kDecBN));
+        pieces.load_index(pre_rows, index, (tile_lo + NS - 1) * kDecBN, min(len_b, tile_hi * kDecBN));
+    }
+    auto issue = [&](int tile, const int (&rows)[TilePieces<HD>::N]) {   // rows: the tile's cache rows, if gathered
         if (MODE == kDecAsyncQ8) {
             if (tile < tile_hi && lane == 0) {
                 const int stage = (tile - tile_lo) % NS;
@@ -840,14 +868,13 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         }
         if (tile < tile_hi) {
             const int stage = (tile - tile_lo) % NS;
+            const uint32_t st = smem_u32(sKV) + stage * 2 * TILE_HALVES * (int)sizeof(__half);
             if (IDX) {
-                // tiles are issued in order: the list entries of this one were requested when the previous one was issued
-                issue_tile_f16_pre<HD>(sKV + stage * 2 * TILE_HALVES, kbase, a.k.nb1, tile * kDecBN, len_b, tid, pre_rows, a.Lk);
-                issue_tile_f16_pre<HD>(sKV + stage * 2 * TILE_HALVES + TILE_HALVES, vbase, a.v.nb1, tile * kDecBN, len_b, tid, pre_rows, a.Lk);
-                if (tile + 1 < tile_hi) load_tile_index<HD>(pre_rows, index, (tile + 1) * kDecBN, len_b, tid);
+                pieces.gather(st, kcol, a.k.nb1, tile * kDecBN, len_b, rows, a.Lk);
+                pieces.gather(st + TILE_HALVES * (int)sizeof(__half), vcol, a.v.nb1, tile * kDecBN, len_b, rows, a.Lk);
             } else {
-                issue_tile_f16<HD, false>(sKV + stage * 2 * TILE_HALVES, kbase, a.k.nb1, tile * kDecBN, len_b, tid);
-                issue_tile_f16<HD, false>(sKV + stage * 2 * TILE_HALVES + TILE_HALVES, vbase, a.v.nb1, tile * kDecBN, len_b, tid);
+                pieces.copy(st, kcol, a.k.nb1, tile * kDecBN, len_b);
+                pieces.copy(st + TILE_HALVES * (int)sizeof(__half), vcol, a.v.nb1, tile * kDecBN, len_b);
             }
             if (stage_mask && tid < R * 8) {
                 const int rr = tid >> 3, ch = tid & 7;
@@ -862,21 +889,19 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         cp_async_commit();
     };
     if (MODE != kDecSync) {
+        if constexpr (IDX) {
 #pragma unroll
-        for (int s0 = 0; s0 < NS - 1; s0++) issue(tile_lo + s0);
-    }
-
-    // Q rows (tiny): one 8-element chunk per loop step
-    for (int idx = tid; idx < kDecRows * (HD / 8); idx += kThreads) {
-        const int rr = idx / (HD / 8), ch = idx % (HD / 8);
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (rr < R) {
-            int iq, hq;
-            row_to_query(a, hk, rr, iq, hq);
-            val = load8_as_half(a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3,
-                                a.q.type, ch * 8, a.hd, a.q.vec16);
+            for (int s0 = 0; s0 < NS - 1; s0++) issue(tile_lo + s0, first_rows[s0]);
+        } else {
+#pragma unroll 1
+            for (int s0 = 0; s0 < NS - 1; s0++) issue(tile_lo + s0, pre_rows);
         }
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (rr * (HD / 8) + swz<HD>(rr, ch)) * 16) = val;
+    }
+#pragma unroll
+    for (int i = 0; i < Q_PER; i++) {
+        const int idx = tid + i * kThreads, rr = idx / (HD / 8), ch = idx % (HD / 8);
+        if (q_f32) q_val[i] = f32x8_to_half(q_val[i], q_hi[i]);
+        if (rr < kDecRows) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (rr * (HD / 8) + swz<HD>(rr, ch)) * 16) = q_val[i];
     }
     __syncthreads();
     uint32_t qf[HD / 16][4];
@@ -916,7 +941,8 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         } else if (MODE == kDecAsyncF16) {
             cp_async_wait<NS - 2>();
             __syncthreads();             // tile `tile` has landed for every thread; stage of tile-1 is free
-            issue(tile + NS - 1);
+            issue(tile + NS - 1, pre_rows);
+            if (IDX && tile + NS < tile_hi) pieces.load_index(pre_rows, index, (tile + NS) * kDecBN, len_b);
             const int stage = (tile - tile_lo) % NS;
             sK = sKV + stage * 2 * TILE_HALVES, sV = sK + TILE_HALVES;
         } else {
@@ -945,7 +971,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
             const int stage = (tile - tile_lo) % NS;
             dequant_tile_q8<HD>(sRaw + stage * 2 * RAW_BYTES + RAW_BYTES, sKV, len_b - k0, warp, lane);
             __syncwarp();
-            issue(tile + NS - 1);        // overwrites the raw stage of tile-1, which this warp dequantised an iteration ago
+            issue(tile + NS - 1, pre_rows);        // overwrites the raw stage of tile-1, which this warp dequantised an iteration ago
         }
         float rmax[2] = {ninf, ninf};
         // common case (no mask, no softcap, every key of the tile visible to every row): one multiply per score
@@ -1458,15 +1484,23 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
     // with the lengths, ahead of everything that waits for them.
     static_assert(8 * (HD / 8) <= 32 * NW, "one chunk per thread");
     const int q_row = tid / (HD / 8), q_ch = tid % (HD / 8);
-    uint4 q_val = make_uint4(0u, 0u, 0u, 0u);
+    // (raw 16-byte pieces where the rows allow it: the conversion would wait for them ahead of the copies)
+    uint4 q_val = make_uint4(0u, 0u, 0u, 0u), q_hi = q_val;
+    const bool q_f32 = a.q.type == B200_TYPE_F32 && a.q.vec16;
     if (q_row < R) {
         int iq, hq;
         row_to_query(a, hk, q_row, iq, hq);
-        q_val = load8_as_half(a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3, a.q.type, q_ch * 8, a.hd, a.q.vec16);
+        const uint8_t* rowp = a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3;
+        if (q_f32) {
+            q_val = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch);
+            q_hi = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch + 1);
+        } else {
+            q_val = load8_as_half(rowp, a.q.type, q_ch * 8, a.hd, a.q.vec16);
+        }
     }
     const int kmax = tq_b > 0 ? len_b : 0;
     const int n_tiles = (kmax + KT - 1) / KT;
-    const int tps = (n_tiles + a.n_splits - 1) / a.n_splits;
+    const int tps = div_splits(a, n_tiles + a.n_splits - 1);
     const int tile_lo = split * tps, tile_hi = min(n_tiles, tile_lo + tps);
     // lanes 2s (K) and 2s+1 (V) of a warp copy the raw bytes of the warp's 16 keys of tile `tile0 + s`; lane 2s also
     // announces both copies to the stage's barrier.  Copies stop at the stream's length (whole 16-byte units).
@@ -1488,6 +1522,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
     auto issue = [&](int tile) { issue_lanes(tile, 1); };
     issue_lanes(tile_lo, NS);
     Q8T_TRACE(2);
+    if (q_f32) q_val = f32x8_to_half(q_val, q_hi);
     if (tid < 8 * (HD / 8)) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (q_row * (HD / 8) + swz<HD>(q_row, q_ch)) * 16) = q_val;
     __syncthreads();
     float* s_qd = &s_l[0][0];   // the block sums of the query rows borrow s_l, free until the epilogue
@@ -1821,6 +1856,7 @@ void launch_split(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const Fatt
     // (its CTAs wait on the device before they touch memory), which hides the launch latency between the layers of a
     // decode step (+0.8 % on the 64-segment decode launches, +1 % at 32 streams).
     FattnArgs ac = a;
+    ac.splits_mul = (65536 + a.n_splits - 1) / a.n_splits;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
