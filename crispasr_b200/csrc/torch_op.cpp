@@ -19,25 +19,44 @@
 namespace {
 
 // Interned names of the optional arguments, compared by pointer first (keyword names of call sites are interned).
-enum Key { kScale, kMaxBias, kSoftcap, kKvType, kCausal, kNPast, kKvLen, kQv, kR, kRelposF32, kBiasU, kBiasV, kKvIndex, kQLen, kKeys };
+enum Key { kScale, kMaxBias, kSoftcap, kKvType, kCausal, kNPast, kKvLen, kQv, kR, kRelposF32, kBiasU, kBiasV, kKvIndex, kQLen, kOut, kWorkspace, kStream, kQ, kK, kV, kMask, kKeys };
 const char* const kKeyNames[kKeys] = {"scale", "max_bias", "softcap", "kv_type", "causal", "n_past", "kv_len", "q_v", "r",
-                                      "relpos_bias_f32", "pos_bias_u", "pos_bias_v", "kv_index", "q_len"};
+                                      "relpos_bias_f32", "pos_bias_u", "pos_bias_v", "kv_index", "q_len", "out", "workspace", "stream", "q", "k", "v", "mask"};
 PyObject* g_keys[kKeys];
 
 struct Kwargs {
     PyObject* v[kKeys] = {};   // borrowed; null = absent or None
-    bool parse(PyObject* kw) {
-        if (!kw || kw == Py_None) return true;
-        PyObject *name, *value;
-        Py_ssize_t pos = 0;
-        while (PyDict_Next(kw, &pos, &name, &value)) {
+    // `values`: those of the keyword names, behind the positional arguments of a vector call
+    bool parse(PyObject* names, PyObject* const* values) {
+        const Py_ssize_t n = names ? PyTuple_GET_SIZE(names) : 0;
+        for (Py_ssize_t j = 0; j < n; j++) {
+            PyObject* name = PyTuple_GET_ITEM(names, j);
             int hit = -1;
             for (int i = 0; i < kKeys && hit < 0; i++)
                 if (name == g_keys[i]) hit = i;
             for (int i = 0; i < kKeys && hit < 0; i++)
                 if (PyUnicode_Compare(name, g_keys[i]) == 0) hit = i;
             if (PyErr_Occurred()) return false;
-            if (hit >= 0 && value != Py_None) v[hit] = value;   // other names are ignored, as they always were
+            if (hit >= 0) v[hit] = values[j] == Py_None ? nullptr : values[j];   // other names are ignored, as they always were
+        }
+        return true;
+    }
+    // q, k, v, mask: by position or by name
+    bool operands(PyObject* const* a, Py_ssize_t n, const char* where, PyObject* (&op)[4]) const {
+        if (n > 4) {
+            PyErr_Format(PyExc_TypeError, "%s() takes from 3 to 4 positional arguments but %zd were given", where, n);
+            return false;
+        }
+        for (int i = 0; i < 4; i++) {
+            if (i < n && v[kQ + i]) {
+                PyErr_Format(PyExc_TypeError, "%s() got multiple values for argument '%s'", where, kKeyNames[kQ + i]);
+                return false;
+            }
+            op[i] = i < n ? a[i] : v[kQ + i];
+            if (!op[i] && i < 3) {
+                PyErr_Format(PyExc_TypeError, "%s() missing required argument '%s'", where, kKeyNames[kQ + i]);
+                return false;
+            }
         }
         return true;
     }
@@ -215,70 +234,86 @@ void* scratch_alloc(void* user, size_t bytes) {
     return s->buf.data_ptr();
 }
 
-// (q, k, v, mask, out, workspace, stream, kw) -> the output tensor
-PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 8) {
-        PyErr_SetString(PyExc_TypeError, "launch takes 8 arguments");
-        return nullptr;
-    }
+const char kLaunchDoc[] =
+    "flash_attn_ext(q, k, v, mask=None, *, out=None, workspace=None, stream=None, **kw)\n--\n\n"
+    "Device tensors in, device tensor out; asynchronous on `stream` (default: torch's current stream).\n"
+    "`workspace` (uint8 device tensor) is allocated here when the launch needs one and none is given.";
+
+PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names) {
     HANDLE_TH_ERRORS
-    const at::Tensor* q = tensor_of(a[0], "q");
+    Kwargs kw;
+    PyObject* in[4];
+    if (!kw.parse(names, a + n) || !kw.operands(a, n, "flash_attn_ext", in)) return nullptr;
+    const at::Tensor* q = tensor_of(in[0], "q");
     if (!q) return nullptr;
     if (!q->is_cuda()) {
         PyErr_SetString(PyExc_ValueError, "flash_attn_ext takes CUDA tensors; use flash_attn_ext_host for host buffers");
         return nullptr;
     }
     const c10::cuda::CUDAGuard guard(q->device());
+    PyObject* out = kw.v[kOut];
     at::Tensor made;
-    if (a[4] == Py_None) {
+    if (!out) {
         if (q->dim() != 4) {
             PyErr_SetString(PyExc_ValueError, "q is (B, H, Tq, hd)");
             return nullptr;
         }
         made = at::detail::empty_cuda({q->size(0), q->size(2), q->size(1), q->size(3)}, at::kFloat, q->device(), std::nullopt);
     }
-    const at::Tensor* dst = a[4] == Py_None ? &made : tensor_of(a[4], "out");
-    Kwargs kw;
+    const at::Tensor* dst = out ? tensor_of(out, "out") : &made;
     Operands op;
-    if (!dst || !kw.parse(a[7]) || !op.fill(a[0], a[1], a[2], a[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
+    if (!dst || !op.fill(in[0], in[1], in[2], in[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
     Scratch ws{at::Tensor(), q->device(), nullptr, 0};
-    if (a[5] != Py_None) {
-        const at::Tensor* w = tensor_of(a[5], "workspace");
+    if (kw.v[kWorkspace]) {
+        const at::Tensor* w = tensor_of(kw.v[kWorkspace], "workspace");
         if (!w) return nullptr;
         ws.given = w->data_ptr(), ws.given_bytes = (size_t)w->numel();
     }
     void* st = nullptr;
-    if (a[6] == Py_None) st = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
-    else if (!stream_of(a[6], &st)) return nullptr;
+    if (!kw.v[kStream]) st = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
+    else if (!stream_of(kw.v[kStream], &st)) return nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS   // a full launch queue blocks: other host threads go on meanwhile
     rc = b200_fattn_launch_alloc(&op.q, &op.k, &op.v, op.mask_p(), &op.dst, &op.params, &op.ext, scratch_alloc, &ws, st);
     Py_END_ALLOW_THREADS
     if (rc) return raise_code(rc, "b200_fattn_launch");
-    if (a[4] == Py_None) return THPVariable_Wrap(std::move(made));
-    Py_INCREF(a[4]);
-    return a[4];
+    if (!out) return THPVariable_Wrap(std::move(made));
+    Py_INCREF(out);
+    return out;
     END_HANDLE_TH_ERRORS
 }
 
-// (q, k, v, mask, out, kw): host buffers in, host buffer out; `out` is made by the caller
-PyObject* forward_host_py(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 6) {
-        PyErr_SetString(PyExc_TypeError, "forward_host takes 6 arguments");
-        return nullptr;
-    }
+const char kHostDoc[] =
+    "flash_attn_ext_host(q, k, v, mask=None, *, out=None, **kw)\n--\n\n"
+    "Host (CPU, ideally pinned) tensors in, host tensor out: H2D, compute, D2H inside one C call.";
+
+PyObject* forward_host_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names) {
     HANDLE_TH_ERRORS
-    const at::Tensor *q = tensor_of(a[0], "q"), *dst = q ? tensor_of(a[4], "out") : nullptr;
     Kwargs kw;
+    PyObject* in[4];
+    if (!kw.parse(names, a + n) || !kw.operands(a, n, "flash_attn_ext_host", in)) return nullptr;
+    const at::Tensor* q = tensor_of(in[0], "q");
+    if (!q) return nullptr;
+    PyObject* out = kw.v[kOut];
+    at::Tensor made;
+    if (!out) {
+        if (q->dim() != 4) {
+            PyErr_SetString(PyExc_ValueError, "q is (B, H, Tq, hd)");
+            return nullptr;
+        }
+        made = at::empty({q->size(0), q->size(2), q->size(1), q->size(3)}, q->options().dtype(at::kFloat));
+    }
+    const at::Tensor* dst = out ? tensor_of(out, "out") : &made;
     Operands op;
-    if (!dst || !kw.parse(a[5]) || !op.fill(a[0], a[1], a[2], a[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
+    if (!dst || !op.fill(in[0], in[1], in[2], in[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS
     rc = b200_fattn_forward_host(&op.q, &op.k, &op.v, op.mask_p(), &op.dst, &op.params, &op.ext);
     Py_END_ALLOW_THREADS
     if (rc) return raise_code(rc, "b200_fattn_forward_host");
-    Py_INCREF(a[4]);
-    return a[4];
+    if (!out) return THPVariable_Wrap(std::move(made));
+    Py_INCREF(out);
+    return out;
     END_HANDLE_TH_ERRORS
 }
 
@@ -310,8 +345,8 @@ PyObject* kv_append_py(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyMethodDef kMethods[] = {
-    {"launch", (PyCFunction)(void (*)(void))launch_py, METH_FASTCALL, "flash_attn_ext on device tensors"},
-    {"forward_host", (PyCFunction)(void (*)(void))forward_host_py, METH_FASTCALL, "flash_attn_ext on host tensors"},
+    {"flash_attn_ext", (PyCFunction)(void (*)(void))launch_py, METH_FASTCALL | METH_KEYWORDS, kLaunchDoc},
+    {"flash_attn_ext_host", (PyCFunction)(void (*)(void))forward_host_py, METH_FASTCALL | METH_KEYWORDS, kHostDoc},
     {"kv_append", (PyCFunction)(void (*)(void))kv_append_py, METH_FASTCALL, "rows of a KV cache"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_op", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

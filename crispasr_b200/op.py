@@ -101,29 +101,20 @@ def workspace_bytes(q, k, v, mask=None, **kw) -> int:
     return n.value
 
 
-_OP = None
+try:
+    # the torch-facing call path in native code (csrc/torch_op.cpp): a decode step is a row of calls of a few microseconds
+    # each, and a wrapper in Python would cost a tenth of them
+    import torch  # noqa: F401  (the module links against torch's libraries)
 
+    from ._torch_op import flash_attn_ext, flash_attn_ext_host, kv_append as _kv_append
+except ImportError as _why:  # not built yet (or no torch): importing the package works, calling does not
+    _missing = str(_why)
 
-def _native():
-    """The torch-facing call path (csrc/torch_op.cpp); raises if it has not been built, there is no fallback."""
-    global _OP
-    if _OP is None:
-        import torch  # noqa: F401  (the module links against torch's libraries)
+    def _unbuilt(*_args, **_kw):
         _lib()
-        from . import _torch_op
-        _OP = _torch_op
-    return _OP
-
-
-def flash_attn_ext(q, k, v, mask=None, *, out=None, workspace=None, stream=None, **kw):
-    """Device tensors in, device tensor out; asynchronous on `stream` (default: torch's current stream).
-    `workspace` (uint8 device tensor) is allocated here when the launch needs one and none is given."""
-    return (_OP or _native()).launch(q, k, v, mask, out, workspace, stream, kw)
-
-
-def flash_attn_ext_host(q, k, v, mask=None, *, out=None, **kw):
-    """Host (CPU, ideally pinned) tensors in, host tensor out: H2D, compute, D2H inside one C call."""
-    return (_OP or _native()).forward_host(q, k, v, mask, out if out is not None else _dst_like(q), kw)
+        raise ImportError(f"crispasr_b200._torch_op: {_missing}: build it with `python -m crispasr_b200.build` "
+                          "(there is no fallback implementation)")
+    flash_attn_ext = flash_attn_ext_host = _kv_append = _unbuilt
 
 
 class KvCache:
@@ -160,7 +151,7 @@ class KvCache:
 
     def append(self, layer, k_new, v_new, pos=None, pos0=0, stream=None):
         """k_new/v_new: float32 CUDA tensors (n_streams, n_kv, n_new, hd)."""
-        (_OP or _native()).kv_append(self._h.value or 0, layer, k_new, v_new, pos, pos0, stream)
+        _kv_append(self._h.value or 0, layer, k_new, v_new, pos, pos0, stream)
 
     def copy_stream(self, dst_stream, src_stream, n_rows, stream=None):
         """Fork a hypothesis: rows [0, n_rows) of every layer/head from one stream to another (kv_snapshot_pool)."""
