@@ -1212,8 +1212,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     const int rb0 = a.Tq - 1 - q0 - 127;  // first R row of half-block 0 (may be negative: TMA zero-fills)
 
     // half-block m of R -> ring slot m % 2.  The ring is laid out panel-major, [panel 0: slot 0 | slot 1][panel 1:
-    // slot 0 | slot 1] (16 KB each), so that per 64-column panel the 256 rows of both slots are contiguous and the
-    // band GEMM can address them as one N = 256 operand.
+    // slot 0 | slot 1] (16 KB each).
     auto load_r = [&](int m) {
         const int slot = m & 1;
         mbar_arrive_expect_tx(bar_r_full + 8 * slot, TILE_BYTES);

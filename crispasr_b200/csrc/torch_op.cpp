@@ -3,9 +3,9 @@
 //
 // A decode step of a small model is a few launches of 4-8 us each, so what a call costs on the host decides the step:
 // the same work in Python (about sixty attribute reads and ctypes objects per call, the operator planned twice) took
-// 27-33 us per call, this module 4-5 us, most of it the kernel launch and the output allocation.  A 6-layer step of
-// Whisper base.en (12 calls) 400 -> 58 us, a 30-layer Q8_0 decoder step (60 calls) 1604 -> 492 us: both are bound by
-// their kernels now.
+// 27-33 us per call, this module 4 us, most of it the kernel launch and the output allocation.  A 6-layer step of Whisper
+// base.en (12 calls) 400 -> 58 us and, as vector calls without a Python function in front, 54 us; a 30-layer Q8_0 decoder
+// step (60 calls) 1604 -> 492 us before its kernels became faster.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -18,10 +18,12 @@
 
 namespace {
 
-// Interned names of the optional arguments, compared by pointer first (keyword names of call sites are interned).
-enum Key { kScale, kMaxBias, kSoftcap, kKvType, kCausal, kNPast, kKvLen, kQv, kR, kRelposF32, kBiasU, kBiasV, kKvIndex, kQLen, kOut, kWorkspace, kStream, kQ, kK, kV, kMask, kKeys };
+// Interned names of the arguments, compared by pointer first (keyword names of call sites are interned).
+enum Key { kScale, kMaxBias, kSoftcap, kKvType, kCausal, kNPast, kKvLen, kQv, kR, kRelposF32, kBiasU, kBiasV, kKvIndex, kQLen, kOut,
+           kWorkspace, kStream, kQ, kK, kV, kMask, kKeys };
 const char* const kKeyNames[kKeys] = {"scale", "max_bias", "softcap", "kv_type", "causal", "n_past", "kv_len", "q_v", "r",
-                                      "relpos_bias_f32", "pos_bias_u", "pos_bias_v", "kv_index", "q_len", "out", "workspace", "stream", "q", "k", "v", "mask"};
+                                      "relpos_bias_f32", "pos_bias_u", "pos_bias_v", "kv_index", "q_len", "out", "workspace", "stream",
+                                      "q", "k", "v", "mask"};
 PyObject* g_keys[kKeys];
 
 struct Kwargs {
