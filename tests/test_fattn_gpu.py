@@ -847,3 +847,29 @@ def test_host_entry_point_pinned_result(b200, orc, B, H, Hkv, Tq, Lk, hd, q_f32)
     ref = orc.flash_attn_ext(q, k, v, scale=hd ** -0.5, kv_len=lens)
     assert_close(out.numpy(), ref, "host entry point, pinned result")
     assert_close(b200.flash_attn_ext_host(*args, **kw).numpy(), ref, "host entry point, pageable result")
+
+
+@pytest.mark.parametrize("T,H", [(256, 6), (1000, 4)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("pos", [14, 15, 20, 30, 63, 78, 79, 94, 255])
+def test_prefill_one_key_far_above_the_others(b200, orc, T, H, causal, pos):
+    """head_dim 64 prefill with one key 60 to 400 nats above all others (the log2-domain distance passes 127, where a float's
+    exponent ends), in each kind of column of the first and of a later 64-key step; T = 256 with a CTA per query tile,
+    T = 1000 with the key steps shared by a cluster.  Every row that sees the key is that key's value row."""
+    gaps = [60.0, 88.9, 95.0, 120.0, 200.0, 400.0]
+    for lo in range(0, len(gaps), H):
+        part = gaps[lo:lo + H]
+        rng = np.random.default_rng(pos + T)
+        n = len(part)
+        q = (1.0 + 0.01 * rng.standard_normal((1, n, T, 64))).astype(np.float16)
+        k, v = randn_f16(rng, (1, n, T, 64), 0.01), randn_f16(rng, (1, n, T, 64))
+        k[0, :, pos] = (np.array(part) / (0.125 * 64))[:, None].astype(np.float16)   # score = gap (1 +- 0.01)
+        kw = dict(scale=0.125, causal=causal)
+        got = gpu_op(b200, q, k, v, **kw)
+        assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+        assert_close(got, orc.flash_attn_ext(q, k, v, **kw), f"key {pos} {part} nats above, T={T} causal={causal}")
+        # all other keys together weigh less than T e^-59 of it: the row is V[pos], |V| < 5, times P / l.  The key's score in
+        # the log2 domain (at most 590) is exact in the product but rounded as the reference (2^-15): l is 1 to 2.2e-5
+        seen = slice(pos, T) if causal else slice(0, T)
+        assert np.abs(got[0, seen] - v[0, :, pos].astype(np.float32)[None]).max() <= 5 * 2.2e-5 + 1e-5
+    assert b200.lib().b200_device_status() == 0
