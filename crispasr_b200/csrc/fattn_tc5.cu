@@ -261,27 +261,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
-// 2^t of a pair on the FMA pipe: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds and leaves n in the low bits), a
-// degree-4 minimax polynomial of 2^f (computed here by weighted least squares; relative error 2.7e-6, a hundredth of the
-// rounding of P to f16), the exponent added as an integer.  Any t may come: against a reference that is far below the
-// score t has no bound, and the caller finds that out from the sum of the results.  t below -126 gives 2^-126 (0 as f16), t
-// above 126 gives 2^126: an exponent field that ran over would be a NaN or a small negative number, which no sum shows.
-__device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p1) {
-    t0 = fminf(fmaxf(t0, -126.0f), 126.0f), t1 = fminf(fmaxf(t1, -126.0f), 126.0f);
-    const uint64_t magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f), neg1 = pack2(-1.0f, -1.0f);
-    const uint64_t x = pack2(t0, t1), r = add2(x, magic), n = add2(r, nmagic), f = fma2(n, neg1, x);
-    const float C0 = 0.9999992847442627f, C1 = 0.6931217908859253f, C2 = 0.240247443318367f, C3 = 0.05591785907745361f, C4 = 0.009570102207362652f;
-    uint64_t p = fma2(f, pack2(C4, C4), pack2(C3, C3));
-    p = fma2(p, f, pack2(C2, C2));
-    p = fma2(p, f, pack2(C1, C1));
-    p = fma2(p, f, pack2(C0, C0));
-    float a, b, ra, rb;
-    unpack2(p, a, b);
-    unpack2(r, ra, rb);
-    p0 = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
-    p1 = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
-}
-
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {
     uint4 out;

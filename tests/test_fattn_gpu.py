@@ -873,3 +873,22 @@ def test_prefill_one_key_far_above_the_others(b200, orc, T, H, causal, pos):
         seen = slice(pos, T) if causal else slice(0, T)
         assert np.abs(got[0, seen] - v[0, :, pos].astype(np.float32)[None]).max() <= 5 * 2.2e-5 + 1e-5
     assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("T,H", [(256, 6), (1000, 4)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("pos", [14, 20, 31, 79, 255])
+def test_prefill_keeps_a_nan(b200, T, H, causal, bad, pos):
+    """A key row of NaN, or of +inf against positive query rows (inf - inf), in each kind of column of a key step: every row
+    that sees the key is NaN, every other row is finite."""
+    rng = np.random.default_rng(pos + T)
+    q = np.abs(randn_f16(rng, (1, H, T, 64))) + np.float16(0.1)
+    k, v = randn_f16(rng, (1, H, T, 64)), randn_f16(rng, (1, H, T, 64))
+    k[0, :, pos] = bad
+    got = gpu_op(b200, q, k, v, scale=0.125, causal=causal)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    first = pos if causal else 0
+    assert np.isnan(got[0, first:]).all()
+    assert np.isfinite(got[0, :first]).all()
+    assert b200.lib().b200_device_status() == 0
