@@ -261,6 +261,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     return d;
 }
 
+// What a row without a finite reference subtracts: any finite score gives P = +inf, which the row's sum shows, however far
+// below 0 the score lies (against 0 a row of scores below -126 would underflow unseen); a score of -inf still gives 0.
+constexpr float kNoReference = -1e30f;
+
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {
     uint4 out;
@@ -1529,7 +1533,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                     }
                     m_ref = m_new;
                 }
-                const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                const float m_use = (m_ref == -INFINITY) ? kNoReference : m_ref;
                 const uint64_t nm2 = pack2(-m_use, -m_use);
                 uint64_t ls[2] = {0ull, 0ull};
                 auto chunk = [&](const uint32_t (&sx)[16], int q) {

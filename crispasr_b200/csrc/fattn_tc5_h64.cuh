@@ -233,7 +233,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
             // kept - one instruction in six of this loop; only a row whose sum passes 2^12 has its tile's maximum taken,
             // O and l rescaled and P redone (947 -> 925 us at 64 windows).
             for (int attempt = 0; attempt < 2; attempt++) {
-                const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
+                const float m_use = (m_ref == -INFINITY) ? kNoReference : m_ref;
                 uint64_t ls2[2] = {0ull, 0ull};
                 const uint64_t nm2 = pack2(-m_use, -m_use);
                 uint32_t sA[16], sB[16];

@@ -892,3 +892,43 @@ def test_prefill_keeps_a_nan(b200, T, H, causal, bad, pos):
     assert np.isnan(got[0, first:]).all()
     assert np.isfinite(got[0, :first]).all()
     assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("hidden", [16, 64, 128, 200])
+@pytest.mark.parametrize("T", [300, 1000])
+def test_prefill_low_scores_behind_keys_of_minus_infinity(b200, orc, hidden, T):
+    """The first keys of every row score -inf, the others about -100: they carry the row although none of them would be seen
+    against a reference of 0 (2^-144)."""
+    rng = np.random.default_rng(hidden + T)
+    q = (1.0 + 0.02 * rng.standard_normal((1, 4, T, 64))).astype(np.float16)
+    k, v = (-12.5 + 0.02 * rng.standard_normal((1, 4, T, 64))).astype(np.float16), randn_f16(rng, (1, 4, T, 64))
+    k[:, :, :hidden] = -np.inf
+    got = gpu_op(b200, q, k, v, scale=0.125)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, orc.flash_attn_ext(q, k, v, scale=0.125), f"{hidden} keys of -inf, T={T}")
+    assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("hidden", [64, 128, 200])
+@pytest.mark.parametrize("low", ["scores", "mask"])
+def test_relpos_low_scores_behind_masked_keys(b200, orc, hidden, low):
+    """Fused bias with an explicit mask whose first keys are -inf, the others' scores about -100, or their mask the lowest
+    finite F16: the visible keys carry the row."""
+    rng = np.random.default_rng(hidden)
+    T = 400
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T)
+    mask = np.zeros((1, 1, T, T), np.float16)
+    if low == "scores":
+        # (F16 numbers in whatever type: the kernels round F32 keys to F16, at this size by more than the tolerance)
+        q_u = (1.0 + 0.02 * rng.standard_normal(q_u.shape)).astype(np.float16).astype(q_u.dtype)
+        k = (-100.0 / 128 ** 0.5 + 0.02 * rng.standard_normal(k.shape)).astype(np.float16).astype(k.dtype)
+    else:
+        mask[:] = np.finfo(np.float16).min
+    mask[..., :hidden] = -np.inf
+    kw = dict(scale=128 ** -0.5, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, mask, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    ref = orc.flash_attn_ext(q_u, k, v, mask, **kw)
+    # against a mask of -65504 a logit is rounded to 2^-8 (the sum in fp32): 0.4 % of P
+    assert_close(got, ref, f"{low} behind {hidden} masked keys", **(dict(max_abs=2e-2, rel_l2=1e-2) if low == "mask" else {}))
+    assert b200.lib().b200_device_status() == 0
