@@ -264,6 +264,13 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // What a row without a finite reference subtracts: any finite score gives P = +inf, which the row's sum shows, however far
 // below 0 the score lies (against 0 a row of scores below -126 would underflow unseen); a score of -inf still gives 0.
 constexpr float kNoReference = -1e30f;
+// Sum of a row over a step's 64 keys (rel-pos kernel: over half of a tile's 128) above which the reference is taken anew from
+// the maximum.  Not a question of range (f16 holds P up to 2^16) but of precision: a key that carries the row has P = 1, exact
+// in f16, only if it is the reference itself.  64 equal scores sum to 64, so the bound lies above that; random scores of unit
+// variance stay below 30 (a bound of 32 redoes most steps: 1230 us at 64 windows).  Error against 64 bits (relative 2-norm, in
+// brackets that of a maximum kept within 2^8, and of a bound of 2^12 with a reference from 16 scores): variance 1, 1500 keys
+// 2.063e-4 (2.063e-4, 2.068e-4), variance 4, 700 keys 1.88e-4 (1.97e-4, 2.05e-4), variance 64 1.16e-4 (1.18e-4, 1.59e-4).
+constexpr float kRedoSum = 96.0f, kRedoSumRelpos = 256.0f;
 
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {
@@ -1388,7 +1395,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         const uint32_t rot = 4u * ((lane + 3u * (lane >> 3)) & 7u);
         const uint32_t x_col0 = 96 - 32 * (warp & 3) + 64 * ch;   // first X column this thread's warp can need
         const uint64_t l2e2 = pack2(kLog2e, kLog2e), c2 = pack2(bscale * kLog2e, bscale * kLog2e);
-        float m_ref = -INFINITY, l_run = 0.0f, l_max = 0.0f;   // l_max: half-row sum that calls for a new reference
+        float m_ref = -INFINITY, l_run = 0.0f;
         bool ok = true;
         // Explicit F16 mask added on top of the bias (bucket padding of src/canary_ctc.cpp:370-382, the local-attention
         // window of src/core/fastconformer.h:887-895): this thread's row of [Lk, Tq, 1|H, 1|B];
@@ -1492,10 +1499,10 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                     }
                 }
             };
-            // The reference need not be the maximum: P only has to stay inside f16, and the half-row sums (needed anyway)
-            // bound it.  The two threads of a row exchange them - the exchange also says that both have read their S columns,
-            // which the P stores overwrite - and only when one passes 2^12 (or in the first tile) is the row's maximum taken,
-            // O and l rescaled and P computed again.  Both warps of a pair see the same sums and take the same branch.
+            // The reference need not be the maximum: the half-row sums (needed anyway) bound P.  The two threads of a row
+            // exchange them - the exchange also says that both have read their S columns, which the P stores overwrite - and
+            // only when one passes kRedoSumRelpos (or in the first tile) is the row's maximum taken, O and l rescaled and P
+            // computed again.  Both warps of a pair see the same sums and take the same branch.
             uint32_t preg[32];
             float lsum;
             bool take_max = j == 0;
@@ -1563,11 +1570,10 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 lsum = l0 + l1;
                 if (tid == 0) TC5_TRACE(0, j, 3);
                 const float other = exchange(lsum);
-                if (!ok || take_max || !__any_sync(0xffffffffu, fmaxf(lsum, other) > l_max)) break;
+                if (!ok || take_max || !__any_sync(0xffffffffu, fmaxf(lsum, other) > kRedoSumRelpos)) break;
                 take_max = true;
             }
             if (!ok) break;
-            l_max = m_ref == -INFINITY ? 0.0f : 4096.0f;
             l_run += lsum;
             tmem_st32(tmem_P + lane_base + ch * 32, preg);
             tmem_wait_st();

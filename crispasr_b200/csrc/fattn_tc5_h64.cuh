@@ -211,27 +211,39 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
         float m_ref = -INFINITY, l_run = 0.0f;
         const uint64_t c2 = pack2(c, c);
         bool ok = true;
+        auto step_max = [&](int n_valid) {   // maximum of this row's scores of the step
+            float mx = -INFINITY;
+#pragma unroll 1
+            for (int half = 0; half < 2; half++) {
+                uint32_t x[32];
+                tmem_ld32(tmem_S + lane_base + half * 32, x);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                    mx = max3(mx, half * 32 + i < n_valid ? __uint_as_float(x[i]) : -INFINITY, half * 32 + i + 1 < n_valid ? __uint_as_float(x[i + 1]) : -INFINITY);
+            }
+            return mx;
+        };
         for (int j = 0; j < n_tiles; j++) {
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
             tc_fence_after();
             const int n_valid = kend - (t0 + j) * kH64Keys;   // columns >= n_valid of this row are masked
             const bool full_tile = __all_sync(0xffffffffu, n_valid >= kH64Keys);
-            if (j == 0) {   // a first reference maximum: that of the row's first 16 scores (the lazy check below corrects it)
-                uint32_t s0[16];
-                tmem_ld16(tmem_S + lane_base, s0);
+            if (j == 0) {   // a first reference: the maximum of the row's first 32 scores (the check below corrects it)
+                uint32_t x[32];
+                tmem_ld32(tmem_S + lane_base, x);
                 tmem_wait_ld();
                 float mx = -INFINITY;
 #pragma unroll
-                for (int i = 0; i < 16; i++) mx = fmaxf(mx, i < n_valid ? __uint_as_float(s0[i]) : -INFINITY);
+                for (int i = 0; i < 32; i += 2) mx = max3(mx, i < n_valid ? __uint_as_float(x[i]) : -INFINITY, i + 1 < n_valid ? __uint_as_float(x[i + 1]) : -INFINITY);
                 m_ref = mx * c;
             }
             uint32_t preg[32];
             float lsum = 0.0f;
-            // P = exp2(S*c - m_ref) against a reference maximum that need not be the maximum: what has to hold is that P
-            // stays inside f16, and the tile's row sum (needed anyway) bounds every P of the row.  No running maximum is
-            // kept - one instruction in six of this loop; only a row whose sum passes 2^12 has its tile's maximum taken,
-            // O and l rescaled and P redone (947 -> 925 us at 64 windows).
+            // P = exp2(S*c - m_ref) against a reference that need not be the maximum: the step's row sum (needed anyway) bounds
+            // every P of the row.  No running maximum is kept - one instruction in six of this loop; only a row whose sum passes
+            // kRedoSum has the step's maximum taken, O and l rescaled and P redone (947 -> 925 us at 64 windows).
             for (int attempt = 0; attempt < 2; attempt++) {
                 const float m_use = (m_ref == -INFINITY) ? kNoReference : m_ref;
                 uint64_t ls2[2] = {0ull, 0ull};
@@ -273,17 +285,9 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                 float l0, l1;
                 unpack2(add2(ls2[0], ls2[1]), l0, l1);
                 lsum = l0 + l1;
-                if (!__any_sync(0xffffffffu, lsum > 4096.0f || (m_ref == -INFINITY && lsum > 0.0f))) break;
+                if (!__any_sync(0xffffffffu, lsum > kRedoSum)) break;
                 // O is at rest: the commit behind S[j] covers P[j-1].V[j-1]
-                float mx = -INFINITY;
-#pragma unroll
-                for (int q4 = 0; q4 < 4; q4++) {
-                    tmem_ld16(tmem_S + lane_base + q4 * 16, sA);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 16; i++) mx = fmaxf(mx, q4 * 16 + i < n_valid ? __uint_as_float(sA[i]) : -INFINITY);
-                }
-                const float m_new = fmaxf(m_ref, mx * c);
+                const float m_new = fmaxf(m_ref, step_max(n_valid) * c);
                 const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
                 l_run *= alpha;
                 if (j > 0) {

@@ -932,3 +932,30 @@ def test_relpos_low_scores_behind_masked_keys(b200, orc, hidden, low):
     # against a mask of -65504 a logit is rounded to 2^-8 (the sum in fp32): 0.4 % of P
     assert_close(got, ref, f"{low} behind {hidden} masked keys", **(dict(max_abs=2e-2, rel_l2=1e-2) if low == "mask" else {}))
     assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("form", ["hd64", "hd64 shared", "relpos"])
+@pytest.mark.parametrize("pos", [30, 80, 200])
+def test_prefill_rounds_no_weight_of_a_row_that_one_key_carries(b200, form, pos):
+    """Key 0 stands 2^8.2 to 2^11.9 below key `pos` and everything else e^-30 below key 0: key `pos` carries the row and its P
+    has to be exact.  What may be wrong is the F16 rounding of key 0's P (2^-12 of 2^-8.2) and fp32 rounding of l and of the
+    logits (2^-19), times |V| < 5; a rounded P of key `pos` would be off by up to 2^-12."""
+    rng = np.random.default_rng(pos)
+    hd, T, H = (128, 300, 8) if form == "relpos" else (64, 1000 if "shared" in form else 256, 4)
+    scale = 1.0 / 16
+    q = np.zeros((1, H, T, hd), np.float16)
+    k, v = np.zeros((1, H, T, hd), np.float16), randn_f16(rng, (1, H, T, hd))
+    # q = (64, gap): k[0] = (1, 0) scores 4, k[pos] = (1, 1) scores 4 + gap / 16, the others (-7, 0) -28
+    q[..., 0], k[..., 0] = 64.0, -7.0
+    gap = np.linspace(8.2, 11.9, T) / np.log2(np.e) / scale
+    q[..., 1] = gap.astype(np.float16)
+    k[:, :, 0, 0], k[:, :, pos, 0], k[:, :, pos, 1] = 1.0, 1.0, 1.0
+    kw = dict(scale=scale)
+    if form == "relpos":
+        kw.update(q_v=q, r=np.zeros((1, H, 2 * T - 1, hd), np.float16))
+    got = gpu_op(b200, q, k, v, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    w0 = np.exp(-q[0, :, :, 1].astype(np.float64) * scale)                       # key 0 against key `pos`
+    v64 = v[0].astype(np.float64)
+    want = (v64[:, pos][:, None] + w0[..., None] * v64[:, 0][:, None]) / (1.0 + w0)[..., None]
+    assert np.abs(got[0].transpose(1, 0, 2) - want).max() <= 5 * (2.0 ** -20 + 2.0 ** -18)
