@@ -272,6 +272,32 @@ constexpr float kNoReference = -1e30f;
 // 2.063e-4 (2.063e-4, 2.068e-4), variance 4, 700 keys 1.88e-4 (1.97e-4, 2.05e-4), variance 64 1.16e-4 (1.18e-4, 1.59e-4).
 constexpr float kRedoSum = 96.0f, kRedoSumRelpos = 256.0f;
 
+// x bounded to [-126, 126]; a NaN stays one (fmaxf and fminf would drop it).
+__device__ __forceinline__ float clamp126(float x) {
+    float y;
+    asm("max.NaN.f32 %0, %1, 0fC2FC0000;\n\tmin.NaN.f32 %0, %0, 0f42FC0000;" : "=f"(y) : "f"(x));
+    return y;
+}
+// 2^t of a pair on the FMA pipe: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds and leaves n in the low bits), a
+// degree-4 minimax polynomial of 2^f (computed here by weighted least squares; relative error 2.7e-6, a hundredth of the
+// rounding of P to f16), times 2^n (which keeps a NaN, where adding n to the exponent field would not).  Any t may come:
+// against a reference that is far below the score t has no bound, and the caller finds that out from the sum of the
+// results.  t below -126 gives 2^-126 (0 as f16), t above 126 gives 2^126: an exponent field that ran over would be a small
+// negative number, which no sum shows.
+__device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p1) {
+    const uint64_t magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f), neg1 = pack2(-1.0f, -1.0f);
+    const uint64_t x = pack2(clamp126(t0), clamp126(t1)), r = add2(x, magic), n = add2(r, nmagic), f = fma2(n, neg1, x);
+    const float C0 = 0.9999992847442627f, C1 = 0.6931217908859253f, C2 = 0.240247443318367f, C3 = 0.05591785907745361f, C4 = 0.009570102207362652f;
+    uint64_t p = fma2(f, pack2(C4, C4), pack2(C3, C3));
+    p = fma2(p, f, pack2(C2, C2));
+    p = fma2(p, f, pack2(C1, C1));
+    p = fma2(p, f, pack2(C0, C0));
+    float ra, rb;
+    unpack2(r, ra, rb);
+    const float e0 = __uint_as_float((__float_as_uint(ra) << 23) + 0x3F800000u), e1 = __uint_as_float((__float_as_uint(rb) << 23) + 0x3F800000u);   // 2^n
+    unpack2(mul2(p, pack2(e0, e1)), p0, p1);
+}
+
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {
     uint4 out;

@@ -39,9 +39,10 @@ __device__ __forceinline__ float2 ld_peer_v2(uint32_t p) {
     return v;
 }
 
-// All exponentials go to the exponential unit.  Every eighth pair as a polynomial on the FMA pipe measured 1044 against 1054 us
-// at 64 windows and the same at 8 (144 us) once its argument is bounded on both sides and keeps a NaN: not worth a second
-// definition of P.
+// Every eighth pair of exponentials goes to the FMA pipe: 64 windows of the large encoder 1086 -> 1074 us, 8 windows 141.1 ->
+// 139.4, four windows 74.5 -> 71.5; every fourth pair costs more issue slots (and power) than the unit's time it frees (990
+// against 917 us in a burst).
+constexpr int kH64PolyEvery = 8;
 
 // QTMA: F16 query rows arrive by one tensor copy (else the softmax warps load and convert them); OTMA: the output leaves by
 // tensor stores (else by the threads).  SPLIT: the CTAs of a cluster share one query tile, each takes a range of its key
@@ -265,7 +266,9 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                         const float s0 = __uint_as_float(sx[i]), s1 = __uint_as_float(sx[i + 1]);
                         float t0, t1;
                         unpack2(fma2(pack2(s0, s1), c2, nm2), t0, t1);
-                        const float p0 = ex2(t0), p1 = ex2(t1);
+                        float p0, p1;
+                        if ((i >> 1) % kH64PolyEvery == kH64PolyEvery - 1) poly_ex2(t0, t1, p0, p1);
+                        else p0 = ex2(t0), p1 = ex2(t1);
                         ls2[(i >> 1) & 1] = add2(ls2[(i >> 1) & 1], pack2(p0, p1));
                         p8[i >> 1] = cvt_f16x2(p0, p1);
                     }
