@@ -1784,27 +1784,38 @@ bool q_box_ok(const FattnArgs& a) {
            a.q.nb3 > 0;
 }
 
-// How many CTAs (a cluster of 1, 2, 4 or 8) share a query tile's `steps` key steps, for a launch of `tiles` query tiles on
-// 148 SMs with four places each.  A step takes 0.77 us in a CTA that has an SM to itself - its own hand-off chain - and
-// 0.92 / 1.2 / 1.48 us in one of two / three / four; sharing a tile costs 3 us (two cluster barriers, O through shared memory,
-// the merge).  One window of the base encoder (8 heads, 96 tiles of 24 steps): one CTA per tile 23.7 us, two 19.9, four
-// 16.9, eight (two waves) 22.1; 700 frames of 6 heads (36 tiles of 11) 13.2 / 11.8 / 10.5 / 11.5; 600 frames of 20 heads (100
-// tiles of 10) 12.0 / 13.3 / 13.3 / 19.7.
-int h64_splits(long tiles, int steps) {
-    constexpr double kStepUs[5] = {0.77, 0.77, 0.92, 1.2, 1.48};
+// How a head_dim 64 launch without a mask runs, from its query tiles and its keys: n >= 1 CTAs (a cluster of 1, 2, 4 or 8)
+// of the four-CTA kernel share a tile's 64-key steps, 0 = the two-CTA kernel with 128-key tiles.  A CTA's time is a start and its
+// steps, both by how many CTAs its SM holds; sharing a tile costs 3.4 us more (two cluster barriers, O through shared
+// memory, the merge).  Clusters do not fill every SM: 72 of two and 32 of four or eight CTAs run side by side before
+// SMs take a second CTA.  The two-CTA kernel has the shorter chain per key when an SM holds one CTA.
+// Fitted to 172 shapes (1 to 6 windows, 6 to 20 heads, 150 to 1500 frames; device time by CUDA graph): never more than 6 % above
+// the best of the five.  In us, two-CTA kernel / one / two / four / eight CTAs per tile: 64 tiles of 16 steps 15.0 / 16.7 / 13.5 /
+// 12.0 / 14.8; 96 of 24 20.3 / 23.2 / 19.4 / 16.6 / 21.7; 96 of 8 9.9 / 10.4 / 12.3 / 12.0 / 17.5; 144 of 24 20.8 / 23.4 / 19.9 /
+// 24.0 / 28.9; 144 of 16 15.6 / 17.2 / 16.3 / 20.1 / 26.0; 192 of 24 25.6 / 26.2 / 24.2 / 27.8 / 35.9; 288 of 11 15.4 / 15.3 / 19.9 /
+// 28.3 / 44.4.
+int h64_plan(long tiles, int keys, bool causal) {
+    constexpr double kStepUs[5] = {0.0, 0.83, 0.93, 1.2, 1.49}, kStartUs[5] = {0.0, 3.7, 4.8, 5.9, 6.6};
+    const int steps = (keys + kH64Keys - 1) / kH64Keys, pairs = (keys + kTile - 1) / kTile;   // 64-key steps, 128-key tiles
+    // A causal launch is as long as its last query tiles, which start first; up to two CTAs per SM (an eighth more when the
+    // tiles that wait are short against the rest) the two-CTA kernel runs those faster: 160 tiles of 16 steps 15.3 / 18.0 us,
+    // 240 of 24 21.4 / 24.3, 288 of 8 10.9 / 11.5, 320 of 16 17.9 / 18.9; but 240 of 5 9.2 / 9.2, 320 of 8 14.6 / 12.5.
+    if (causal && tiles > 148 && tiles <= (pairs >= 8 ? 333 : 296) && pairs >= 4) return 0;
+    if (tiles > 2 * 148) return 1;
     int best = 1;
     double best_cost = 0.0;
     for (int n = 1; n <= 8; n *= 2) {
-        const long per_sm = (tiles * n + 147) / 148;
-        if (n > 1 && per_sm > 4) break;   // more than one wave
-        const double cost = (steps + n - 1) / n * kStepUs[per_sm < 4 ? per_sm : 4] + (n > 1 ? 2.9 + 0.2 * n : 0.0);
+        const long places = n == 1 ? 148 : (n == 2 ? 144 : 128), per_sm = (tiles * n + places - 1) / places;
+        if (per_sm > 4) break;   // more than one wave
+        const double cost = (steps + n - 1) / n * kStepUs[per_sm] + kStartUs[per_sm] + (n > 1 ? 3.4 : 0.0);
         // (a clear gain only: where it is even, the result of an entry stays what it is inside a larger batch, bit for bit)
-        if (n == 1 || cost < 0.93 * best_cost) best = n, best_cost = cost;
+        if (n == 1 || cost < 0.96 * best_cost) best = n, best_cost = cost;
     }
-    return best;
+    const double two_cta = 4.5 + 1.32 * pairs;   // one CTA per SM; with two per SM it gains no more than 2 %
+    return tiles <= 148 && two_cta < 0.98 * best_cost ? 0 : best;
 }
 
-int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
+int launch_h64(const FattnArgs& a, int n_split, cudaStream_t st, char* errbuf, size_t errlen) {
     CUtensorMap tmK, tmV;
     if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq, kH64Keys)) {
         snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V");
@@ -1815,7 +1826,7 @@ int launch_h64(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen)
     const bool o_tma = gqa_box(a) && !a.dst_on_host && (uintptr_t)a.dst % 16 == 0 && encode_o_map(&tmO, a);
     FattnArgs as = a;
     const int n_q = (a.Tq * a.gqa + kTile - 1) / kTile;
-    as.n_splits = h64_splits((long)n_q * a.Hkv * a.B, (a.Lk + kH64Keys - 1) / kH64Keys);
+    as.n_splits = n_split;
     dim3 grid(n_q * as.n_splits, a.Hkv, a.B);
     auto go = [&](auto kern, bool (&smem_set)[64]) {
         cudaError_t e = set_smem_once(kern, kH64Smem, smem_set);
@@ -1858,12 +1869,11 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     auto args = [&](auto launch) { e = launch(grid, smem, st, a, tmK, tmV, tmQ, tmO); };
     constexpr int QRAW = RAW_INST ? 2 : 0;
 #define B200_GO(...) args(launch_inst<fattn_prefill_tc5_kernel<__VA_ARGS__>, FattnArgs, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap>)
-    // head_dim 64 comes here with an explicit mask only
     if (a.has_mask) {
         if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, true, QRAW, true); else B200_GO(HD, NSTG, true, QRAW, false); }
         else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, true, 1, true); else B200_GO(HD, NSTG, true, 1, false); }
         else { if (o_tma) B200_GO(HD, NSTG, true, 0, true); else B200_GO(HD, NSTG, true, 0, false); }
-    } else if constexpr (HD == 128) {
+    } else {
         if (q_tma == 2) { if (o_tma) B200_GO(HD, NSTG, false, QRAW, true); else B200_GO(HD, NSTG, false, QRAW, false); }
         else if (q_tma == 1) { if (o_tma) B200_GO(HD, NSTG, false, 1, true); else B200_GO(HD, NSTG, false, 1, false); }
         else { if (o_tma) B200_GO(HD, NSTG, false, 0, true); else B200_GO(HD, NSTG, false, 0, false); }
@@ -1898,8 +1908,10 @@ bool tc5_supported(const FattnArgs& a) {
 
 int launch_prefill_tc5(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
     if (a.relpos) return launch_relpos(a, st, errbuf, errlen);
-    if (a.hd == 64 && !a.has_mask) return launch_h64(a, st, errbuf, errlen);
-    if (a.hd == 64) return launch_t<64, 2>(a, st, errbuf, errlen);
+    if (a.hd == 64) {
+        const int n = a.has_mask ? 0 : h64_plan((long)((a.Tq * a.gqa + kTile - 1) / kTile) * a.Hkv * a.B, a.Lk, a.causal != 0);
+        return n ? launch_h64(a, n, st, errbuf, errlen) : launch_t<64, 2>(a, st, errbuf, errlen);
+    }
     return launch_t<128, 1>(a, st, errbuf, errlen);
 }
 

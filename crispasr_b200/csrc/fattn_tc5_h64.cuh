@@ -47,7 +47,7 @@ constexpr int kH64PolyEvery = 8;
 // QTMA: F16 query rows arrive by one tensor copy (else the softmax warps load and convert them); OTMA: the output leaves by
 // tensor stores (else by the threads).  SPLIT: the CTAs of a cluster share one query tile, each takes a range of its key
 // steps; at the end they leave their O rows and (m, l) in shared memory and each merges and writes a share of the rows.
-// For launches with fewer tiles than the SMs can run at full pace (h64_splits): a lone CTA per SM spends 0.75 us per step,
+// For launches with fewer tiles than the SMs can run at full pace (h64_plan): a lone CTA per SM spends 0.75 us per step,
 // its own hand-off chain, which two CTAs per SM hide for each other and four CTAs fill.
 template <bool QTMA, bool OTMA, bool SPLIT = false>
 __global__ void __launch_bounds__(kH64Threads, 4)

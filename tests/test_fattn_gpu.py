@@ -959,3 +959,26 @@ def test_prefill_rounds_no_weight_of_a_row_that_one_key_carries(b200, form, pos)
     v64 = v[0].astype(np.float64)
     want = (v64[:, pos][:, None] + w0[..., None] * v64[:, 0][:, None]) / (1.0 + w0)[..., None]
     assert np.abs(got[0].transpose(1, 0, 2) - want).max() <= 5 * (2.0 ** -20 + 2.0 ** -18)
+
+
+@pytest.mark.parametrize("S,H,gqa,T", [(1, 6, 1, 500), (3, 8, 1, 500), (2, 12, 2, 700), (1, 20, 1, 1000), (5, 8, 4, 900)])
+@pytest.mark.parametrize("form", ["plain", "causal", "lengths"])
+@pytest.mark.parametrize("q_f32", [False, True])
+def test_prefill_few_tiles_forms(b200, orc, S, H, gqa, T, form, q_f32):
+    """head_dim 64 launches on both sides of each line of the choice between the four-CTA kernel, its shared tiles and the
+    two-CTA kernel: 24 to 320 query tiles, F16 and F32 queries, grouped heads, causal, ragged lengths."""
+    rng = np.random.default_rng(S * T + H)
+    q, k, v = randn_f16(rng, (S, H, T, 64)), randn_f16(rng, (S, H // gqa, T, 64)), randn_f16(rng, (S, H // gqa, T, 64))
+    if q_f32:
+        q = q.astype(np.float32)
+    kw = dict(scale=0.125)
+    if form == "causal":
+        kw.update(causal=True, n_past=0)
+    if form == "lengths":
+        kw.update(kv_len=np.linspace(1, T, S).astype(np.int32))
+    rows = np.unique(np.linspace(0, T - 1, 60).astype(np.int32))
+    got = gpu_op(b200, q, k, v, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    ref = orc.flash_attn_ext(q, k, v, rows=rows, **kw)
+    assert_close(got[:, rows], ref[:, rows], f"S={S} H={H} gqa={gqa} T={T} {form}")
+    assert b200.lib().b200_device_status() == 0
