@@ -8,6 +8,8 @@
 // step (60 calls) 1604 -> 492 us before its kernels became faster.
 #include <Python.h>
 
+#include <exception>
+
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -224,6 +226,7 @@ struct Scratch {
     c10::Device device;
     void* given;
     size_t given_bytes;
+    std::exception_ptr error;   // what the allocator raised: it must not pass through the C entry point, the caller gets it behind that
 };
 void* scratch_alloc(void* user, size_t bytes) {
     Scratch* s = (Scratch*)user;
@@ -231,6 +234,7 @@ void* scratch_alloc(void* user, size_t bytes) {
     try {
         s->buf = at::detail::empty_cuda({(int64_t)bytes}, at::kByte, s->device, std::nullopt);
     } catch (...) {
+        s->error = std::current_exception();
         return nullptr;
     }
     return s->buf.data_ptr();
@@ -265,7 +269,7 @@ PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names
     const at::Tensor* dst = out ? tensor_of(out, "out") : &made;
     Operands op;
     if (!dst || !op.fill(in[0], in[1], in[2], in[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
-    Scratch ws{at::Tensor(), q->device(), nullptr, 0};
+    Scratch ws{at::Tensor(), q->device(), nullptr, 0, nullptr};
     if (kw.v[kWorkspace]) {
         const at::Tensor* w = tensor_of(kw.v[kWorkspace], "workspace");
         if (!w) return nullptr;
@@ -278,6 +282,7 @@ PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names
     Py_BEGIN_ALLOW_THREADS   // a full launch queue blocks: other host threads go on meanwhile
     rc = b200_fattn_launch_alloc(&op.q, &op.k, &op.v, op.mask_p(), &op.dst, &op.params, &op.ext, scratch_alloc, &ws, st);
     Py_END_ALLOW_THREADS
+    if (ws.error) std::rethrow_exception(ws.error);   // torch.OutOfMemoryError, as from any other allocation
     if (rc) return raise_code(rc, "b200_fattn_launch");
     if (!out) return THPVariable_Wrap(std::move(made));
     Py_INCREF(out);

@@ -982,3 +982,22 @@ def test_prefill_few_tiles_forms(b200, orc, S, H, gqa, T, form, q_f32):
     ref = orc.flash_attn_ext(q, k, v, rows=rows, **kw)
     assert_close(got[:, rows], ref[:, rows], f"S={S} H={H} gqa={gqa} T={T} {form}")
     assert b200.lib().b200_device_status() == 0
+
+
+def test_workspace_out_of_memory_is_torchs_error(b200):
+    """A workspace that the caching allocator cannot provide (here: beyond the process's share of the card) raises
+    torch.OutOfMemoryError, on which servers free their caches and try again."""
+    q = torch.randn(1, 20, 64, 64, device="cuda")
+    k, v = (torch.randn(1, 20, 16384, 64, device="cuda") for _ in "kv")   # converted to F16: 84 MB of workspace
+    out = torch.empty(1, 64, 20, 64, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (32 << 20)) / total)
+        with pytest.raises(torch.OutOfMemoryError):
+            b200.flash_attn_ext(q, k, v, scale=0.125, out=out)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert b200.flash_attn_ext(q, k, v, scale=0.125, out=out) is out
+    torch.cuda.synchronize()
