@@ -226,12 +226,18 @@ struct Scratch {
     c10::Device device;
     void* given;
     size_t given_bytes;
+    void* stream;   // the launch's
     std::exception_ptr error;   // what the allocator raised: it must not pass through the C entry point, the caller gets it behind that
 };
 void* scratch_alloc(void* user, size_t bytes) {
     Scratch* s = (Scratch*)user;
     if (s->given && s->given_bytes >= bytes) return s->given;
     try {
+        // The block comes from the pool of the stream that uses it: one of the current stream's pool may still be in use by
+        // that stream's earlier work, and would be handed out again while this launch is in flight.
+        c10::cuda::OptionalCUDAStreamGuard on_stream;
+        if (s->stream != (void*)c10::cuda::getCurrentCUDAStream(s->device.index()).stream())
+            on_stream.reset_stream(c10::cuda::getStreamFromExternal((cudaStream_t)s->stream, s->device.index()));
         s->buf = at::detail::empty_cuda({(int64_t)bytes}, at::kByte, s->device, std::nullopt);
     } catch (...) {
         s->error = std::current_exception();
@@ -243,7 +249,8 @@ void* scratch_alloc(void* user, size_t bytes) {
 const char kLaunchDoc[] =
     "flash_attn_ext(q, k, v, mask=None, *, out=None, workspace=None, stream=None, **kw)\n--\n\n"
     "Device tensors in, device tensor out; asynchronous on `stream` (default: torch's current stream).\n"
-    "`workspace` (uint8 device tensor) is allocated here when the launch needs one and none is given.";
+    "`workspace` (uint8 device tensor) is allocated here, for `stream`, when the launch needs one and none is given; the\n"
+    "result comes from the current stream's pool, as any tensor made here would.";
 
 PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names) {
     HANDLE_TH_ERRORS
@@ -269,7 +276,7 @@ PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names
     const at::Tensor* dst = out ? tensor_of(out, "out") : &made;
     Operands op;
     if (!dst || !op.fill(in[0], in[1], in[2], in[3], kw) || !describe(*dst, -1, &op.dst)) return nullptr;
-    Scratch ws{at::Tensor(), q->device(), nullptr, 0, nullptr};
+    Scratch ws{at::Tensor(), q->device(), nullptr, 0, nullptr, nullptr};
     if (kw.v[kWorkspace]) {
         const at::Tensor* w = tensor_of(kw.v[kWorkspace], "workspace");
         if (!w) return nullptr;
@@ -278,6 +285,7 @@ PyObject* launch_py(PyObject*, PyObject* const* a, Py_ssize_t n, PyObject* names
     void* st = nullptr;
     if (!kw.v[kStream]) st = c10::cuda::getCurrentCUDAStream(q->device().index()).stream();
     else if (!stream_of(kw.v[kStream], &st)) return nullptr;
+    ws.stream = st;
     int rc;
     Py_BEGIN_ALLOW_THREADS   // a full launch queue blocks: other host threads go on meanwhile
     rc = b200_fattn_launch_alloc(&op.q, &op.k, &op.v, op.mask_p(), &op.dst, &op.params, &op.ext, scratch_alloc, &ws, st);

@@ -1001,3 +1001,28 @@ def test_workspace_out_of_memory_is_torchs_error(b200):
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert b200.flash_attn_ext(q, k, v, scale=0.125, out=out) is out
     torch.cuda.synchronize()
+
+
+def test_workspace_of_a_launch_on_another_stream(b200, orc):
+    """A call on an explicit stream takes its workspace from that stream's pool: a block that the current stream has freed but
+    still reads (behind a delay) is not written, and the result does not depend on what the current stream allocates next."""
+    rng = np.random.default_rng(5)
+    q, k, v = (rng.standard_normal((1, 8, n, 64)).astype(np.float32) for n in (200, 9000, 9000))
+    dq, dk, dv = (torch.from_numpy(x).cuda() for x in (q, k, v))
+    out = torch.empty(1, 200, 8, 64, device="cuda")
+    n = b200.workspace_bytes(dq, dk, dv, scale=0.125)
+    assert n > 10 << 20
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    x = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+    y = torch.empty_like(x)
+    side.wait_stream(torch.cuda.current_stream())
+    torch.cuda._sleep(200_000_000)      # about 0.1 s on the current stream; the launch below does not wait for it
+    y.copy_(x)
+    del x
+    b200.flash_attn_ext(dq, dk, dv, scale=0.125, out=out, stream=side.cuda_stream)
+    z = torch.full((n,), 9, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    assert bool((y == 7).all()) and bool((z == 9).all())
+    assert_close(out.cpu().numpy(), orc.flash_attn_ext(q, k.astype(np.float16), v.astype(np.float16), scale=0.125), "launch on another stream")
