@@ -156,12 +156,21 @@ bool last_extent(PyObject* o, int32_t* out) {
     return !PyErr_Occurred();
 }
 
-// Stream handle: None (the caller picks), an integer, or a ctypes pointer.
+// Stream handle: None (the caller picks), an integer, a ctypes pointer, or an object that has one for ctypes (`_as_parameter_`:
+// torch.cuda.Stream).
 bool stream_of(PyObject* o, void** out) {
     if (PyLong_Check(o)) {
         *out = PyLong_AsVoidPtr(o);
         return !PyErr_Occurred();
     }
+    if (PyObject* as = PyObject_GetAttrString(o, "_as_parameter_")) {
+        const bool ok = PyLong_Check(as) || PyObject_HasAttrString(as, "value");
+        if (!ok) PyErr_SetString(PyExc_TypeError, "stream is an integer, a ctypes pointer or a torch.cuda.Stream");
+        const bool got = ok && stream_of(as, out);
+        Py_DECREF(as);
+        return got;
+    }
+    PyErr_Clear();
     PyObject* value = PyObject_GetAttrString(o, "value");
     if (!value) return false;
     *out = value == Py_None ? nullptr : PyLong_AsVoidPtr(value);
@@ -236,8 +245,9 @@ void* scratch_alloc(void* user, size_t bytes) {
         // The block comes from the pool of the stream that uses it: one of the current stream's pool may still be in use by
         // that stream's earlier work, and would be handed out again while this launch is in flight.
         c10::cuda::OptionalCUDAStreamGuard on_stream;
-        if (s->stream != (void*)c10::cuda::getCurrentCUDAStream(s->device.index()).stream())
-            on_stream.reset_stream(c10::cuda::getStreamFromExternal((cudaStream_t)s->stream, s->device.index()));
+        const cudaStream_t st = s->stream == (void*)cudaStreamLegacy ? nullptr : (cudaStream_t)s->stream;
+        if (st != c10::cuda::getCurrentCUDAStream(s->device.index()).stream())
+            on_stream.reset_stream(c10::cuda::getStreamFromExternal(st, s->device.index()));
         s->buf = at::detail::empty_cuda({(int64_t)bytes}, at::kByte, s->device, std::nullopt);
     } catch (...) {
         s->error = std::current_exception();
