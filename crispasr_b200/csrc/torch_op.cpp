@@ -356,9 +356,14 @@ PyObject* kv_append_py(PyObject*, PyObject* const* a, Py_ssize_t n) {
     b200_tensor tk, tv;
     if (!v || !describe(*k, -1, &tk) || !describe(*v, -1, &tv)) return nullptr;
     const int32_t* pos = nullptr;
+    if (a[4] != Py_None && !tensor_of(a[4], "pos")) return nullptr;   // (read by the kernel: a numpy array has no device address)
     if (a[4] != Py_None && !address_of(a[4], &pos)) return nullptr;
+    if (a[6] == Py_None && !k->is_cuda()) {
+        PyErr_SetString(PyExc_ValueError, "kv_append takes CUDA tensors");
+        return nullptr;
+    }
     void* st = nullptr;
-    if (a[6] == Py_None) st = c10::cuda::getCurrentCUDAStream(k->is_cuda() ? k->device().index() : (c10::DeviceIndex)-1).stream();
+    if (a[6] == Py_None) st = c10::cuda::getCurrentCUDAStream(k->device().index()).stream();
     else if (!stream_of(a[6], &st)) return nullptr;
     int rc;
     Py_BEGIN_ALLOW_THREADS

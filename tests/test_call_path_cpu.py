@@ -2,6 +2,7 @@
 at a null cache)."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
@@ -32,3 +33,13 @@ def test_streams_that_are_refused(b200, stream):
     x = torch.zeros(1, 1, 1, 64)
     with pytest.raises((TypeError, AttributeError)):
         b200.op._kv_append(0, 0, x, x, None, 0, stream)
+
+
+def test_append_refuses_host_rows_and_host_positions(b200):
+    """Rows in host memory on the default stream, and positions that are no tensor, never reach the kernel."""
+    x = torch.zeros(1, 1, 1, 64)
+    with pytest.raises(ValueError):
+        b200.op._kv_append(0, 0, x, x, None, 0, None)
+    with pytest.raises(TypeError):
+        b200.op._kv_append(0, 0, x, x, np.zeros(1, np.int32), 0, 0)
+    _append(b200, pos=torch.zeros(1, dtype=torch.int32))
