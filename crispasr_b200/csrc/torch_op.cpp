@@ -29,7 +29,7 @@ const char* const kKeyNames[kKeys] = {"scale", "max_bias", "softcap", "kv_type",
 PyObject* g_keys[kKeys];
 
 struct Kwargs {
-    PyObject* v[kKeys] = {};   // borrowed; null = absent or None
+    PyObject* v[kKeys] = {};   // borrowed; null = absent, or None where that is a value (a number has to be one)
     // `values`: those of the keyword names, behind the positional arguments of a vector call
     bool parse(PyObject* names, PyObject* const* values) {
         const Py_ssize_t n = names ? PyTuple_GET_SIZE(names) : 0;
@@ -41,7 +41,8 @@ struct Kwargs {
             for (int i = 0; i < kKeys && hit < 0; i++)
                 if (PyUnicode_Compare(name, g_keys[i]) == 0) hit = i;
             if (PyErr_Occurred()) return false;
-            if (hit >= 0) v[hit] = values[j] == Py_None ? nullptr : values[j];   // other names are ignored, as they always were
+            const bool number = hit == kScale || hit == kMaxBias || hit == kSoftcap || hit == kNPast;
+            if (hit >= 0) v[hit] = values[j] == Py_None && !number ? nullptr : values[j];   // other names are ignored, as they always were
         }
         return true;
     }
@@ -66,8 +67,11 @@ struct Kwargs {
     }
     bool number(Key k, double dflt, double* out) const {
         if (!v[k]) return *out = dflt, true;
-        *out = PyFloat_AsDouble(v[k]);
-        return !(*out == -1.0 && PyErr_Occurred());
+        PyObject* f = PyNumber_Float(v[k]);   // float(x): texts as well
+        if (!f) return false;
+        *out = PyFloat_AS_DOUBLE(f);
+        Py_DECREF(f);
+        return true;
     }
     bool integer(Key k, long* out) const {
         if (!v[k]) return *out = 0, true;
@@ -126,15 +130,20 @@ bool describe(const at::Tensor& x, long type, b200_tensor* t) {
     return true;
 }
 
-// Address of an index table: a torch tensor's, or a numpy array's.
+// Address of an index table: a torch tensor's, that of any other object with data_ptr(), or a numpy array's.
 bool address_of(PyObject* o, const int32_t** out) {
     if (THPVariable_Check(o)) {
         *out = (const int32_t*)THPVariable_Unpack(o).data_ptr();
         return true;
     }
-    PyObject* ct = PyObject_GetAttrString(o, "ctypes");
-    PyObject* data = ct ? PyObject_GetAttrString(ct, "data") : nullptr;
-    Py_XDECREF(ct);
+    PyObject* data = nullptr;
+    if (PyObject_HasAttrString(o, "data_ptr")) {
+        data = PyObject_CallMethod(o, "data_ptr", nullptr);
+    } else {
+        PyObject* ct = PyObject_GetAttrString(o, "ctypes");
+        data = ct ? PyObject_GetAttrString(ct, "data") : nullptr;
+        Py_XDECREF(ct);
+    }
     if (!data) return false;
     *out = (const int32_t*)PyLong_AsVoidPtr(data);
     Py_DECREF(data);
@@ -350,13 +359,21 @@ PyObject* kv_append_py(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     HANDLE_TH_ERRORS
     b200_kv_cache* kv = (b200_kv_cache*)PyLong_AsVoidPtr(a[0]);
-    const long layer = PyLong_AsLong(a[1]), pos0 = PyLong_AsLong(a[5]);
+    const long layer = PyLong_AsLong(a[1]);
+    if (PyErr_Occurred()) return nullptr;
+    PyObject* p0 = PyNumber_Long(a[5]);   // int(pos0): floats as well
+    if (!p0) return nullptr;
+    const long pos0 = PyLong_AsLong(p0);
+    Py_DECREF(p0);
     if (PyErr_Occurred()) return nullptr;
     const at::Tensor *k = tensor_of(a[2], "k_new"), *v = k ? tensor_of(a[3], "v_new") : nullptr;
     b200_tensor tk, tv;
     if (!v || !describe(*k, -1, &tk) || !describe(*v, -1, &tv)) return nullptr;
     const int32_t* pos = nullptr;
-    if (a[4] != Py_None && !tensor_of(a[4], "pos")) return nullptr;   // (read by the kernel: a numpy array has no device address)
+    if (a[4] != Py_None && !PyObject_HasAttrString(a[4], "data_ptr")) {   // (read by the kernel: a numpy array has no device address)
+        PyErr_Format(PyExc_TypeError, "pos is a torch tensor, not %s", Py_TYPE(a[4])->tp_name);
+        return nullptr;
+    }
     if (a[4] != Py_None && !address_of(a[4], &pos)) return nullptr;
     if (a[6] == Py_None && !k->is_cuda()) {
         PyErr_SetString(PyExc_ValueError, "kv_append takes CUDA tensors");

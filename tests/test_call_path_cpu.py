@@ -43,3 +43,46 @@ def test_append_refuses_host_rows_and_host_positions(b200):
     with pytest.raises(TypeError):
         b200.op._kv_append(0, 0, x, x, np.zeros(1, np.int32), 0, 0)
     _append(b200, pos=torch.zeros(1, dtype=torch.int32))
+
+
+@pytest.mark.parametrize("pos0", [3, 3.0, np.int64(3), torch.tensor(3)])
+def test_append_positions_are_whatever_int_takes(b200, pos0):
+    _append(b200, pos0=pos0)
+
+
+def _host_call(b200, **kw):
+    """A call on host tensors: returns, or ends at the missing device, once its arguments are converted."""
+    x = torch.zeros(1, 1, 2, 64)
+    try:
+        b200.flash_attn_ext_host(x, x, x, **kw)
+    except b200.B200Error as e:
+        assert e.code in (abi.E_NO_DEVICE, abi.E_CUDA), e
+
+
+class _Table:
+    """An index table that is no tensor but knows its address."""
+
+    def __init__(self):
+        self.t = torch.ones(1, dtype=torch.int32)
+
+    def data_ptr(self):
+        return self.t.data_ptr()
+
+
+@pytest.mark.parametrize("kw", [dict(scale="0.125"), dict(scale=torch.tensor(0.125)), dict(scale=np.float32(0.125)), dict(scale=1, n_past="2"),
+                                dict(scale=1, n_past=1.0), dict(scale=1, causal=None, kv_len=None, kv_type=None, mask=None),
+                                dict(scale=1, kv_len=np.ones(1, np.int32)), dict(scale=1, kv_len=_Table())])
+def test_values_that_are_taken(b200, kw):
+    """float() and int() of what is given, None where an argument may be left out, tables by address."""
+    _host_call(b200, **kw)
+
+
+@pytest.mark.parametrize("kw", [dict(scale=None), dict(scale=1, max_bias=None), dict(scale=1, softcap=None), dict(scale=1, n_past=None)])
+def test_none_is_no_number(b200, kw):
+    with pytest.raises(TypeError):
+        _host_call(b200, **kw)
+
+
+def test_scale_is_required(b200):
+    with pytest.raises(KeyError):
+        _host_call(b200)
