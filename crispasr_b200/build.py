@@ -1,8 +1,9 @@
-"""Builds libb200_fattn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and _torch_op.so, the
-torch-facing call path over its C-ABI, with the host compiler."""
+"""Builds libb200_fattn.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and, where torch is installed,
+_torch_op.so, the torch-facing call path over its C-ABI, with the host compiler."""
 from __future__ import annotations
 
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -51,8 +52,13 @@ def built_hash() -> str | None:
         return None
 
 
+def have_torch() -> bool:
+    """Whether torch can be imported; the C library needs none."""
+    return importlib.util.find_spec("torch") is not None
+
+
 def needs_build() -> bool:
-    return built_hash() != source_hash() or not os.path.exists(TORCH_OP)
+    return built_hash() != source_hash() or (have_torch() and not os.path.exists(TORCH_OP))
 
 
 def _torch_op_command() -> list[str]:
@@ -76,6 +82,18 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError(
             f"{LIB} is missing or was built from other sources (recorded {built_hash()}, tree {source_hash()}) "
             "and there is no nvcc to rebuild it with")
+    if force or built_hash() != source_hash():
+        _build_library(verbose)
+    if have_torch():
+        subprocess.run(_torch_op_command(), check=True)
+    elif os.path.exists(TORCH_OP):
+        os.remove(TORCH_OP)   # of other sources
+    with open(STAMP, "w") as f:
+        f.write(source_hash() + "\n")
+    return LIB
+
+
+def _build_library(verbose: bool) -> None:
     objs = []
     procs = []
     os.makedirs(os.path.join(HERE, "build"), exist_ok=True)
@@ -96,10 +114,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed")
     link = [_nvcc(), "-shared", "-o", LIB, *objs, "-lcudart", "-Xcompiler", "-fPIC"]
     subprocess.run(link, check=True)
-    subprocess.run(_torch_op_command(), check=True)
-    with open(STAMP, "w") as f:
-        f.write(source_hash() + "\n")
-    return LIB
 
 
 if __name__ == "__main__":

@@ -3,6 +3,7 @@ with error codes (never aborts), plans kernels, and the segment scheduler's host
 import ctypes as C
 import os
 import re
+import sys
 import threading
 
 import numpy as np
@@ -385,3 +386,32 @@ def test_beam_cells_to_union_lists_each_visible_cell_once(b200, orc):
     assert np.array_equal(got[:, :n[0]], mask[:, seen])
     assert np.all(np.isneginf(got[:, n[0]:])) and np.all(idx[n[0]:] == 0)   # the tail is masked out and points at a valid row
     assert L.b200_beam_cells_to_union(*args, idx.ctypes.data, 8, n.ctypes.data, cmask.ctypes.data) == abi.E_LIMIT
+
+
+def test_the_library_is_built_without_torch(monkeypatch, tmp_path):
+    """Where there is no torch the C library is compiled, linked and stamped, and is not compiled again."""
+    from crispasr_b200 import build
+    ran = []
+
+    class Done:
+        returncode = 0
+
+        def __init__(self, cmd, **kw):
+            ran.append(cmd)
+            if "-o" in cmd:
+                open(cmd[cmd.index("-o") + 1], "w").close()
+
+        def communicate(self):
+            return "", None
+    for name, path in (("LIB", "lib.so"), ("TORCH_OP", "op.so"), ("STAMP", "lib.so.srchash")):
+        monkeypatch.setattr(build, name, str(tmp_path / path))
+    real = build.HERE
+    monkeypatch.setattr(build, "source_hash", lambda: "abc")
+    monkeypatch.setattr(build, "sources", lambda: [os.path.join(real, "csrc", "segment_sched.cpp")])
+    monkeypatch.setattr(build, "HERE", str(tmp_path))
+    monkeypatch.setattr(build.subprocess, "Popen", Done)
+    monkeypatch.setattr(build.subprocess, "run", Done)
+    monkeypatch.setattr(build.shutil, "which", lambda _: "/bin/true")
+    monkeypatch.setitem(sys.modules, "torch", None)   # import torch raises ImportError, find_spec finds nothing
+    assert build.build() == build.LIB and len(ran) == 2   # one object, one link
+    assert not build.needs_build() and build.build() == build.LIB and len(ran) == 2
