@@ -37,8 +37,16 @@ def lib() -> C.CDLL:
     return _LIB
 
 
-from .op import (flash_attn_ext, flash_attn_ext_host, plan, supports, workspace_bytes, KvCache,  # noqa: E402
-                 SegmentScheduler)
+from .op import plan, supports, workspace_bytes, KvCache, SegmentScheduler  # noqa: E402
+
+
+def __getattr__(name):
+    if name not in ("flash_attn_ext", "flash_attn_ext_host"):   # native functions: op.py loads them, and torch, on first use
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    from . import op
+    globals()[name] = fn = getattr(op, name)
+    return fn
+
 
 __all__ = ["abi", "lib", "B200Error", "flash_attn_ext", "flash_attn_ext_host", "plan", "supports",
            "workspace_bytes", "KvCache", "SegmentScheduler", "LIB_PATH"]

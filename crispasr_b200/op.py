@@ -101,20 +101,33 @@ def workspace_bytes(q, k, v, mask=None, **kw) -> int:
     return n.value
 
 
-try:
-    # the torch-facing call path in native code (csrc/torch_op.cpp): a decode step is a row of calls of a few microseconds
-    # each, and a wrapper in Python would cost a tenth of them
-    import torch  # noqa: F401  (the module links against torch's libraries)
+# The torch-facing call path is native code (csrc/torch_op.cpp): a decode step is a row of calls of a few microseconds each,
+# and a wrapper in Python would cost a tenth of them.  It links against torch, which is imported with the first use of one
+# of its functions: the rest of the package needs none.
+_NATIVE = {"flash_attn_ext": "flash_attn_ext", "flash_attn_ext_host": "flash_attn_ext_host", "_kv_append": "kv_append"}
 
-    from ._torch_op import flash_attn_ext, flash_attn_ext_host, kv_append as _kv_append
-except ImportError as _why:  # not built yet (or no torch): importing the package works, calling does not
-    _missing = str(_why)
 
-    def _unbuilt(*_args, **_kw):
-        _lib()
-        raise ImportError(f"crispasr_b200._torch_op: {_missing}: build it with `python -m crispasr_b200.build` "
-                          "(there is no fallback implementation)")
-    flash_attn_ext = flash_attn_ext_host = _kv_append = _unbuilt
+def _load_native():
+    try:
+        import torch  # noqa: F401
+
+        from . import _torch_op
+        globals().update({name: getattr(_torch_op, native) for name, native in _NATIVE.items()})
+    except ImportError as why:  # not built yet (or no torch): importing the package works, calling does not
+        missing = str(why)
+
+        def unbuilt(*_args, **_kw):
+            _lib()
+            raise ImportError(f"crispasr_b200._torch_op: {missing}: build it with `python -m crispasr_b200.build` "
+                              "(there is no fallback implementation)")
+        globals().update(dict.fromkeys(_NATIVE, unbuilt))
+
+
+def __getattr__(name):
+    if name not in _NATIVE:
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    _load_native()
+    return globals()[name]
 
 
 class KvCache:
@@ -151,7 +164,9 @@ class KvCache:
 
     def append(self, layer, k_new, v_new, pos=None, pos0=0, stream=None):
         """k_new/v_new: float32 CUDA tensors (n_streams, n_kv, n_new, hd)."""
-        _kv_append(self._h.value or 0, layer, k_new, v_new, pos, pos0, stream)
+        if "_kv_append" not in globals():
+            _load_native()
+        _kv_append(self._h.value or 0, layer, k_new, v_new, pos, pos0, stream)  # noqa: F821
 
     def copy_stream(self, dst_stream, src_stream, n_rows, stream=None):
         """Fork a hypothesis: rows [0, n_rows) of every layer/head from one stream to another (kv_snapshot_pool)."""

@@ -1,12 +1,17 @@
 """What the native call path takes and refuses as arguments (no GPU: a call that gets through ends at the missing device or
 at a null cache)."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 import torch
 
 from crispasr_b200 import abi
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _append(b200, stream=0, pos=None, pos0=0):
@@ -86,3 +91,17 @@ def test_none_is_no_number(b200, kw):
 def test_scale_is_required(b200):
     with pytest.raises(KeyError):
         _host_call(b200)
+
+
+def test_importing_the_package_imports_no_torch():
+    """torch comes with the first use of a function that takes tensors, which is then the native one itself."""
+    code = ("import sys, crispasr_b200 as b200\n"
+            "from crispasr_b200 import abi, KvCache, SegmentScheduler\n"
+            "assert 'torch' not in sys.modules\n"
+            "f = b200.flash_attn_ext\n"
+            "assert 'torch' in sys.modules and b200.flash_attn_ext is f is b200.op.flash_attn_ext and type(f).__name__ == 'builtin_function_or_method'\n"
+            "from crispasr_b200 import flash_attn_ext_host\n"
+            "try: b200.nothing\n"
+            "except AttributeError: print('ok')\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr
