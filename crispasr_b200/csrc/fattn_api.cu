@@ -9,10 +9,12 @@
 #include <mutex>
 #include <vector>
 
+#include <cuda.h>
 #include <nvtx3/nvToolsExt.h>
 
 #include "fattn_common.cuh"
 #include "fattn_tc5.cuh"
+#include "host_range.h"
 
 namespace b200 {
 
@@ -441,20 +443,33 @@ struct Arena {
 };
 thread_local Arena g_arena;
 
+// The allocation or registration that holds an address of unified memory.
+bool allocation_of(uintptr_t p, uintptr_t* start, size_t* size) {
+    typedef CUresult (*PointerAttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+    static const PointerAttributeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &qres) == cudaSuccess &&
+                        qres == cudaDriverEntryPointSuccess;
+        return ok ? (PointerAttributeFn)f : nullptr;
+    }();
+    CUdeviceptr base = 0;
+    if (!fn || fn(&base, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+        fn(size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+        return false;
+    *start = (uintptr_t)base;
+    return true;
+}
+
 // The address at which kernels of the current device reach pinned host memory [p, p + bytes), or null.
 void* mapped_host(void* p, size_t bytes) {
     cudaPointerAttributes at;
-    void* dev = nullptr;
-    for (size_t off : {(size_t)0, bytes - 1}) {
-        if (cudaPointerGetAttributes(&at, (uint8_t*)p + off) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-        if (off == 0) dev = at.devicePointer;
-        else if ((uint8_t*)at.devicePointer != (uint8_t*)dev + off) return nullptr;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    return dev;
+    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
+    return inside_one_allocation(allocation_of, (uintptr_t)at.devicePointer, bytes) ? at.devicePointer : nullptr;
 }
 
 // Bytes spanned by a strided tensor (offset of the last element + one element/block).
