@@ -780,7 +780,18 @@ B200_API int b200_fattn_forward_host(const b200_tensor* q, const b200_tensor* k,
     const size_t dst_bytes = (size_t)dst->ne[0] * dst->ne[1] * dst->ne[2] * dst->ne[3] * 4;
     // A pinned result is written by the kernels themselves, row by row over the link: no copy is left behind the last kernel,
     // and none shares the copy engines with the uploads (12 uploads and 4 downloads together took 1213 us, 896 and 590 alone).
-    float* const dst_host = (float*)mapped_host(dst->data, dst_bytes);
+    // Not where the result overlaps an operand that is still to be uploaded when the first chunk is written: entries of an
+    // operand that is updated in place stay apart, heads of one entry do not.
+    Meets meets = Meets::kNot;
+    for (int i = 0; i < NIN; i++)
+        if (in[i]) {
+            b200_tensor one = *in[i];
+            one.ne[3] = 1;
+            const Meets m = result_meets((uintptr_t)dst->data, dst->nb[3], (size_t)dst->ne[3], (uintptr_t)in[i]->data, in[i]->nb[3], span_bytes(&one),
+                                         (size_t)in[i]->ne[3]);
+            if (m > meets) meets = m;
+        }
+    float* const dst_host = meets == Meets::kAnyhow ? nullptr : (float*)mapped_host(dst->data, dst_bytes);
     const size_t dst_off = dst_host ? 0 : bump(dst_bytes);
 
     // The call is pipelined over chunks - batch entries, or heads of one - that are independent: the upload of chunk i + 1
@@ -795,10 +806,10 @@ B200_API int b200_fattn_forward_host(const b200_tensor* q, const b200_tensor* k,
         for (int d = dim; d < 4; d++) one.ne[d] = 1;
         return t->ne[dim] == 1 || t->nb[dim] >= span_bytes(&one);
     };
-    bool by_batch = B >= 2 && k->ne[3] == B;
+    bool by_batch = B >= 2 && k->ne[3] == B && meets != Meets::kAnyhow;
     for (int i = 0; i < NIN && by_batch; i++)
         if (in[i] && in[i]->ne[3] != 1 && (in[i]->ne[3] != B || !outermost(in[i], 3))) by_batch = false;
-    bool by_heads = dst_host != nullptr && (by_batch || B == 1) && (!mask || mask->ne[2] == 1) && !plan.args.relpos && plan.args.n2 == 0;
+    bool by_heads = dst_host != nullptr && meets == Meets::kNot && (by_batch || B == 1) && (!mask || mask->ne[2] == 1) && !plan.args.relpos && plan.args.n2 == 0;
     for (int i = 0; i < 3 && by_heads; i++) by_heads = outermost(in[i], 2);
     static const int forced_chunks = [] {  // B200_HOST_CHUNKS=1..16 overrides the pipeline depth
         const char* e = getenv("B200_HOST_CHUNKS");

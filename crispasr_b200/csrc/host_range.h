@@ -14,4 +14,13 @@ bool inside_one_allocation(Query query, uintptr_t p, size_t bytes) {
     return query(p, &start, &size) && start <= p && p - start <= size && bytes <= size - (p - start);
 }
 
+// How a result [dst, dst + n * stride) of n entries meets an operand of m entries, [p, p + (m - 1) * entry_stride + entry_bytes).
+// kByEntry: entry i of the operand lies inside entry i of the result (an update in place): entries stay independent.
+enum class Meets { kNot, kByEntry, kAnyhow };
+inline Meets result_meets(uintptr_t dst, size_t stride, size_t n, uintptr_t p, size_t entry_stride, size_t entry_bytes, size_t m) {
+    const size_t span = (m - 1) * entry_stride + entry_bytes;
+    if (p >= dst + n * stride || dst >= p + span) return Meets::kNot;
+    return m == n && p >= dst && p - dst + entry_bytes <= stride && (n == 1 || entry_stride == stride) ? Meets::kByEntry : Meets::kAnyhow;
+}
+
 }  // namespace b200

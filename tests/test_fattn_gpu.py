@@ -1026,3 +1026,17 @@ def test_workspace_of_a_launch_on_another_stream(b200, orc):
     torch.cuda.synchronize()
     assert bool((y == 7).all()) and bool((z == 9).all())
     assert_close(out.cpu().numpy(), orc.flash_attn_ext(q, k.astype(np.float16), v.astype(np.float16), scale=0.125), "launch on another stream")
+
+
+@pytest.mark.parametrize("B,H,T", [(1, 20, 1500), (3, 20, 1500)])
+def test_host_entry_point_result_over_its_query(b200, orc, B, H, T):
+    """The result may take the place of the query: the heads of an entry, which lie apart in the query and side by side in the
+    result, then have to be uploaded before any of them is written."""
+    rng = np.random.default_rng(B)
+    q, k, v = (randn_f16(rng, (B, H, T, 64)) for _ in "qkv")
+    hq = torch.from_numpy(q.astype(np.float32)).pin_memory()
+    hk, hv = torch.from_numpy(k).pin_memory(), torch.from_numpy(v).pin_memory()
+    out = hq.view(B, T, H, 64)
+    assert b200.flash_attn_ext_host(hq, hk, hv, scale=0.125, out=out) is out
+    rows = np.arange(0, T, 37)
+    assert_close(out.numpy()[:, rows], orc.flash_attn_ext(q, k, v, scale=0.125, rows=rows)[:, rows], "result in place of the query")
