@@ -76,6 +76,12 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// An ordinary load.  Not __ldg: the non-coherent path asks for data that nobody writes while the kernel lives, and a kernel
+// launched with programmatic stream serialisation lives while the kernel before it (an append to the cache, say) still
+// writes; griddepcontrol.wait makes those writes visible to ordinary loads.
+template <typename T>
+__device__ __forceinline__ T load_global(const T* p) { return *p; }
+
 // Eight Q elements [c0, c0+8) of one row plus eight fp32 bias values, as packed f16: the sum is formed in fp32
 // and rounded once (an F32 add followed by the conversion to F16). F16 and F32 rows only; c0 + 8 <= head_dim.
 __device__ __forceinline__ uint4 load8_plus_bias_as_half(const uint8_t* rowp, int type, int c0, bool vec16,
@@ -84,7 +90,7 @@ __device__ __forceinline__ uint4 load8_plus_bias_as_half(const uint8_t* rowp, in
     if (type == B200_TYPE_F16) {
         uint32_t w[4];
         if (vec16) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(rowp + 2 * c0));
+            const uint4 u = load_global(reinterpret_cast<const uint4*>(rowp + 2 * c0));
             w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
         } else {
             const uint16_t* h = reinterpret_cast<const uint16_t*>(rowp + 2 * c0);
@@ -97,15 +103,15 @@ __device__ __forceinline__ uint4 load8_plus_bias_as_half(const uint8_t* rowp, in
             f[2 * i] = p.x, f[2 * i + 1] = p.y;
         }
     } else if (vec16) {
-        const float4 x = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0));
-        const float4 y = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
+        const float4 x = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0));
+        const float4 y = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
         f[0] = x.x, f[1] = x.y, f[2] = x.z, f[3] = x.w, f[4] = y.x, f[5] = y.y, f[6] = y.z, f[7] = y.w;
     } else {
 #pragma unroll
         for (int i = 0; i < 8; i++) f[i] = *reinterpret_cast<const float*>(rowp + 4 * (c0 + i));
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) f[i] = __fadd_rn(f[i], __ldg(bias8 + i));
+    for (int i = 0; i < 8; i++) f[i] = __fadd_rn(f[i], load_global(bias8 + i));
     uint4 out;
     out.x = pack_half2(f[0], f[1]), out.y = pack_half2(f[2], f[3]);
     out.z = pack_half2(f[4], f[5]), out.w = pack_half2(f[6], f[7]);

@@ -83,7 +83,7 @@ __device__ __forceinline__ uint4 load8_as_half(const uint8_t* rowp, int type, in
     uint4 out = make_uint4(0u, 0u, 0u, 0u);
     if (c0 >= hd) return out;
     if (type == B200_TYPE_F16) {
-        if (vec16 && c0 + 8 <= hd) return __ldg(reinterpret_cast<const uint4*>(rowp + 2 * c0));
+        if (vec16 && c0 + 8 <= hd) return load_global(reinterpret_cast<const uint4*>(rowp + 2 * c0));
         __half tmp[8];
 #pragma unroll
         for (int i = 0; i < 8; i++)
@@ -92,8 +92,8 @@ __device__ __forceinline__ uint4 load8_as_half(const uint8_t* rowp, int type, in
     } else if (type == B200_TYPE_F32) {
         float f[8];
         if (vec16 && c0 + 8 <= hd) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0));
-            const float4 b = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
+            const float4 a = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0));
+            const float4 b = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
             f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
         } else {
 #pragma unroll
@@ -136,7 +136,7 @@ __device__ __forceinline__ void load_tile(__half* sm, const uint8_t* base, int64
         const int grow = row0 + row;
         uint4 val = make_uint4(0u, 0u, 0u, 0u);
         if (grow >= row_lo && grow < row_hi) {
-            const int src = index ? min(max(__ldg(index + grow), 0), pool_rows - 1) : grow;
+            const int src = index ? min(max(load_global(index + grow), 0), pool_rows - 1) : grow;
             val = load8_as_half(base + (int64_t)src * nb1, type, ch * 8, hd, vec16);
         }
         *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sm) + (row * CPR + swz<HD>(row, ch)) * 16) = val;
@@ -165,7 +165,7 @@ __device__ __forceinline__ void load_tile_bias(__half* sm, const uint8_t* base, 
                         const float x = type == B200_TYPE_F16
                                             ? __half2float(*reinterpret_cast<const __half*>(rowp + 2 * (c0 + i)))
                                             : *reinterpret_cast<const float*>(rowp + 4 * (c0 + i));
-                        f[i] = __fadd_rn(x, __ldg(bias + c0 + i));
+                        f[i] = __fadd_rn(x, load_global(bias + c0 + i));
                     }
                 }
                 val.x = pack_half2(f[0], f[1]), val.y = pack_half2(f[2], f[3]);
@@ -474,7 +474,7 @@ struct TilePieces {
 #pragma unroll
         for (int i = 0; i < N; i++) {
             const int grow = row0 + row + i * kRows;
-            idx[i] = grow < row_hi ? __ldg(index + grow) : 0;   // clamped where it is used: nothing here waits for the load
+            idx[i] = grow < row_hi ? load_global(index + grow) : 0;   // clamped where it is used: nothing here waits for the load
         }
     }
 };
@@ -841,8 +841,8 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
             row_to_query(a, hk, rr, iq, hq);
             const uint8_t* rowp = a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3;
             if (q_f32) {
-                q_val[i] = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * ch);
-                q_hi[i] = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * ch + 1);
+                q_val[i] = load_global(reinterpret_cast<const uint4*>(rowp) + 2 * ch);
+                q_hi[i] = load_global(reinterpret_cast<const uint4*>(rowp) + 2 * ch + 1);
             } else {
                 q_val[i] = load8_as_half(rowp, a.q.type, ch * 8, a.hd, a.q.vec16);
             }
@@ -1492,8 +1492,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
         row_to_query(a, hk, q_row, iq, hq);
         const uint8_t* rowp = a.q.p + (int64_t)iq * a.q.nb1 + (int64_t)hq * a.q.nb2 + (int64_t)b * a.q.nb3;
         if (q_f32) {
-            q_val = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch);
-            q_hi = __ldg(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch + 1);
+            q_val = load_global(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch);
+            q_hi = load_global(reinterpret_cast<const uint4*>(rowp) + 2 * q_ch + 1);
         } else {
             q_val = load8_as_half(rowp, a.q.type, q_ch * 8, a.hd, a.q.vec16);
         }
@@ -2074,9 +2074,9 @@ __global__ void __launch_bounds__(256) kv_to_f16_kernel(const View src0, uint8_t
             if (row0 + u * RPW < Lk) {
                 const uint8_t* rowp = base + (int64_t)(row0 + u * RPW) * src.nb1;
                 const uint32_t* p = reinterpret_cast<const uint32_t*>(rowp + off + 2 * odd);
-                w[u][0] = __ldg(p), w[u][1] = __ldg(p + 1);
-                w[u][2] = odd ? 0u : (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p + 2));
-                d[u] = __ldg(reinterpret_cast<const uint16_t*>(rowp + 34 * blk));
+                w[u][0] = load_global(p), w[u][1] = load_global(p + 1);
+                w[u][2] = odd ? 0u : (uint32_t)load_global(reinterpret_cast<const uint16_t*>(p + 2));
+                d[u] = load_global(reinterpret_cast<const uint16_t*>(rowp + 34 * blk));
             }
         const uint32_t fs = odd ? 0u : 16u;
         const __half2 bias = __float2half2_rn(1152.0f);

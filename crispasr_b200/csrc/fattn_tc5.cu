@@ -302,7 +302,7 @@ __device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {
     uint4 out;
     if (type == B200_TYPE_F16) {
-        if (vec16) return __ldg(reinterpret_cast<const uint4*>(rowp + 2 * c0));
+        if (vec16) return load_global(reinterpret_cast<const uint4*>(rowp + 2 * c0));
         const uint16_t* h = reinterpret_cast<const uint16_t*>(rowp + 2 * c0);
         out.x = h[0] | ((uint32_t)h[1] << 16), out.y = h[2] | ((uint32_t)h[3] << 16);
         out.z = h[4] | ((uint32_t)h[5] << 16), out.w = h[6] | ((uint32_t)h[7] << 16);
@@ -310,8 +310,8 @@ __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, 
     }
     float f[8];
     if (vec16) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0));
-        const float4 b = __ldg(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
+        const float4 a = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0));
+        const float4 b = load_global(reinterpret_cast<const float4*>(rowp + 4 * c0 + 16));
         f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
     } else {
 #pragma unroll
@@ -365,12 +365,12 @@ __device__ __forceinline__ void load_mask64(uint4 (&mv)[8], const uint8_t* mptr,
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         if (q * 8 + 8 <= avail && ((reinterpret_cast<uintptr_t>(mptr) & 15) == 0)) {
-            mv[q] = __ldg(reinterpret_cast<const uint4*>(mptr + q * 16));
+            mv[q] = load_global(reinterpret_cast<const uint4*>(mptr + q * 16));
         } else {   // the end of the row, or a row that does not start on a 16-byte boundary (mask rows hold exactly Lk values)
             uint16_t hv[8];
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                hv[i] = (q * 8 + i < avail) ? __ldg(reinterpret_cast<const uint16_t*>(mptr + (q * 8 + i) * 2)) : (uint16_t)0;
+                hv[i] = (q * 8 + i < avail) ? load_global(reinterpret_cast<const uint16_t*>(mptr + (q * 8 + i) * 2)) : (uint16_t)0;
             mv[q] = make_uint4(hv[0] | ((uint32_t)hv[1] << 16), hv[2] | ((uint32_t)hv[3] << 16), hv[4] | ((uint32_t)hv[5] << 16),
                                hv[6] | ((uint32_t)hv[7] << 16));
         }
@@ -442,13 +442,13 @@ __device__ __forceinline__ void load_q_row(uint8_t* tile, int r, const uint8_t* 
         for (int c = 0; c < HD / 8; c++) v[c] = make_uint4(0u, 0u, 0u, 0u);
     } else if (type == B200_TYPE_F16 && vec16) {
 #pragma unroll
-        for (int c = 0; c < HD / 8; c++) v[c] = __ldg(reinterpret_cast<const uint4*>(rowp) + c);
+        for (int c = 0; c < HD / 8; c++) v[c] = load_global(reinterpret_cast<const uint4*>(rowp) + c);
     } else if (type == B200_TYPE_F32 && vec16) {
 #pragma unroll
         for (int c0 = 0; c0 < HD / 8; c0 += 4) {  // 4 chunks = 8 float4 in flight
             float4 f[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = __ldg(reinterpret_cast<const float4*>(rowp) + c0 * 2 + i);
+            for (int i = 0; i < 8; i++) f[i] = load_global(reinterpret_cast<const float4*>(rowp) + c0 * 2 + i);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 v[c0 + i].x = pack_half2(f[2 * i].x, f[2 * i].y), v[c0 + i].y = pack_half2(f[2 * i].z, f[2 * i].w);
@@ -489,7 +489,7 @@ __device__ __forceinline__ void load_q_rows_f32_coalesced(uint8_t* tile, int war
         for (int k = 0; k < 16; k++) {
             const int src = (batch * 16 + k) * RPI + sub;
             const uintptr_t p = (uintptr_t)__shfl_sync(0xffffffffu, plo, src) | ((uintptr_t)__shfl_sync(0xffffffffu, phi, src) << 32);
-            f[k] = p ? __ldg(reinterpret_cast<const float4*>(p) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            f[k] = p ? load_global(reinterpret_cast<const float4*>(p) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int k = 0; k < 16; k++) {
@@ -512,7 +512,7 @@ __device__ __forceinline__ void load_q_rows_f16_coalesced(uint8_t* tile, int war
     for (int k = 0; k < 32 / RPI; k++) {
         const int src = k * RPI + sub;
         const uintptr_t p = (uintptr_t)__shfl_sync(0xffffffffu, plo, src) | ((uintptr_t)__shfl_sync(0xffffffffu, phi, src) << 32);
-        v[k] = p ? __ldg(reinterpret_cast<const uint4*>(p) + cc) : make_uint4(0u, 0u, 0u, 0u);
+        v[k] = p ? load_global(reinterpret_cast<const uint4*>(p) + cc) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int k = 0; k < 32 / RPI; k++) {
@@ -1103,7 +1103,7 @@ __device__ __forceinline__ void load_relpos_q(uint8_t* tile_u, uint8_t* tile_v, 
     if (BIAS) {
 #pragma unroll
         for (int i = 0; i < N; i += 4) {
-            const float4 x = __ldg(reinterpret_cast<const float4*>(bias_u + c + i)), y = __ldg(reinterpret_cast<const float4*>(bias_v + c + i));
+            const float4 x = load_global(reinterpret_cast<const float4*>(bias_u + c + i)), y = load_global(reinterpret_cast<const float4*>(bias_v + c + i));
             bu[i] = x.x, bu[i + 1] = x.y, bu[i + 2] = x.z, bu[i + 3] = x.w;
             bv[i] = y.x, bv[i + 1] = y.y, bv[i + 2] = y.z, bv[i + 3] = y.w;
         }
@@ -1113,7 +1113,7 @@ __device__ __forceinline__ void load_relpos_q(uint8_t* tile_u, uint8_t* tile_v, 
     for (int k = 0; k < K; k++) {
         const int r = warp * 16 + k * RPI + (F16 ? lane >> 4 : 0);
         v[k] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < rows) v[k] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)(q0 + r) * nb1 + c * (F16 ? 2 : 4)));
+        if (r < rows) v[k] = load_global(reinterpret_cast<const uint4*>(base + (int64_t)(q0 + r) * nb1 + c * (F16 ? 2 : 4)));
     }
 #pragma unroll
     for (int k = 0; k < K; k++) {

@@ -415,3 +415,16 @@ def test_the_library_is_built_without_torch(monkeypatch, tmp_path):
     monkeypatch.setitem(sys.modules, "torch", None)   # import torch raises ImportError, find_spec finds nothing
     assert build.build() == build.LIB and len(ran) == 2   # one object, one link
     assert not build.needs_build() and build.build() == build.LIB and len(ran) == 2
+
+
+def test_kernels_that_overlap_their_predecessor_load_coherently():
+    """Sources whose kernels are launched with programmatic stream serialisation use no non-coherent load: their operands may
+    still be written when they start."""
+    csrc = os.path.join(ROOT, "crispasr_b200", "csrc")
+    seen = 0
+    for f in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        if "griddepcontrol.wait" in text or f == "fattn_common.cuh":
+            seen += 1
+            assert not re.search(r"__ldg\s*\(|ld\.global\.nc|__restrict__", text), f
+    assert seen >= 5
