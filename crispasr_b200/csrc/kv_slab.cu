@@ -114,6 +114,10 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
             uint32_t q[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) q[i] = round_away(__fmul_rn(f[i], id));
+            if (isinf(id)) {   // amax below 4e-37: 1/d is beyond a float, and x * (1/d) an infinity or NaN, converted as such
+#pragma unroll
+                for (int i = 0; i < 8; i++) q[i] = (uint32_t)(int)roundf(__fmul_rn(f[i], id));
+            }
             const uint32_t w0 = low_bytes(q[0], q[1], q[2], q[3]), w1 = low_bytes(q[4], q[5], q[6], q[7]);
             const uint32_t dbits = __half_as_ushort(__float2half_rn(d));
             const uint32_t left = __shfl_up_sync(0xffffffffu, w1, 1);

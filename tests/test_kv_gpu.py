@@ -253,3 +253,26 @@ def test_append_row_shapes(b200, orc, type_, hd, n_new):
         want[1, :, ctx - 2:ctx - 2 + n1] = enc[1][:, :n1]
         assert np.array_equal(raw, want)
     kv.close()
+
+
+@pytest.mark.parametrize("amax", [1e-36, 4e-37, 3e-37, 1e-38, 1e-43])
+def test_append_blocks_of_tiny_values(b200, amax):
+    """Blocks whose scale d = amax / 127 is so small that 1 / d leaves the range of a float: x * (1 / d) is an infinity, or NaN
+    for 0, and its conversion to an integer saturates: bytes 0xFF for positive, 0x00 for negative x and for 0."""
+    kv = b200.KvCache(abi.Q8_0, 64, 1, n_layers=1, max_ctx=32, n_streams=1)
+    x = np.zeros((1, 1, 2, 64), np.float32)
+    x[0, 0, 0, ::3], x[0, 0, 1, ::2], x[0, 0, 1, 1::4] = amax, amax, -amax
+    t = torch.from_numpy(x).cuda()
+    kv.append(0, t, t)
+    torch.cuda.synchronize()
+    with np.errstate(all="ignore"):
+        d = np.float32(amax) / np.float32(127)
+        inv = np.float32(1) / d if d else np.float32(0)
+        p = x * inv
+        r = np.where(np.isfinite(p), np.trunc(np.where(np.isfinite(p), p, 0) + np.copysign(np.float32(0.5), p)), 0)
+    q = np.where(p == np.inf, 0xFF, np.where(np.isfinite(p), r.astype(np.int64) & 0xFF, 0)).astype(np.uint8)
+    for s in kv.view(0, 2):
+        raw = _read_slab(s, 2 * s.nb[1]).reshape(2, 2, 34)
+        assert (raw[..., :2].view(np.float16)[..., 0] == np.float16(d)).all()
+        assert np.array_equal(raw[..., 2:].reshape(2, 64), q[0, 0])
+    kv.close()
