@@ -701,9 +701,9 @@ __device__ __forceinline__ void decode_write_out(const FattnArgs& a, const float
             row_to_query(a, hk, rr, iq, hq);
             const float inv = (L > 0.0f && iq < tq_b) ? 1.0f / L : 0.0f;
             float* drow = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + hq) * a.hd;
-            if (a.hd == HD) {
+            if (a.hd == HD && (HD > 32 || (reinterpret_cast<uintptr_t>(drow) & 15) == 0)) {   // (head_dim 32 has no rule on the result's alignment)
                 *reinterpret_cast<float4*>(drow + 4 * cg) = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
-            } else {   // a head dim padded up to HD: the row is a.hd floats long
+            } else {   // the row is a.hd floats long: a head dim padded up to HD, or an unaligned result
                 const float vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                 for (int j = 0; j < 4; j++)

@@ -1040,3 +1040,22 @@ def test_host_entry_point_result_over_its_query(b200, orc, B, H, T):
     assert b200.flash_attn_ext_host(hq, hk, hv, scale=0.125, out=out) is out
     rows = np.arange(0, T, 37)
     assert_close(out.numpy()[:, rows], orc.flash_attn_ext(q, k, v, scale=0.125, rows=rows)[:, rows], "result in place of the query")
+
+
+@pytest.mark.parametrize("kv_kind", ["f16", "q8_0"])
+def test_head_dim_32_into_an_unaligned_result(b200, orc, kv_kind):
+    """The result of head_dim 32 may start on any 4-byte boundary, decode steps without splits included."""
+    rng = np.random.default_rng(1)
+    q, k = randn_f16(rng, (2, 4, 3, 32)), rng.standard_normal((2, 2, 40, 32)).astype(np.float32)
+    kw = dict(scale=32 ** -0.5)
+    if kv_kind == "q8_0":
+        kv, kw["kv_type"] = orc.quantize_q8_0(k), abi.Q8_0
+    else:
+        kv = k.astype(np.float16)
+    out = torch.empty(2 * 3 * 4 * 32 + 1, device="cuda")[1:].view(2, 3, 4, 32)
+    assert out.data_ptr() % 16 == 4
+    dkv = torch.from_numpy(kv).cuda()
+    b200.flash_attn_ext(torch.from_numpy(q).cuda(), dkv, dkv, out=out, **kw)
+    torch.cuda.synchronize()
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_DECODE_SPLIT
+    assert_close(out.cpu().numpy(), orc.flash_attn_ext(q, kv, kv, **kw), f"unaligned result, {kv_kind}")
