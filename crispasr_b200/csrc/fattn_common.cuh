@@ -76,11 +76,30 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// An ordinary load.  Not __ldg: the non-coherent path asks for data that nobody writes while the kernel lives, and a kernel
-// launched with programmatic stream serialisation lives while the kernel before it (an append to the cache, say) still
-// writes; griddepcontrol.wait makes those writes visible to ordinary loads.
+// An ordinary load, in its place behind griddepcontrol.wait.  Not __ldg: the non-coherent path asks for data that nobody
+// writes while the kernel lives, and a kernel launched with programmatic stream serialisation lives while the kernel before
+// it (an append to the cache, say) still writes; the wait makes those writes visible to ordinary loads.  As volatile
+// assembly, which stays where it was written: as a plain expression the compiler moved the query loads of a decode CTA (one
+// step of the base decoder 54 -> 62 us).
 template <typename T>
-__device__ __forceinline__ T load_global(const T* p) { return *p; }
+__device__ __forceinline__ T load_global(const T* p) {
+    T r;
+    if constexpr (sizeof(T) == 16) {
+        uint32_t x[4];
+        asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "l"(p) : "memory");
+        memcpy(&r, x, 16);
+    } else if constexpr (sizeof(T) == 4) {
+        uint32_t x;
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+        memcpy(&r, &x, 4);
+    } else {
+        static_assert(sizeof(T) == 2, "16, 4 or 2 bytes");
+        uint16_t x;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(x) : "l"(p) : "memory");
+        memcpy(&r, &x, 2);
+    }
+    return r;
+}
 
 // Eight Q elements [c0, c0+8) of one row plus eight fp32 bias values, as packed f16: the sum is formed in fp32
 // and rounded once (an F32 add followed by the conversion to F16). F16 and F32 rows only; c0 + 8 <= head_dim.
