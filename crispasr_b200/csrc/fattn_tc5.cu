@@ -98,6 +98,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     atomicExch(&g_tc5_status, 1);
     return false;
 }
+// One answer for all lanes: the issuing warps elect a lane behind their waits, which needs every lane there, also when a wait
+// ran out for some.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -791,6 +794,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             };
             bool ok = mbar_wait(bar_k_full, 0, s_abort);
             if (ok && q_tma) ok = mbar_wait(q_raw ? bar_q_conv : bar_q_full, 0, s_abort);
+            ok = warp_all(ok);
             if (ok) {
                 TC5_TRACE(1, 0, 0);
                 tc_fence_after();
@@ -807,9 +811,9 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 const bool more = j + 1 < n_tiles;
                 ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
                 if (ok && more) ok = mbar_wait(bar_k_full + 8 * nslot, nuse & 1, s_abort);
-                if (!ok) break;
                 TC5_TRACE(1, j, 2);
-                ok = mbar_wait(bar_p_ready, j & 1, s_abort);
+                if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
+                ok = warp_all(ok);
                 if (!ok) break;
                 TC5_TRACE(1, j, 3);
                 tc_fence_after();
@@ -836,9 +840,11 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 __syncwarp();
                 TC5_TRACE(1, j, 4);
             }
-            if (!ok && lane == 0) {
-                // make sure no MMA of this CTA is still running before TMEM is released
-                tc_commit(bar_o_done);
+            if (!ok) {
+                // make sure no MMA of this CTA is still running before TMEM is released (the commit comes from the lane that
+                // issued them)
+                if (elect_one()) tc_commit(bar_o_done);
+                __syncwarp();
                 for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
             }
             __syncwarp();
@@ -1355,6 +1361,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             };
             bool ok = mbar_wait(bar_r_full, 0, s_abort) && mbar_wait(bar_r_full + 8, 0, s_abort) &&
                       mbar_wait(bar_k_full, 0, s_abort);
+            ok = warp_all(ok);
             if (ok) {
                 tc_fence_after();
                 if (elect_one()) {
@@ -1370,6 +1377,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                     // half-block j+2 is in its slot, and the columns of half-block j have been read
                     ok = mbar_wait(bar_r_full + 8 * (j & 1), ((j + 2) >> 1) & 1, s_abort) &&
                          mbar_wait(bar_x_free, j & 1, s_abort);
+                    ok = warp_all(ok);
                     if (!ok) break;
                     TC5_TRACE(1, j, 0);
                     tc_fence_after();
@@ -1380,6 +1388,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 ok = mbar_wait(bar_v_full, j & 1, s_abort);
                 if (ok && more) ok = mbar_wait(bar_k_full, (j + 1) & 1, s_abort);
                 if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
+                ok = warp_all(ok);
                 if (!ok) break;
                 TC5_TRACE(1, j, 2);
                 tc_fence_after();
@@ -1395,8 +1404,9 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 __syncwarp();
                 TC5_TRACE(1, j, 3);
             }
-            if (!ok && lane == 0) {
-                tc_commit(bar_o_done);
+            if (!ok) {
+                if (elect_one()) tc_commit(bar_o_done);
+                __syncwarp();
                 for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
             }
             __syncwarp();

@@ -158,6 +158,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
             int k_issued = min(2, n_tiles), v_issued = 1;
             const bool any = !SPLIT || n_tiles > 0;   // a split beyond the last step has nothing to do
             bool ok = !any || ((!QTMA || mbar_wait(bar_q, 0, s_abort)) && mbar_wait(bar_k, 0, s_abort));
+            ok = warp_all(ok);
             if (ok && any) {
                 tc_fence_after();
                 if (elect_one()) {
@@ -171,6 +172,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                 ok = mbar_wait(bar_v + 8 * (j & 1), (j >> 1) & 1, s_abort);
                 if (ok && more) ok = mbar_wait(bar_k + 8 * ((j + 1) & 1), ((j + 1) >> 1) & 1, s_abort);
                 if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
+                ok = warp_all(ok);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t vd = v_lo + (j & 1) * (kH64KvBytes >> 4);
@@ -187,9 +189,11 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
                 if (j > 0 && more) v_issued = j + 2;
                 if (j + 2 < n_tiles) k_issued = j + 3;
             }
-            if (!ok && lane == 0) {
-                // no MMA and no copy of this CTA may still be running when its memory is released
-                tc_commit(bar_o_done);
+            if (!ok) {
+                // no MMA and no copy of this CTA may still be running when its memory is released (the commit comes from the
+                // lane that issued the MMAs)
+                if (elect_one()) tc_commit(bar_o_done);
+                __syncwarp();
                 for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
                 if (QTMA)
                     for (uint32_t it = 0; it < 4096 && !mbar_try_wait(bar_q, 0); ++it) __nanosleep(256);
