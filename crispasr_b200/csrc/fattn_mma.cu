@@ -61,16 +61,6 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Same product with the accumulator rows g+8 in caller-chosen registers: when those rows are padding (all zeros in
-// A and in C) a few shared zero registers stand in for them and the real accumulator needs half the registers.
-__device__ __forceinline__ void mma16816_lo(float& c0, float& c1, float& z0, float& z1, const uint32_t (&a)[4], uint32_t b0,
-                                            uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c0), "+f"(c1), "+f"(z0), "+f"(z1)
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
 // 2^x on the exponential unit, one instruction (exp2f adds a range fix-up that P in f16 does not need; -inf -> 0).
 __device__ __forceinline__ float fast_ex2(float x) {
     float y;
@@ -1120,11 +1110,9 @@ constexpr int kDecRegStages = 3;
 
 // PLAIN: no explicit mask, no softcap, no causal bound (single-token decode): only kv_len limits the keys.  A separate
 // instantiation, so the common case carries none of the general path's registers and code.
-// LOW (with PLAIN): at most 8 live rows (Tq * gqa <= 8), so rows g+8 of every fragment are padding and their softmax
-// arithmetic is skipped.
-template <int HD, bool PLAIN, bool LOW = false>
+// (Plain calls of at most 8 query rows are the keys-on-M kernel's, below.)
+template <int HD, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const FattnArgs a) {
-    constexpr int NR = LOW ? 1 : 2, NE = 2 * NR;   // live row halves / accumulator elements per n-tile
     constexpr int NBLK = HD / 32, RB = NBLK * 34;
     constexpr int RAW_BYTES = kDecBN * RB;   // one raw K or V tile
     constexpr int NS = kDecRegStages;
@@ -1222,7 +1210,6 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
     float o[HD / 8][4];   // n-tile 4*blk + j, column n <-> dim 32blk + 4n + j
 #pragma unroll
     for (int i = 0; i < HD / 8; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    float zpad[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};   // LOW: stand-ins for the padding rows of O (stay 0)
     const __half2 bias = __float2half2_rn(1152.0f);
     auto cvt2 = [&](uint32_t packed, __half2 d2) {   // {0x64 q1' 0x64 q0'} -> {d*q0, d*q1}
         const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&packed), bias), d2);
@@ -1276,7 +1263,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
 #pragma unroll
             for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-                for (int e = 0; e < NE; e++) {
+                for (int e = 0; e < 4; e++) {
                     s[nt][e] *= c;
                     rmax[e >> 1] = fmaxf(rmax[e >> 1], s[nt][e]);
                 }
@@ -1285,7 +1272,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
 #pragma unroll
             for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-                for (int e = 0; e < NE; e++) {
+                for (int e = 0; e < 4; e++) {
                     const int ik = k0 + warp * 16 + nt * 8 + 2 * t + (e & 1);
                     s[nt][e] = ik < len_b ? s[nt][e] * c : ninf;
                     rmax[e >> 1] = fmaxf(rmax[e >> 1], s[nt][e]);
@@ -1311,7 +1298,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
         // when a row's tile maximum outgrew it by 2^8, so P <= 256 stays inside f16 and most tiles skip the rescale.
         float alpha[2] = {1.0f, 1.0f}, muse[2] = {0.0f, 0.0f};
 #pragma unroll
-        for (int rI = 0; rI < NR; rI++) {
+        for (int rI = 0; rI < 2; rI++) {
             const float mt = quad_max(rmax[rI]);
             const float mnew = (mt > m_run[rI] + 8.0f) ? mt : m_run[rI];   // -inf + 8 = -inf: the first finite maximum is taken
             muse[rI] = mnew == ninf ? 0.0f : mnew;
@@ -1323,10 +1310,6 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
         for (int nt = 0; nt < 2; nt++)
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                if (e >= NE) {
-                    s[nt][e] = 0.0f;   // padding rows: P = 0
-                    continue;
-                }
                 const float p = fast_ex2(s[nt][e] - muse[e >> 1]);
                 s[nt][e] = p;
                 l_run[e >> 1] += p;
@@ -1341,7 +1324,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
 #pragma unroll
             for (int i = 0; i < HD / 8; i++) {
                 o[i][0] *= alpha[0], o[i][1] *= alpha[0];
-                if (!LOW) o[i][2] *= alpha[1], o[i][3] *= alpha[1];
+                o[i][2] *= alpha[1], o[i][3] *= alpha[1];
             }
         }
 
@@ -1369,14 +1352,10 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
             // pair the two keys of an operand register: x = {k0.j, k1.j, k0.j', k1.j'}
             const uint32_t x01a = __byte_perm(w[0], w[1], 0x5140), x01b = __byte_perm(w[0], w[1], 0x7362);
             const uint32_t x23a = __byte_perm(w[2], w[3], 0x5140), x23b = __byte_perm(w[2], w[3], 0x7362);
-            if (LOW) mma16816_lo(o[4 * blk + 0][0], o[4 * blk + 0][1], zpad[0][0], zpad[0][1], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x5140), d23));
-            else mma16816(o[4 * blk + 0], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x5140), d23));
-            if (LOW) mma16816_lo(o[4 * blk + 1][0], o[4 * blk + 1][1], zpad[1][0], zpad[1][1], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x7362), d23));
-            else mma16816(o[4 * blk + 1], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x7362), d23));
-            if (LOW) mma16816_lo(o[4 * blk + 2][0], o[4 * blk + 2][1], zpad[2][0], zpad[2][1], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x5140), d23));
-            else mma16816(o[4 * blk + 2], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x5140), d23));
-            if (LOW) mma16816_lo(o[4 * blk + 3][0], o[4 * blk + 3][1], zpad[3][0], zpad[3][1], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x7362), d23));
-            else mma16816(o[4 * blk + 3], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x7362), d23));
+            mma16816(o[4 * blk + 0], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x5140), d23));
+            mma16816(o[4 * blk + 1], pf, cvt2(__byte_perm(x01a, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23a, 0x64646464u, 0x7362), d23));
+            mma16816(o[4 * blk + 2], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x5140), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x5140), d23));
+            mma16816(o[4 * blk + 3], pf, cvt2(__byte_perm(x01b, 0x64646464u, 0x7362), d01), cvt2(__byte_perm(x23b, 0x64646464u, 0x7362), d23));
         }
         __syncwarp();       // every lane is done with this stage's bytes
         issue(tile + NS);   // the next tile that lives in this stage: NS-1 tiles stay in flight during the arithmetic
@@ -1400,7 +1379,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
     // thread four consecutive dims of rows g and g + 8 (dim = 32 blk + 4 (2t + e) + n-tile), one 16-byte store each;
     // rows at or beyond R are never read.
 #pragma unroll
-    for (int rI = 0; rI < NR; rI++) {
+    for (int rI = 0; rI < 2; rI++) {
         if (g + rI * 8 >= R) continue;
 #pragma unroll
         for (int blk = 0; blk < HD / 32; blk++)
@@ -2000,13 +1979,13 @@ int launch_decode_q8reg(const FattnArgs& a, cudaStream_t st) {
         else go(fattn_decode_q8t_kernel<HD, 4>, 4, set[1]);
         if (e != cudaSuccess) return (int)e;
     } else if (!a.has_mask && a.softcap == 0.0f && !a.causal) {
-        auto kern = fattn_decode_q8reg_kernel<HD, true, false>;
+        auto kern = fattn_decode_q8reg_kernel<HD, true>;
         static bool smem_set[64] = {false};
         e = set_smem_once(kern, smem_attr, smem_set);
         if (e != cudaSuccess) return (int)e;
         launch_split(kern, grid, smem, st, a);
     } else {
-        auto kern = fattn_decode_q8reg_kernel<HD, false, false>;
+        auto kern = fattn_decode_q8reg_kernel<HD, false>;
         static bool smem_set[64] = {false};
         e = set_smem_once(kern, smem_attr, smem_set);
         if (e != cudaSuccess) return (int)e;

@@ -129,16 +129,6 @@ __device__ __forceinline__ void tma_store_commit_and_wait_read() {
 // Shared-memory matrix descriptor, SWIZZLE_128B, descriptor version 1 (sm_100).
 //   K-major operand : rows of 128 bytes, 8-row groups 1024 bytes apart  -> LBO = 16 B (unused), SBO = 1024 B
 //   MN-major operand: 64-element chunks `lbo` bytes apart, 8-k groups 1024 bytes apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;   // version
-    d |= (uint64_t)2 << 61;   // SWIZZLE_128B
-    return d;
-}
-
 // The two 32-bit words of a descriptor.  Only the low word carries the address (bits 0-13, in 16-byte units),
 // so stepping through an operand is one 32-bit add: the issuing thread's instruction latency, not the tensor
 // pipe, bounds how fast small MMAs can be issued.
@@ -468,12 +458,6 @@ __device__ __forceinline__ void load_q_row(uint8_t* tile, int r, const uint8_t* 
         *reinterpret_cast<uint4*>(dst_row + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) = v[c];
 }
 
-struct Tc5Smem {
-    // offsets from the 1024-byte aligned base of dynamic shared memory
-    template <int HD, int NSTG>
-    static constexpr int tile_bytes() { return kPanelBytes * (HD / 64); }
-};
-
 // Coalesced forms of the two per-row transfers of a CTA.  A thread that moves its own row makes every warp instruction
 // touch 32 rows (32 sectors for 16 bytes each); here a warp instruction covers whole rows, the row pointers travel by
 // shuffle from the lanes that own them (lane i of warp w owns row 32w + i).
@@ -569,15 +553,12 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     uint8_t* misc = smem_gen + (1 + 2 * NSTG) * TILE_BYTES + 32 * NSTG + 64;
     // q_tma: 0 = the softmax warps load and convert the Q tile; 1 = F16 rows by one tensor copy into the operand tile;
     // 2 = F32 rows by tensor copies into stages that are not needed yet, converted from there by the softmax warps.
-    // head_dim 128 (the form that is launched): the raw tile (64 KB) takes the K and the V stage, so the first K tile
+    // The raw tile (64 KB) takes the K and the V stage, so the first K tile
     // waits for the conversion too - still ahead of a register pass, whose global loads a CTA next to one in its key
     // loop issues at a few tens of clocks per instruction (T = 407 GQA prefill with an F32 Q: 4807 -> 5034 streams/s).
-    // head_dim 64 (the raw tile in the two V stages) measured 1459 against 1481 segments/s for the register pass on the
-    // encoder and is not launched.
-    constexpr bool RAW_OK = QMODE == 2 && ((HD == 64 && NSTG == 2) || (HD == 128 && NSTG == 1));
-    static_assert(QMODE != 2 || RAW_OK, "the raw form needs stages to park the tile in");
-    constexpr int RAW_OFF = HD == 64 ? (1 + NSTG) * TILE_BYTES : TILE_BYTES;   // V stages / K stage onwards
-    constexpr bool q_raw = RAW_OK;
+    constexpr bool q_raw = QMODE == 2;
+    static_assert(!q_raw || (HD == 128 && NSTG == 1), "the raw tile takes the stages of head_dim 128");
+    constexpr int RAW_OFF = TILE_BYTES;   // the K stage onwards
     // head_dim 64 leaves 64 spare TMEM columns: P gets its own, so S of the next tile can be issued before P.V
     constexpr bool SEP_P = (HD == 64);
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
@@ -660,7 +641,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
         // the first NSTG tiles need no empty-slot wait: start their copies before the CTA-wide set-up barrier
         for (int j = 0; j < NSTG && j < n_tiles; j++) {
-            if (q_raw && HD == 128) continue;   // the K stage holds raw Q rows for now
+            if (q_raw) continue;   // the K stage holds raw Q rows for now
             mbar_arrive_expect_tx(bar_k_full + 8 * j, TILE_BYTES);
 #pragma unroll
             for (int p = 0; p < PANELS; p++)
@@ -699,7 +680,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     const uint32_t tmem_S = tmem_base;            // cols [0,128)
     const uint32_t tmem_P = SEP_P ? tmem_base + kTile + HD : tmem_base;  // f16x2: cols [192,256) (hd 64) or aliasing S [0,64)
     const uint32_t tmem_O = tmem_base + kTile;    // cols [128,128+HD)
-    if constexpr (RAW_OK) {
+    if constexpr (q_raw) {
         if (q_raw && warp < 4) {
             // raw F32 row r (panels of 128-byte swizzled rows) -> F16 row r of the operand tile: HD / 4 loads, HD / 2
             // conversions, HD / 8 stores per thread, all from shared memory
@@ -726,17 +707,15 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         // ================= TMA producer =================
         if (lane == 0) {
             bool ok = true;
-            int issued_k = (q_raw && HD == 128) ? 0 : min(NSTG, n_tiles), issued_v = q_raw ? 0 : min(NSTG, n_tiles);
+            int issued_k = q_raw ? 0 : min(NSTG, n_tiles), issued_v = q_raw ? 0 : min(NSTG, n_tiles);
             if (q_raw) {
                 ok = mbar_wait(bar_q_conv, 0, s_abort);
                 for (int j = 0; j < NSTG && j < n_tiles && ok; j++) {
-                    if (HD == 128) {
-                        mbar_arrive_expect_tx(bar_k_full + 8 * j, TILE_BYTES);
+                    mbar_arrive_expect_tx(bar_k_full + 8 * j, TILE_BYTES);
 #pragma unroll
-                        for (int p = 0; p < PANELS; p++)
-                            tma_load_4d(sK + j * TILE_BYTES + p * kPanelBytes, &tmK, bar_k_full + 8 * j, p * 64, j * kTile, hk, bk);
-                        issued_k = j + 1;
-                    }
+                    for (int p = 0; p < PANELS; p++)
+                        tma_load_4d(sK + j * TILE_BYTES + p * kPanelBytes, &tmK, bar_k_full + 8 * j, p * 64, j * kTile, hk, bk);
+                    issued_k = j + 1;
                     mbar_arrive_expect_tx(bar_v_full + 8 * j, TILE_BYTES);
 #pragma unroll
                     for (int p = 0; p < PANELS; p++)
