@@ -22,13 +22,6 @@ namespace b200 {
 int decode_ctas_per_sm(const FattnArgs& a, bool cluster = false);   // resident CTAs of the split kernel per SM for these operands, as a cluster launch with its receive area if asked (defined below)
 
 __device__ int g_mma_status = 0;  // 0 ok, 1 = a bounded wait of a kernel in this file ran out
-#ifdef B200_Q8T_TRACE
-__device__ long long g_q8t_trace[16];
-#define Q8T_TRACE(k) do { if (blockIdx.x == 0 && blockIdx.y == 3 && blockIdx.z == B200_Q8T_TRACE && threadIdx.x == 0) g_q8t_trace[k] = clock64(); } while (0)
-#else
-#define Q8T_TRACE(k) do { } while (0)
-#endif
-
 namespace {
 
 constexpr int kThreads = 128;
@@ -1432,7 +1425,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-    Q8T_TRACE(0);
     const int bk = b / a.bq;
     const int R = a.Tq * a.gqa;  // <= 8; row rr -> (iq = rr / gqa, head hk*gqa + rr % gqa)
     const float ninf = -INFINITY;
@@ -1444,19 +1436,16 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
     // A CTA of this kernel shares its SM with three others in their key loops, where a lone thread gets an issue slot
     // every few tens of clocks: the set-up below is spread over lanes so that its chain of dependent instructions is
     // short - lane i initialises barrier i, lanes 2s and 2s+1 request the K and the V bytes of stage s.
-    Q8T_TRACE(14);
     if (lane < NS) {
         mbar_init(smem_u32(&s_bar[warp][lane]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
-    Q8T_TRACE(15);
     // Launched with programmatic stream serialisation: everything above (kernel parameters, this CTA's own shared
     // memory) ran while the previous kernel of the stream drained; from here on that kernel has completed and flushed
     // (a no-op under an ordinary launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    Q8T_TRACE(1);
     const int len_b = clamp_len(a, b);
     const int tq_b = q_rows_of(a, b);
     // Q rows (tiny): the eight rows this kernel has, one 8-element chunk per thread; rows >= R are zero.  Requested together
@@ -1500,7 +1489,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
     };
     auto issue = [&](int tile) { issue_lanes(tile, 1); };
     issue_lanes(tile_lo, NS);
-    Q8T_TRACE(2);
     if (q_f32) q_val = f32x8_to_half(q_val, q_hi);
     if (tid < 8 * (HD / 8)) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (q_row * (HD / 8) + swz<HD>(q_row, q_ch)) * 16) = q_val;
     __syncthreads();
@@ -1540,7 +1528,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
         if (pair < 8 * NBLK && c4 == 0) s_qd[pair] = -1152.0f * sum;
         __syncthreads();
     }
-    Q8T_TRACE(3);
     float negc[NBLK][2];
 #pragma unroll
     for (int blk = 0; blk < NBLK; blk++)
@@ -1556,13 +1543,10 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
     const __half2 bias = __float2half2_rn(1152.0f);
     const float c = a.scale * kLog2e;
 
-    Q8T_TRACE(4);
     for (int tile = tile_lo; tile < tile_hi; tile++) {
         const int k0 = tile * KT;
         const int stage = (tile - tile_lo) % NS;
         if (!mbar_wait_bounded(smem_u32(&s_bar[warp][stage]), (uint32_t)((tile - tile_lo) / NS) & 1u)) break;
-        if (tile == tile_lo) Q8T_TRACE(5);
-        if (tile == tile_lo + 1) Q8T_TRACE(6);
         const uint8_t* rawK = sRaw + stage * 2 * RAW_BYTES + 16 * warp * RB;   // this warp's 16 keys
         const uint8_t* rawV = rawK + RAW_BYTES;
         const int rows_valid = len_b - (k0 + 16 * warp);   // keys at or beyond it hold stale bytes: their scale reads as 0
@@ -1686,7 +1670,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
         issue(tile + NS);
     }
 
-    Q8T_TRACE(7);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // ---- merge the four warps' (m, l, O) in shared memory (same slabs as the kernel above) ----
     constexpr int SLAB_STRIDE = HD + 4;
@@ -1705,7 +1688,6 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
         s_l[warp][2 * t] = lq[0], s_l[warp][2 * t + 1] = lq[1];
     }
     __syncthreads();  // the warps' (m, l) are visible, and all warps are done with the raw stages (the merge slabs alias them)
-    Q8T_TRACE(8);
     // Each warp parks its accumulators as they are (scaled to its OWN running maximum): a thread's accumulators of one
     // block are four consecutive dims (4g .. 4g+3) of rows 2t and 2t+1, one 16-byte store per (block, row), conflict-free
     // (quarter-warps cover eight different 16-byte slots of a 128-byte line); rows at or beyond R are never read.
@@ -1717,12 +1699,8 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
             *reinterpret_cast<float4*>(slab + (warp * 8 + 2 * t + j) * SLAB_STRIDE + 32 * blk + 4 * g) =
                 make_float4(o[blk][0][j], o[blk][0][2 + j], o[blk][1][j], o[blk][1][2 + j]);
     }
-    Q8T_TRACE(12);
     __syncthreads();
-    Q8T_TRACE(9);
-    Q8T_TRACE(13);
     decode_write_out<HD, NW, 8>(a, slab, s_m, s_l, sRaw + NS * 2 * RAW_BYTES, R, b, hk, split, tq_b, tid);
-    Q8T_TRACE(10);
 }
 
 // One warp per (batch, kv-head, row): log-sum-exp merge of the split partials.
@@ -2151,12 +2129,6 @@ size_t decode_split_ws_bytes(int B, int Hkv, int n_splits, int hd) {
 }
 
 bool decode_uses_cluster_merge(const FattnArgs& a) { return use_cluster_merge(a); }
-
-#ifdef B200_Q8T_TRACE
-extern "C" __attribute__((visibility("default"))) int b200_dbg_q8t_trace(long long* out) {
-    return (int)cudaMemcpyFromSymbol(out, g_q8t_trace, sizeof(long long) * 16);
-}
-#endif
 
 int mma_read_status(int* status) {
     int v = 0;

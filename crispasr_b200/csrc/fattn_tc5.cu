@@ -31,16 +31,6 @@ namespace b200 {
 
 __device__ int g_tc5_status = 0;  // 0 ok, 1 = a bounded wait ran out in some CTA
 
-#ifdef B200_TC5_TRACE
-__device__ long long g_tc5_trace[3][64][8];
-#ifndef B200_TC5_TRACE_Z
-#define B200_TC5_TRACE_Z 0
-#endif
-#define TC5_TRACE(role, j, k) do { if (blockIdx.x == 1 && blockIdx.y == 3 && blockIdx.z == B200_TC5_TRACE_Z && (j) < 64) g_tc5_trace[role][j][k] = clock64(); } while (0)
-#else
-#define TC5_TRACE(role, j, k) do { } while (0)
-#endif
-
 namespace {
 
 constexpr int kTile = 128;              // query rows per CTA and keys per step
@@ -606,7 +596,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     }
 
     // ---- set-up ----
-    if (tid == 0) TC5_TRACE(2, 60, 0);
     if (tid == 4 * 32) {
         for (int i = 0; i < NSTG; i++) {
             mbar_init(bar_k_full + 8 * i, 1);
@@ -658,7 +647,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        if (lane == 0) TC5_TRACE(2, 61, 0);
     }
     if (warp < 4 && !q_tma) {
         // Q tile -> shared memory (thread r writes row r)
@@ -669,14 +657,11 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         else if (a.q.type == B200_TYPE_F16 && a.q.vec16) load_q_rows_f16_coalesced<HD>(smem_gen, warp, lane, q0 + r < rows_total ? rowp : nullptr);
         else load_q_row<HD>(smem_gen, r, rowp, a.q.type, a.q.vec16 != 0, q0 + r < rows_total);
         fence_proxy_async();
-        if (tid == 0) TC5_TRACE(2, 61, 1);
     }
-    if (tid == 4 * 32) TC5_TRACE(2, 61, 2);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
-    if (tid == 0) TC5_TRACE(2, 60, 1);
     const uint32_t tmem_S = tmem_base;            // cols [0,128)
     const uint32_t tmem_P = SEP_P ? tmem_base + kTile + HD : tmem_base;  // f16x2: cols [192,256) (hd 64) or aliasing S [0,64)
     const uint32_t tmem_O = tmem_base + kTile;    // cols [128,128+HD)
@@ -728,7 +713,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 const int k0 = j * kTile;
                 ok = mbar_wait(bar_k_empty + 8 * slot, (use - 1) & 1, s_abort);
                 if (!ok) break;
-                TC5_TRACE(2, j, 0);
                 mbar_arrive_expect_tx(bar_k_full + 8 * slot, TILE_BYTES);
 #pragma unroll
                 for (int p = 0; p < PANELS; p++)
@@ -736,7 +720,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 issued_k = j + 1;
                 ok = mbar_wait(bar_v_empty + 8 * slot, (use - 1) & 1, s_abort);
                 if (!ok) break;
-                TC5_TRACE(2, j, 1);
                 mbar_arrive_expect_tx(bar_v_full + 8 * slot, TILE_BYTES);
 #pragma unroll
                 for (int p = 0; p < PANELS; p++)
@@ -775,14 +758,12 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             if (ok && q_tma) ok = mbar_wait(q_raw ? bar_q_conv : bar_q_full, 0, s_abort);
             ok = warp_all(ok);
             if (ok) {
-                TC5_TRACE(1, 0, 0);
                 tc_fence_after();
                 if (elect_one()) {
                     issue_s(0);
                     tc_commit(bar_k_empty);
                 }
                 __syncwarp();
-                TC5_TRACE(1, 0, 1);
             }
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int slot = j % NSTG, use = j / NSTG;
@@ -790,11 +771,9 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 const bool more = j + 1 < n_tiles;
                 ok = mbar_wait(bar_v_full + 8 * slot, use & 1, s_abort);
                 if (ok && more) ok = mbar_wait(bar_k_full + 8 * nslot, nuse & 1, s_abort);
-                TC5_TRACE(1, j, 2);
                 if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
                 ok = warp_all(ok);
                 if (!ok) break;
-                TC5_TRACE(1, j, 3);
                 tc_fence_after();
                 if (elect_one()) {
                     // with P in its own columns the next S goes first: the softmax threads wake after 4 MMAs, not 12
@@ -817,7 +796,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                     if (!more) tc_commit(bar_o_done);
                 }
                 __syncwarp();
-                TC5_TRACE(1, j, 4);
             }
             if (!ok) {
                 // make sure no MMA of this CTA is still running before TMEM is released (the commit comes from the lane that
@@ -849,7 +827,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         for (int j = 0; j < n_tiles; j++) {
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
-            if (tid == 0) TC5_TRACE(0, j, 0);
             tc_fence_after();
             const int n_valid = kend - j * kTile;  // columns >= n_valid of this row are masked
             const bool full_tile = __all_sync(0xffffffffu, n_valid >= kTile);
@@ -941,14 +918,11 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                     tmem_ld32(tmem_S + lane_base + hh * 64 + 32, sreg[1]);
                     if (SEP_P && hh == 1 && j > 0 && !pv_waited && !pv_probe) pv_probe = mbar_test(bar_pv_done, (j - 1) & 1);
                     tmem_wait_ld();
-                    if (tid == 0) TC5_TRACE(0, j, 3 + 2 * hh);
                     uint4 mv[8];
                     load_mask64(mv, mrow + (int64_t)(j * kTile + hh * 64) * 2, a.Lk - (j * kTile + hh * 64));
                     if (full_tile) softmax64_masked<false>(sreg, mv, preg[hh], c, m_use, 0, 0, mx, lsum);
                     else softmax64_masked<true>(sreg, mv, preg[hh], c, m_use, hh * 64, n_valid, mx, lsum);
-                    if (tid == 0) TC5_TRACE(0, j, 4 + 2 * hh);
                 }
-                if (tid == 0 && attempt == 1) TC5_TRACE(0, j, 7);
                 const float m_tile = HASMASK ? mx + m_use : mx * c_exp;   // (the masked form tracks the maximum of x = logit - m)
                 const bool grow = m_tile > m_ref + kRescaleThreshold;
                 if (!__any_sync(0xffffffffu, grow)) break;
@@ -982,17 +956,14 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 if (!ok) break;
                 tc_fence_after();
             }
-            if (tid == 0) TC5_TRACE(0, j, 1);
             tmem_st32(tmem_P + lane_base, preg[0]);
             tmem_st32(tmem_P + lane_base + 32, preg[1]);
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
-            if (tid == 0) TC5_TRACE(0, j, 2);
         }
         if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
-        if (tid == 0) TC5_TRACE(2, 60, 2);
         if (ok) {
             tc_fence_after();
             // dead rows are written as literal zeros (whatever the padding row of Q held never reaches dst), rows
@@ -1044,7 +1015,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     }
 
     // ---- teardown ----
-    if (tid == 0) TC5_TRACE(2, 60, 3);
     tc_fence_before();
     __syncthreads();
     if (warp == 5) {
@@ -1193,9 +1163,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
     }
     // launched with programmatic stream serialisation: nothing is read before the previous kernel has completed
-    if (tid == 0) TC5_TRACE(2, 60, 0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) TC5_TRACE(2, 60, 1);
 
     int len_b = a.Lk;
     if (a.kv_len) {
@@ -1276,13 +1244,11 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             }
         }
         fence_proxy_async();
-        if (tid == 0) TC5_TRACE(2, 60, 2);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
-    if (tid == 0) TC5_TRACE(2, 60, 3);
     const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + 128, tmem_X = tmem_base + 256;
 
     if (warp == 8) {
@@ -1358,18 +1324,15 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                          mbar_wait(bar_x_free, j & 1, s_abort);
                     ok = warp_all(ok);
                     if (!ok) break;
-                    TC5_TRACE(1, j, 0);
                     tc_fence_after();
                     if (elect_one()) issue_x(j + 2);
                     __syncwarp();
-                    TC5_TRACE(1, j, 1);
                 }
                 ok = mbar_wait(bar_v_full, j & 1, s_abort);
                 if (ok && more) ok = mbar_wait(bar_k_full, (j + 1) & 1, s_abort);
                 if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
                 ok = warp_all(ok);
                 if (!ok) break;
-                TC5_TRACE(1, j, 2);
                 tc_fence_after();
                 if (elect_one()) {
                     mma_ts(tmem_O, tmem_P, desc64(v_lo, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
@@ -1381,7 +1344,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                     else tc_commit(bar_o_done);
                 }
                 __syncwarp();
-                TC5_TRACE(1, j, 3);
             }
             if (!ok) {
                 if (elect_one()) tc_commit(bar_o_done);
@@ -1438,7 +1400,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             // ---- phase A: the 64 bias values of this half row, fp32 registers holding f16-rounded numbers ----
             ok = mbar_wait(bar_x_full, j & 1, s_abort);
             if (!ok) break;
-            if (tid == 0) TC5_TRACE(0, j, 0);
             tc_fence_after();
             uint32_t bias2[32];   // the 64 bias values as packed pairs
             auto bounce_chunk = [&](const uint32_t (&xr)[32], int k) {
@@ -1481,7 +1442,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 bounce_chunk(xa[2], 2);
                 read_quarter(1);
             }
-            if (tid == 0) TC5_TRACE(0, j, 1);
             float u[HASMASK ? 64 : 1];   // with an explicit mask: bias + mask, in fp32
             if constexpr (HASMASK) {
                 uint4 mv[8];
@@ -1496,7 +1456,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             // ---- phase B: P = exp2(S*scale*log2(e) + bias*log2(e) - m_ref) ----
             ok = mbar_wait(bar_s_full, j & 1, s_abort);
             if (!ok) break;
-            if (tid == 0) TC5_TRACE(0, j, 2);
             tc_fence_after();
             const int n_valid = len_b - j * kTile;
             const bool full_tile = n_valid >= kTile;   // uniform over the CTA: only the last tile is partial
@@ -1583,7 +1542,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
                 float l0, l1;
                 unpack2(add2(ls[0], ls[1]), l0, l1);
                 lsum = l0 + l1;
-                if (tid == 0) TC5_TRACE(0, j, 3);
                 const float other = exchange(lsum);
                 if (!ok || take_max || !__any_sync(0xffffffffu, fmaxf(lsum, other) > kRedoSumRelpos)) break;
                 take_max = true;
@@ -1595,10 +1553,8 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
-            if (tid == 0) TC5_TRACE(0, j, 4);
         }
         if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
-        if (tid == 0) TC5_TRACE(2, 60, 4);
         if (ok) {
             tc_fence_after();
             const float l_tot = l_run + exchange(l_run);   // a failed wait has set the abort flag: the host reports it
@@ -1622,7 +1578,6 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         }
     }
 
-    if (tid == 0) TC5_TRACE(2, 60, 5);
     tc_fence_before();
     __syncthreads();
     if (warp == 9) {
@@ -1903,12 +1858,6 @@ int launch_prefill_tc5(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t
     }
     return launch_t<128, 1>(a, st, errbuf, errlen);
 }
-
-#ifdef B200_TC5_TRACE
-extern "C" __attribute__((visibility("default"))) int b200_dbg_trace(long long* out) {
-    return (int)cudaMemcpyFromSymbol(out, g_tc5_trace, sizeof(long long) * 3 * 64 * 8);
-}
-#endif
 
 int tc5_read_status(int* status) {
     int v = 0;
