@@ -1948,9 +1948,13 @@ int launch_decode_q8reg(const FattnArgs& a, cudaStream_t st) {
     cudaError_t e;
     if (q8t_form(a)) {
         auto go = [&](auto kern, int nw, bool (&smem_set)[64]) {
-            const size_t main = q8t_smem(HD, nw);
+            // A cluster launch of more than two CTAs per SM asks for the receive area of at least four rows: at head_dim 128
+            // three CTAs fit an SM then, as the cost model counts.  With less a fourth fits, and clusters pile up on some SMs
+            // while others have room (384 CTAs, 8 streams x 8 KV heads of one row, 663 keys: 6.2 us per launch, 7.0 without).
+            const int R = a.Tq * a.gqa, rows = (long)a.n_splits * a.Hkv * a.B > 2 * 148 && R < 4 ? 4 : R;
+            const size_t main = q8t_smem(HD, nw), push = use_cluster_merge(a) ? cluster_push_bytes(HD, rows) : 0;
             e = set_smem_once(kern, main + cluster_push_bytes(HD, 8), smem_set);
-            if (e == cudaSuccess) launch_split(kern, grid, main + (use_cluster_merge(a) ? cluster_push_bytes(HD, a.Tq * a.gqa) : 0), st, a, 32 * nw);
+            if (e == cudaSuccess) launch_split(kern, grid, main + push, st, a, 32 * nw);
         };
         static bool set[2][64] = {};
         if (a.wide) go(fattn_decode_q8t_kernel<HD, 8>, 8, set[0]);
