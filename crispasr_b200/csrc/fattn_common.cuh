@@ -101,6 +101,26 @@ __device__ __forceinline__ T load_global(const T* p) {
     return r;
 }
 
+// Waits for the kernels before this one; the result is 0.  An address that it was added to is one that no load can be
+// formed from ahead of the wait.
+__device__ __forceinline__ uint32_t wait_for_predecessors() {
+    uint32_t zero;
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero) : : "memory");
+    return zero;
+}
+// Loads from such an address: coherent ones, which the compiler may move among the instructions of a loop (mask rows at head_dim
+// 64: volatile 1-2 % and plain expressions 5-8 % slower).
+__device__ __forceinline__ uint4 load_behind_wait(const uint4* p) {
+    uint4 x;
+    asm("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ uint16_t load_behind_wait(const uint16_t* p) {
+    uint16_t x;
+    asm("ld.global.u16 %0, [%1];" : "=h"(x) : "l"(p));
+    return x;
+}
+
 // Eight Q elements [c0, c0+8) of one row plus eight fp32 bias values, as packed f16: the sum is formed in fp32
 // and rounded once (an F32 add followed by the conversion to F16). F16 and F32 rows only; c0 + 8 <= head_dim.
 __device__ __forceinline__ uint4 load8_plus_bias_as_half(const uint8_t* rowp, int type, int c0, bool vec16,

@@ -348,12 +348,12 @@ __device__ __forceinline__ void load_mask64(uint4 (&mv)[8], const uint8_t* mptr,
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         if (q * 8 + 8 <= avail && ((reinterpret_cast<uintptr_t>(mptr) & 15) == 0)) {
-            mv[q] = load_global(reinterpret_cast<const uint4*>(mptr + q * 16));
+            mv[q] = load_behind_wait(reinterpret_cast<const uint4*>(mptr + q * 16));
         } else {   // the end of the row, or a row that does not start on a 16-byte boundary (mask rows hold exactly Lk values)
             uint16_t hv[8];
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                hv[i] = (q * 8 + i < avail) ? load_global(reinterpret_cast<const uint16_t*>(mptr + (q * 8 + i) * 2)) : (uint16_t)0;
+                hv[i] = (q * 8 + i < avail) ? load_behind_wait(reinterpret_cast<const uint16_t*>(mptr + (q * 8 + i) * 2)) : (uint16_t)0;
             mv[q] = make_uint4(hv[0] | ((uint32_t)hv[1] << 16), hv[2] | ((uint32_t)hv[3] << 16), hv[4] | ((uint32_t)hv[5] << 16),
                                hv[6] | ((uint32_t)hv[7] << 16));
         }
@@ -557,7 +557,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // launched with programmatic stream serialisation: nothing is read or written before the previous kernel of the
     // stream (e.g. the K/V conversion pass) has completed and flushed
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t behind_wait = wait_for_predecessors();
     // Causal launches hand out the query tiles with the most KV tiles first (longest-processing-time order over
     // the whole grid: the tile index becomes the slowest-varying coordinate, reversed), which shortens the tail of
     // short prefills; otherwise consecutive CTAs are the query tiles of one head, which share K/V in L2.
@@ -820,7 +820,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         float m_ref = -INFINITY, l_run = 0.0f;
         bool ok = true;
         // explicit mask row of this query ([Lk, Tq, 1|H, 1|B] F16); rows past Tq reuse row 0
-        const uint8_t* mrow = HASMASK ? a.mask.p + (int64_t)(iq < a.Tq ? iq : 0) * a.mask.nb1 +
+        const uint8_t* mrow = HASMASK ? a.mask.p + behind_wait + (int64_t)(iq < a.Tq ? iq : 0) * a.mask.nb1 +
                                             (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3
                                       : nullptr;
         const float c_exp = HASMASK ? 1.0f : c;   // with a mask the scores are moved to the log2 domain by apply_mask64
@@ -1163,7 +1163,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
     }
     // launched with programmatic stream serialisation: nothing is read before the previous kernel has completed
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t behind_wait = wait_for_predecessors();
 
     int len_b = a.Lk;
     if (a.kv_len) {
@@ -1377,7 +1377,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         // Explicit F16 mask added on top of the bias (bucket padding of src/canary_ctc.cpp:370-382, the local-attention
         // window of src/core/fastconformer.h:887-895): this thread's row of [Lk, Tq, 1|H, 1|B];
         // rows past Tq (the padding rows of the last query tile) read row 0.
-        const uint8_t* mrow = HASMASK ? a.mask.p + (int64_t)(iq < a.Tq ? iq : 0) * a.mask.nb1 +
+        const uint8_t* mrow = HASMASK ? a.mask.p + behind_wait + (int64_t)(iq < a.Tq ? iq : 0) * a.mask.nb1 +
                                             (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3
                                       : nullptr;
         // Publish a value, meet the partner warp at the pair barrier (bounded wait), read the partner's value.

@@ -424,7 +424,7 @@ def test_kernels_that_overlap_their_predecessor_load_coherently():
     seen = 0
     for f in sorted(os.listdir(csrc)):
         text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
-        if "griddepcontrol.wait" in text or f == "fattn_common.cuh":
+        if "griddepcontrol.wait" in text or "wait_for_predecessors()" in text:
             seen += 1
             assert not re.search(r"__ldg\s*\(|ld\.global\.nc|__restrict__", text), f
     assert seen >= 5
