@@ -179,11 +179,10 @@ def test_cfg3_large_v3_encoder_segments(b200, orc, kernel):
         assert b200.lib().b200_device_status() == 0
 
 
-@pytest.mark.parametrize("env", ["B200_PREFILL_EARLY=1", "B200_PREFILL_EARLY=2", "B200_PREFILL_SPLIT=1", "B200_PREFILL_PAIR=1"])
-def test_opt_in_prefill_variants(env):
-    """The head_dim 64 prefill variants that are kept for A/B runs (early score issue, split rows, paired tiles) are
-    selected per process by an environment variable: each runs an encoder-shaped and a causal case against the oracle
-    in a child process."""
+@pytest.mark.parametrize("env", ["B200_HOST_CHUNKS=1", "B200_HOST_CHUNKS=16", "B200_DECODE_CLUSTER_MERGE=0", "B200_DECODE_CTAS_PER_SM=1"])
+def test_switches_read_once_per_process(env):
+    """Each of the library's environment variables is read once per process: decode steps that split their keys and
+    host-buffer calls run against the oracle in a child process that has it set."""
     import subprocess
     import sys
 
@@ -192,7 +191,7 @@ def test_opt_in_prefill_variants(env):
     r = subprocess.run([sys.executable, os.path.join(root, "tests", "variant_case.py")], env={**os.environ, name: value},
                        capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
-    assert r.stdout.count("OK") == 2, r.stdout
+    assert r.stdout.count("OK") == 4, r.stdout
 
 
 def test_voxtral_audio_encoder_f32_kv(b200, orc, kernel):
