@@ -1145,7 +1145,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
     uint8_t* misc = smem_gen + 6 * TILE_BYTES + 2 * kTile * kBncStride + 136;
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
     volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
-    volatile float* s_xchg = reinterpret_cast<volatile float*>(misc + 8);   // [2][128]: row maximum exchange of a thread pair
+    volatile float* s_xchg = reinterpret_cast<volatile float*>(misc + 8);   // [2][128]: exchange of row sums between the two threads of a row
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int q0 = blockIdx.x * kTile, h = blockIdx.y, b = blockIdx.z;
@@ -1354,9 +1354,9 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUten
         }
     } else {
         // ================= softmax / bias / epilogue: thread (r, ch) owns columns [64ch, 64ch+64) of row r ========
-        // Eight softmax warps: warps w and w+4 see the same 32 TMEM lanes. The two threads of a row agree on the
-        // running maximum through shared memory and a 64-thread named barrier once per tile; each keeps a partial
-        // row sum and owns half of the O columns.
+        // Eight softmax warps: warps w and w+4 see the same 32 TMEM lanes. The two threads of a row exchange
+        // their half-row sums through shared memory and an mbarrier of 64 arrivals once per tile (their maxima only where
+        // the reference is taken anew); each keeps a partial row sum and owns half of the O columns.
         const int r = tid & 127, ch = tid >> 7;
         const int iq = q0 + r;
         const uint32_t my_pair_bar = bar_pair + 8 * (warp & 3);

@@ -16,8 +16,9 @@
 // P[j-1].V[j-1] are complete), issues P[j].V[j] and S[j+1], then refills the K slot of S[j] and the V slot of step j - 1:
 // no "slot empty" barriers exist.
 //
-// 64 windows of the large encoder (T = 1500): 1277 -> 917 us (577 -> 804 TFLOP/s, 0.56 of the sustained GEMM rate), at the
-// 1000 W limit (1.65 GHz; 1.9 GHz before): 1.2 k clk per 128 x 128 scores.
+// 64 windows of the large encoder (T = 1500): 1277 -> 917 us in a burst (577 -> 804 TFLOP/s, 0.56 of the sustained GEMM rate,
+// 1.2 k clk per 128 x 128 scores); in a long run 1065-1080 us at the 1000 W limit, whose 1.59-1.65 GHz (1.9 GHz before) make
+// that 1.4 k clk.
 constexpr int kH64Keys = 64;
 constexpr int kH64Threads = 160;
 constexpr int kH64KvBytes = kH64Keys * 128;   // one K or V tile

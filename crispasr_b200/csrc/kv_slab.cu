@@ -28,8 +28,8 @@ namespace {
 // the launch when one does; what the first form (one thread per pair or element, three 64-bit divisions each, 16-bit
 // stores, a launch each for K and V) spent its time on was index arithmetic: 407 rows x 64 heads of head_dim 128 into
 // Q8_0 66 us, this one 9.7 us, against 5.2 us of memory time (F16 7.7 us; 1500 rows 28 and 22 us: 4.4 and 6.6 TB/s; what
-// Q8_0 adds is the arithmetic of its blocks).  One row per head: two launches of 2.8 us -> one, hidden under the set-up
-// of the attention behind it.
+// Q8_0 adds is the arithmetic of its blocks).  One row per head: two launches of 2.8 us -> one of 2.0, on which the
+// attention behind it waits (its set-up runs meanwhile).
 struct AppendArgs {
     const uint8_t* src[2];                   // K, V
     int64_t snb1[2], snb2[2], snb3[2];
