@@ -223,7 +223,9 @@ B200_API int b200_fattn_launch_alloc(const b200_tensor* q, const b200_tensor* k,
  * heads of an entry, are independent, so the call is pipelined over chunks of them (their number follows from the
  * bytes of the result; environment variable B200_HOST_CHUNKS = 1..16 sets it): the upload of one chunk overlaps the
  * kernel and the write-back of the previous one.  Pinned host buffers are needed for that overlap to happen; into a
- * pinned `dst` the kernels write the result themselves, anything else is staged and copied back.
+ * pinned `dst` (inside one allocation) the kernels write the result themselves, anything else is staged and copied back.
+ * `dst` may overlap an operand: entry by entry (an update in place) the chunks stay, in any other way the call runs as
+ * one chunk whose result is copied back behind all uploads.
  */
 B200_API int b200_fattn_forward_host(const b200_tensor* q, const b200_tensor* k, const b200_tensor* v,
                                      const b200_tensor* mask, const b200_tensor* dst,
