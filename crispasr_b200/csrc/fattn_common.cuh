@@ -108,6 +108,9 @@ __device__ __forceinline__ uint32_t wait_for_predecessors() {
     asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero) : : "memory");
     return zero;
 }
+// The next kernel of the stream may become resident from here on (if it was launched with programmatic serialisation; it waits
+// for this grid's completion before it touches memory).
+__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Loads from such an address: coherent ones, which the compiler may move among the instructions of a loop (mask rows at head_dim
 // 64: volatile 1-2 % and plain expressions 5-8 % slower).
 __device__ __forceinline__ uint4 load_behind_wait(const uint4* p) {

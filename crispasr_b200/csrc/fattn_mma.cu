@@ -887,6 +887,12 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         if (rr < kDecRows) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(sQ) + (rr * (HD / 8) + swz<HD>(rr, ch)) * 16) = q_val[i];
     }
     __syncthreads();
+    // One split per unit: a launch of so many units that nothing needs sharing.  The next kernel of the stream (the cache append of
+    // the next layer) then becomes resident under this one's key loop instead of behind it: 32 streams of head_dim 128, 30
+    // layers 485 -> 474 us, 60 streams of 200 keys, 20 layers 277 -> 262.  Split units gain nothing by it (pairs: 16 segments
+    // under a dense mask, 8 layers 176 -> 181 us): what waits there takes the room of clusters that are still to start.
+    const bool early = a.n_splits == 1;
+    if (early) let_dependents_launch();
     uint32_t qf[HD / 16][4];
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ks++) ldsm_x4(qf[ks], tile_addr<HD>(sQ, lane & 15, ks * 2 + (lane >> 4)));
@@ -1055,8 +1061,8 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
     }
     if (MODE == kDecAsyncF16) cp_async_wait<0>();
 
-    // the merge kernel (if any) may start launching: it waits for this grid's completion before reading anything
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // split units: the merge kernel (if any) may start launching; it waits for this grid's completion before reading anything
+    if (!early) let_dependents_launch();
     // ---- merge the four warps' (m, l, O) in shared memory ----
     constexpr int SLAB_STRIDE = HD + 4;
     float* slab = reinterpret_cast<float*>(smem_raw);   // [4][16][SLAB_STRIDE]
