@@ -374,6 +374,7 @@ int do_launch_untraced(Plan& plan, void* workspace, size_t ws_bytes, cudaStream_
             ce = launch_kv_to_f16(a.r, rbuf, a.hd, 2 * a.Tq - 1, a.H, a.r_ne3, st);
             c = with_f16_r(c, rbuf);
         }
+        c.behind_cast = 1;
         if (ce != 0) return cuda_fail((cudaError_t)ce, "operand conversion launch");
         const int rc = launch_prefill_tc5(c, st, g_cuda_err, sizeof(g_cuda_err));
         if (rc != B200_OK) return rc;
