@@ -420,6 +420,13 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A value that the previous kernel of the stream may still write, read past L1, which would keep the old one.
+__device__ __forceinline__ int32_t peek(const int32_t* p) {
+    int32_t v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // The 16-byte pieces of a 64-row F16 tile that one thread copies: column chunk tid % (HD/8) of every kRows-th row from
 // tid / (HD/8) on.  The row step is a multiple of 8, so the place in the swizzled tile advances by a constant and the
 // source by one addition.  With a row, an index and a 64-bit product worked out per piece, issuing the first three tiles took
@@ -508,11 +515,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 // (32 segments +10 %).  Over a Q8_0 cache, whose copies a CTA starts with a few instructions, it measured nothing.
 constexpr int kPrefetchTiles = 2;
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-__device__ __forceinline__ int32_t peek(const int32_t* p) {
-    int32_t v;
-    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
 // x / n_splits: the cluster forms (at most eight splits) without a division.
 __device__ __forceinline__ int div_splits(const FattnArgs& a, int x) {
     return a.n_splits == 1 ? x : (a.n_splits <= 8 && x < 4096 ? (x * a.splits_mul) >> 16 : x / a.n_splits);
@@ -522,15 +524,6 @@ __device__ __forceinline__ uint4 f32x8_to_half(const uint4& a, const uint4& b) {
     return make_uint4(pack_half2(__uint_as_float(a.x), __uint_as_float(a.y)), pack_half2(__uint_as_float(a.z), __uint_as_float(a.w)),
                       pack_half2(__uint_as_float(b.x), __uint_as_float(b.y)), pack_half2(__uint_as_float(b.z), __uint_as_float(b.w)));
 }
-// Logical keys [lo, hi) of this CTA's first tiles, as far as they can be told before the wait.
-__device__ __forceinline__ void peek_range(const FattnArgs& a, int b, int split, int& lo, int& hi) {
-    const int cap = a.kv_index ? a.kv_index_stride : a.Lk;
-    const int len = a.kv_len ? min(max(peek(a.kv_len + b), 0), cap) : cap;
-    const int n_tiles = (len + kDecBN - 1) / kDecBN, tps = div_splits(a, n_tiles + a.n_splits - 1);
-    lo = split * tps * kDecBN;
-    hi = min(len, lo + min(tps, kPrefetchTiles) * kDecBN);
-}
-
 // Raw bytes of this warp's 16 Q8_0 rows [row0 + 16*warp, +16) of a 64-row K tile and V tile: two contiguous,
 // 16-byte aligned ranges of at most 16 * (HD/32*34) bytes, one bulk copy each, issued by lane 0.  Only the bytes of
 // rows below row_hi are requested (rounded up to 16: the same footprint as 16-byte chunk copies; the rest of the
@@ -778,11 +771,34 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         }
         __syncwarp();
     }
-    // (rows of head_dim 128 split over a cluster, ahead of which a cache append runs, measured 0.5 us slower with it)
-    if (MODE == kDecAsyncF16 && (HD <= 64 || a.n_splits == 1)) {
+    // The length that says which keys the first tiles are is read ahead of the wait, for the prefetch; behind the wait it nearly always is
+    // what it was, so the first copies are issued by it while it is read again, and once more where it turns out to have changed.
+    // (3 streams of 300 keys, head_dim 128, 20 layers: 113 -> 108 us; 8 streams of 900 185 -> 182.  Of index lists, too, it costs more
+    // than it gives: every thread reads its entries of four tiles twice.)
+    const TilePieces<HD> pieces(tid);
+    const int n_logical = a.kv_index ? a.kv_index_stride : a.Lk;   // logical keys: a mask row holds one value per logical key
+    const bool ahead = MODE == kDecAsyncF16 && !IDX && !a.causal && !a.q_len;
+    int len_ahead = n_logical, lo_ahead = 0, hi_ahead = 0;
+    if (MODE == kDecAsyncF16) {
+        if (a.kv_len) len_ahead = min(max(peek(a.kv_len + b), 0), n_logical);
+        const int n = (len_ahead + kDecBN - 1) / kDecBN, tps = div_splits(a, n + a.n_splits - 1);
+        lo_ahead = split * tps, hi_ahead = min(n, lo_ahead + tps);
+    }
+    // staged mask: the row of the mask this thread copies pieces of (the head and batch broadcasts are remainders by
+    // run-time values: computed once, not per tile)
+    const uint8_t* mask_row = nullptr;
+    if (stage_mask && tid < R * 8) {
+        int iq, hq;
+        row_to_query(a, hk, tid >> 3, iq, hq);
+        mask_row = a.mask.p + (int64_t)iq * a.mask.nb1 + (int64_t)(hq % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3;
+    }
+    // (Rows of head_dim 128 split over a cluster, ahead of which a cache append runs, measured 0.5 us slower with it.  CTAs beyond those
+    // that start together have nothing to wait for, and would ask for every line twice: 60 streams of 200 keys, 20 layers, 269 ->
+    // 260 us, 40 of 300, 10 layers, 134 -> 128.)
+    const bool first_wave = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < 2 * 148;
+    if (MODE == kDecAsyncF16 && (HD <= 64 || a.n_splits == 1) && first_wave) {
         constexpr int LPR = HD * 2 / 128 > 0 ? HD * 2 / 128 : 1;   // 128-byte lines per row
-        int lo, hi;
-        peek_range(a, b, split, lo, hi);
+        const int lo = lo_ahead * kDecBN, hi = min(len_ahead, min(hi_ahead, lo_ahead + kPrefetchTiles) * kDecBN);
         for (int i = tid; i < (hi - lo) * LPR; i += kThreads) {
             const int key = lo + i / LPR, row = IDX ? min(max(peek(index + key), 0), a.Lk - 1) : key;
             prefetch_l2(kbase + (int64_t)row * a.k.nb1 + (i % LPR) * 128);
@@ -793,23 +809,8 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
     // memory) ran while the previous kernel of the stream drained; from here on that kernel has completed and flushed
     // (a no-op under an ordinary launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int len_b = clamp_len(a, b);
+    const int len_raw = a.kv_len ? load_global(a.kv_len + b) : n_logical;
     const int tq_b = q_rows_of(a, b);   // query rows at or beyond it give zeros
-    int kmax = tq_b > 0 ? len_b : 0;    // an entry without live rows reads no keys
-    const int n_past = n_past_of(a, len_b, tq_b);
-    if (a.causal) kmax = min(kmax, n_past + tq_b);
-    const int n_tiles = (kmax + kDecBN - 1) / kDecBN;
-    const int tps = div_splits(a, n_tiles + a.n_splits - 1);
-    const int tile_lo = split * tps, tile_hi = min(n_tiles, tile_lo + tps);
-    // staged mask: the row of the mask this thread copies pieces of (the head and batch broadcasts are remainders by
-    // run-time values: computed once, not per tile)
-    const int n_logical = a.kv_index ? a.kv_index_stride : a.Lk;   // a mask row holds one value per logical key
-    const uint8_t* mask_row = nullptr;
-    if (stage_mask && tid < R * 8) {
-        int iq, hq;
-        row_to_query(a, hk, tid >> 3, iq, hq);
-        mask_row = a.mask.p + (int64_t)iq * a.mask.nb1 + (int64_t)(hq % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3;
-    }
     // Q rows (tiny): requested ahead of the copies, stored behind them; rows >= R are zero
     constexpr int Q_PER = (kDecRows * (HD / 8) + kThreads - 1) / kThreads;
     // (raw 16-byte pieces where the rows allow it: the conversion would wait for them ahead of the copies)
@@ -831,16 +832,11 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
             }
         }
     }
-    const TilePieces<HD> pieces(tid);
     const uint8_t *kcol = kbase + tid % (HD / 8) * 16, *vcol = vbase + tid % (HD / 8) * 16;
     // gathered keys: the cache rows of the first tiles, requested together, then of the next tile to be issued
     int first_rows[IDX ? NS - 1 : 1][TilePieces<HD>::N], pre_rows[TilePieces<HD>::N];
-    if (IDX) {
-#pragma unroll
-        for (int s0 = 0; s0 < NS - 1; s0++) pieces.load_index(first_rows[s0], index, (tile_lo + s0) * kDecBN, min(len_b, tile_hi * kDecBN));
-        pieces.load_index(pre_rows, index, (tile_lo + NS - 1) * kDecBN, min(len_b, tile_hi * kDecBN));
-    }
-    auto issue = [&](int tile, const int (&rows)[TilePieces<HD>::N]) {   // rows: the tile's cache rows, if gathered
+    // rows: the tile's cache rows, if gathered; [tile_lo, tile_hi) this CTA's tiles of `len_b` keys
+    auto issue_of = [&](int tile, const int (&rows)[TilePieces<HD>::N], int tile_lo, int tile_hi, int len_b) {
         if (MODE == kDecAsyncQ8) {
             if (tile < tile_hi && lane == 0) {
                 const int stage = (tile - tile_lo) % NS;
@@ -871,11 +867,29 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         }
         cp_async_commit();
     };
+    if (ahead) {
+#pragma unroll 1
+        for (int s0 = 0; s0 < NS - 1; s0++) issue_of(lo_ahead + s0, pre_rows, lo_ahead, hi_ahead, len_ahead);
+    }
+    const int len_b = min(max(len_raw, 0), n_logical);
+    int kmax = tq_b > 0 ? len_b : 0;    // an entry without live rows reads no keys
+    const int n_past = n_past_of(a, len_b, tq_b);
+    if (a.causal) kmax = min(kmax, n_past + tq_b);
+    const int n_tiles = (kmax + kDecBN - 1) / kDecBN;
+    const int tps = div_splits(a, n_tiles + a.n_splits - 1);
+    const int tile_lo = split * tps, tile_hi = min(n_tiles, tile_lo + tps);
+    auto issue = [&](int tile, const int (&rows)[TilePieces<HD>::N]) { issue_of(tile, rows, tile_lo, tile_hi, len_b); };
+    if (IDX) {
+#pragma unroll
+        for (int s0 = 0; s0 < NS - 1; s0++) pieces.load_index(first_rows[s0], index, (tile_lo + s0) * kDecBN, min(len_b, tile_hi * kDecBN));
+        pieces.load_index(pre_rows, index, (tile_lo + NS - 1) * kDecBN, min(len_b, tile_hi * kDecBN));
+    }
     if (MODE != kDecSync) {
         if constexpr (IDX) {
 #pragma unroll
             for (int s0 = 0; s0 < NS - 1; s0++) issue(tile_lo + s0, first_rows[s0]);
-        } else {
+        } else if (!ahead || len_b != len_ahead) {
+            if (MODE == kDecAsyncF16) cp_async_wait<0>();   // each thread writes the same places of the ring again: no barrier is needed
 #pragma unroll 1
             for (int s0 = 0; s0 < NS - 1; s0++) issue(tile_lo + s0, pre_rows);
         }

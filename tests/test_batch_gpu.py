@@ -305,3 +305,48 @@ def test_slot_table_drives_a_decode_batch(b200, orc):
     assert step(True) == 4
     L.b200_batch_destroy(h)
     kvc.close()
+
+
+class _Memory:
+    """Device memory owned by `keep`, as int32 words for torch."""
+
+    def __init__(self, keep, ptr, n):
+        self.keep = keep
+        self.__cuda_array_interface__ = dict(data=(ptr, False), shape=(n,), typestr="<i4", strides=None, version=3)
+
+
+@pytest.mark.parametrize("kv,hd,gqa,B", [("f16", 128, 4, 2), ("f16", 128, 4, 40), ("f16", 64, 1, 3), ("q8_0", 128, 4, 2), ("q8_0", 64, 2, 24)])
+def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B):
+    """The decode kernels read kv_len ahead of their dependency wait and again behind it.  Here the table lies in a cache
+    row that an append of the same stream writes directly before the launch, behind a long kernel: what is read ahead is the
+    old length, longer, shorter, of another tile count or zero."""
+    rng = np.random.default_rng(hd + B)
+    Hkv, Lk = 8, 448
+    H = Hkv * gqa
+    q = randn_f16(rng, (B, H, 1, hd))
+    kf, vf = (rng.standard_normal((B, Hkv, Lk, hd)).astype(np.float32) for _ in "kv")
+    k, v = (orc.quantize_q8_0(kf), orc.quantize_q8_0(vf)) if kv == "q8_0" else (kf.astype(np.float16), vf.astype(np.float16))
+    kw = dict(scale=hd ** -0.5, **(dict(kv_type=abi.Q8_0) if kv == "q8_0" else {}))
+    dq, dk, dv = (torch.from_numpy(x).cuda() for x in (q, k, v))
+    table = b200.KvCache(abi.F16, 128, 1, 1, 32, 1)
+    words = torch.as_tensor(_Memory(table, table.view(0, 1)[0].data, 64), device="cuda")
+    slow = torch.randn((8, 20, 1500, 64), device="cuda").half()
+    lens = [[(37 * (i + 1) * (t + 3)) % (Lk + 1) for i in range(B)] for t in range(6)] + [[Lk] * B, [0] * B, [64] * B, [65] * B, [1] * B]
+    rows = []
+    for ls in lens:   # 32-bit words as pairs of f16, as the float32 values that an append turns into those bits
+        bits = np.zeros(128, np.uint16)
+        bits[:2 * B:2] = ls
+        rows.append(torch.from_numpy(bits.view(np.float16).astype(np.float32).reshape(1, 1, 1, 128)).cuda())
+    torch.cuda.synchronize()
+    got = []
+    for row in rows:
+        b200.flash_attn_ext(slow, slow, slow, scale=0.125)
+        table.append(0, row, row, pos0=0)
+        got.append(b200.flash_attn_ext(dq, dk, dv, kv_len=words[:B], **kw))
+    torch.cuda.synchronize()
+    for ls, out in zip(lens, got):
+        ref = np.zeros((B, 1, H, hd), np.float32)
+        for i, n in enumerate(ls):
+            if n:
+                ref[i] = orc.flash_attn_ext(q[i:i + 1], k[i:i + 1, :, :n], v[i:i + 1, :, :n], **kw)[0]
+        assert_close(out.cpu().numpy(), ref, "lengths %s" % ls[:4])
