@@ -73,12 +73,20 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
     // launched with programmatic stream serialisation: the attention of this layer may set itself up meanwhile, and
     // nothing is touched before the previous kernel of the stream has completed
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = a.hd / 8, rpw = 32 / lpr;   // lanes per row (4, 8, 12, 16); rows per warp instruction
     const int sub = lane / lpr, c = (lane - sub * lpr) * 8;
     const int which = blockIdx.y, sh = blockIdx.x / a.chunks, chunk = blockIdx.x - sh * a.chunks, s = sh / a.n_kv, h = sh - s * a.n_kv;
     const int n_new = a.n_new[which];
+    // One token per stream: its rows are brought into L2 while the previous kernel still runs (a prefetch returns nothing, and L2 is where
+    // that kernel's writes arrive too).  Rows that are not there yet cost a trip to memory on the chain of a decode step otherwise: 32
+    // streams of an F16 cache, 30 layers, 470 -> 458 us; 20 streams, 20 layers, 157 -> 148.
+    if (U == 1) {
+        const int row = (chunk * (blockDim.x >> 5) + warp) * rpw + sub;
+        if (sub < rpw && row < n_new && (c & 31) == 0)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.src[which] + (int64_t)h * a.snb2[which] + (int64_t)s * a.snb3[which] + (int64_t)row * a.snb1[which] + c * 4));
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int p0 = a.pos ? a.pos[s] : a.pos0;
     const int row_lo = max(0, -p0), row_hi = sub < rpw ? min(n_new, a.ctx_rows - p0) : 0;   // out-of-range rows are dropped, never written
     const uint8_t* src = a.src[which] + (int64_t)h * a.snb2[which] + (int64_t)s * a.snb3[which] + (int64_t)c * 4;
