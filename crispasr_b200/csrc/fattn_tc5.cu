@@ -1681,7 +1681,7 @@ bool encode_r_map(CUtensorMap* m, const FattnArgs& a) {
 }
 
 // Launch that may begin while the previous kernel of the stream drains, if that kernel allows it
-// (griddepcontrol.launch_dependents: the K/V conversion pre-pass does).  The kernels wait for the predecessor's
+// (griddepcontrol.launch_dependents: the conversion pre-pass, the cache append and others do).  The kernels wait for the predecessor's
 // completion (griddepcontrol.wait) before they read anything it may have written.
 // `cluster` > 1: so many CTAs along x form a thread-block cluster.
 template <typename Kern, typename... Args>
