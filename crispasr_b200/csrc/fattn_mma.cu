@@ -914,9 +914,12 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
     __syncthreads();
     // One split per unit: a launch of so many units that nothing needs sharing.  The next kernel of the stream (the cache append of
     // the next layer) then becomes resident under this one's key loop instead of behind it: 32 streams of head_dim 128, 30
-    // layers 485 -> 474 us, 60 streams of 200 keys, 20 layers 277 -> 262.  Split units gain nothing by it (pairs: 16 segments
-    // under a dense mask, 8 layers 176 -> 181 us): what waits there takes the room of clusters that are still to start.
-    const bool early = a.n_splits == 1;
+    // layers 485 -> 474 us, 60 streams of 200 keys, 20 layers 277 -> 262.  What waits there takes places next to CTAs that still run, so
+    // the next launch starts unevenly spread over the SMs.  Short units of few rows do not feel that; others lose by it (us per
+    // launch, late / early): 9 to 16 rows, head_dim 128, 24 streams of 600 keys 13.9 / 15.0, 40 with a causal bound 27.8 / 28.5
+    // (37, which fill the places, 18.3 / 17.9); head_dim 32, 50 streams of 600 keys 7.4 / 8.1 (40: 6.9 / 6.5); over a Q8_0 cache of
+    // head_dim 32 13.2 / 14.5.  Split units gain nothing (pairs: 16 segments under a dense mask, 8 layers 176 / 181): it takes the room of clusters that are still to start.
+    const bool early = MODE != kDecAsyncQ8 && HD > 32 && a.n_splits == 1 && R <= 8;
     if (early) let_dependents_launch();
     uint32_t qf[HD / 16][4];
 #pragma unroll
