@@ -42,6 +42,7 @@ struct FattnArgs {
     // split-KV
     int32_t n_splits;
     int32_t splits_mul;  // (x * splits_mul) >> 16 == x / n_splits for x < 4096 and up to eight splits
+    int32_t prefetch_q;   // split-KV: the CTAs bring their query rows into L2 ahead of the dependency wait
     int32_t behind_cast;  // the kernel before this one is the call's own conversion of K and V (or R)
     int32_t wide;  // split-KV over a Q8_0 cache: eight warps per CTA instead of four
     float* ws_o;   // [B][Hkv][n_splits][16][hd]

@@ -627,8 +627,8 @@ __device__ __forceinline__ void row_to_query(const FattnArgs& a, int hk, int rr,
     else iq = rr / a.gqa, hq = hk * a.gqa + rr % a.gqa;
 }
 
-// The query rows of a decode CTA into L2 ahead of the wait, a thread per row (F16 caches: one segment of the large decoder 296 -> 286 us
-// per step of 64 launches; over a Q8_0 cache, where the append and not the queries are on the chain, 243 -> 245).
+// The query rows of a decode CTA into L2 ahead of the wait, a thread per row (one segment of the large decoder 296 -> 286 us per step
+// of 64 launches; see launch_split for which launches gain by it).
 __device__ __forceinline__ void prefetch_queries(const FattnArgs& a, int b, int hk, int R, int tid) {
     if (tid >= R) return;
     int iq, hq;
@@ -815,7 +815,7 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
             prefetch_l2(vbase + (int64_t)row * a.v.nb1 + (i % LPR) * 128);
         }
     }
-    if (first_wave) prefetch_queries(a, b, hk, R, tid);
+    if (MODE != kDecAsyncQ8 && first_wave && a.prefetch_q) prefetch_queries(a, b, hk, R, tid);
     // Launched with programmatic stream serialisation: everything above (kernel parameters, this CTA's own shared
     // memory) ran while the previous kernel of the stream drained; from here on that kernel has completed and flushed
     // (a no-op under an ordinary launch).
@@ -1848,6 +1848,12 @@ void launch_split(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const Fatt
     // decode step (+0.8 % on the 64-segment decode launches, +1 % at 32 streams).
     FattnArgs ac = a;
     ac.splits_mul = (65536 + a.n_splits - 1) / a.n_splits;
+    // Not where split units come in more CTAs than start together: the wait is over for most of them, and what the first ones ask for
+    // competes with keys (us per launch with / without: Whisper cross-attention, 12 and 14 windows of 20 heads, three splits,
+    // 21.9 / 21.6 and 24.3 / 23.9, 36 of 8 heads 24.8 / 24.4).  Unsplit units and gathered keys, whose copies wait for their list, keep it
+    // (44 streams of 60 keys 5.95 / 6.07, 80 index lists of 20 heads 22.8 / 23.2).  The kernels over a Q8_0 cache go without: the append
+    // and not the queries is on their chain (20 layers 243 us without, 245 with; head_dim 32, 4 streams, 6.3 and 6.6 per launch).
+    ac.prefetch_q = a.n_splits == 1 || a.kv_index || (long)grid.x * grid.y * grid.z <= 2 * 148;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
