@@ -784,14 +784,17 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
     // The length that says which keys the first tiles are is read ahead of the wait, for the prefetch; behind the wait it nearly always is
     // what it was, so the first copies are issued by it while it is read again, and once more where it turns out to have changed.
     // (3 streams of 300 keys, head_dim 128, 20 layers: 113 -> 108 us; 8 streams of 900 185 -> 182.  Of index lists, too, it costs more
-    // than it gives: every thread reads its entries of four tiles twice.)
+    // than it gives: every thread reads its entries of four tiles twice.)  The general form may have a causal bound, which depends on
+    // no more than the length then.  (4 streams x 4 tokens, 600 keys, 7.4 us; left out of it, while it carried the code, 7.8.)
     const TilePieces<HD> pieces(tid);
     const int n_logical = a.kv_index ? a.kv_index_stride : a.Lk;   // logical keys: a mask row holds one value per logical key
-    const bool ahead = MODE == kDecAsyncF16 && !IDX && !a.causal && !a.q_len;
+    constexpr bool kGeneral = !PLAIN && !STAGE_MASK;
+    const bool ahead = MODE == kDecAsyncF16 && !IDX && (kGeneral || !a.causal) && !a.q_len;
     int len_ahead = n_logical, lo_ahead = 0, hi_ahead = 0;
     if (MODE == kDecAsyncF16) {
         if (a.kv_len) len_ahead = min(max(peek(a.kv_len + b), 0), n_logical);
-        const int n = (len_ahead + kDecBN - 1) / kDecBN, tps = div_splits(a, n + a.n_splits - 1);
+        const int bound = kGeneral && a.causal ? min(len_ahead, a.n_past + a.Tq) : len_ahead;   // without q_len tables n_past is the call's
+        const int n = (bound + kDecBN - 1) / kDecBN, tps = div_splits(a, n + a.n_splits - 1);
         lo_ahead = split * tps, hi_ahead = min(n, lo_ahead + tps);
     }
     // staged mask: the row of the mask this thread copies pieces of (the head and batch broadcasts are remainders by

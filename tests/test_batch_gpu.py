@@ -315,18 +315,25 @@ class _Memory:
         self.__cuda_array_interface__ = dict(data=(ptr, False), shape=(n,), typestr="<i4", strides=None, version=3)
 
 
-@pytest.mark.parametrize("kv,hd,gqa,B", [("f16", 128, 4, 2), ("f16", 128, 4, 40), ("f16", 64, 1, 3), ("q8_0", 128, 4, 2), ("q8_0", 64, 2, 24)])
-def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B):
-    """The decode kernels read kv_len ahead of their dependency wait and again behind it.  Here the table lies in a cache
-    row that an append of the same stream writes directly before the launch, behind a long kernel: what is read ahead is the
-    old length, longer, shorter, of another tile count or zero."""
+@pytest.mark.parametrize("kv,hd,gqa,B,Tq,form", [
+    ("f16", 128, 4, 2, 1, "plain"), ("f16", 128, 4, 40, 1, "plain"), ("f16", 64, 1, 3, 1, "plain"), ("q8_0", 128, 4, 2, 1, "plain"),
+    ("q8_0", 64, 2, 24, 1, "plain"),
+    # a causal bound cuts the tile range that the length gives: none, some or all of it lies behind the bound
+    ("f16", 128, 4, 3, 4, "causal"), ("f16", 64, 1, 40, 3, "causal"), ("f16", 32, 2, 24, 2, "causal")])
+def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B, Tq, form):
+    """The decode kernels over F16 rows read kv_len ahead of their dependency wait, copy by it and read it again behind the wait.
+    Here the table lies in a cache row that an append of the same stream writes directly before the launch, behind a long
+    kernel: what is read ahead is the old length, longer, shorter, of another tile count or zero.  (The kernels over a Q8_0
+    cache read it behind the wait only.)"""
     rng = np.random.default_rng(hd + B)
     Hkv, Lk = 8, 448
     H = Hkv * gqa
-    q = randn_f16(rng, (B, H, 1, hd))
+    q = randn_f16(rng, (B, H, Tq, hd))
     kf, vf = (rng.standard_normal((B, Hkv, Lk, hd)).astype(np.float32) for _ in "kv")
     k, v = (orc.quantize_q8_0(kf), orc.quantize_q8_0(vf)) if kv == "q8_0" else (kf.astype(np.float16), vf.astype(np.float16))
     kw = dict(scale=hd ** -0.5, **(dict(kv_type=abi.Q8_0) if kv == "q8_0" else {}))
+    if form == "causal":
+        kw.update(causal=True, n_past=150)
     dq, dk, dv = (torch.from_numpy(x).cuda() for x in (q, k, v))
     table = b200.KvCache(abi.F16, 128, 1, 1, 32, 1)
     words = torch.as_tensor(_Memory(table, table.view(0, 1)[0].data, 64), device="cuda")
@@ -345,7 +352,7 @@ def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B):
         got.append(b200.flash_attn_ext(dq, dk, dv, kv_len=words[:B], **kw))
     torch.cuda.synchronize()
     for ls, out in zip(lens, got):
-        ref = np.zeros((B, 1, H, hd), np.float32)
+        ref = np.zeros((B, Tq, H, hd), np.float32)
         for i, n in enumerate(ls):
             if n:
                 ref[i] = orc.flash_attn_ext(q[i:i + 1], k[i:i + 1, :, :n], v[i:i + 1, :, :n], **kw)[0]
