@@ -805,11 +805,16 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         row_to_query(a, hk, tid >> 3, iq, hq);
         mask_row = a.mask.p + (int64_t)iq * a.mask.nb1 + (int64_t)(hq % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3;
     }
-    // (Rows of head_dim 128 split over a cluster, ahead of which a cache append runs, measured 0.5 us slower with it.  CTAs beyond those
-    // that start together have nothing to wait for, and would ask for every line twice: 60 streams of 200 keys, 20 layers, 269 ->
-    // 260 us, 40 of 300, 10 layers, 134 -> 128.)
+    // (Rows of head_dim 128 split over a cluster, ahead of which a cache append runs, measured 0.5 us slower with it.  CTAs beyond the
+    // first ones have little to wait for, and ask for every line twice: head_dim 128, two CTAs per SM, 60 streams of 200 keys, 20
+    // layers, 269 -> 260 us, 40 of 300, 10 layers, 134 -> 128.  At head_dim 64 three CTAs per SM start together; those beyond two, too,
+    // are better off without (prefetch by the first two / by all three per SM, us per launch: unsplit units, 50 streams of 300 keys
+    // 6.34 / 6.52, 55 6.55 / 6.81; cross-attention of 5 rows, split, 3 windows of 20 heads 6.84 / 7.00, 7 windows 11.69 / 11.86),
+    // except split units of few rows, which are through their queries sooner (1 row, 3 windows 6.45 / 6.32, 4 windows 7.65 / 7.50, 8
+    // of 12 heads 8.42 / 8.30; 3 rows, 4 windows 7.56 / 7.41; but 1 row, 7 windows 11.66 / 11.84, and in the general form, with a
+    // softcap, 4 windows 10.16 / 10.33).)
     const bool first_wave = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < 2 * 148;
-    if (MODE == kDecAsyncF16 && (HD <= 64 || a.n_splits == 1) && first_wave) {
+    if (MODE == kDecAsyncF16 && (HD <= 64 || a.n_splits == 1) && (first_wave || (!kGeneral && a.n_splits > 1 && R < 4))) {
         constexpr int LPR = HD * 2 / 128 > 0 ? HD * 2 / 128 : 1;   // 128-byte lines per row
         const int lo = lo_ahead * kDecBN, hi = min(len_ahead, min(hi_ahead, lo_ahead + kPrefetchTiles) * kDecBN);
         for (int i = tid; i < (hi - lo) * LPR; i += kThreads) {
