@@ -110,9 +110,13 @@ __device__ __forceinline__ uint32_t wait_for_predecessors() {
     asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero) : : "memory");
     return zero;
 }
-// The next kernel of the stream may become resident from here on (if it was launched with programmatic serialisation; it waits
-// for this grid's completion before it touches memory).
+// The next kernel of the stream may become resident from here on, if it was launched with programmatic serialisation.  Ahead of
+// its own griddepcontrol.wait, which every thread of every such kernel executes and which returns when this grid has completed, a kernel
+// does two things with global memory: it asks for lines to be brought into L2 (prefetch_l2 and the tensor-copy prefetch: they return
+// nothing, and L2 is where this grid's writes arrive too), and it reads lengths and index entries past L1, whose values are clamped to
+// the operand before they become an address and read again behind the wait.  No other load, and no store.
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Loads from such an address: coherent ones, which the compiler may move among the instructions of a loop (mask rows at head_dim
 // 64: volatile 1-2 % and plain expressions 5-8 % slower).
 __device__ __forceinline__ uint4 load_behind_wait(const uint4* p) {

@@ -514,7 +514,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
 // launch, four segments 9.2 -> 8.4, 16 segments 19.6 -> 19.0); eight tiles per CTA compete with the copies of the others
 // (32 segments +10 %).  Over a Q8_0 cache, whose copies a CTA starts with a few instructions, it measured nothing.
 constexpr int kPrefetchTiles = 2;
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // x / n_splits: the cluster forms (at most eight splits) without a division.
 __device__ __forceinline__ int div_splits(const FattnArgs& a, int x) {
     return a.n_splits == 1 ? x : (a.n_splits <= 8 && x < 4096 ? (x * a.splits_mul) >> 16 : x / a.n_splits);
@@ -1397,7 +1396,7 @@ __global__ void __launch_bounds__(kThreads, 4) fattn_decode_q8reg_kernel(const F
     }
 
     // the merge kernel (if any) may start launching: it waits for this grid's completion before reading anything
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    let_dependents_launch();
     // ---- merge the four warps' (m, l, O) in shared memory ----
     constexpr int SLAB_STRIDE = HD + 4;
     float* slab = reinterpret_cast<float*>(smem_raw);   // [4][16][SLAB_STRIDE]
@@ -1712,7 +1711,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) fattn_decode_q8t_kernel(cons
         issue(tile + NS);
     }
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    let_dependents_launch();
     // ---- merge the four warps' (m, l, O) in shared memory (same slabs as the kernel above) ----
     constexpr int SLAB_STRIDE = HD + 4;
     float* slab = reinterpret_cast<float*>(smem_raw);   // [NW][8][SLAB_STRIDE]
@@ -2050,7 +2049,7 @@ template <int TYPE, bool VEC16, int HD>
 __global__ void __launch_bounds__(256) kv_to_f16_kernel(const View src0, uint8_t* dst0, const View src1, uint8_t* dst1, int Lk, int Hkv, int chunks) {
     // launched with programmatic stream serialisation: the attention kernel may start its set-up, and nothing is read
     // before the previous kernel of the stream (a cache append) has completed
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    let_dependents_launch();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int LPR = HD / 8, RPW = 32 / LPR;   // lanes per row, rows per warp instruction
     const View& src = blockIdx.y ? src1 : src0;

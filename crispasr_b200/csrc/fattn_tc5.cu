@@ -103,7 +103,7 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
-// The box of such a load into L2 only; see prefetch_line.
+// The box of such a load into L2 only, with no copy to shared memory.
 __device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
                  ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
@@ -287,10 +287,6 @@ __device__ __forceinline__ void poly_ex2(float t0, float t1, float& p0, float& p
     const float e0 = __uint_as_float((__float_as_uint(ra) << 23) + 0x3F800000u), e1 = __uint_as_float((__float_as_uint(rb) << 23) + 0x3F800000u);   // 2^n
     unpack2(mul2(p, pack2(e0, e1)), p0, p1);
 }
-
-// One 128-byte line into L2.  For operands asked for while the previous kernel of the stream still runs: a prefetch returns nothing, and
-// L2 is where that kernel's writes arrive too, so it needs no ordering.
-__device__ __forceinline__ void prefetch_line(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Eight Q elements [c0, c0+8) of one row as packed f16 (F32 rows are rounded to nearest even).
 __device__ __forceinline__ uint4 q_chunk(const uint8_t* rowp, int type, int c0, bool vec16) {

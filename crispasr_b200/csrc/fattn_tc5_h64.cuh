@@ -83,8 +83,8 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     // it measured nothing.)
     if (kPrefetchQ && a.behind_cast && warp < 4 && q0 + tid < a.Tq * a.gqa) {
         const uint8_t* rowp = a.q.p + (int64_t)((q0 + tid) / a.gqa) * a.q.nb1 + (int64_t)(hk * a.gqa + (q0 + tid) % a.gqa) * a.q.nb2 + (int64_t)b * a.q.nb3;
-        prefetch_line(rowp);
-        if (a.q.type == B200_TYPE_F32) prefetch_line(rowp + 128);
+        prefetch_l2(rowp);
+        if (a.q.type == B200_TYPE_F32) prefetch_l2(rowp + 128);
     }
     if (kPrefetchQ) asm volatile("griddepcontrol.wait;" ::: "memory");
     const int bk = b / a.bq;

@@ -72,7 +72,7 @@ template <bool Q8, bool V16, int U>
 __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
     // launched with programmatic stream serialisation: the attention of this layer may set itself up meanwhile, and
     // nothing is touched before the previous kernel of the stream has completed
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    let_dependents_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = a.hd / 8, rpw = 32 / lpr;   // lanes per row (4, 8, 12, 16); rows per warp instruction
     const int sub = lane / lpr, c = (lane - sub * lpr) * 8;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
     if (U == 1) {
         const int row = (chunk * (blockDim.x >> 5) + warp) * rpw + sub;
         if (sub < rpw && row < n_new && (c & 31) == 0)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.src[which] + (int64_t)h * a.snb2[which] + (int64_t)s * a.snb3[which] + (int64_t)row * a.snb1[which] + c * 4));
+            prefetch_l2(a.src[which] + (int64_t)h * a.snb2[which] + (int64_t)s * a.snb3[which] + (int64_t)row * a.snb1[which] + c * 4);
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int p0 = a.pos ? a.pos[s] : a.pos0;
