@@ -507,12 +507,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
-// The first tiles of a decode CTA, asked for while the CTA waits for the previous kernel of the stream: a prefetch returns
-// nothing, and L2 is where that kernel's writes arrive too, so it needs no ordering.  The lengths and index lists that say
-// what to ask for may still change (they are read again after the wait); they are read past L1, which would keep the old
-// values.  Two tiles: the first copies after the wait then hit L2 (one segment of the large decoder 6.6 -> 6.2 us per
-// launch, four segments 9.2 -> 8.4, 16 segments 19.6 -> 19.0); eight tiles per CTA compete with the copies of the others
-// (32 segments +10 %).  Over a Q8_0 cache, whose copies a CTA starts with a few instructions, it measured nothing.
+// The first tiles of a decode CTA, asked for while the CTA waits for the previous kernel of the stream (let_dependents_launch says
+// what may run there).  Two tiles: the first copies after the wait then hit L2 (one segment of the large decoder 6.6 -> 6.2 us per
+// launch, four segments 9.2 -> 8.4); eight tiles per CTA compete with the copies of the others (32 segments +10 %).  Over a Q8_0
+// cache, whose copies a CTA starts with a few instructions, it measured nothing.
 constexpr int kPrefetchTiles = 2;
 // x / n_splits: the cluster forms (at most eight splits) without a division.
 __device__ __forceinline__ int div_splits(const FattnArgs& a, int x) {
@@ -823,9 +821,9 @@ __global__ void __launch_bounds__(kThreads, MODE == kDecAsyncQ8 ? 4 : 1) fattn_d
         }
     }
     if (MODE != kDecAsyncQ8 && first_wave && a.prefetch_q) prefetch_queries(a, b, hk, R, tid);
-    // Launched with programmatic stream serialisation: everything above (kernel parameters, this CTA's own shared
-    // memory) ran while the previous kernel of the stream drained; from here on that kernel has completed and flushed
-    // (a no-op under an ordinary launch).
+    // Launched with programmatic stream serialisation: everything above (kernel parameters, this CTA's own shared memory, prefetches,
+    // lengths that are read again below) ran while the previous kernel of the stream drained; from here on that kernel has completed
+    // and flushed (a no-op under an ordinary launch).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int len_raw = a.kv_len ? load_global(a.kv_len + b) : n_logical;
     const int tq_b = q_rows_of(a, b);   // query rows at or beyond it give zeros
@@ -1851,8 +1849,8 @@ bool use_cluster_merge(const FattnArgs& a) {
 template <typename Kern>
 void launch_split(Kern kern, dim3 grid, size_t smem, cudaStream_t st, const FattnArgs& a, int threads = kThreads) {
     // Programmatic stream serialisation: the grid may become resident while the previous kernel of the stream drains
-    // (its CTAs wait on the device before they touch memory), which hides the launch latency between the layers of a
-    // decode step (+0.8 % on the 64-segment decode launches, +1 % at 32 streams).
+    // (its CTAs wait on the device; let_dependents_launch says what they do before), which hides the launch latency between the
+    // layers of a decode step (+0.8 % on the 64-segment decode launches, +1 % at 32 streams).
     FattnArgs ac = a;
     ac.splits_mul = (65536 + a.n_splits - 1) / a.n_splits;
     // Not where split units come in more CTAs than start together: the wait is over for most of them, and what the first ones ask for

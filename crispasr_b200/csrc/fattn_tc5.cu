@@ -576,8 +576,12 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     }
     // While the previous kernel runs (behind a conversion of K and V, say, which lets this one become resident early) the query tile is
     // brought into L2, from where its copy behind the wait is half as far: 8 streams x 407 tokens over a Q8_0 cache, F32
-    // queries, 53.6 -> 51.9 us per layer; 16 x 100 tokens 18.1 -> 17.5.  (The tile of the CTA that follows on this SM, asked for as
-    // well, cost the gain again: it competes with the copies that are waited for.)
+    // queries, 53.6 -> 51.9 us per layer; 16 x 100 tokens 18.1 -> 17.5.  Behind any other kernel, and in CTAs of later waves, it runs
+    // ahead of the TMEM allocation and the barriers: F32 queries gain 2 % (16 x 407 tokens over F16 rows 75.0 -> 73.8, 1 x 407 14.3 ->
+    // 14.0), F16 queries as much as they lose (1 x 407 12.4 -> 12.35, 16 x 407 60.7 -> 60.5, masked rows of head_dim 64, 1 x 224, 12.9
+    // -> 12.75; but 16 x 100 16.8 -> 17.0, 16 x 750 not causal 102.4 -> 103.3, where leaving out the CTAs of later waves gave half
+    // of that back and took the other gains).  (The tile of the CTA that follows on this SM, asked for as well, cost the gain again:
+    // it competes with the copies that are waited for.)
     if (QMODE && tid == 4 * 32) {
         constexpr int kCols = QMODE == 2 ? 32 : 64;
 #pragma unroll

@@ -66,7 +66,8 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
     volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // launched with programmatic stream serialisation: nothing is read or written before the previous kernel has completed
+    // launched with programmatic stream serialisation: but for the query prefetch below, nothing is read or written before the previous
+    // kernel has completed
     constexpr bool kPrefetchQ = !QTMA && !SPLIT;
     if (!kPrefetchQ) asm volatile("griddepcontrol.wait;" ::: "memory");
     // tile order and GQA packing as in fattn_prefill_tc5_kernel
@@ -78,7 +79,7 @@ fattn_prefill_tc5_h64_kernel(const FattnArgs a, const __grid_constant__ CUtensor
         hk = (lin % hb) % gridDim.y, b = (lin % hb) / gridDim.y;
     }
     // Behind a conversion of K and V, which lets this kernel become resident early, the query rows that the threads will load are brought
-    // into L2 meanwhile: four windows of 20 heads, all F32, 89.8 -> 87.4 us, ten of 500 frames 44.0 -> 41.2.  (Behind a kernel that
+    // into L2 meanwhile: four windows of 20 heads, all F32, 89.1 -> 86.7 us per launch in a graph, ten of 500 frames 44.8 -> 42.2.  (Behind a kernel that
     // does not, and where a cluster shares a tile, it only delays: one window of 8 heads 17.0 -> 17.3.  For tiles that come by one copy
     // it measured nothing.)
     if (kPrefetchQ && a.behind_cast && warp < 4 && q0 + tid < a.Tq * a.gqa) {

@@ -70,17 +70,19 @@ __device__ __forceinline__ uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c
 // the upper half of its left neighbour's last word (the first lane the scale) and the row leaves in 32-bit stores.
 template <bool Q8, bool V16, int U>
 __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
-    // launched with programmatic stream serialisation: the attention of this layer may set itself up meanwhile, and
-    // nothing is touched before the previous kernel of the stream has completed
+    // launched with programmatic stream serialisation: the attention of this layer may set itself up meanwhile; rows are read and
+    // written behind the wait, when the previous kernel of the stream has completed
     let_dependents_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lpr = a.hd / 8, rpw = 32 / lpr;   // lanes per row (4, 8, 12, 16); rows per warp instruction
     const int sub = lane / lpr, c = (lane - sub * lpr) * 8;
     const int which = blockIdx.y, sh = blockIdx.x / a.chunks, chunk = blockIdx.x - sh * a.chunks, s = sh / a.n_kv, h = sh - s * a.n_kv;
     const int n_new = a.n_new[which];
-    // One token per stream: its rows are brought into L2 while the previous kernel still runs (a prefetch returns nothing, and L2 is where
-    // that kernel's writes arrive too).  Rows that are not there yet cost a trip to memory on the chain of a decode step otherwise: 32
-    // streams of an F16 cache, 30 layers, 470 -> 458 us; 20 streams, 20 layers, 157 -> 148.
+    // A warp's first rows (all it has where one token per stream enters) are brought into L2 while the previous kernel still runs.  Rows that
+    // are not there yet cost a trip to memory on the chain of a decode step otherwise: 32 streams of an F16 cache, 30 layers, 470 ->
+    // 458 us; 20 streams, 20 layers, 157 -> 148.  A few rows per stream gain as much, in one wave of CTAs or several (the append alone,
+    // 16 streams of 4 rows 1.7 -> 1.45 us, 256 of 8 6.8 -> 5.7, 64 of 30 6.1 -> 5.3).  The form of
+    // two rows in flight per warp was not measured with it.
     if (U == 1) {
         const int row = (chunk * (blockDim.x >> 5) + warp) * rpw + sub;
         if (sub < rpw && row < n_new && (c & 31) == 0)
