@@ -319,14 +319,19 @@ class _Memory:
     ("f16", 128, 4, 2, 1, "plain"), ("f16", 128, 4, 40, 1, "plain"), ("f16", 64, 1, 3, 1, "plain"), ("q8_0", 128, 4, 2, 1, "plain"),
     ("q8_0", 64, 2, 24, 1, "plain"),
     # a causal bound cuts the tile range that the length gives: none, some or all of it lies behind the bound
-    ("f16", 128, 4, 3, 4, "causal"), ("f16", 64, 1, 40, 3, "causal"), ("f16", 32, 2, 24, 2, "causal")])
+    ("f16", 128, 4, 3, 4, "causal"), ("f16", 64, 1, 40, 3, "causal"), ("f16", 32, 2, 24, 2, "causal"),
+    # mask pieces travel with the key tiles and are issued again with them: at most eight rows, more, and head_dim 32
+    ("f16", 64, 1, 3, 5, "mask"), ("f16", 128, 4, 2, 4, "mask"), ("f16", 64, 1, 40, 5, "mask"), ("f16", 32, 1, 3, 5, "mask"),
+    ("f16", 64, 1, 3, 1, "softcap"), ("f16", 32, 2, 40, 1, "plain"),
+    # nine splits of eleven tiles through the workspace: some of them without a tile
+    ("f16", 64, 1, 2, 1, "9 splits"), ("f16", 128, 4, 2, 4, "9 splits")])
 def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B, Tq, form):
     """The decode kernels over F16 rows read kv_len ahead of their dependency wait, copy by it and read it again behind the wait.
     Here the table lies in a cache row that an append of the same stream writes directly before the launch, behind a long
     kernel: what is read ahead is the old length, longer, shorter, of another tile count or zero.  (The kernels over a Q8_0
     cache read it behind the wait only.)"""
     rng = np.random.default_rng(hd + B)
-    Hkv, Lk = 8, 448
+    Hkv, Lk = 8, 700 if form == "9 splits" else 448
     H = Hkv * gqa
     q = randn_f16(rng, (B, H, Tq, hd))
     kf, vf = (rng.standard_normal((B, Hkv, Lk, hd)).astype(np.float32) for _ in "kv")
@@ -334,6 +339,13 @@ def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B, T
     kw = dict(scale=hd ** -0.5, **(dict(kv_type=abi.Q8_0) if kv == "q8_0" else {}))
     if form == "causal":
         kw.update(causal=True, n_past=150)
+    if form == "softcap":
+        kw["softcap"] = 5.0
+    mask = None
+    if form == "mask":
+        mask = np.where(rng.random((1, 1, Tq, Lk)) < 0.4, -np.inf, rng.standard_normal((1, 1, Tq, Lk))).astype(np.float16)
+        mask[..., 0] = 0.0   # a row of one key sees it
+    dmask = None if mask is None else torch.from_numpy(mask).cuda()
     dq, dk, dv = (torch.from_numpy(x).cuda() for x in (q, k, v))
     table = b200.KvCache(abi.F16, 128, 1, 1, 32, 1)
     words = torch.as_tensor(_Memory(table, table.view(0, 1)[0].data, 64), device="cuda")
@@ -349,11 +361,16 @@ def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B, T
     for row in rows:
         b200.flash_attn_ext(slow, slow, slow, scale=0.125)
         table.append(0, row, row, pos0=0)
-        got.append(b200.flash_attn_ext(dq, dk, dv, kv_len=words[:B], **kw))
+        assert b200.lib().b200_set_decode_splits(9 if form == "9 splits" else 0) == 0
+        try:
+            got.append(b200.flash_attn_ext(dq, dk, dv, dmask, kv_len=words[:B], **kw))
+        finally:
+            b200.lib().b200_set_decode_splits(0)
     torch.cuda.synchronize()
     for ls, out in zip(lens, got):
         ref = np.zeros((B, Tq, H, hd), np.float32)
         for i, n in enumerate(ls):
             if n:
-                ref[i] = orc.flash_attn_ext(q[i:i + 1], k[i:i + 1, :, :n], v[i:i + 1, :, :n], **kw)[0]
+                m = None if mask is None else mask[..., :n]
+                ref[i] = orc.flash_attn_ext(q[i:i + 1], k[i:i + 1, :, :n], v[i:i + 1, :, :n], m, **kw)[0]
         assert_close(out.cpu().numpy(), ref, "lengths %s" % ls[:4])
