@@ -320,6 +320,7 @@ class _Memory:
     ("q8_0", 64, 2, 24, 1, "plain"),
     # a causal bound cuts the tile range that the length gives: none, some or all of it lies behind the bound
     ("f16", 128, 4, 3, 4, "causal"), ("f16", 64, 1, 40, 3, "causal"), ("f16", 32, 2, 24, 2, "causal"),
+    ("f16", 64, 1, 3, 4, "causal from -2"), ("f16", 128, 4, 3, 4, "causal from -300"),   # rows that see no key give zeros
     # mask pieces travel with the key tiles and are issued again with them: at most eight rows, more, and head_dim 32
     ("f16", 64, 1, 3, 5, "mask"), ("f16", 128, 4, 2, 4, "mask"), ("f16", 64, 1, 40, 5, "mask"), ("f16", 32, 1, 3, 5, "mask"),
     ("f16", 64, 1, 3, 1, "softcap"), ("f16", 32, 2, 40, 1, "plain"),
@@ -337,8 +338,8 @@ def test_lengths_written_by_the_kernel_right_before(b200, orc, kv, hd, gqa, B, T
     kf, vf = (rng.standard_normal((B, Hkv, Lk, hd)).astype(np.float32) for _ in "kv")
     k, v = (orc.quantize_q8_0(kf), orc.quantize_q8_0(vf)) if kv == "q8_0" else (kf.astype(np.float16), vf.astype(np.float16))
     kw = dict(scale=hd ** -0.5, **(dict(kv_type=abi.Q8_0) if kv == "q8_0" else {}))
-    if form == "causal":
-        kw.update(causal=True, n_past=150)
+    if form.startswith("causal"):
+        kw.update(causal=True, n_past=int(form[len("causal from"):] or 150))
     if form == "softcap":
         kw["softcap"] = 5.0
     mask = None
