@@ -204,6 +204,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st64(uint32_t taddr, const uint32_t (&r)[64]) {
+    uint32_t lo[32], hi[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) lo[i] = r[i], hi[i] = r[32 + i];
+    tmem_st32(taddr, lo);
+    tmem_st32(taddr + 32, hi);
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -1043,570 +1050,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     }
 }
 
-// ------------------------------------------------------------------------------------------------------
-// Relative-position variant (FastConformer, head_dim 128): logits = scale*Q_u.K^T + f16(scale * relshift(Q_v.R^T)).
-//
-// Per 128x128 tile the bias needs X = Q_v[128 x hd] . R_band[256 x hd]^T with R_band = R rows
-// [rb, rb+256), rb = (Tq-1) + k0 - q0 - 127; the bias of (row i, key j) is X[i][j - i + 127] (the rel-shift).
-// X is one more accumulator in TMEM (256 columns; S 128, O 128 -> all 512 columns, one CTA per SM).
-// A tcgen05.ld reads the same columns for every lane, so the per-row shift cannot be done in the load:
-// each softmax thread loads the 96 columns its warp can need for half a tile, rounds scale*x to f16 (the
-// reference's rounding point), parks them in its own row of a shared-memory buffer and reads 64 of them
-// back from its row-dependent offset.  Only the thread itself touches its row: no barrier is involved.
-// Consecutive KV tiles share half of the band, so R arrives in 128-row half-blocks through a 2-slot ring
-// (half-block m = rows rb_0 + 128m ..; tile j uses half-blocks j and j+1), and so does X: the product of a half-block is
-// computed once, into the 128 columns that the half-block two before it leaves.
-// MMA order: X_0 X_1 S[0] | per tile j: X_(j+2) as soon as the softmax threads have drained tile j's columns; then, once
-// P[j] is in TMEM, PV[j] and S[j+1].
-//
-// What bounds it: the chain of one tile through the eight softmax warps (extraction of the bias 1.35 k clk, exponentials
-// 1.7 k, hand-offs 0.9 k = 4.0 k), against 1.5 k of MMA and 1.0 k of exponential unit; TMEM and shared memory are full,
-// there is no room for a second query tile.  2 recordings of 7500 frames: 985 -> 856 us (both products per band half, a
-// separate maximum pass, and the R copies queued behind the V copies cost the rest); 8 utterances of up to 138 frames 29 ->
-// 16 us, a mask over 3000 frames 209 -> 186 us (the query tile by whole rows: 7 k clk of a CTA's start).
-// ------------------------------------------------------------------------------------------------------
-// 128-element query rows -> swizzled f16 operand tiles, 16 rows per warp, a warp instruction covers whole rows: lane l reads
-// float4 l of one F32 row, or 16 bytes l % 16 of two F16 rows; all loads in flight at once.  BIAS: two tiles from one read,
-// Q + bias_u and Q + bias_v, sums formed in fp32 and rounded once.  Rows at or beyond `rows` (of the tile) are zero.
-// (A thread per half row read 32 rows per instruction, 16 bytes each, and the biases element by element.)
-template <bool F16, bool BIAS>
-__device__ __forceinline__ void load_relpos_q(uint8_t* tile_u, uint8_t* tile_v, const uint8_t* base, int64_t nb1, int q0, int rows, const float* bias_u,
-                                              const float* bias_v, int warp, int lane) {
-    constexpr int N = F16 ? 8 : 4, RPI = F16 ? 2 : 1, K = 16 / RPI;   // elements per lane; rows per instruction; instructions
-    const int c = (F16 ? lane & 15 : lane) * N;
-    float bu[N], bv[N];
-    if (BIAS) {
-#pragma unroll
-        for (int i = 0; i < N; i += 4) {
-            const float4 x = load_global(reinterpret_cast<const float4*>(bias_u + c + i)), y = load_global(reinterpret_cast<const float4*>(bias_v + c + i));
-            bu[i] = x.x, bu[i + 1] = x.y, bu[i + 2] = x.z, bu[i + 3] = x.w;
-            bv[i] = y.x, bv[i + 1] = y.y, bv[i + 2] = y.z, bv[i + 3] = y.w;
-        }
-    }
-    uint4 v[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int r = warp * 16 + k * RPI + (F16 ? lane >> 4 : 0);
-        v[k] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < rows) v[k] = load_global(reinterpret_cast<const uint4*>(base + (int64_t)(q0 + r) * nb1 + c * (F16 ? 2 : 4)));
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-        const int r = warp * 16 + k * RPI + (F16 ? lane >> 4 : 0);
-        const uint32_t off = (c >> 6) * kPanelBytes + r * 128 + ((((c & 63) >> 3) ^ (r & 7)) << 4) + (c & 4) * 2;
-        if (F16 && !BIAS) {
-            *reinterpret_cast<uint4*>(tile_u + off) = v[k];
-            continue;
-        }
-        float f[N];
-        const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (F16) {
-                const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-                f[(2 * i) % N] = p.x, f[(2 * i + 1) % N] = p.y;
-            } else {
-                f[i] = __uint_as_float(w[i]);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < (BIAS ? 2 : 1); t++) {
-            uint32_t o[N / 2];
-#pragma unroll
-            for (int i = 0; i < N; i += 2) {
-                const float x = BIAS && r < rows ? __fadd_rn(f[i], t ? bv[i] : bu[i]) : f[i];
-                const float y = BIAS && r < rows ? __fadd_rn(f[i + 1], t ? bv[i + 1] : bu[i + 1]) : f[i + 1];
-                o[i >> 1] = pack_half2(x, y);
-            }
-            uint8_t* p = (t ? tile_v : tile_u) + off;
-            if constexpr (F16) *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2 % (N / 2)], o[3 % (N / 2)]);
-            else *reinterpret_cast<uint2*>(p) = make_uint2(o[0], o[1]);
-        }
-    }
-}
-
-// 32 bytes of one row per lane: whole sectors without a staging pass through shared memory (`wide`: 32-byte aligned rows).
-__device__ __forceinline__ void store8(float* p, const uint32_t* r, float f, bool wide) {
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]) * f;
-    if (wide) {
-        asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
-                     "f"(v[6]), "f"(v[7])
-                     : "memory");
-    } else {
-        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-    }
-}
-
-constexpr int kBncStride = 128;  // bytes per bounce row: a ring of 64 f16 values
-
-constexpr int kThreadsRelpos = 320;  // 8 softmax warps (two threads per query row), TMA warp, MMA warp
-
-template <bool HASMASK>
-__global__ void __launch_bounds__(kThreadsRelpos, 1)
-fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap tmK,
-                                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmR) {
-    constexpr int HD = 128;
-    constexpr int TILE_BYTES = 2 * kPanelBytes;  // 128 rows x 128 halves
-    constexpr uint32_t IDESC_S = idesc_f16(kTile, false);
-    constexpr uint32_t IDESC_PV = idesc_f16(HD, true);
-
-    extern __shared__ uint8_t smem_dyn[];
-    const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
-    uint8_t* smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));
-    const uint32_t sQ = smem_base, sQv = sQ + TILE_BYTES, sK = sQv + TILE_BYTES, sV = sK + TILE_BYTES,
-                   sR = sV + TILE_BYTES, sBnc = sR + 2 * TILE_BYTES, sBar = sBnc + 2 * kTile * kBncStride;
-    const uint32_t bar_k_full = sBar, bar_k_empty = sBar + 8, bar_v_full = sBar + 16, bar_v_empty = sBar + 24,
-                   bar_r_full = sBar + 32 /* [2] */, bar_r_empty = sBar + 48 /* [2] */, bar_s_full = sBar + 64,
-                   bar_x_full = sBar + 72, bar_x_free = sBar + 80, bar_p_ready = sBar + 88, bar_o_done = sBar + 96,
-                   bar_pair = sBar + 104 /* [4]: the two warps that share 32 TMEM lanes */;
-    uint8_t* misc = smem_gen + 6 * TILE_BYTES + 2 * kTile * kBncStride + 136;
-    volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
-    volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
-    volatile float* s_xchg = reinterpret_cast<volatile float*>(misc + 8);   // [2][128]: exchange of row sums between the two threads of a row
-
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int q0 = blockIdx.x * kTile, h = blockIdx.y, b = blockIdx.z;
-    const int hk = h / a.gqa, bk = b / a.bq;
-    const int rb3 = a.r_ne3 > 1 ? b : 0;
-    if (tid == 8 * 32) {
-        for (int i = 0; i < 17; i++) {
-            const uint32_t bar = sBar + 8 * i;
-            mbar_init(bar, (bar == bar_x_free || bar == bar_p_ready) ? 8 : (bar >= bar_pair ? 64 : 1));   // 8 = one arrival per softmax warp
-        }
-        *s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
-    }
-    // launched with programmatic stream serialisation: nothing is read before the previous kernel has completed
-    const uint32_t behind_wait = wait_for_predecessors();
-
-    int len_b = a.Lk;
-    if (a.kv_len) {
-        const int v = a.kv_len[b];
-        len_b = v < 0 ? 0 : (v > a.Lk ? a.Lk : v);
-    }
-    const int tq_b = q_rows_of(a, b);   // query rows at or beyond it are padding of a batched launch: zeros
-    const int n_tiles = (len_b > 0 && q0 < tq_b) ? (len_b + kTile - 1) / kTile : 0;
-    if (n_tiles == 0) {
-        if (tid < kTile && q0 + tid < a.Tq) {
-            float4* out = reinterpret_cast<float4*>(a.dst + (((int64_t)b * a.Tq + q0 + tid) * a.dst_heads + h) * HD);
-#pragma unroll
-            for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        return;
-    }
-    const int rb0 = a.Tq - 1 - q0 - 127;  // first R row of half-block 0 (may be negative: TMA zero-fills)
-
-    // half-block m of R -> ring slot m % 2.  The ring is laid out panel-major, [panel 0: slot 0 | slot 1][panel 1:
-    // slot 0 | slot 1] (16 KB each).
-    auto load_r = [&](int m) {
-        const int slot = m & 1;
-        mbar_arrive_expect_tx(bar_r_full + 8 * slot, TILE_BYTES);
-        tma_load_4d(sR + slot * kPanelBytes, &tmR, bar_r_full + 8 * slot, 0, rb0 + kTile * m, h, rb3);
-        tma_load_4d(sR + 2 * kPanelBytes + slot * kPanelBytes, &tmR, bar_r_full + 8 * slot, 64, rb0 + kTile * m, h, rb3);
-    };
-    auto load_kv = [&](int j, bool is_v) {
-        const uint32_t bar = is_v ? bar_v_full : bar_k_full;
-        const uint32_t dst = is_v ? sV : sK;
-        mbar_arrive_expect_tx(bar, TILE_BYTES);
-        tma_load_4d(dst, is_v ? &tmV : &tmK, bar, 0, j * kTile, hk, bk);
-        tma_load_4d(dst + kPanelBytes, is_v ? &tmV : &tmK, bar, 64, j * kTile, hk, bk);
-    };
-
-    // ---- set-up ----
-    if (tid == 8 * 32) {
-        load_r(0);
-        load_r(1);
-        load_kv(0, false);
-        load_kv(0, true);
-    }
-    if (warp == 9) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(const_cast<uint32_t*>(s_tmem_base))),
-                     "r"(512u)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (warp < 8) {
-        // Q_u and Q_v tiles -> shared memory.  Aligned rows: warp w takes rows [16w, 16w + 16) whole (load_relpos_q); with
-        // the position biases folded in, one read of Q serves both tiles.  Otherwise thread (r, ch) moves half of row r.
-        const uint8_t* q_base = a.q.p + (int64_t)h * a.q.nb2 + (int64_t)b * a.q.nb3;
-        const uint8_t* qv_base = a.qv.p + (int64_t)h * a.qv.nb2 + (int64_t)b * a.qv.nb3;
-        const int rows = a.Tq - q0;
-        if (a.bias_u != nullptr && a.q.vec16 && ((reinterpret_cast<uintptr_t>(a.bias_u) | reinterpret_cast<uintptr_t>(a.bias_v)) & 15) == 0) {
-            if (a.q.type == B200_TYPE_F32) load_relpos_q<false, true>(smem_gen, smem_gen + TILE_BYTES, q_base, a.q.nb1, q0, rows, a.bias_u + h * HD, a.bias_v + h * HD, warp, lane);
-            else load_relpos_q<true, true>(smem_gen, smem_gen + TILE_BYTES, q_base, a.q.nb1, q0, rows, a.bias_u + h * HD, a.bias_v + h * HD, warp, lane);
-        } else if (a.bias_u == nullptr && a.q.vec16 && a.qv.vec16) {
-            if (a.q.type == B200_TYPE_F32) load_relpos_q<false, false>(smem_gen, nullptr, q_base, a.q.nb1, q0, rows, nullptr, nullptr, warp, lane);
-            else load_relpos_q<true, false>(smem_gen, nullptr, q_base, a.q.nb1, q0, rows, nullptr, nullptr, warp, lane);
-            if (a.qv.type == B200_TYPE_F32) load_relpos_q<false, false>(smem_gen + TILE_BYTES, nullptr, qv_base, a.qv.nb1, q0, rows, nullptr, nullptr, warp, lane);
-            else load_relpos_q<true, false>(smem_gen + TILE_BYTES, nullptr, qv_base, a.qv.nb1, q0, rows, nullptr, nullptr, warp, lane);
-        } else {
-            const int r = tid & 127, ch = tid >> 7;
-            const int iq = q0 + r;
-#pragma unroll 1
-            for (int which = 0; which < 2; which++) {
-                const View& qv = which ? a.qv : a.q;
-                const uint8_t* rowp = (which ? qv_base : q_base) + (int64_t)iq * qv.nb1;
-                const float* bias = which ? a.bias_v : a.bias_u;
-#pragma unroll 1
-                for (int c = 0; c < HD / 16; c++) {
-                    const int cc = ch * (HD / 16) + c;
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (iq < a.Tq) v = bias != nullptr ? load8_plus_bias_as_half(rowp, qv.type, cc * 8, qv.vec16 != 0, bias + h * HD + cc * 8)
-                                                       : q_chunk(rowp, qv.type, cc * 8, qv.vec16 != 0);
-                    *reinterpret_cast<uint4*>(smem_gen + which * TILE_BYTES + r * 128 + (cc >> 3) * kPanelBytes + (((cc & 7) ^ (r & 7)) << 4)) = v;
-                }
-            }
-        }
-        fence_proxy_async();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
-    const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + 128, tmem_X = tmem_base + 256;
-
-    if (warp == 8) {
-        // ================= TMA producer =================
-        if (lane == 0) {
-            bool ok = true;
-            // half-block m goes into the slot half-block m - 2 leaves when its product is complete
-            auto next_r = [&](int m) {
-                ok = mbar_wait(bar_r_empty + 8 * (m & 1), ((m >> 1) - 1) & 1, s_abort);
-                if (ok) load_r(m);
-                return ok;
-            };
-            if (n_tiles > 1) next_r(2);
-            for (int j = 1; j < n_tiles && ok; j++) {
-                // two tiles ahead: behind the copy of V[j - 1], which waits for a product of its own
-                if (j + 2 <= n_tiles && !next_r(j + 2)) break;
-                ok = mbar_wait(bar_k_empty, (j - 1) & 1, s_abort);
-                if (!ok) break;
-                load_kv(j, false);
-                ok = mbar_wait(bar_v_empty, (j - 1) & 1, s_abort);
-                if (!ok) break;
-                load_kv(j, true);
-            }
-            if (!ok) {  // drain: bounded wait for copies still in flight
-                for (uint32_t it = 0; it < 65536; ++it) __nanosleep(64);
-            }
-        }
-    } else if (warp == 9) {
-        // ================= MMA issuer =================
-        {
-            // X_m = Q_v . R_m^T, the product of half-block m, lives in X columns [128 (m & 1), +128): tile j reads those of
-            // half-blocks j and j + 1, and only half-block j + 2 is new to tile j + 1.
-            const uint32_t q_lo = smem_desc_lo(sQ, 16), qv_lo = smem_desc_lo(sQv, 16), k_lo = smem_desc_lo(sK, 16), r_lo = smem_desc_lo(sR, 16),
-                           v_lo = smem_desc_lo(sV, kPanelBytes);
-            constexpr uint32_t desc_hi = smem_desc_hi(1024);
-            auto issue_x = [&](int m) {
-#pragma unroll
-                for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                    const uint32_t roff16 = (uint32_t)(((ks >> 2) * 2 * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(tmem_X + (m & 1) * kTile, desc64(qv_lo + off16, desc_hi), desc64(r_lo + (m & 1) * (kPanelBytes >> 4) + roff16, desc_hi), IDESC_S,
-                           ks > 0 ? 1u : 0u);
-                }
-                if (m > 0) tc_commit(bar_x_full);   // (tile 0 needs half-blocks 0 and 1)
-                tc_commit(bar_r_empty + 8 * (m & 1));
-            };
-            auto issue_s = [&]() {
-#pragma unroll
-                for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(k_lo + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
-                }
-                tc_commit(bar_s_full);
-                tc_commit(bar_k_empty);
-            };
-            bool ok = mbar_wait(bar_r_full, 0, s_abort) && mbar_wait(bar_r_full + 8, 0, s_abort) &&
-                      mbar_wait(bar_k_full, 0, s_abort);
-            ok = warp_all(ok);
-            if (ok) {
-                tc_fence_after();
-                if (elect_one()) {
-                    issue_x(0);
-                    issue_x(1);
-                    issue_s();
-                }
-                __syncwarp();
-            }
-            for (int j = 0; j < n_tiles && ok; j++) {
-                const bool more = j + 1 < n_tiles;
-                if (more) {
-                    // half-block j+2 is in its slot, and the columns of half-block j have been read
-                    ok = mbar_wait(bar_r_full + 8 * (j & 1), ((j + 2) >> 1) & 1, s_abort) &&
-                         mbar_wait(bar_x_free, j & 1, s_abort);
-                    ok = warp_all(ok);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) issue_x(j + 2);
-                    __syncwarp();
-                }
-                ok = mbar_wait(bar_v_full, j & 1, s_abort);
-                if (ok && more) ok = mbar_wait(bar_k_full, (j + 1) & 1, s_abort);
-                if (ok) ok = mbar_wait(bar_p_ready, j & 1, s_abort);
-                ok = warp_all(ok);
-                if (!ok) break;
-                tc_fence_after();
-                if (elect_one()) {
-                    mma_ts(tmem_O, tmem_P, desc64(v_lo, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
-#pragma unroll
-                    for (int ks = 1; ks < kTile / 16; ks++)
-                        mma_ts(tmem_O, tmem_P + ks * 8, desc64(v_lo + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
-                    tc_commit(bar_v_empty);
-                    if (more) issue_s();
-                    else tc_commit(bar_o_done);
-                }
-                __syncwarp();
-            }
-            if (!ok) {
-                if (elect_one()) tc_commit(bar_o_done);
-                __syncwarp();
-                for (uint32_t it = 0; it < 65536 && !mbar_try_wait(bar_o_done, 0); ++it) __nanosleep(256);
-            }
-            __syncwarp();
-        }
-    } else {
-        // ================= softmax / bias / epilogue: thread (r, ch) owns columns [64ch, 64ch+64) of row r ========
-        // Eight softmax warps: warps w and w+4 see the same 32 TMEM lanes. The two threads of a row exchange
-        // their half-row sums through shared memory and an mbarrier of 64 arrivals once per tile (their maxima only where
-        // the reference is taken anew); each keeps a partial row sum and owns half of the O columns.
-        const int r = tid & 127, ch = tid >> 7;
-        const int iq = q0 + r;
-        const uint32_t my_pair_bar = bar_pair + 8 * (warp & 3);
-        uint32_t pair_phase = 0;
-        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        const float bscale = a.relscale;   // == a.scale: the tcgen05 path is not taken with a softcap
-        const uint64_t bscale2 = pack2(bscale, bscale);
-        const int shift = 31 - lane;       // band offset of this row inside the warp's columns
-        // Bounce ring of this thread: 64 f16 values (two 32-column chunks) = 32 words.
-        uint8_t* const bnc_gen = smem_gen + (sBnc - smem_base) + tid * kBncStride;
-        // rotation in words: 16-byte stores of the same logical chunk by the 8 lanes of a quarter-warp, and 4-byte
-        // loads of logical word (const - lane/2) by all 32 lanes, both hit 32 distinct banks (found by enumeration)
-        const uint32_t rot = 4u * ((lane + 3u * (lane >> 3)) & 7u);
-        const uint32_t x_col0 = 96 - 32 * (warp & 3) + 64 * ch;   // first X column this thread's warp can need
-        const uint64_t l2e2 = pack2(kLog2e, kLog2e), c2 = pack2(bscale * kLog2e, bscale * kLog2e);
-        float m_ref = -INFINITY, l_run = 0.0f;
-        bool ok = true;
-        // Explicit F16 mask added on top of the bias (bucket padding of src/canary_ctc.cpp:370-382, the local-attention
-        // window of src/core/fastconformer.h:887-895): this thread's row of [Lk, Tq, 1|H, 1|B];
-        // rows past Tq (the padding rows of the last query tile) read row 0.
-        const uint8_t* mrow = HASMASK ? a.mask.p + behind_wait + (int64_t)(iq < a.Tq ? iq : 0) * a.mask.nb1 +
-                                            (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3
-                                      : nullptr;
-        // Publish a value, meet the partner warp at the pair barrier (bounded wait), read the partner's value.
-        // One slot per thread is enough for the row sums: between two of them lies either an exchange of maxima or the wait
-        // for the next S tile, which the tensor pipe only produces after the P*V product that needed the partner's arrival
-        // on bar_p_ready (behind its read).  The maxima travel through the first word of the thread's own bounce ring, free
-        // between the extraction of the bias and the next tile; an exchange of sums always follows them.
-        auto exchange_at = [&](volatile float* mine, volatile float* theirs, float v) {
-            *mine = v;
-            mbar_arrive(my_pair_bar);
-            ok = mbar_wait(my_pair_bar, pair_phase, s_abort);
-            pair_phase ^= 1;
-            return *theirs;
-        };
-        auto exchange = [&](float v) { return exchange_at(s_xchg + ch * 128 + r, s_xchg + (ch ^ 1) * 128 + r, v); };
-        auto exchange_max = [&](float v) {
-            return exchange_at(reinterpret_cast<volatile float*>(bnc_gen), reinterpret_cast<volatile float*>(smem_gen + (sBnc - smem_base) + (tid ^ 128) * kBncStride), v);
-        };
-        for (int j = 0; j < n_tiles; j++) {
-            // ---- phase A: the 64 bias values of this half row, fp32 registers holding f16-rounded numbers ----
-            ok = mbar_wait(bar_x_full, j & 1, s_abort);
-            if (!ok) break;
-            tc_fence_after();
-            uint32_t bias2[32];   // the 64 bias values as packed pairs
-            auto bounce_chunk = [&](const uint32_t (&xr)[32], int k) {
-                // scale*x rounded to f16 (the reference's cast of its mask), 32 values = 16 words, into ring half k&1
-                uint32_t w[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    float x0, x1;
-                    unpack2(mul2(pack2(__uint_as_float(xr[2 * i]), __uint_as_float(xr[2 * i + 1])), bscale2), x0, x1);
-                    w[i] = cvt_f16x2(x0, x1);
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i += 4)
-                    *reinterpret_cast<uint4*>(bnc_gen + ((((k & 1) * 16 + i + rot) & 31) << 2)) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
-            };
-            auto read_quarter = [&](int qq) {  // half-row columns [32qq, 32qq+32): ring halves shift .. shift+31 of chunks qq, qq+1
-                const uint32_t h0 = (uint32_t)(qq * 32 + shift);
-                const uint32_t fs = (h0 & 1u) * 16u;
-                uint32_t prev = *reinterpret_cast<const uint32_t*>(bnc_gen + ((((h0 >> 1) + rot) & 31) << 2));
-#pragma unroll
-                for (int p2 = 0; p2 < 16; p2++) {
-                    const uint32_t next = *reinterpret_cast<const uint32_t*>(bnc_gen + ((((h0 >> 1) + p2 + 1 + rot) & 31) << 2));
-                    bias2[qq * 16 + p2] = __funnelshift_r(prev, next, fs);
-                    prev = next;
-                }
-            };
-            {
-                const uint32_t xswap = (j & 1) ? 128u : 0u;  // half-block j lives in columns 128 (j & 1) ..
-                uint32_t xa[3][32];
-#pragma unroll
-                for (int k = 0; k < 3; k++) tmem_ld32(tmem_X + lane_base + ((x_col0 + k * 32 + xswap) & 255u), xa[k]);
-                tmem_wait_ld();
-                // the columns of half-block j are free the moment every warp holds its 96 values in registers
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_x_free);
-                bounce_chunk(xa[0], 0);
-                bounce_chunk(xa[1], 1);
-                read_quarter(0);
-                bounce_chunk(xa[2], 2);
-                read_quarter(1);
-            }
-            float u[HASMASK ? 64 : 1];   // with an explicit mask: bias + mask, in fp32
-            if constexpr (HASMASK) {
-                uint4 mv[8];
-                load_mask64(mv, mrow + (int64_t)(j * kTile + ch * 64) * 2, a.Lk - (j * kTile + ch * 64));
-#pragma unroll
-                for (int i = 0; i < 64; i += 2) {
-                    const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias2[i >> 1])), m2 = mask_pair(mv, i);
-                    u[i] = b2.x + m2.x, u[i + 1] = b2.y + m2.y;
-                }
-            }
-
-            // ---- phase B: P = exp2(S*scale*log2(e) + bias*log2(e) - m_ref) ----
-            ok = mbar_wait(bar_s_full, j & 1, s_abort);
-            if (!ok) break;
-            tc_fence_after();
-            const int n_valid = len_b - j * kTile;
-            const bool full_tile = n_valid >= kTile;   // uniform over the CTA: only the last tile is partial
-            // logits (log2 domain) of 16 columns, minus `m`
-            auto logits16 = [&](const uint32_t (&sx)[16], int q, uint64_t nm2, float (&x)[16]) {
-#pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    float2 b2;
-                    if constexpr (HASMASK) b2 = make_float2(u[q * 16 + i], u[q * 16 + i + 1]);
-                    else b2 = __half22float2(*reinterpret_cast<const __half2*>(&bias2[q * 8 + (i >> 1)]));
-                    unpack2(fma2(pack2(__uint_as_float(sx[i]), __uint_as_float(sx[i + 1])), c2, fma2(pack2(b2.x, b2.y), l2e2, nm2)), x[i], x[i + 1]);
-                    if (!full_tile) {
-                        if (ch * 64 + q * 16 + i >= n_valid) x[i] = -INFINITY;
-                        if (ch * 64 + q * 16 + i + 1 >= n_valid) x[i + 1] = -INFINITY;
-                    }
-                }
-            };
-            // The reference need not be the maximum: the half-row sums (needed anyway) bound P.  The two threads of a row
-            // exchange them - the exchange also says that both have read their S columns, which the P stores overwrite - and
-            // only when one passes kRedoSumRelpos (or in the first tile) is the row's maximum taken, O and l rescaled and P
-            // computed again.  Both warps of a pair see the same sums and take the same branch.
-            uint32_t preg[32];
-            float lsum;
-            bool take_max = j == 0;
-#pragma unroll 1
-            for (;;) {
-                uint32_t sA[16], sB[16];
-                if (take_max) {
-                    float mx = -INFINITY;
-#pragma unroll 1
-                    for (int q = 0; q < 4; q++) {
-                        // (bias2 is indexed by a run-time q here: the four cases are spelled out)
-                        tmem_ld16(tmem_S + lane_base + ch * 64 + q * 16, sA);
-                        tmem_wait_ld();
-                        float x[16];
-                        if (q == 0) logits16(sA, 0, 0ull, x);
-                        else if (q == 1) logits16(sA, 1, 0ull, x);
-                        else if (q == 2) logits16(sA, 2, 0ull, x);
-                        else logits16(sA, 3, 0ull, x);
-#pragma unroll
-                        for (int i = 0; i < 16; i++) mx = fmaxf(mx, x[i]);
-                    }
-                    const float m_new = fmaxf(m_ref, fmaxf(mx, exchange_max(mx)));
-                    if (!ok) break;
-                    const float alpha = (m_ref == -INFINITY) ? 0.0f : ex2(m_ref - m_new);
-                    l_run *= alpha;
-                    if (j > 0) {
-#pragma unroll 1
-                        for (int q4 = 0; q4 < 4; q4++) {
-                            tmem_ld16(tmem_O + lane_base + ch * 64 + q4 * 16, sA);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 16; i++) sA[i] = __float_as_uint(__uint_as_float(sA[i]) * alpha);
-                            tmem_st16(tmem_O + lane_base + ch * 64 + q4 * 16, sA);
-                        }
-                    }
-                    m_ref = m_new;
-                }
-                const float m_use = (m_ref == -INFINITY) ? kNoReference : m_ref;
-                const uint64_t nm2 = pack2(-m_use, -m_use);
-                uint64_t ls[2] = {0ull, 0ull};
-                auto chunk = [&](const uint32_t (&sx)[16], int q) {
-                    float x[16];
-                    logits16(sx, q, nm2, x);
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        const float p0 = ex2(x[i]), p1 = ex2(x[i + 1]);
-                        ls[(i >> 1) & 1] = add2(ls[(i >> 1) & 1], pack2(p0, p1));
-                        preg[q * 8 + (i >> 1)] = cvt_f16x2(p0, p1);
-                    }
-                };
-                const uint32_t s_cols = tmem_S + lane_base + ch * 64;
-                tmem_ld16(s_cols, sA);
-                tmem_ld16(s_cols + 16, sB);
-                tmem_wait_ld();
-                chunk(sA, 0);
-                tmem_ld16(s_cols + 32, sA);
-                chunk(sB, 1);
-                tmem_wait_ld();
-                tmem_ld16(s_cols + 48, sB);
-                chunk(sA, 2);
-                tmem_wait_ld();
-                chunk(sB, 3);
-                float l0, l1;
-                unpack2(add2(ls[0], ls[1]), l0, l1);
-                lsum = l0 + l1;
-                const float other = exchange(lsum);
-                if (!ok || take_max || !__any_sync(0xffffffffu, fmaxf(lsum, other) > kRedoSumRelpos)) break;
-                take_max = true;
-            }
-            if (!ok) break;
-            l_run += lsum;
-            tmem_st32(tmem_P + lane_base + ch * 32, preg);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_p_ready);
-        }
-        if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
-        if (ok) {
-            tc_fence_after();
-            const float l_tot = l_run + exchange(l_run);   // a failed wait has set the abort flag: the host reports it
-            const float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-            float* out = a.dst + (((int64_t)b * a.Tq + iq) * a.dst_heads + h) * HD + ch * 64;
-            const bool wide = (reinterpret_cast<uintptr_t>(a.dst) & 31) == 0;
-#pragma unroll
-            for (int q4 = 0; q4 < 2; q4++) {
-                uint32_t oreg[32];
-                tmem_ld32(tmem_O + lane_base + ch * 64 + q4 * 32, oreg);
-                tmem_wait_ld();
-                if (iq >= tq_b) {   // padding row of a batched launch: literal zeros
-#pragma unroll
-                    for (int i = 0; i < 32; i++) oreg[i] = 0u;
-                }
-                if (iq < a.Tq) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) store8(out + q4 * 32 + i, oreg + i, inv, wide);
-                }
-            }
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 9) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
-    }
-}
-
-
 // ---- host side ----------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1666,14 +1109,14 @@ bool encode_o_map(CUtensorMap* m, const FattnArgs& a) {
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// R as a rank-4 F16 tensor [hd, 2T-1, H, 1|B]; box = 64 columns x 128 rows.
-bool encode_r_map(CUtensorMap* m, const FattnArgs& a) {
+// R as a rank-4 F16 tensor [hd, 2T-1, H, 1|B]; box = 64 columns x `rows` rows.
+bool encode_r_map(CUtensorMap* m, const FattnArgs& a, int rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const int64_t nb3 = a.r_ne3 > 1 ? a.r.nb3 : a.r.nb2 * a.H;
     const cuuint64_t dims[4] = {(cuuint64_t)a.hd, (cuuint64_t)(2 * a.Tq - 1), (cuuint64_t)a.H, (cuuint64_t)a.r_ne3};
     const cuuint64_t strides[3] = {(cuuint64_t)a.r.nb1, (cuuint64_t)a.r.nb2, (cuuint64_t)nb3};
-    const cuuint32_t box[4] = {64, (cuuint32_t)kTile, 1, 1};
+    const cuuint32_t box[4] = {64, (cuuint32_t)rows, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<uint8_t*>(a.r.p), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1705,20 +1148,24 @@ cudaError_t launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStrea
     return launch_pdl_cluster(kern, grid, 1, threads, smem, st, args...);
 }
 
+#include "fattn_tc5_relpos.cuh"
+
 int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errlen) {
     CUtensorMap tmK, tmV, tmR;
     if (!encode_kv_map(&tmK, a.k, a.hd, a.Lk, a.Hkv, a.B / a.bq) || !encode_kv_map(&tmV, a.v, a.hd, a.Lk, a.Hkv, a.B / a.bq) ||
-        !encode_r_map(&tmR, a)) {
+        !encode_r_map(&tmR, a, kRelBlock)) {
         snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V/R");
         return B200_E_CUDA;
     }
-    const size_t smem = 1024 + (size_t)6 * 2 * kPanelBytes + (size_t)2 * kTile * kBncStride + 136 + 8 + 2 * 128 * sizeof(float) + 16;
+    const __half d = __float2half_rn(1.0f / a.scale);   // in range: tc5_supported
+    const float inv_d = 1.0f / __half2float(d);
+    const uint32_t d16 = __half_as_ushort(d);
     cudaError_t e;
     dim3 grid((a.Tq + kTile - 1) / kTile, a.H, a.B);
     static bool set[2][64] = {};
     auto go = [&](auto kern, bool (&smem_set)[64]) {
-        e = set_smem_once(kern, smem, smem_set);
-        if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsRelpos, smem, st, a, tmK, tmV, tmR);
+        e = set_smem_once(kern, kRelSmem, smem_set);
+        if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsRelpos, kRelSmem, st, a, inv_d, d16, tmK, tmV, tmR);
     };
     if (a.has_mask) go(fattn_prefill_tc5_relpos_kernel<true>, set[0]);
     else go(fattn_prefill_tc5_relpos_kernel<false>, set[1]);
@@ -1862,6 +1309,7 @@ bool tc5_supported(const FattnArgs& a) {
     if (a.relpos) {
         // fused bias: head_dim 128, F16 R with TMA-legal strides, no causal mask, bias rounded to F16
         if (a.hd != 128 || a.causal || a.relpos_f32) return false;
+        if (a.scale < 0x1p-14f || a.scale > 0x1p13f) return false;   // 1 / scale is an F16 number in the kernel
         if (a.r.type != B200_TYPE_F16 || !a.r.vec16 || a.r.nb1 <= 0 || a.r.nb2 <= 0) return false;
     }
     const int64_t lim = (int64_t)1 << 40;

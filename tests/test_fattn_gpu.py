@@ -692,6 +692,48 @@ def test_cfg5_relpos_with_explicit_masks_on_the_tensor_core_path(b200, orc, T):
     assert b200.lib().b200_device_status() == 0
 
 
+@pytest.mark.parametrize("T", [1, 2, 63, 64, 65, 127, 128, 129, 191, 193, 256, 257, 385, 640])
+@pytest.mark.parametrize("spread", [1.0, 4.0])
+def test_relpos_edges_of_tiles_and_growing_scores(b200, orc, T, spread):
+    """Sizes around the kernel's 64-column blocks and 128-key tiles; keys scaled by 4 make scores outgrow the reference of the
+    running softmax in later tiles (the bias, whose F16 rounding is the kernel's own, stays as it is)."""
+    rng = np.random.default_rng(461)
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    k *= np.float32(spread)
+    ref = orc.flash_attn_ext(q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, ref, f"rel-pos T={T} spread={spread}")
+    assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("T", [136, 140, 142, 141, 264, 267])
+def test_relpos_mask_rows_of_every_alignment(b200, orc, T):
+    """Mask rows on 16-, 8-, 4- and 2-byte boundaries, with a partial last tile."""
+    rng = np.random.default_rng(462)
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    qi, ki = np.arange(T)[:, None], np.arange(T)[None, :]
+    mask = (np.where(np.abs(qi - ki) <= 40, 0.0, -np.inf) + rng.standard_normal((T, T)) * 0.5).astype(np.float16)[None, None]
+    ref = orc.flash_attn_ext(q_u, k, v, mask, scale=128 ** -0.5, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, mask, scale=128 ** -0.5, q_v=q_v, r=r)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, ref, f"rel-pos with a mask, T={T}")
+    assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -16, 0.04, 0.125, 1.0, 2.0 ** 14])
+def test_relpos_scales(b200, orc, scale):
+    """Scales whose inverse is an F16 number, is not one, or is none within F16's range (the general kernel takes those)."""
+    rng = np.random.default_rng(463)
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, 150, H=2, d_model=256)
+    f = np.float32(min(1.0, 128 ** -0.5 / scale))   # scores of ordinary size also under a large scale
+    q_u, q_v = (q_u * f).astype(np.float16).astype(np.float32), (q_v * f).astype(np.float16).astype(np.float32)
+    ref = orc.flash_attn_ext(q_u, k, v, scale=scale, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, scale=scale, q_v=q_v, r=r)
+    assert (b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5) == (2.0 ** -14 <= scale <= 2.0 ** 13)
+    assert_close(got, ref, f"rel-pos scale={scale}")
+
+
 def test_relpos_table_built_on_the_device_and_cached(b200, orc):
     """R = attn_pos_w . pos_enc (src/core/fastconformer.h:118-130, :843, :851) built by the library for a (layer, T)
     equals the oracle's make_pos_enc @ W to within one F16 rounding, attention with the library's table meets the
