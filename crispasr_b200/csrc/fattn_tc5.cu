@@ -557,12 +557,11 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     uint8_t* misc = smem_gen + (1 + 2 * NSTG) * TILE_BYTES + 32 * NSTG + 64;
     // q_tma: 0 = the softmax warps load and convert the Q tile; 1 = F16 rows by one tensor copy into the operand tile;
     // 2 = F32 rows by tensor copies into stages that are not needed yet, converted from there by the softmax warps.
-    // The raw tile (64 KB) takes the K and the V stage, so the first K tile
-    // waits for the conversion too - still ahead of a register pass, whose global loads a CTA next to one in its key
-    // loop issues at a few tens of clocks per instruction (T = 407 GQA prefill with an F32 Q: 4807 -> 5034 streams/s).
+    // The raw tile (64 KB) takes the V stage (columns 0 to 63) and the operand tile itself (64 to 127): a softmax thread holds its whole
+    // row in registers before any of them writes the operand tile, and the first K tile is on its way meanwhile.
     constexpr bool q_raw = QMODE == 2;
     static_assert(!q_raw || (HD == 128 && NSTG == 1), "the raw tile takes the stages of head_dim 128");
-    constexpr int RAW_OFF = TILE_BYTES;   // the K stage onwards
+    constexpr int RAW_PANEL_OFF[4] = {2 * TILE_BYTES, 2 * TILE_BYTES + kPanelBytes, 0, kPanelBytes};   // 32 columns each
     // head_dim 64 leaves 64 spare TMEM columns: P gets its own, so S of the next tile can be issued before P.V
     constexpr bool SEP_P = (HD == 64);
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
@@ -643,7 +642,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             mbar_arrive_expect_tx(bar_q_full, (HD / 32) * kPanelBytes);
 #pragma unroll
             for (int p = 0; p < HD / 32; p++)
-                tma_load_4d(sQ + RAW_OFF + p * kPanelBytes, &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
+                tma_load_4d(sQ + RAW_PANEL_OFF[p], &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
         } else if (q_tma) {
             // F16 query rows go straight into the operand layout: one copy instead of a pass through the softmax warps'
             // registers, which a CTA sharing its SM with another one in its key loop executes at a few tens of clocks
@@ -657,12 +656,11 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
         // the first NSTG tiles need no empty-slot wait: start their copies before the CTA-wide set-up barrier
         for (int j = 0; j < NSTG && j < n_tiles; j++) {
-            if (q_raw) continue;   // the K stage holds raw Q rows for now
             mbar_arrive_expect_tx(bar_k_full + 8 * j, TILE_BYTES);
 #pragma unroll
             for (int p = 0; p < PANELS; p++)
                 tma_load_4d(sK + j * TILE_BYTES + p * kPanelBytes, &tmK, bar_k_full + 8 * j, p * 64, j * kTile, hk, bk);
-            if (q_raw) continue;   // the V stages hold the raw Q tile for now
+            if (q_raw) continue;   // the V stage holds raw Q rows for now
             mbar_arrive_expect_tx(bar_v_full + 8 * j, TILE_BYTES);
 #pragma unroll
             for (int p = 0; p < PANELS; p++)
@@ -696,19 +694,23 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         if (q_raw && warp < 4) {
             // raw F32 row r (panels of 128-byte swizzled rows) -> F16 row r of the operand tile: HD / 4 loads, HD / 2
             // conversions, HD / 8 stores per thread, all from shared memory
-            if (mbar_wait(bar_q_full, 0, s_abort)) {
-                const int r = tid;
-                const uint8_t* raw = smem_gen + RAW_OFF + r * 128;
-                uint8_t* qrow = smem_gen + r * 128;
+            const bool there = mbar_wait(bar_q_full, 0, s_abort);
+            const int r = tid;
+            uint4 row[HD / 8];
 #pragma unroll
-                for (int c = 0; c < HD / 8; c++) {   // F16 chunk c = columns 8c .. 8c+7 = F32 chunks 2c, 2c+1 of raw panel c / 4
-                    const int f0 = (2 * c) & 7;
-                    const float4 x0 = *reinterpret_cast<const float4*>(raw + (c >> 2) * kPanelBytes + ((f0 ^ (r & 7)) << 4));
-                    const float4 x1 = *reinterpret_cast<const float4*>(raw + (c >> 2) * kPanelBytes + (((f0 + 1) ^ (r & 7)) << 4));
-                    *reinterpret_cast<uint4*>(qrow + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) =
-                        make_uint4(pack_half2(x0.x, x0.y), pack_half2(x0.z, x0.w), pack_half2(x1.x, x1.y), pack_half2(x1.z, x1.w));
-                }
-                fence_proxy_async();   // the operand tile is read, and the V stages are overwritten, through the async proxy
+            for (int c = 0; c < HD / 8; c++) {   // F16 chunk c = columns 8c .. 8c+7 = F32 chunks 2c, 2c+1 of raw panel c / 4
+                const int f0 = (2 * c) & 7;
+                const uint8_t* raw = smem_gen + RAW_PANEL_OFF[c >> 2] + r * 128;
+                const float4 x0 = *reinterpret_cast<const float4*>(raw + ((f0 ^ (r & 7)) << 4));
+                const float4 x1 = *reinterpret_cast<const float4*>(raw + (((f0 + 1) ^ (r & 7)) << 4));
+                row[c] = make_uint4(pack_half2(x0.x, x0.y), pack_half2(x0.z, x0.w), pack_half2(x1.x, x1.y), pack_half2(x1.z, x1.w));
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");   // the operand tile is written over raw columns 64 to 127 of all rows
+#pragma unroll
+            for (int c = 0; c < HD / 8; c++)
+                *reinterpret_cast<uint4*>(smem_gen + r * 128 + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) = row[c];
+            if (there) {
+                fence_proxy_async();   // the operand tile is read, and the V stage is overwritten, through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_q_conv);
             }
@@ -719,15 +721,10 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         // ================= TMA producer =================
         if (lane == 0) {
             bool ok = true;
-            int issued_k = q_raw ? 0 : min(NSTG, n_tiles), issued_v = q_raw ? 0 : min(NSTG, n_tiles);
+            int issued_k = min(NSTG, n_tiles), issued_v = q_raw ? 0 : min(NSTG, n_tiles);
             if (q_raw) {
                 ok = mbar_wait(bar_q_conv, 0, s_abort);
                 for (int j = 0; j < NSTG && j < n_tiles && ok; j++) {
-                    mbar_arrive_expect_tx(bar_k_full + 8 * j, TILE_BYTES);
-#pragma unroll
-                    for (int p = 0; p < PANELS; p++)
-                        tma_load_4d(sK + j * TILE_BYTES + p * kPanelBytes, &tmK, bar_k_full + 8 * j, p * 64, j * kTile, hk, bk);
-                    issued_k = j + 1;
                     mbar_arrive_expect_tx(bar_v_full + 8 * j, TILE_BYTES);
 #pragma unroll
                     for (int p = 0; p < PANELS; p++)
