@@ -204,13 +204,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-__device__ __forceinline__ void tmem_st64(uint32_t taddr, const uint32_t (&r)[64]) {
-    uint32_t lo[32], hi[32];
-#pragma unroll
-    for (int i = 0; i < 32; i++) lo[i] = r[i], hi[i] = r[32 + i];
-    tmem_st32(taddr, lo);
-    tmem_st32(taddr + 32, hi);
-}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -1174,6 +1167,7 @@ int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errl
 }
 
 #include "fattn_tc5_h64.cuh"
+#include "fattn_tc5_h128.cuh"
 
 // One instantiation per kernel: its own "shared-memory attribute raised" flags per device.
 template <auto Kern, typename... Args>
@@ -1275,6 +1269,21 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     // launch_inst is instantiated per kernel (the kernels share one function-pointer type, so a generic lambda would
     // share its "attribute set" flags between them)
     auto args = [&](auto launch) { e = launch(grid, smem, st, a, tmK, tmV, tmQ, tmO); };
+    if constexpr (HD == 128) {
+        // more than two full waves (of two CTAs per SM): CTAs that go on to the next tile themselves
+        if (!a.has_mask && q_tma && o_tma && (long)grid.x * grid.y * grid.z > 4 * 148) {
+            const size_t smem_h128 = 1024 + (size_t)3 * TILE_BYTES + 112;
+            static bool set[2][64] = {};
+            auto go = [&](auto kern, bool (&smem_set)[64]) {
+                cudaError_t e = set_smem_once(kern, smem_h128, smem_set);
+                return e == cudaSuccess ? launch_pdl(kern, grid, kThreadsTc5, smem_h128, st, a, tmK, tmV, tmQ, tmO) : e;
+            };
+            e = q_tma == 2 ? go(fattn_prefill_tc5_h128_kernel<true>, set[0]) : go(fattn_prefill_tc5_h128_kernel<false>, set[1]);
+            if (e == cudaSuccess) return B200_OK;
+            snprintf(errbuf, errlen, "tcgen05 prefill launch: %s", cudaGetErrorString(e));
+            return B200_E_CUDA;
+        }
+    }
     constexpr int QRAW = RAW_INST ? 2 : 0;
 #define B200_GO(...) args(launch_inst<fattn_prefill_tc5_kernel<__VA_ARGS__>, FattnArgs, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap>)
     if (a.has_mask) {

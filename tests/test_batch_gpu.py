@@ -220,6 +220,36 @@ def test_batched_units_of_different_lengths_equal_per_unit_launches(b200, orc, f
     assert L.b200_device_status() == 0
 
 
+@pytest.mark.parametrize("qdtype", [np.float32, np.float16])
+@pytest.mark.parametrize("causal", [True, False])
+def test_head_dim_128_launch_of_more_than_two_waves(b200, orc, qdtype, causal):
+    """A launch whose CTAs go on to further tiles (more than 592 of them): units of 0 to 70 new tokens, tiles without keys among
+    them, bit for bit what launches of a few units each give, and some of them against the oracle."""
+    rng = np.random.default_rng(51)
+    B, H, Hkv, Tq, Lk = 40, 16, 8, 70, 300
+    qlens = [int(x) for x in rng.integers(0, Tq + 1, B)]
+    klens = [min(Lk, n + int(x)) for n, x in zip(qlens, rng.integers(0, 231, B))]
+    qlens[3], klens[5], klens[6], qlens[6] = 0, 0, Lk, Tq
+    qlens[5] = 0 if causal else qlens[5]
+    q = randn_f16(rng, (B, H, Tq, 128)).astype(qdtype)
+    k, v = randn_f16(rng, (B, Hkv, Lk, 128)), randn_f16(rng, (B, Hkv, Lk, 128))
+    kw = dict(scale=128 ** -0.5, causal=True) if causal else dict(scale=128 ** -0.5)
+    got = gpu_op(b200, q, k, v, q_len=qlens, kv_len=klens, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert (B * Hkv * -(-Tq * (H // Hkv) // 128)) > 592
+    for b in range(0, B, 4):
+        few = slice(b, b + 4)
+        alone = gpu_op(b200, q[few], k[few], v[few], q_len=qlens[few], kv_len=klens[few], **kw)
+        assert np.array_equal(got[few], alone), f"units {b} to {b + 3}"
+    for b in (3, 5, 6, 17):
+        nq, nk = qlens[b], klens[b]
+        assert not got[b, nq:].any()
+        if nq and nk:
+            okw = dict(kw, n_past=nk - nq) if causal else kw
+            assert_close(got[b:b + 1, :nq], orc.flash_attn_ext(q[b:b + 1, :, :nq], k[b:b + 1, :, :nk], v[b:b + 1, :, :nk], **okw), f"unit {b}")
+    assert b200.lib().b200_device_status() == 0
+
+
 def test_slot_table_drives_a_decode_batch(b200, orc):
     """b200_batch over a Q8_0 cache with 6 stream slots: streams join with different cache lengths, every step
     appends one row per resident stream and attends with the tables b200_batch_tables uploads; a stream that
