@@ -107,6 +107,15 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const AppendArgs a) {
                 x[u][0] = load4<V16>(p), x[u][1] = load4<V16>(p + 16);
             }
         }
+        // The rows of the next turn into L2 meanwhile: 16 x 407 rows of 8 heads into F16 15.5 -> 14.5 us, 8 x 1500 27.1 -> 26.0.  (Into Q8_0, whose
+        // arithmetic covers the loads, 1 %, and the attention behind 8 x 407 rows then starts 0.3 us later.)
+        if (U > 1 && !Q8) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int row = row0 + (U + u) * step + sub;
+                if (row < row_hi && (c & 31) == 0) prefetch_l2(src + (int64_t)row * a.snb1[which]);
+            }
+        }
 #pragma unroll
         for (int u = 0; u < U; u++) {
             uint8_t* row_out = dst + (int64_t)(row0 + u * step + sub) * a.dnb1;
