@@ -31,7 +31,7 @@
 // the bias one tile ahead of the softmax.
 //
 // 2 recordings of 7500 frames 874 -> 640 us in a burst (4.0 -> 3.0 k clk per 128 x 128 scores), 942 -> 728 in a long run at the 1000 W limit; one of
-// 1000 frames 25.0 -> 19.2, 8 utterances of up to 138 13.1 -> 12.4, a mask over 3000 frames 188 -> 148.
+// 1000 frames 25.0 -> 19.2, 8 utterances of up to 138 13.1 -> 12.4, a mask over 3000 frames 188 -> 122.
 // What bounds it: per tile the softmax warps take 2.5 k clk (exponentials 1.5 k, where the exponential unit needs 1.0 k; the meeting of the
 // two warps of a row, the P store and the wait for the next scores the rest), and the columns of a score tile are free again 3 k clk
 // after its P is there (P.V, S, bias and three hand-offs); the products of a tile keep the tensor pipe busy for 2.0 to 2.5 k.  Instruction
@@ -133,32 +133,54 @@ __device__ __forceinline__ uint32_t cvt_f16x2_sat(float lo, float hi) {
     return y;
 }
 
-// 64 mask values of a row as 32 pairs; those at or beyond `avail` (the end of the mask row) read as 0 and are never
-// touched.  `align` is what the start and the strides of the mask are multiples of: one answer for all rows, so that the warp stays
-// together, which the tensor memory instructions behind these loads need.  (load_global: an assembly load that is not volatile may be
-// executed ahead of the test of its alignment.)
-__device__ __forceinline__ void load_mask_row(uint32_t (&mv)[32], const uint8_t* mptr, int avail, int align) {
+// 64 mask values of a row as 32 pairs; those at or beyond `avail` (the end of the mask row) read as 0 and are never touched.  `align` is
+// what the start and the strides of the mask are multiples of: one answer for all rows, so that the warp stays together, which the tensor
+// memory instructions behind these loads need.  (load_global: an assembly load that is not volatile may be executed ahead of the test of
+// its alignment.)  A warp load of 32 rows occupies L1 32 times whatever its width, and what shared memory leaves of L1 does not hold
+// the tile's rows: rows on no 16-byte boundary are read as the nine 16-byte words around them and shifted into place, unless some of those
+// reach beyond the mask [lo, hi) (4 x 1501 frames 307 -> 134 us, 11 utterances of up to 246 frames 47.8 -> 37.3, by 4- and 2-byte loads before; the
+// aligned form as a block of its own 2 x 3000 frames 245 -> 200).
+__device__ __forceinline__ void load_mask_row(uint32_t (&mv)[32], const uint8_t* mptr, int avail, int align, const uint8_t* lo, const uint8_t* hi) {
+    const uint32_t skew = (uint32_t)reinterpret_cast<uintptr_t>(mptr) & 15u;
+    if (align >= 16 && avail >= 64) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const uint4 v = load_global(reinterpret_cast<const uint4*>(mptr) + q);
+            mv[4 * q] = v.x, mv[4 * q + 1] = v.y, mv[4 * q + 2] = v.z, mv[4 * q + 3] = v.w;
+        }
+        return;
+    }
+    if (avail >= 64 && __all_sync(0xffffffffu, mptr - skew >= lo && mptr - skew + 144 <= hi)) {
+        uint32_t w[36];
+#pragma unroll
+        for (int q = 0; q < 9; q++) {
+            const uint4 v = load_global(reinterpret_cast<const uint4*>(mptr - skew) + q);
+            w[4 * q] = v.x, w[4 * q + 1] = v.y, w[4 * q + 2] = v.z, w[4 * q + 3] = v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < 34; i++) w[i] = skew & 8u ? w[i + 2] : w[i];
+#pragma unroll
+        for (int i = 0; i < 33; i++) w[i] = skew & 4u ? w[i + 1] : w[i];
+#pragma unroll
+        for (int i = 0; i < 32; i++) mv[i] = __funnelshift_r(w[i], w[i + 1], (skew & 2u) * 8u);
+        return;
+    }
 #pragma unroll
     for (int g = 0; g < 8; g++) {   // 16 bytes each
         const uint8_t* p = mptr + g * 16;
         uint32_t* m = mv + g * 4;
-        if (avail >= g * 8 + 8 && align >= 8) {
-            if (align >= 16) {
-                const uint4 v = load_global(reinterpret_cast<const uint4*>(p));
-                m[0] = v.x, m[1] = v.y, m[2] = v.z, m[3] = v.w;
-            } else {
-                const uint2 v0 = load_global(reinterpret_cast<const uint2*>(p)), v1 = load_global(reinterpret_cast<const uint2*>(p + 8));
-                m[0] = v0.x, m[1] = v0.y, m[2] = v1.x, m[3] = v1.y;
-            }
+        if (avail >= g * 8 + 8 && align >= 16) {
+            const uint4 v = load_global(reinterpret_cast<const uint4*>(p));
+            m[0] = v.x, m[1] = v.y, m[2] = v.z, m[3] = v.w;
         } else if (avail >= g * 8 + 8 && align >= 4) {
 #pragma unroll
             for (int i = 0; i < 4; i++) m[i] = load_global(reinterpret_cast<const uint32_t*>(p + i * 4));
         } else {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const uint32_t lo = g * 8 + 2 * i < avail ? load_global(reinterpret_cast<const uint16_t*>(p + i * 4)) : (uint16_t)0;
-                const uint32_t hi = g * 8 + 2 * i + 1 < avail ? load_global(reinterpret_cast<const uint16_t*>(p + i * 4 + 2)) : (uint16_t)0;
-                m[i] = lo | (hi << 16);
+                const uint32_t l = g * 8 + 2 * i < avail ? load_global(reinterpret_cast<const uint16_t*>(p + i * 4)) : (uint16_t)0;
+                const uint32_t h = g * 8 + 2 * i + 1 < avail ? load_global(reinterpret_cast<const uint16_t*>(p + i * 4 + 2)) : (uint16_t)0;
+                m[i] = l | (h << 16);
             }
         }
     }
@@ -522,7 +544,8 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint
                                             (int64_t)(h % a.mask_ne2) * a.mask.nb2 + (int64_t)(b % a.mask_ne3) * a.mask.nb3 + ch * 128
                                       : nullptr;
         const uint32_t mask_bits = (uint32_t)(reinterpret_cast<uintptr_t>(a.mask.p) | a.mask.nb1 | a.mask.nb2 | a.mask.nb3);
-        const int mask_align = (mask_bits & 15) == 0 ? 16 : ((mask_bits & 7) == 0 ? 8 : ((mask_bits & 3) == 0 ? 4 : 2));
+        const int mask_align = (mask_bits & 15) == 0 ? 16 : ((mask_bits & 3) == 0 ? 4 : 2);
+        const uint8_t* mask_end = a.mask.p + (int64_t)(a.mask_ne3 - 1) * a.mask.nb3 + (int64_t)(a.mask_ne2 - 1) * a.mask.nb2 + (int64_t)(a.Tq - 1) * a.mask.nb1 + (int64_t)a.Lk * 2;
         // The two warps of 32 rows meet at a hardware barrier (a fraction of an mbarrier's latency).  Both take part in every meeting, also when
         // a wait of theirs ran out: kFailed tells the other one, and both leave.
         constexpr uint32_t kFailed = 2u;
@@ -550,7 +573,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint
             bool take_max = j == 0, waited = false;
 #pragma unroll 1
             for (;;) {
-                if constexpr (HASMASK) load_mask_row(pm, mrow + (int64_t)j * kTile * 2, a.Lk - j * kTile - ch * 64, mask_align);
+                if constexpr (HASMASK) load_mask_row(pm, mrow + (int64_t)j * kTile * 2, a.Lk - j * kTile - ch * 64, mask_align, a.mask.p, mask_end);
                 if (!waited) {
                     ok = warp_all(s_there || mbar_wait(bar_s_full + 8 * (j & 1), (j >> 1) & 1, s_abort));
                     tc_fence_after();
