@@ -679,9 +679,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // The next launch may become resident as this one's CTAs leave: F16 rows, 1 x 100 tokens 6.8 -> 6.3 us per launch, 1 x 407 11.9 -> 11.4, 16 x 100
-    // 15.5 -> 15.0.  Not where the next one is likely a conversion again, whose CTAs take the room of this one's.
-    if (!a.behind_cast) let_dependents_launch();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *s_tmem_base, 0);
     const uint32_t tmem_S = tmem_base;            // cols [0,128)
     const uint32_t tmem_P = SEP_P ? tmem_base + kTile + HD : tmem_base;  // f16x2: cols [192,256) (hd 64) or aliasing S [0,64)
