@@ -1147,15 +1147,12 @@ int launch_relpos(const FattnArgs& a, cudaStream_t st, char* errbuf, size_t errl
         snprintf(errbuf, errlen, "cuTensorMapEncodeTiled failed for K/V/R");
         return B200_E_CUDA;
     }
-    const __half d = __float2half_rn(1.0f / a.scale);   // in range: tc5_supported
-    const float inv_d = 1.0f / __half2float(d);
-    const uint32_t d16 = __half_as_ushort(d);
     cudaError_t e;
     dim3 grid((a.Tq + kTile - 1) / kTile, a.H, a.B);
     static bool set[2][64] = {};
     auto go = [&](auto kern, bool (&smem_set)[64]) {
         e = set_smem_once(kern, kRelSmem, smem_set);
-        if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsRelpos, kRelSmem, st, a, inv_d, d16, tmK, tmV, tmR);
+        if (e == cudaSuccess) e = launch_pdl(kern, grid, kThreadsRelpos, kRelSmem, st, a, 1.0f / a.scale, tmK, tmV, tmR);
     };
     if (a.has_mask) go(fattn_prefill_tc5_relpos_kernel<true>, set[0]);
     else go(fattn_prefill_tc5_relpos_kernel<false>, set[1]);
@@ -1315,7 +1312,7 @@ bool tc5_supported(const FattnArgs& a) {
     if (a.relpos) {
         // fused bias: head_dim 128, F16 R with TMA-legal strides, no causal mask, bias rounded to F16
         if (a.hd != 128 || a.causal || a.relpos_f32) return false;
-        if (a.scale < 0x1p-14f || a.scale > 0x1p13f) return false;   // 1 / scale is an F16 number in the kernel
+        if (a.scale < 0x1p-14f || a.scale > 0x1p13f) return false;   // (bias / scale goes into the score columns: far inside F32's range)
         if (a.r.type != B200_TYPE_F16 || !a.r.vec16 || a.r.nb1 <= 0 || a.r.nb2 <= 0) return false;
     }
     const int64_t lim = (int64_t)1 << 40;

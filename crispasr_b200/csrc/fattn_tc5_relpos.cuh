@@ -3,26 +3,24 @@
 //
 // The bias of (query i, key J) is X[i][J - i + 127], X = Q_v . R_band^T with R_band row 0 = R row (Tq - 1) - q0 - 127: one more
 // matrix product, whose columns have to be shifted by a different amount in every row.  A tcgen05.ld reads the same columns
-// for all lanes, so the shift goes through shared memory, and the tensor cores add the result to the scores:
+// for all lanes, so the shift goes through shared memory:
 //
-//   four warps take the blocks of 64 X columns out of tensor memory as they are produced, each element once, round them to F16 and
-//   store them at their key's place in a ring [128 query rows][4 panels of 64 keys] in shared memory that has the layout of
-//   an A operand.  S += ring . (d * identity): products with a 16 x 16 identity, 16 keys each.  The softmax warps then see
-//   finished scores, and their loop is that of a call without a bias.
+//   four warps take the blocks of 64 X columns out of tensor memory as they are produced, each element once, round scale * x to F16 (where
+//   the reference rounds, src/core/fastconformer.h:918) and store it at its key's place in a ring [128 query rows][4 panels of 64 keys].
+//   A tile of 128 keys that is complete goes back, divided by scale, into the columns of its score tile, and the score product
+//   adds to them.  The softmax warps then see finished scores, and their loop is that of a call without a bias.
+//
+// A row of the ring is written and read by one thread.  An infinite bias or a NaN stays with its own key, and what the table holds for keys
+// at or beyond kv_len goes no further than the score columns that the softmax warps overwrite.
 //
 // Tile row r holds query 4 * (r % 32) + r / 32 of the tile: the rows of a warp differ by multiples of four keys, and a warp that
 // starts its TMEM columns at 3 - (r / 32) has every group of four values on an 8-byte boundary of its row, whatever the lane.
 // (With neighbouring queries in neighbouring lanes every row went through a bounce buffer and back, shifted by 2 bytes where needed.)
-// d is 1 / scale as an F16 number, and what is rounded to F16 is x / d: the rounding is as fine as that of scale * x, which is what
-// the reference rounds (src/core/fastconformer.h:918), and not the same in the last place.  Relative error (2-norm) against 64 bits
-// without any rounding, before and now: 8 ragged utterances of 138 frames 2.261e-4, 2.263e-4; 1500 frames 2.856e-4, 2.852e-4; 2500
-// frames 2.947e-4, 2.953e-4.  (1 / scale as the sum of two F16 numbers has the reference's own roundings; a product with the identity
-// costs 64 clocks whatever its width, and 2 x 7500 frames took 805 instead of 680 us.  Added by the softmax warps: 889.)
 //
 //   warps 0-7   softmax, epilogue: thread (r, ch) owns columns [64 ch, + 64) of tile row r (TMEM lane r)
 //   warps 8-11  bias, as above; Q_v into tensor memory
 //   warp  12    copies of K and V
-//   warp  13    TMEM allocation; S products and the bias
+//   warp  13    TMEM allocation; S products
 //   warp  14    copies of R, X products
 //   warp  15    P.V products
 //   TMEM       [0,128) [128,256) S of even and odd tiles, P as f16x2 over the first 64 of its columns; [256,384) O; [384,448) X;
@@ -30,22 +28,26 @@
 // Key tiles of 128: tile t takes X blocks 2t .. 2t + 3 and its bias is complete when the last of them is stored.  Scores run two tiles,
 // the bias one tile ahead of the softmax.
 //
-// 2 recordings of 7500 frames 874 -> 640 us in a burst (4.0 -> 3.0 k clk per 128 x 128 scores), 942 -> 728 in a long run at the 1000 W limit; one of
-// 1000 frames 25.0 -> 19.2, 8 utterances of up to 138 13.1 -> 12.4, a mask over 3000 frames 188 -> 122.
-// What bounds it: per tile the softmax warps take 2.5 k clk (exponentials 1.5 k, where the exponential unit needs 1.0 k; the meeting of the
-// two warps of a row, the P store and the wait for the next scores the rest), and the columns of a score tile are free again 3 k clk
-// after its P is there (P.V, S, bias and three hand-offs); the products of a tile keep the tensor pipe busy for 2.0 to 2.5 k.  Instruction
-// fetch counts: five kinds of warps that each run straight-line code once per tile (hit rate of the instruction cache 79 %, 86 % with the
-// partial tile's -inf and the first tile's maximum taken out of the hot loop).  So slower variants were, in us for 2 x 7500: one warp for S
-// and P.V 711, X in two buffers with R in two slots 906, the first four X blocks back to back 690 to 710, one lane per warp that polls the
-// barriers 1219, four softmax warps with whole rows 785.
+// Relative error (2-norm) against 64 bits with the operator's own rounding of the bias: 8 ragged utterances of 138 frames 1.64e-4, 1500 frames
+// 2.04e-4, 2500 frames 2.05e-4, 7500 frames 2.06e-4, the figures of a kernel that adds the rounded bias in its softmax warps.  The bias as an
+// operand of the tensor cores, times 1 / scale as an F16 number in an identity matrix, is not that value: rounded as x * scale / d, d being that
+// number, 2.5e-4, 3.2e-4, 3.3e-4, 3.5e-4, growing with the bias, and a NaN reaches the other keys of its product (2 x 7500 frames 645 us).
+//
+// 2 recordings of 7500 frames, bias added by the softmax warps / here: 875 -> 745 us in a burst, 945 -> 835 in a long run at the 1000 W limit; one
+// of 1000 frames 25.0 -> 21.6, 8 utterances of up to 138 13.5 -> 12.8, a mask over 3000 frames 189 -> 135.
+// What bounds it: 128 x 128 scores take 3.3 k clk, the softmax warps 2.5 k of them (exponentials 1.5 k, where the exponential unit needs 1.0 k;
+// the meeting of the two warps of a row, the P store and the wait for the next scores the rest).  The columns of a score tile are free again 3 k
+// clk after its P is there (P.V, bias, S and three hand-offs), and a block of X, of which a tile takes two, comes 1.5 k clk after the one
+// before it has left its columns.  So the bias of a tile waits for P.V with the next block of X already taken out and its successor on the
+// way (waiting ahead of that block 790, and with a wait of its own for the upper columns, which P leaves earlier, 837).
+// Instruction fetch counts: five kinds of warps that each run straight-line code once per tile.
 constexpr int kThreadsRelpos = 512;
 constexpr int kRelBlock = 64;                          // X columns per step
 constexpr int kRelRSlots = 4;                          // R blocks in flight
 constexpr int kRelRBytes = kRelBlock * 2 * 128;        // 64 rows x 128 halves
 constexpr int kRelTile = 2 * kPanelBytes;              // 128 rows x 128 halves
 constexpr int kRelRingOff = kRelTile, kRelKOff = kRelRingOff + 2 * kRelTile, kRelVOff = kRelKOff + kRelTile, kRelROff = kRelVOff + kRelTile,
-              kRelIdOff = kRelROff + kRelRSlots * kRelRBytes, kRelBarOff = kRelIdOff + 512, kRelMiscOff = kRelBarOff + 24 * 8;
+              kRelBarOff = kRelROff + kRelRSlots * kRelRBytes, kRelMiscOff = kRelBarOff + 24 * 8;
 constexpr size_t kRelSmem = 1024 + (size_t)kRelMiscOff + 16 + 64 + 2 * kTile * sizeof(float);
 static_assert(kRelSmem <= 232448, "shared memory of a CTA");
 
@@ -125,13 +127,6 @@ __device__ __forceinline__ void store8(float* p, const uint32_t* r, float f, boo
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
-// {hi, lo} -> packed f16x2, values beyond the range of F16 at its ends (an infinity would be a NaN in the other columns of the
-// product with the identity); a NaN stays one.
-__device__ __forceinline__ uint32_t cvt_f16x2_sat(float lo, float hi) {
-    uint32_t y;
-    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(y) : "f"(hi), "f"(lo));
-    return y;
-}
 
 // 64 mask values of a row as 32 pairs; those at or beyond `avail` (the end of the mask row) read as 0 and are never touched.  `align` is
 // what the start and the strides of the mask are multiples of: one answer for all rows, so that the warp stays together, which the tensor
@@ -194,22 +189,20 @@ __device__ __forceinline__ bool mbar_wait_all(uint32_t b0, uint32_t p0, uint32_t
 
 template <bool HASMASK>
 __global__ void __launch_bounds__(kThreadsRelpos, 1)
-fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint32_t d16, const __grid_constant__ CUtensorMap tmK,
+fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const __grid_constant__ CUtensorMap tmK,
                                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmR) {
     constexpr int HD = 128;
-    constexpr uint32_t IDESC_S = idesc_f16(kTile, false), IDESC_X = idesc_f16(kRelBlock, false), IDESC_B = idesc_f16(16, false),
-                       IDESC_PV = idesc_f16(HD, true);
+    constexpr uint32_t IDESC_S = idesc_f16(kTile, false), IDESC_X = idesc_f16(kRelBlock, false), IDESC_PV = idesc_f16(HD, true);
 
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_dyn + (smem_base - smem_u32(smem_dyn));
-    const uint32_t sQ = smem_base, sRing = smem_base + kRelRingOff, sK = smem_base + kRelKOff, sV = smem_base + kRelVOff, sR = smem_base + kRelROff,
-                   sId = smem_base + kRelIdOff, sBar = smem_base + kRelBarOff;
+    const uint32_t sQ = smem_base, sK = smem_base + kRelKOff, sV = smem_base + kRelVOff, sR = smem_base + kRelROff,
+                   sBar = smem_base + kRelBarOff;
     const uint32_t bar_k_full = sBar /* [2]: halves of the head dimension */, bar_k_empty = sBar + 16 /* [2] */, bar_v_full = sBar + 32,
                    bar_v_empty = sBar + 40, bar_r_full = sBar + 48 /* [4] */, bar_s_full = sBar + 80 /* [2] */, bar_p_ready = sBar + 96 /* [2] */,
-                   bar_o_done = sBar + 112, bar_x_full = sBar + 120, bar_x_free = sBar + 128, bar_b_full = sBar + 136, bar_b_free = sBar + 144,
-                   bar_qv = sBar + 152, bar_drain = sBar + 160 /* [2] */,
-                   bar_pv = sBar + 176 /* [2]: P.V of even and odd tiles */;
+                   bar_o_done = sBar + 112, bar_x_full = sBar + 120, bar_x_free = sBar + 128, bar_b_full = sBar + 136 /* [2] */,
+                   bar_qv = sBar + 152, bar_drain = sBar + 160 /* [2] */, bar_pv = sBar + 176 /* [2]: P.V of even and odd tiles */;
     uint8_t* misc = smem_gen + kRelMiscOff;
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
     volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
@@ -223,24 +216,16 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint
     if (tid == 14 * 32) {
         for (int i = 0; i < 24; i++) {
             const uint32_t bar = sBar + 8 * i;
-            // one arrival per warp of the softmax or the bias group (P has a barrier for each of the two score tiles: a softmax warp may be a
-            // tile ahead of another one)
-            mbar_init(bar, bar == bar_p_ready || bar == bar_p_ready + 8 ? 8 : (bar == bar_x_free || bar == bar_b_full || bar == bar_qv ? 4 : 1));
+            // one arrival per warp of the softmax or the bias group (P and the bias have a barrier for each of the two score tiles: a warp may be
+            // a tile ahead of another one)
+            const bool four = bar == bar_x_free || bar == bar_b_full || bar == bar_b_full + 8 || bar == bar_qv;
+            mbar_init(bar, bar == bar_p_ready || bar == bar_p_ready + 8 ? 8 : (four ? 4 : 1));
         }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmR)) : "memory");
-    }
-    if (warp == 12) {
-        // d * I of 16 x 16, as four 8 x 8 core matrices (rows of 16 bytes) of which the two on the diagonal are not zero
-#pragma unroll
-        for (int i = lane; i < 128; i += 32) {   // word i: core i / 32, row (i % 32) / 4, elements 2 (i % 4), + 1
-            const int core = i >> 5, row = (i & 31) >> 2, e = (i & 3) * 2;
-            reinterpret_cast<uint32_t*>(smem_gen + kRelIdOff)[i] = (core == 0 || core == 3) && e == (row & ~1) ? (row & 1 ? d16 << 16 : d16) : 0u;
-        }
-        fence_proxy_async();
     }
     // launched with programmatic stream serialisation: nothing is read before the previous kernel has completed
     const uint32_t behind_wait = wait_for_predecessors();
@@ -366,35 +351,23 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint
             }
         }
     } else if (warp == 13) {
-        // ================= scores: Q_u.K^T plus the bias, two tiles ahead =================
-        const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), ring_lo = smem_desc_lo(sRing, 16);
-        const uint64_t id_desc = desc64(smem_desc_lo(sId, 128), (256u >> 4) | (1u << 14));   // no swizzle: core matrices 128 bytes apart along K, 256 along N
+        // ================= scores: Q_u.K^T onto the bias, two tiles ahead =================
+        const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16);
         for (int j = 0; j < n_tiles; j++) {
             const uint32_t s = tmem_S + (j & 1) * kTile;
-            // K[j] is there and P[j - 2].V[j - 2], whose P lies in the columns of S[j], has completed
-            ok = warp_all(mbar_wait_all(bar_k_full, j & 1, bar_k_full + 8, j & 1, j < 2 ? bar_k_full : bar_pv + 8 * (j & 1), j < 2 ? j & 1 : ((j >> 1) - 1) & 1, s_abort));
+            // K[j] is there, and the bias in the columns of S[j] (behind P[j - 2].V[j - 2], whose P lay in them)
+            ok = warp_all(mbar_wait_all(bar_k_full, j & 1, bar_k_full + 8, j & 1, bar_b_full + 8 * (j & 1), (j >> 1) & 1, s_abort));
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ks++) {
                     const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(s, desc64(q_lo + off16, desc_hi), desc64(k_lo + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
+                    mma_ss(s, desc64(q_lo + off16, desc_hi), desc64(k_lo + off16, desc_hi), IDESC_S, 1u);
                     if (ks == 3) tc_commit(bar_k_empty);
                 }
                 tc_commit(bar_k_empty + 8);
-            }
-            __syncwarp();
-            ok = warp_all(mbar_wait(bar_b_full, j & 1, s_abort));
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-#pragma unroll
-                for (int ks = 0; ks < kTile / 16; ks++)
-                    mma_ss(s + ks * 16, desc64(ring_lo + ((j & 1) * kRelTile >> 4) + (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4), desc_hi), id_desc,
-                           IDESC_B, 1u);
                 tc_commit(bar_s_full + 8 * (j & 1));
-                tc_commit(bar_b_free);
             }
             __syncwarp();
         }
@@ -487,48 +460,81 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_d, const uint
             off[g] = (2u + (u >> 4)) * kPanelBytes + r * 128 + ((((u >> 1) & 7) ^ (r & 7)) << 4) + (u & 1) * 8;
         }
         uint32_t carry[4] = {0u, 0u, 0u, 0u};
-        const uint64_t inv_d2 = pack2(inv_d, inv_d);
-        auto scaled = [&](float x0, float x1) {   // x / d, rounded to f16
-            unpack2(mul2(pack2(x0, x1), inv_d2), x0, x1);
-            return cvt_f16x2_sat(x0, x1);
+        const uint64_t scale2 = pack2(a.scale, a.scale), inv_scale2 = pack2(inv_scale, inv_scale);
+        auto scaled = [&](float x0, float x1) {   // f16(scale * x), the reference's rounding
+            unpack2(mul2(pack2(x0, x1), scale2), x0, x1);
+            return cvt_f16x2(x0, x1);
         };
-        for (int m = 0; m < n_blocks; m++) {
-            ok = warp_all(mbar_wait(bar_x_full, m & 1, s_abort));   // (the tensor memory instructions want the warp together)
-            if (!ok) break;
-            tc_fence_after();
-            uint32_t first[4], xa[32], xb[32], o[32];
-            tmem_ld4(tmem_X + lane_base - 1 - w, first);         // (columns before the block's own are not used)
-            tmem_ld32(tmem_X + lane_base + 3 - w, xa);
-            tmem_ld32(tmem_X + lane_base + 35 - w, xb);          // (nor the last ones: they wait for the next block)
-            tmem_wait_ld();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_x_free);
-            {
-                float e[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) e[k] = __uint_as_float(k <= w ? carry[k] : first[k]);
-                o[0] = scaled(e[0], e[1]), o[1] = scaled(e[2], e[3]);
-            }
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) o[2 + (i >> 1)] = scaled(__uint_as_float(xa[i]), __uint_as_float(xa[i + 1]));
-#pragma unroll
-            for (int i = 0; i < 28; i += 2) o[18 + (i >> 1)] = scaled(__uint_as_float(xb[i]), __uint_as_float(xb[i + 1]));
-#pragma unroll
-            for (int k = 0; k < 4; k++) carry[k] = xb[28 + k];
-            if (m >= 4 && !(m & 1)) {   // the first of the two panels of tile m / 2 - 2, which are written from here on
-                ok = warp_all(mbar_wait(bar_b_free, (m / 2 - 2) & 1, s_abort));
+        // Tile t is complete with block 2t + 3.  Its columns of the score tile start from bias / scale; they are free once P[t - 2].V[t - 2], whose P
+        // lies in them, has completed, which is awaited with the next block of X already out of tensor memory (not for the first two tiles).
+        int m = 0, t = 0;
+        while (t < n_tiles) {
+            const bool complete = m >= 2 * t + 4, block = m < n_blocks && !(complete && t < 2);
+            uint32_t o[32], pv_there = 0;
+            if (block) {
+                ok = warp_all(mbar_wait(bar_x_full, m & 1, s_abort));   // (the tensor memory instructions want the warp together)
                 if (!ok) break;
-            }
-#pragma unroll
-            for (int g = 0; g < 16; g++) {
-                *reinterpret_cast<uint2*>(ring_row + (off[g] & (4 * kPanelBytes - 1))) = make_uint2(o[2 * g], o[2 * g + 1]);
-                off[g] += kPanelBytes;
-            }
-            if (m >= 3 && (m & 1)) {
-                fence_proxy_async();
+                tc_fence_after();
+                uint32_t first[4], xa[32], xb[32];
+                tmem_ld4(tmem_X + lane_base - 1 - w, first);         // (columns before the block's own are not used)
+                tmem_ld32(tmem_X + lane_base + 3 - w, xa);
+                tmem_ld32(tmem_X + lane_base + 35 - w, xb);          // (nor the last ones: they wait for the next block)
+                tmem_wait_ld();
+                tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_b_full);
+                if (lane == 0) mbar_arrive(bar_x_free);
+                if (complete) pv_there = mbar_test(bar_pv + 8 * (t & 1), ((t >> 1) - 1) & 1);
+                {
+                    float e[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) e[k] = __uint_as_float(k <= w ? carry[k] : first[k]);
+                    o[0] = scaled(e[0], e[1]), o[1] = scaled(e[2], e[3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) o[2 + (i >> 1)] = scaled(__uint_as_float(xa[i]), __uint_as_float(xa[i + 1]));
+#pragma unroll
+                for (int i = 0; i < 28; i += 2) o[18 + (i >> 1)] = scaled(__uint_as_float(xb[i]), __uint_as_float(xb[i + 1]));
+#pragma unroll
+                for (int k = 0; k < 4; k++) carry[k] = xb[28 + k];
+            }
+            if (complete) {
+                if (t >= 2) {
+                    ok = warp_all(pv_there || mbar_wait(bar_pv + 8 * (t & 1), ((t >> 1) - 1) & 1, s_abort));
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                const uint8_t* row = ring_row + (t & 1) * kRelTile + r * 128;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    uint32_t f[32];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int cc = 4 * q + i;
+                        const uint4 v = *reinterpret_cast<const uint4*>(row + (cc >> 3) * kPanelBytes + (((cc & 7) ^ (r & 7)) << 4));
+                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&w4[k]));
+                            float f0, f1;
+                            unpack2(mul2(pack2(x.x, x.y), inv_scale2), f0, f1);
+                            f[8 * i + 2 * k] = __float_as_uint(f0), f[8 * i + 2 * k + 1] = __float_as_uint(f1);
+                        }
+                    }
+                    tmem_st32(tmem_S + (t & 1) * kTile + lane_base + q * 32, f);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_b_full + 8 * (t & 1));
+                t++;
+            }
+            if (block) {
+#pragma unroll
+                for (int g = 0; g < 16; g++) {
+                    *reinterpret_cast<uint2*>(ring_row + (off[g] & (4 * kPanelBytes - 1))) = make_uint2(o[2 * g], o[2 * g + 1]);
+                    off[g] += kPanelBytes;
+                }
+                m++;
             }
         }
     } else {

@@ -734,6 +734,61 @@ def test_relpos_scales(b200, orc, scale):
     assert_close(got, ref, f"rel-pos scale={scale}")
 
 
+@pytest.mark.parametrize("size", [4.0, 8.0, 16.0])
+@pytest.mark.parametrize("T", [150, 700])
+def test_relpos_bias_of_any_size_is_rounded_once(b200, orc, T, size):
+    """f16(scale * x) of a bias of standard deviation `size`: a step of F16 grows with it, so that a rounding elsewhere than the
+    operator's (of x / d, say, times d afterwards) shows."""
+    rng = np.random.default_rng(464)
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    r = (r.astype(np.float32) * np.float32(size / orc.relpos_mask(q_v, r, 128 ** -0.5).astype(np.float32).std())).astype(np.float16)
+    ref = orc.flash_attn_ext(q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, ref, f"rel-pos T={T} bias of {size}")
+    assert b200.lib().b200_device_status() == 0
+
+
+@pytest.mark.parametrize("T,valid", [(150, 131), (300, 257), (300, 127), (100, 3)])
+def test_relpos_table_rows_of_dead_keys_hold_anything(b200, orc, T, valid):
+    """Rows of the table that only keys at or beyond kv_len reach (bucket padding) hold NaN: no living key sees them."""
+    rng = np.random.default_rng(465)
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    pad = np.zeros((1, 1, T, T), np.float16)
+    pad[..., valid:] = -np.inf
+    ref = orc.flash_attn_ext(q_u, k, v, pad, scale=128 ** -0.5, q_v=q_v, r=r)
+    r[:, :, T - 1 + valid:] = np.nan
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r, kv_len=[valid])
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, ref, f"rel-pos T={T} kv_len={valid}")
+    assert b200.lib().b200_device_status() == 0
+
+
+def test_relpos_bias_beyond_f16_is_an_infinity(b200, orc):
+    """A bias of -inf (scale * x below the range of F16) removes its key, and that key only; one just inside the range is itself."""
+    rng = np.random.default_rng(466)
+    T = 200
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    q_v[..., 0] = 16.0
+    for distance, x in ((5, -60000.0), (-31, -60000.0), (70, -46000.0)):   # scale * 16 * x: -84853 (twice) and -65054
+        r[:, :, T - 1 + distance] = 0.0
+        r[:, :, T - 1 + distance, 0] = x
+    bias = orc.relpos_mask(q_v, r, 128 ** -0.5)
+    assert np.isneginf(bias).sum() == 2 * (T - 5 + T - 31) and not np.isnan(bias).any()
+    ref = orc.flash_attn_ext(q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    assert_close(got, ref, "rel-pos with biases of -inf")
+    # query 10: every key removed but one
+    r[:] = 0.0
+    r[:, :, :, 0] = -60000.0
+    r[:, :, T - 1 + 7, 0] = 0.0
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r)
+    assert_close(got[0, 10], v[0, :, 17], "one key left", max_abs=0.0, rel_l2=0.0)
+    assert not got[0, T - 1].any()                       # no key left: zeros, as under a mask
+    assert b200.lib().b200_device_status() == 0
+
+
 def test_relpos_table_built_on_the_device_and_cached(b200, orc):
     """R = attn_pos_w . pos_enc (src/core/fastconformer.h:118-130, :843, :851) built by the library for a (layer, T)
     equals the oracle's make_pos_enc @ W to within one F16 rounding, attention with the library's table meets the
