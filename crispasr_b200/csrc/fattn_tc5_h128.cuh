@@ -116,6 +116,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                 for (int i = 0; i < HD / 4; i++) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (tid == 4 * 32) ask_for_next_block(s_next, bar_next);
+            if (turn == 0) __syncthreads();   // a first tile without keys: nobody else has seen the set-up of the barriers yet
             return 0;
         }
         auto load_kv = [&](const CUtensorMap& tm, uint32_t stage, uint32_t bar, int j) {

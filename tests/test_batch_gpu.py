@@ -250,6 +250,29 @@ def test_head_dim_128_launch_of_more_than_two_waves(b200, orc, qdtype, causal):
     assert b200.lib().b200_device_status() == 0
 
 
+@pytest.mark.parametrize("qdtype", [np.float32, np.float16])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("live", [12, 1, 0])
+def test_head_dim_128_launch_whose_first_tiles_have_no_keys(b200, qdtype, causal, live):
+    """More than 592 tiles, and the CTAs of the first waves start with tiles of units without queries or without keys: bit for bit what
+    launches of a few units each give."""
+    rng = np.random.default_rng(52)
+    B, H, Hkv, Tq, Lk = 48, 16, 8, 70, 140
+    qlens = [0] * (B - live) + [int(x) for x in rng.integers(1, Tq + 1, live)]
+    klens = [0] * (B - live) + [min(Lk, n + int(x)) for n, x in zip(qlens[B - live:], rng.integers(0, 71, live))]
+    for b in range(0, B - live, 2):   # every other empty unit has rows to write or keys to skip
+        qlens[b], klens[b] = (0, Lk) if causal else (Tq, 0)
+    q = randn_f16(rng, (B, H, Tq, 128)).astype(qdtype)
+    k, v = randn_f16(rng, (B, Hkv, Lk, 128)), randn_f16(rng, (B, Hkv, Lk, 128))
+    kw = dict(scale=128 ** -0.5, causal=True) if causal else dict(scale=128 ** -0.5)
+    got = gpu_op(b200, q, k, v, q_len=qlens, kv_len=klens, **kw)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5 and b200.lib().b200_device_status() == 0
+    assert not got[:B - live].any()
+    for b in range(B - live, B, 4):
+        few = slice(b, b + 4)
+        assert np.array_equal(got[few], gpu_op(b200, q[few], k[few], v[few], q_len=qlens[few], kv_len=klens[few], **kw)), f"units {b} to {b + 3}"
+
+
 def test_slot_table_drives_a_decode_batch(b200, orc):
     """b200_batch over a Q8_0 cache with 6 stream slots: streams join with different cache lengths, every step
     appends one row per resident stream and attends with the tables b200_batch_tables uploads; a stream that
