@@ -1267,8 +1267,14 @@ int launch_t(const FattnArgs& a_in, cudaStream_t st, char* errbuf, size_t errlen
     // share its "attribute set" flags between them)
     auto args = [&](auto launch) { e = launch(grid, smem, st, a, tmK, tmV, tmQ, tmO); };
     if constexpr (HD == 128) {
-        // more than two full waves (of two CTAs per SM): CTAs that go on to the next tile themselves
-        if (!a.has_mask && q_tma && o_tma && (long)grid.x * grid.y * grid.z > 4 * 148) {
+        // More than two full waves (of two CTAs per SM): CTAs that go on to the next tile themselves.  They ask for it when they start the one
+        // before, so under a causal bound whoever has the longest tile also gets the longer of the second ones, which takes a third tile
+        // to even out, and the more of them the longer the rows.  us, ordinary kernel / this one, F32 queries: 600 tiles of up to 96 keys
+        // 25.4 / 24.6, 480 keys 32.3 / 29.5, 1920 keys 53.7 / 57.4; 640 tiles of 1280 keys 45.9 / 43.6, 2560 keys 67.8 / 71.0; 680 of 5400
+        // 123 / 131; 704 of 1400 52.7 / 50.4; 752 of 12000 286 / 312; 768 of 3072 89.2 / 86.1; 960 of 5000 165 / 163.  Not causal, 600 tiles of
+        // 128, 384, 1920 keys 27.0, 36.5, 100.2 / 25.8, 35.8, 98.6 (F16 queries 21.3, 33.0, 96.2 / 22.1, 32.8, 94.6).
+        const long tiles = (long)grid.x * grid.y * grid.z;
+        if (!a.has_mask && q_tma && o_tma && tiles > 4 * 148 + (a.causal && a.Lk > 1024 ? (a.Lk - 1024) / 16 : 0)) {
             const size_t smem_h128 = 1024 + (size_t)3 * TILE_BYTES + 112;
             static bool set[2][64] = {};
             auto go = [&](auto kern, bool (&smem_set)[64]) {

@@ -8,7 +8,8 @@
 // 8 streams x 407 tokens over a Q8_0 cache 50.9 -> 48.8 us per layer; F16 rows, F32 queries, 16 x 407 68.0 -> 62.9, 2 x 1600 61.8 -> 60.9, 8 x
 // 1500 not causal 175.7 -> 170.7; F16 queries, 16 x 407 59.6 -> 56.1, 16 x 750 not causal 103.3 -> 99.7.
 // Whoever asks first gets the block, not who is done first: launches of up to two full waves are slower this way (4 x 407 tokens 18.9 ->
-// 20.6, 16 x 100 15.5 -> 16.2) and take the other kernel.  (Asked for behind the last copies the answer is waited for: 16 x 750 111.)
+// 20.6, 16 x 100 15.5 -> 16.2), so are causal ones of long rows with few tiles more (launch_t), and take the other kernel.  (Asked for behind
+// the last copies the answer is waited for: 16 x 750 111.)
 // A kernel of its own because the loop around a tile costs the registers that masks need (2 x 1500 under a mask 148 -> 174).
 // Asks the hardware for a block of this grid that has not been launched yet and will not be: the caller does its work (16 bytes at `dst`,
 // announced on `bar`).  Not again after an answer that there is none.

@@ -273,6 +273,18 @@ def test_head_dim_128_launch_whose_first_tiles_have_no_keys(b200, qdtype, causal
         assert np.array_equal(got[few], gpu_op(b200, q[few], k[few], v[few], q_len=qlens[few], kv_len=klens[few], **kw)), f"units {b} to {b + 3}"
 
 
+@pytest.mark.parametrize("B,T", [(9, 1100), (7, 1408), (5, 1920)])
+def test_head_dim_128_causal_launches_of_long_rows_around_two_waves(b200, B, T):
+    """648, 616 and 600 tiles, on either side of where a launch goes over to CTAs that take several: the same bits as one unit alone."""
+    rng = np.random.default_rng(53)
+    q, k, v = randn_f16(rng, (B, 8, T, 128)), randn_f16(rng, (B, 8, T, 128)), randn_f16(rng, (B, 8, T, 128))
+    got = gpu_op(b200, q, k, v, scale=128 ** -0.5, causal=True)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5
+    for b in (0, B - 1):
+        assert np.array_equal(got[b:b + 1], gpu_op(b200, q[b:b + 1], k[b:b + 1], v[b:b + 1], scale=128 ** -0.5, causal=True)), f"unit {b}"
+    assert b200.lib().b200_device_status() == 0
+
+
 def test_slot_table_drives_a_decode_batch(b200, orc):
     """b200_batch over a Q8_0 cache with 6 stream slots: streams join with different cache lengths, every step
     appends one row per resident stream and attends with the tables b200_batch_tables uploads; a stream that
