@@ -245,8 +245,12 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const 
         }
         return;
     }
-    const int n_blocks = 2 * n_tiles + 2;
-    const int rb0 = a.Tq - 1 - q0 - 127;  // R row of X column 0 (may be negative: the copies fill with zeros)
+    // X blocks: 2 n_tiles + 2, but for the first one, which only rows from 64 on need (J - i + 127 < 64 with J >= 0), and the last one, which only
+    // keys of the last tile from 64 on need, where there are none.  They are numbered from the first one taken, block m0; what the
+    // ring holds in the places left out goes to dead rows and keys.
+    const int m0 = tq_b - q0 <= 64 ? 1 : 0;
+    const int n_blocks = 2 * n_tiles + (len_b - (n_tiles - 1) * kTile <= 64 ? 1 : 2) - m0;
+    const int rb0 = a.Tq - 1 - q0 - 127 + kRelBlock * m0;  // R row of the first block's first column (may be negative: the copies fill with zeros)
 
     auto load_r = [&](int m) {
         const uint32_t bar = bar_r_full + 8 * (m & (kRelRSlots - 1)), dst = sR + (m & (kRelRSlots - 1)) * kRelRBytes;
@@ -267,7 +271,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const 
     // ---- set-up ----
     if (tid == 14 * 32) {   // (the thread that set the barriers up)
 #pragma unroll 1
-        for (int m = 0; m < kRelRSlots; m++) load_r(m);   // n_blocks >= 4
+        for (int m = 0; m < min(kRelRSlots, n_blocks); m++) load_r(m);
         load_k(0, 0);
         load_k(0, 1);
         load_v(0);
@@ -404,7 +408,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const 
     } else if (warp == 14) {
         // ================= X products and copies of R =================
         const uint32_t r_lo = smem_desc_lo(sR, 16);
-        int r_issued = kRelRSlots;
+        int r_issued = min(kRelRSlots, n_blocks);
         ok = warp_all(mbar_wait(bar_qv, 0, s_abort));
         for (int m = 0; m < n_blocks && ok; m++) {
             ok = mbar_wait(bar_r_full + 8 * (m & (kRelRSlots - 1)), (m / kRelRSlots) & 1, s_abort) && (m == 0 || mbar_wait(bar_x_free, (m - 1) & 1, s_abort));
@@ -457,7 +461,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const 
 #pragma unroll
         for (int g = 0; g < 16; g++) {
             const uint32_t u = g + lane;
-            off[g] = (2u + (u >> 4)) * kPanelBytes + r * 128 + ((((u >> 1) & 7) ^ (r & 7)) << 4) + (u & 1) * 8;
+            off[g] = (2u + m0 + (u >> 4)) * kPanelBytes + r * 128 + ((((u >> 1) & 7) ^ (r & 7)) << 4) + (u & 1) * 8;
         }
         uint32_t carry[4] = {0u, 0u, 0u, 0u};
         const uint64_t scale2 = pack2(a.scale, a.scale), inv_scale2 = pack2(inv_scale, inv_scale);
@@ -469,7 +473,7 @@ fattn_prefill_tc5_relpos_kernel(const FattnArgs a, const float inv_scale, const 
         // lies in them, has completed, which is awaited with the next block of X already out of tensor memory (not for the first two tiles).
         int m = 0, t = 0;
         while (t < n_tiles) {
-            const bool complete = m >= 2 * t + 4, block = m < n_blocks && !(complete && t < 2);
+            const bool complete = m0 + m >= 2 * t + 4 || m == n_blocks, block = m < n_blocks && !(complete && t < 2);
             uint32_t o[32], pv_there = 0;
             if (block) {
                 ok = warp_all(mbar_wait(bar_x_full, m & 1, s_abort));   // (the tensor memory instructions want the warp together)

@@ -764,6 +764,28 @@ def test_relpos_table_rows_of_dead_keys_hold_anything(b200, orc, T, valid):
     assert b200.lib().b200_device_status() == 0
 
 
+@pytest.mark.parametrize("T", [200, 330])
+def test_relpos_batch_of_lengths_around_the_blocks(b200, orc, T):
+    """Utterances whose last tiles hold 64 query rows or keys or fewer, which leave out blocks of 64 table rows, and of one row or key more;
+    their lengths for queries and keys need not be the same."""
+    rng = np.random.default_rng(467)
+    lens = [n for n in (1, 63, 64, 65, 128, 129, 191, 192, 193, 200, 256, 257, 320, 321, 330) if n <= T]
+    qlens, klens = lens + lens, lens + lens[::-1]
+    q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
+    B = len(qlens)
+    roll = lambda x: np.concatenate([np.roll(x, 7 * b, axis=2) for b in range(B)])
+    q_u, q_v, k, v = (roll(x) for x in (q_u, q_v, k, v))
+    got = gpu_op(b200, q_u, k, v, scale=128 ** -0.5, q_v=q_v, r=r, q_len=qlens, kv_len=klens)
+    assert b200.lib().b200_last_kernel() == abi.KERNEL_PREFILL_TC5 and b200.lib().b200_device_status() == 0
+    for b, (nq, nk) in enumerate(zip(qlens, klens)):
+        pad = np.zeros((1, 1, T, T), np.float16)
+        pad[..., nk:] = -np.inf
+        one = slice(b, b + 1)
+        ref = orc.flash_attn_ext(q_u[one], k[one], v[one], pad, scale=128 ** -0.5, q_v=q_v[one], r=r)
+        assert_close(got[one, :nq], ref[:, :nq], f"rel-pos T={T} q_len={nq} kv_len={nk}")
+        assert not got[b, nq:].any()
+
+
 def test_relpos_bias_beyond_f16_is_an_infinity(b200, orc):
     """A bias of -inf (scale * x below the range of F16) removes its key, and that key only; one just inside the range is itself."""
     rng = np.random.default_rng(466)
