@@ -90,16 +90,12 @@ __device__ __forceinline__ T load_global(const T* p) {
         uint32_t x[4];
         asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "l"(p) : "memory");
         memcpy(&r, x, 16);
-    } else if constexpr (sizeof(T) == 8) {
-        uint32_t x[2];
-        asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(x[0]), "=r"(x[1]) : "l"(p) : "memory");
-        memcpy(&r, x, 8);
     } else if constexpr (sizeof(T) == 4) {
         uint32_t x;
         asm volatile("ld.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
         memcpy(&r, &x, 4);
     } else {
-        static_assert(sizeof(T) == 2, "16, 8, 4 or 2 bytes");
+        static_assert(sizeof(T) == 2, "16, 4 or 2 bytes");
         uint16_t x;
         asm volatile("ld.global.u16 %0, [%1];" : "=h"(x) : "l"(p) : "memory");
         memcpy(&r, &x, 2);
