@@ -522,6 +522,145 @@ __device__ __forceinline__ void store_o_rows_coalesced(float* stage, int lane, f
     }
 }
 
+// ---- parts that the two-CTA kernels share (fattn_tc5_h128.cuh) ------------------------------------------
+// A query tile of F32 rows as tensor copies bring it: four panels of 128-byte swizzled rows, 32 columns each.  Columns 0 to 63 lie in the V stage
+// and 64 to 127 in the operand tile itself: a softmax thread holds its whole row in registers before any of them writes the operand
+// tile, and the first K tile is on its way meanwhile.
+__device__ __forceinline__ constexpr int raw_panel_off(int p) { return (p < 2 ? 4 * kPanelBytes : 0) + (p & 1) * kPanelBytes; }
+
+// Raw F32 row r -> F16 row r of the operand tile: 32 loads, 64 conversions, 16 stores per thread, all from shared memory.
+__device__ __forceinline__ void convert_raw_row(uint8_t* smem_gen, int r) {
+    uint4 row[16];
+#pragma unroll
+    for (int c = 0; c < 16; c++) {   // F16 chunk c = columns 8c .. 8c+7 = F32 chunks 2c, 2c+1 of raw panel c / 4
+        const int f0 = (2 * c) & 7;
+        const uint8_t* raw = smem_gen + raw_panel_off(c >> 2) + r * 128;
+        const float4 x0 = *reinterpret_cast<const float4*>(raw + ((f0 ^ (r & 7)) << 4));
+        const float4 x1 = *reinterpret_cast<const float4*>(raw + (((f0 + 1) ^ (r & 7)) << 4));
+        row[c] = make_uint4(pack_half2(x0.x, x0.y), pack_half2(x0.z, x0.w), pack_half2(x1.x, x1.y), pack_half2(x1.z, x1.w));
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");   // the operand tile is written over raw columns 64 to 127 of all rows
+#pragma unroll
+    for (int c = 0; c < 16; c++) *reinterpret_cast<uint4*>(smem_gen + r * 128 + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) = row[c];
+}
+
+// S = Q.K^T of one key tile and O (+)= P.V, by one lane.
+template <int HD>
+__device__ __forceinline__ void issue_scores(uint32_t tmem_S, uint32_t q_lo, uint32_t k_lo) {
+#pragma unroll
+    for (int ks = 0; ks < HD / 16; ks++) {
+        const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
+        mma_ss(tmem_S, desc64(q_lo + off16, smem_desc_hi(1024)), desc64(k_lo + off16, smem_desc_hi(1024)), idesc_f16(kTile, false), ks > 0 ? 1u : 0u);
+    }
+}
+template <int HD>
+__device__ __forceinline__ void issue_pv(uint32_t tmem_O, uint32_t tmem_P, uint32_t v_lo, bool first) {
+    mma_ts(tmem_O, tmem_P, desc64(v_lo, smem_desc_hi(1024)), idesc_f16(HD, true), first ? 0u : 1u);
+#pragma unroll
+    for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(v_lo + ks * (2048 >> 4), smem_desc_hi(1024)), idesc_f16(HD, true), 1u);
+}
+
+// A first reference maximum of a row without a mask: that of its first 32 scores.  It is rarely more than 2^8 below the row's real maximum, and
+// when it is (or when those columns are dead) the check behind softmax_tile has the tile redone against the exact maximum.
+__device__ __forceinline__ float first_maximum(uint32_t s_row, int n_valid) {
+    uint32_t s0[32];
+    tmem_ld32(s_row, s0);
+    tmem_wait_ld();
+    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        const float x0 = (i < n_valid) ? __uint_as_float(s0[i]) : -INFINITY;
+        const float x1 = (i + 1 < n_valid) ? __uint_as_float(s0[i + 1]) : -INFINITY;
+        m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], x0, x1);
+    }
+    return max3(fmaxf(m4[0], m4[1]), m4[2], m4[3]);
+}
+
+// P = exp2(S * c - m) of a row's 128 scores, rounded to f16x2, their sum and the maximum of S, in one pass; columns >= n_valid are dead.  Rolling
+// 32-column chunks: the load of chunk k+2 is issued into the registers chunk k has just left and completes under the exponentials of
+// chunk k+1.  `meanwhile` runs behind the first chunk.
+template <typename F>
+__device__ __forceinline__ void softmax_tile(uint32_t s_row, float c, float m, bool full_tile, int n_valid, uint32_t (&preg)[2][32], float& mx, float& lsum, F meanwhile) {
+    float mx8[8];
+    uint64_t ls4[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+    for (int i = 0; i < 8; i++) mx8[i] = -INFINITY;
+    const uint64_t c2 = pack2(c, c), nm2 = pack2(-m, -m);
+    uint32_t sA[32], sB[32];
+    // a partial tile (the last one, or the diagonal of a causal call) puts -inf into the dead columns first and skips chunks that are
+    // dead for the whole warp: one copy of the arithmetic serves both
+    auto chunk = [&](uint32_t (&sx)[32], uint32_t* p16, int col0) {
+        if (!full_tile) {
+            if (__all_sync(0xffffffffu, col0 >= n_valid)) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) p16[i] = 0u;
+                return;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i++)
+                if (col0 + i >= n_valid) sx[i] = 0xFF800000u;
+        }
+        softmax32(sx, p16, c2, nm2, mx8, ls4);
+    };
+    tmem_ld32(s_row, sA);
+    tmem_ld32(s_row + 32, sB);
+    tmem_wait_ld();
+    chunk(sA, preg[0], 0);
+    tmem_ld32(s_row + 64, sA);
+    meanwhile();
+    chunk(sB, preg[0] + 16, 32);
+    tmem_wait_ld();
+    tmem_ld32(s_row + 96, sB);
+    chunk(sA, preg[1], 64);
+    tmem_wait_ld();
+    chunk(sB, preg[1] + 16, 96);
+    mx = fmaxf(max3(fmaxf(mx8[0], mx8[1]), mx8[2], mx8[3]), max3(fmaxf(mx8[4], mx8[5]), mx8[6], mx8[7]));
+    float l0, l1;
+    unpack2(add2(add2(ls4[0], ls4[1]), add2(ls4[2], ls4[3])), l0, l1);
+    lsum = l0 + l1;
+}
+
+template <int HD>
+__device__ __forceinline__ void rescale_o(uint32_t o_row, float alpha) {
+#pragma unroll
+    for (int q4 = 0; q4 < HD / 32; q4++) {
+        uint32_t oreg[32];
+        tmem_ld32(o_row + q4 * 32, oreg);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
+        tmem_st32(o_row + q4 * 32, oreg);
+    }
+}
+
+// A warp's 32 packed rows x 32 columns of the output are a box [32 columns, gqa heads, 32 / gqa tokens] of dst [hd, H, Tq, B]; the warp parks them
+// as 128-byte rows with the 16-byte chunks swizzled by the row (the copy's own pattern, conflict-free for the stores) and one lane
+// hands each panel to a tensor store, which also clips the tokens beyond Tq.  `stage`: this warp's 32 * HD floats; dead rows are written
+// as literal zeros (whatever the padding row of Q held never reaches dst); `row0`: first packed row of the warp.
+template <int HD>
+__device__ __forceinline__ void store_o_box(const CUtensorMap& tmO, float* stage, uint32_t o_row, float inv, bool row_live, int lane, int row0, int rows_total, int hk,
+                                            int gqa, int b) {
+#pragma unroll
+    for (int q4 = 0; q4 < HD / 32; q4++) {
+        uint32_t oreg[32];
+        tmem_ld32(o_row + q4 * 32, oreg);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(stage + q4 * 32 * 32 + lane * 32 + (((i >> 2) ^ (lane & 7)) << 2)) =
+                row_live ? make_float4(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv,
+                                       __uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0 && row0 < rows_total) {
+#pragma unroll
+        for (int q4 = 0; q4 < HD / 32; q4++) tma_store_4d(&tmO, smem_u32(stage + q4 * 32 * 32), q4 * 32, hk * gqa, row0 / gqa, b);
+        tma_store_commit_and_wait_read();
+    }
+}
+
 // QMODE / OTMA: how the query tile comes in and the output tile goes out (see q_tma below).  Template parameters, not
 // run-time flags: every path compiled into one kernel costs the others (the raw F32 form behind a flag took 5 % off the
 // F16-Q encoder launches and 9 % off the T = 407 prefill).
@@ -534,8 +673,6 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     constexpr bool o_tma = OTMA;
     constexpr int PANELS = HD / 64;
     constexpr int TILE_BYTES = kPanelBytes * PANELS;
-    constexpr uint32_t IDESC_S = idesc_f16(kTile, false);
-    constexpr uint32_t IDESC_PV = idesc_f16(HD, true);
 
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -550,11 +687,8 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     uint8_t* misc = smem_gen + (1 + 2 * NSTG) * TILE_BYTES + 32 * NSTG + 64;
     // q_tma: 0 = the softmax warps load and convert the Q tile; 1 = F16 rows by one tensor copy into the operand tile;
     // 2 = F32 rows by tensor copies into stages that are not needed yet, converted from there by the softmax warps.
-    // The raw tile (64 KB) takes the V stage (columns 0 to 63) and the operand tile itself (64 to 127): a softmax thread holds its whole
-    // row in registers before any of them writes the operand tile, and the first K tile is on its way meanwhile.
     constexpr bool q_raw = QMODE == 2;
     static_assert(!q_raw || (HD == 128 && NSTG == 1), "the raw tile takes the stages of head_dim 128");
-    constexpr int RAW_PANEL_OFF[4] = {2 * TILE_BYTES, 2 * TILE_BYTES + kPanelBytes, 0, kPanelBytes};   // 32 columns each
     // head_dim 64 leaves 64 spare TMEM columns: P gets its own, so S of the next tile can be issued before P.V
     constexpr bool SEP_P = (HD == 64);
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
@@ -635,7 +769,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             mbar_arrive_expect_tx(bar_q_full, (HD / 32) * kPanelBytes);
 #pragma unroll
             for (int p = 0; p < HD / 32; p++)
-                tma_load_4d(sQ + RAW_PANEL_OFF[p], &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
+                tma_load_4d(sQ + raw_panel_off(p), &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
         } else if (q_tma) {
             // F16 query rows go straight into the operand layout: one copy instead of a pass through the softmax warps'
             // registers, which a CTA sharing its SM with another one in its key loop executes at a few tens of clocks
@@ -685,23 +819,8 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
     const uint32_t tmem_O = tmem_base + kTile;    // cols [128,128+HD)
     if constexpr (q_raw) {
         if (q_raw && warp < 4) {
-            // raw F32 row r (panels of 128-byte swizzled rows) -> F16 row r of the operand tile: HD / 4 loads, HD / 2
-            // conversions, HD / 8 stores per thread, all from shared memory
             const bool there = mbar_wait(bar_q_full, 0, s_abort);
-            const int r = tid;
-            uint4 row[HD / 8];
-#pragma unroll
-            for (int c = 0; c < HD / 8; c++) {   // F16 chunk c = columns 8c .. 8c+7 = F32 chunks 2c, 2c+1 of raw panel c / 4
-                const int f0 = (2 * c) & 7;
-                const uint8_t* raw = smem_gen + RAW_PANEL_OFF[c >> 2] + r * 128;
-                const float4 x0 = *reinterpret_cast<const float4*>(raw + ((f0 ^ (r & 7)) << 4));
-                const float4 x1 = *reinterpret_cast<const float4*>(raw + (((f0 + 1) ^ (r & 7)) << 4));
-                row[c] = make_uint4(pack_half2(x0.x, x0.y), pack_half2(x0.z, x0.w), pack_half2(x1.x, x1.y), pack_half2(x1.z, x1.w));
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");   // the operand tile is written over raw columns 64 to 127 of all rows
-#pragma unroll
-            for (int c = 0; c < HD / 8; c++)
-                *reinterpret_cast<uint4*>(smem_gen + r * 128 + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) = row[c];
+            convert_raw_row(smem_gen, tid);
             if (there) {
                 fence_proxy_async();   // the operand tile is read, and the V stage is overwritten, through the async proxy
                 __syncwarp();
@@ -761,14 +880,8 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         // issue order, so PV[j] has consumed P[j] before S[j+1] writes.
         {
             const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), v_lo = smem_desc_lo(sV, kPanelBytes);
-            constexpr uint32_t desc_hi = smem_desc_hi(1024);
             auto issue_s = [&](int slot) {
-                const uint32_t kd = k_lo + slot * (TILE_BYTES >> 4);
-#pragma unroll
-                for (int ks = 0; ks < HD / 16; ks++) {
-                    const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(kd + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
-                }
+                issue_scores<HD>(tmem_S, q_lo, k_lo + slot * (TILE_BYTES >> 4));
                 tc_commit(bar_s_full);
             };
             bool ok = mbar_wait(bar_k_full, 0, s_abort);
@@ -795,10 +908,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 if (elect_one()) {
                     // with P in its own columns the next S goes first: the softmax threads wake after 4 MMAs, not 12
                     if (SEP_P && more) issue_s(nslot);
-                    const uint32_t vd = v_lo + slot * (TILE_BYTES >> 4);
-                    mma_ts(tmem_O, tmem_P, desc64(vd, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
-#pragma unroll
-                    for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(vd + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
+                    issue_pv<HD>(tmem_O, tmem_P, v_lo + slot * (TILE_BYTES >> 4), j == 0);
                     if (SEP_P) {
                         if (more) tc_commit(bar_k_empty + 8 * nslot);   // after the P.V MMAs: off the softmax threads' critical path
                         tc_commit(bar_v_empty + 8 * slot);
@@ -848,9 +958,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
             const int n_valid = kend - j * kTile;  // columns >= n_valid of this row are masked
             const bool full_tile = __all_sync(0xffffffffu, n_valid >= kTile);
             if (j == 0) {
-                // First tile: a first reference maximum.  Without a mask the maximum of the row's first 32 scores
-                // is enough - it is rarely more than 2^8 below the row's real maximum, and when it is (or when those
-                // columns are masked) the lazy-rescale check below redoes the tile against the exact maximum.
+                // First tile: a first reference maximum
                 float mx = -INFINITY;
                 if (HASMASK) {
 #pragma unroll
@@ -863,17 +971,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                         mx = fmaxf(mx, row_max64(sreg, hh * 64, full_tile ? 2 * kTile : n_valid));
                     }
                 } else {
-                    uint32_t s0[32];
-                    tmem_ld32(tmem_S + lane_base, s0);
-                    tmem_wait_ld();
-                    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float x0 = (i < n_valid) ? __uint_as_float(s0[i]) : -INFINITY;
-                        const float x1 = (i + 1 < n_valid) ? __uint_as_float(s0[i + 1]) : -INFINITY;
-                        m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], x0, x1);
-                    }
-                    mx = max3(fmaxf(m4[0], m4[1]), m4[2], m4[3]);
+                    mx = first_maximum(tmem_S + lane_base, n_valid);
                 }
                 m_ref = mx * c_exp;  // c > 0
             }
@@ -888,45 +986,9 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 float mx = -INFINITY;
                 lsum = 0.0f;
                 if constexpr (!HASMASK) {
-                    // rolling 32-column chunks: the load of chunk k+2 is issued into the registers chunk k has just
-                    // left and completes under the exponentials of chunk k+1
-                    float mx8[8];
-                    uint64_t ls4[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-                    for (int i = 0; i < 8; i++) mx8[i] = -INFINITY;
-                    const uint64_t c2 = pack2(c_exp, c_exp), nm2 = pack2(-m_use, -m_use);
-                    uint32_t sA[32], sB[32];
-                    // a partial tile (the last one, or the diagonal of a causal call) puts -inf into the dead columns
-                    // first and skips chunks that are dead for the whole warp: one copy of the arithmetic serves both
-                    auto chunk = [&](uint32_t (&sx)[32], uint32_t* p16, int col0) {
-                        if (!full_tile) {
-                            if (__all_sync(0xffffffffu, col0 >= n_valid)) {
-#pragma unroll
-                                for (int i = 0; i < 16; i++) p16[i] = 0u;
-                                return;
-                            }
-#pragma unroll
-                            for (int i = 0; i < 32; i++)
-                                if (col0 + i >= n_valid) sx[i] = 0xFF800000u;
-                        }
-                        softmax32(sx, p16, c2, nm2, mx8, ls4);
-                    };
-                    tmem_ld32(tmem_S + lane_base, sA);
-                    tmem_ld32(tmem_S + lane_base + 32, sB);
-                    tmem_wait_ld();
-                    chunk(sA, preg[0], 0);
-                    tmem_ld32(tmem_S + lane_base + 64, sA);
-                    if (SEP_P && j > 0 && !pv_waited && !pv_probe) pv_probe = mbar_test(bar_pv_done, (j - 1) & 1);
-                    chunk(sB, preg[0] + 16, 32);
-                    tmem_wait_ld();
-                    tmem_ld32(tmem_S + lane_base + 96, sB);
-                    chunk(sA, preg[1], 64);
-                    tmem_wait_ld();
-                    chunk(sB, preg[1] + 16, 96);
-                    mx = max3(max3(fmaxf(mx8[0], mx8[1]), mx8[2], mx8[3]), max3(fmaxf(mx8[4], mx8[5]), mx8[6], mx8[7]), mx);
-                    float l0, l1;
-                    unpack2(add2(add2(ls4[0], ls4[1]), add2(ls4[2], ls4[3])), l0, l1);
-                    lsum = l0 + l1;
+                    softmax_tile(tmem_S + lane_base, c_exp, m_use, full_tile, n_valid, preg, mx, lsum, [&]() {
+                        if (SEP_P && j > 0 && !pv_waited && !pv_probe) pv_probe = mbar_test(bar_pv_done, (j - 1) & 1);
+                    });
                 } else
 #pragma unroll
                 for (int hh = 0; hh < 2; hh++) {
@@ -953,17 +1015,7 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
                 const float m_new = fmaxf(m_ref, m_tile);
                 const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
                 l_run *= alpha;
-                if (j > 0) {
-#pragma unroll
-                    for (int q4 = 0; q4 < HD / 32; q4++) {
-                        uint32_t oreg[32];
-                        tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-                        tmem_st32(tmem_O + lane_base + q4 * 32, oreg);
-                    }
-                }
+                if (j > 0) rescale_o<HD>(tmem_O + lane_base, alpha);
                 m_ref = m_new;
             }
             if (!ok) break;
@@ -983,36 +1035,13 @@ fattn_prefill_tc5_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap 
         if (ok) ok = mbar_wait(bar_o_done, 0, s_abort);
         if (ok) {
             tc_fence_after();
-            // dead rows are written as literal zeros (whatever the padding row of Q held never reaches dst), rows
-            // outside the tensor not at all.  The K/V stages are free once the last MMA has completed: they stage O.
+            // dead rows are written as literal zeros, rows outside the tensor not at all.  The K/V stages are free once the last MMA has
+            // completed: they stage O.
             const float inv = row_live && l_run > 0.0f ? 1.0f / l_run : 0.0f;
             float* out = (row_live || row_zero) ? a.dst + (((int64_t)b * a.Tq + iq_dst) * a.dst_heads + h) * HD : nullptr;
             float* stage = reinterpret_cast<float*>(smem_gen + TILE_BYTES) + warp * 32 * HD;
             if (o_tma) {
-                // A warp's 32 packed rows x 32 columns are a box [32 columns, gqa heads, 32 / gqa tokens] of
-                // dst [hd, H, Tq, B]; the warp parks them as 128-byte rows with the 16-byte chunks swizzled by the row (the
-                // copy's own pattern, conflict-free for the stores) and one lane hands each panel to a tensor store,
-                // which also clips the tokens beyond Tq.
-#pragma unroll
-                for (int q4 = 0; q4 < HD / 32; q4++) {
-                    uint32_t oreg[32];
-                    tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(stage + q4 * 32 * 32 + lane * 32 + (((i >> 2) ^ (lane & 7)) << 2)) =
-                            row_live ? make_float4(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv,
-                                                   __uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv)
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0 && q0 + warp * 32 < rows_total) {
-#pragma unroll
-                    for (int q4 = 0; q4 < HD / 32; q4++)
-                        tma_store_4d(&tmO, smem_u32(stage + q4 * 32 * 32), q4 * 32, hk * a.gqa, (q0 + warp * 32) / a.gqa, b);
-                    tma_store_commit_and_wait_read();
-                }
+                store_o_box<HD>(tmO, stage, tmem_O + lane_base, inv, row_live, lane, q0 + warp * 32, rows_total, hk, a.gqa, b);
             } else {
 #pragma unroll
                 for (int q4 = 0; q4 < HD / 32; q4++) {

@@ -37,7 +37,6 @@ __global__ void __launch_bounds__(kThreadsTc5, 2)
 fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                               const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmO) {
     constexpr int HD = 128, TILE_BYTES = 2 * kPanelBytes;
-    constexpr uint32_t IDESC_S = idesc_f16(kTile, false), IDESC_PV = idesc_f16(HD, true);
 
     extern __shared__ uint8_t smem_dyn[];
     const uint32_t smem_base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -47,9 +46,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                    bar_p_ready = sBar + 40, bar_o_done = sBar + 48, bar_q_full = sBar + 56, bar_q_conv = sBar + 64, bar_next = sBar + 72;
     const uint32_t s_next = sBar + 96;   // the answer about the next block
     uint8_t* misc = smem_gen + 3 * TILE_BYTES + 80;
-    // The query tile comes by tensor copies: F16 rows into the operand tile, F32 rows (RAW, 64 KB) into the V stage (columns 0 to 63) and the
-    // operand tile itself (64 to 127), from where the softmax threads convert them through their registers.
-    constexpr int RAW_PANEL_OFF[4] = {2 * TILE_BYTES, 2 * TILE_BYTES + kPanelBytes, 0, kPanelBytes};   // 32 columns each
+    // The query tile comes by tensor copies: F16 rows into the operand tile, F32 rows (RAW, 64 KB) as convert_raw_row takes them.
     volatile uint32_t* s_tmem_base = reinterpret_cast<volatile uint32_t*>(misc);
     volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 4);
 
@@ -129,7 +126,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
             mbar_arrive_expect_tx(bar_q_full, RAW ? 2 * TILE_BYTES : TILE_BYTES);
             if (RAW) {
 #pragma unroll
-                for (int p = 0; p < 4; p++) tma_load_4d(sQ + RAW_PANEL_OFF[p], &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
+                for (int p = 0; p < 4; p++) tma_load_4d(sQ + raw_panel_off(p), &tmQ, bar_q_full, p * 32, hk * a.gqa, q0 / a.gqa, b);
             } else {
 #pragma unroll
                 for (int p = 0; p < 2; p++) tma_load_4d(sQ + p * kPanelBytes, &tmQ, bar_q_full, p * 64, hk * a.gqa, q0 / a.gqa, b);
@@ -145,23 +142,8 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
         const uint32_t tmem_S = tmem_base, tmem_P = tmem_base, tmem_O = tmem_base + kTile;   // P as f16x2 over the first 64 columns of S
         if constexpr (RAW) {
             if (warp < 4) {
-                // raw F32 row r (panels of 128-byte swizzled rows) -> F16 row r of the operand tile: HD / 4 loads, HD / 2
-                // conversions, HD / 8 stores per thread, all from shared memory
                 const bool there = mbar_wait(bar_q_full, item & 1, s_abort);
-                const int r = tid;
-                uint4 row[HD / 8];
-#pragma unroll
-                for (int c = 0; c < HD / 8; c++) {   // F16 chunk c = columns 8c .. 8c+7 = F32 chunks 2c, 2c+1 of raw panel c / 4
-                    const int f0 = (2 * c) & 7;
-                    const uint8_t* raw = smem_gen + RAW_PANEL_OFF[c >> 2] + r * 128;
-                    const float4 x0 = *reinterpret_cast<const float4*>(raw + ((f0 ^ (r & 7)) << 4));
-                    const float4 x1 = *reinterpret_cast<const float4*>(raw + (((f0 + 1) ^ (r & 7)) << 4));
-                    row[c] = make_uint4(pack_half2(x0.x, x0.y), pack_half2(x0.z, x0.w), pack_half2(x1.x, x1.y), pack_half2(x1.z, x1.w));
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");   // the operand tile is written over raw columns 64 to 127 of all rows
-#pragma unroll
-                for (int c = 0; c < HD / 8; c++)
-                    *reinterpret_cast<uint4*>(smem_gen + r * 128 + (c >> 3) * kPanelBytes + (((c & 7) ^ (r & 7)) << 4)) = row[c];
+                convert_raw_row(smem_gen, tid);
                 if (there) {
                     fence_proxy_async();   // the operand tile is read, and the V stage is overwritten, through the async proxy
                     __syncwarp();
@@ -211,13 +193,8 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
             // issue order, so PV[j] has consumed P[j] before S[j+1] writes.
             {
                 const uint32_t q_lo = smem_desc_lo(sQ, 16), k_lo = smem_desc_lo(sK, 16), v_lo = smem_desc_lo(sV, kPanelBytes);
-                constexpr uint32_t desc_hi = smem_desc_hi(1024);
                 auto issue_s = [&]() {
-#pragma unroll
-                    for (int ks = 0; ks < HD / 16; ks++) {
-                        const uint32_t off16 = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                        mma_ss(tmem_S, desc64(q_lo + off16, desc_hi), desc64(k_lo + off16, desc_hi), IDESC_S, ks > 0 ? 1u : 0u);
-                    }
+                    issue_scores<HD>(tmem_S, q_lo, k_lo);
                     tc_commit(bar_s_full);
                     tc_commit(bar_k_empty);
                 };
@@ -237,9 +214,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        mma_ts(tmem_O, tmem_P, desc64(v_lo, desc_hi), IDESC_PV, j > 0 ? 1u : 0u);
-#pragma unroll
-                        for (int ks = 1; ks < kTile / 16; ks++) mma_ts(tmem_O, tmem_P + ks * 8, desc64(v_lo + ks * (2048 >> 4), desc_hi), IDESC_PV, 1u);
+                        issue_pv<HD>(tmem_O, tmem_P, v_lo, j == 0);
                         tc_commit(bar_v_empty);
                         if (more) issue_s();
                         if (!more) tc_commit(bar_o_done);
@@ -271,63 +246,16 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                 tc_fence_after();
                 const int n_valid = kend - j * kTile;  // columns >= n_valid of this row are masked
                 const bool full_tile = __all_sync(0xffffffffu, n_valid >= kTile);
-                if (j == 0) {   // a first reference: the maximum of the row's first 32 scores (the check below corrects it)
-                    uint32_t s0[32];
-                    tmem_ld32(tmem_S + lane_base, s0);
-                    tmem_wait_ld();
-                    float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float x0 = (i < n_valid) ? __uint_as_float(s0[i]) : -INFINITY;
-                        const float x1 = (i + 1 < n_valid) ? __uint_as_float(s0[i + 1]) : -INFINITY;
-                        m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], x0, x1);
-                    }
-                    m_ref = max3(fmaxf(m4[0], m4[1]), m4[2], m4[3]) * c;
-                }
+                if (j == 0) m_ref = first_maximum(tmem_S + lane_base, n_valid) * c;
                 uint32_t preg[2][32];
                 float lsum = 0.0f;
                 for (int attempt = 0; attempt < 2; attempt++) {
                     // P = exp2(S*c - m_ref), rounded to f16x2; the tile maximum is tracked in the same pass and
                     // only checked afterwards (lazy rescale).
                     const float m_use = (m_ref == -INFINITY) ? 0.0f : m_ref;
-                    // rolling 32-column chunks: the load of chunk k+2 is issued into the registers chunk k has just
-                    // left and completes under the exponentials of chunk k+1
-                    float mx8[8];
-                    uint64_t ls4[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll
-                    for (int i = 0; i < 8; i++) mx8[i] = -INFINITY;
-                    const uint64_t c2 = pack2(c, c), nm2 = pack2(-m_use, -m_use);
-                    uint32_t sA[32], sB[32];
-                    // a partial tile (the last one, or the diagonal of a causal call) puts -inf into the dead columns
-                    // first and skips chunks that are dead for the whole warp: one copy of the arithmetic serves both
-                    auto chunk = [&](uint32_t (&sx)[32], uint32_t* p16, int col0) {
-                        if (!full_tile) {
-                            if (__all_sync(0xffffffffu, col0 >= n_valid)) {
-#pragma unroll
-                                for (int i = 0; i < 16; i++) p16[i] = 0u;
-                                return;
-                            }
-#pragma unroll
-                            for (int i = 0; i < 32; i++)
-                                if (col0 + i >= n_valid) sx[i] = 0xFF800000u;
-                        }
-                        softmax32(sx, p16, c2, nm2, mx8, ls4);
-                    };
-                    tmem_ld32(tmem_S + lane_base, sA);
-                    tmem_ld32(tmem_S + lane_base + 32, sB);
-                    tmem_wait_ld();
-                    chunk(sA, preg[0], 0);
-                    tmem_ld32(tmem_S + lane_base + 64, sA);
-                    chunk(sB, preg[0] + 16, 32);
-                    tmem_wait_ld();
-                    tmem_ld32(tmem_S + lane_base + 96, sB);
-                    chunk(sA, preg[1], 64);
-                    tmem_wait_ld();
-                    chunk(sB, preg[1] + 16, 96);
-                    const float m_tile = c * fmaxf(max3(fmaxf(mx8[0], mx8[1]), mx8[2], mx8[3]), max3(fmaxf(mx8[4], mx8[5]), mx8[6], mx8[7]));
-                    float l0, l1;
-                    unpack2(add2(add2(ls4[0], ls4[1]), add2(ls4[2], ls4[3])), l0, l1);
-                    lsum = l0 + l1;
+                    float mx;
+                    softmax_tile(tmem_S + lane_base, c, m_use, full_tile, n_valid, preg, mx, lsum, []() {});
+                    const float m_tile = c * mx;
                     const bool grow = m_tile > m_ref + kRescaleThreshold;
                     if (!__any_sync(0xffffffffu, grow)) break;
                     // some row of this warp outgrew its reference maximum: rescale O and l, then redo P
@@ -335,17 +263,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                     const float m_new = fmaxf(m_ref, m_tile);
                     const float alpha = (m_new == -INFINITY) ? 1.0f : ex2(m_ref - m_new);
                     l_run *= alpha;
-                    if (j > 0) {
-#pragma unroll
-                        for (int q4 = 0; q4 < HD / 32; q4++) {
-                            uint32_t oreg[32];
-                            tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i++) oreg[i] = __float_as_uint(__uint_as_float(oreg[i]) * alpha);
-                            tmem_st32(tmem_O + lane_base + q4 * 32, oreg);
-                        }
-                    }
+                    if (j > 0) rescale_o<HD>(tmem_O + lane_base, alpha);
                     m_ref = m_new;
                 }
                 l_run += lsum;
@@ -363,30 +281,7 @@ fattn_prefill_tc5_h128_kernel(const FattnArgs a, const __grid_constant__ CUtenso
                 // completed: they stage O
                 const float inv = row_live && l_run > 0.0f ? 1.0f / l_run : 0.0f;
                 float* stage = reinterpret_cast<float*>(smem_gen + TILE_BYTES) + warp * 32 * HD;
-                // A warp's 32 packed rows x 32 columns are a box [32 columns, gqa heads, 32 / gqa tokens] of
-                // dst [hd, H, Tq, B]; the warp parks them as 128-byte rows with the 16-byte chunks swizzled by the row (the
-                // copy's own pattern, conflict-free for the stores) and one lane hands each panel to a tensor store,
-                // which also clips the tokens beyond Tq.
-#pragma unroll
-                for (int q4 = 0; q4 < HD / 32; q4++) {
-                    uint32_t oreg[32];
-                    tmem_ld32(tmem_O + lane_base + q4 * 32, oreg);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(stage + q4 * 32 * 32 + lane * 32 + (((i >> 2) ^ (lane & 7)) << 2)) =
-                            row_live ? make_float4(__uint_as_float(oreg[i]) * inv, __uint_as_float(oreg[i + 1]) * inv,
-                                                   __uint_as_float(oreg[i + 2]) * inv, __uint_as_float(oreg[i + 3]) * inv)
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0 && q0 + warp * 32 < rows_total) {
-#pragma unroll
-                    for (int q4 = 0; q4 < HD / 32; q4++)
-                        tma_store_4d(&tmO, smem_u32(stage + q4 * 32 * 32), q4 * 32, hk * a.gqa, (q0 + warp * 32) / a.gqa, b);
-                    tma_store_commit_and_wait_read();
-                }
+                store_o_box<HD>(tmO, stage, tmem_O + lane_base, inv, row_live, lane, q0 + warp * 32, rows_total, hk, a.gqa, b);
             }
         }
         return n_tiles;
