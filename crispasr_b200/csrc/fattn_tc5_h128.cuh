@@ -11,6 +11,7 @@
 // 20.6, 16 x 100 15.5 -> 16.2), so are causal ones of long rows with few tiles more (launch_t), and take the other kernel.  (Asked for behind
 // the last copies the answer is waited for: 16 x 750 111.)
 // A kernel of its own because the loop around a tile costs the registers that masks need (2 x 1500 under a mask 148 -> 174).
+
 // Asks the hardware for a block of this grid that has not been launched yet and will not be: the caller does its work (16 bytes at `dst`,
 // announced on `bar`).  Not again after an answer that there is none.
 __device__ __forceinline__ void ask_for_next_block(uint32_t dst, uint32_t bar) {

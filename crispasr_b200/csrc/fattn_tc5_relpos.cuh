@@ -33,13 +33,14 @@
 // operand of the tensor cores, times 1 / scale as an F16 number in an identity matrix, is not that value: rounded as x * scale / d, d being that
 // number, 2.5e-4, 3.2e-4, 3.3e-4, 3.5e-4, growing with the bias, and a NaN reaches the other keys of its product (2 x 7500 frames 645 us).
 //
-// 2 recordings of 7500 frames, bias added by the softmax warps / here: 875 -> 745 us in a burst, 945 -> 835 in a long run at the 1000 W limit; one
-// of 1000 frames 25.0 -> 21.6, 8 utterances of up to 138 13.5 -> 12.8, a mask over 3000 frames 189 -> 135.
+// 2 recordings of 7500 frames, bias added by the softmax warps / here: 873 -> 730 us in a burst, 953 -> 834 in a long run at the 1000 W limit; one
+// of 1000 frames 24.9 -> 21.6, 8 utterances of up to 138 13.0 -> 12.6, a mask over 3000 frames 189 -> 130; of 5 frames 8.5 -> 8.6.
 // What bounds it: 128 x 128 scores take 3.3 k clk, the softmax warps 2.5 k of them (exponentials 1.5 k, where the exponential unit needs 1.0 k;
 // the meeting of the two warps of a row, the P store and the wait for the next scores the rest).  The columns of a score tile are free again 3 k
 // clk after its P is there (P.V, bias, S and three hand-offs), and a block of X, of which a tile takes two, comes 1.5 k clk after the one
 // before it has left its columns.  So the bias of a tile waits for P.V with the next block of X already taken out and its successor on the
-// way (waiting ahead of that block 790, and with a wait of its own for the upper columns, which P leaves earlier, 837).
+// way (745 us before the blocks that nothing needs were left out; waiting ahead of that block 790, and with a wait of its own for the upper
+// columns, which P leaves earlier, 837).
 // Instruction fetch counts: five kinds of warps that each run straight-line code once per tile.
 constexpr int kThreadsRelpos = 512;
 constexpr int kRelBlock = 64;                          // X columns per step
@@ -134,7 +135,7 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
 // its alignment.)  A warp load of 32 rows occupies L1 32 times whatever its width, and what shared memory leaves of L1 does not hold
 // the tile's rows: rows on no 16-byte boundary are read as the nine 16-byte words around them and shifted into place, unless some of those
 // reach beyond the mask [lo, hi) (4 x 1501 frames 307 -> 134 us, 11 utterances of up to 246 frames 47.8 -> 37.3, by 4- and 2-byte loads before; the
-// aligned form as a block of its own 2 x 3000 frames 245 -> 200).
+// aligned form as a block of its own 2 x 3000 frames 245 -> 200; all with the bias as an operand of the tensor cores; now the first takes 145).
 __device__ __forceinline__ void load_mask_row(uint32_t (&mv)[32], const uint8_t* mptr, int avail, int align, const uint8_t* lo, const uint8_t* hi) {
     const uint32_t skew = (uint32_t)reinterpret_cast<uintptr_t>(mptr) & 15u;
     if (align >= 16 && avail >= 64) {

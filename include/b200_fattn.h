@@ -77,6 +77,7 @@ typedef struct b200_fattn_ext {
     /* FastConformer relative-position bias, replacing the materialised F16 mask that
      * src/core/fastconformer.h:880-918 builds (MUL_MAT(R,Q_v) -> rel_shift -> scale -> cast F16):
      *   bias[k,q,h] = f16( scale * sum_c q_v[c,q,h] * r[c, (Tq-1) + k - q, h] )
+     * (beyond the range of F16 an infinity: -inf removes the key; rows of r that only keys at or beyond kv_len reach may hold anything).
      * q_v has the shape and type rules of Q; r is [hd, 2*Tq-1, H, 1|B] F16 or F32. Requires
      * Lk == Tq and either q_v or the two position biases below. May be combined with `mask` (added after the bias) and kv_len. */
     const b200_tensor* q_v;

@@ -696,7 +696,7 @@ def test_cfg5_relpos_with_explicit_masks_on_the_tensor_core_path(b200, orc, T):
 @pytest.mark.parametrize("spread", [1.0, 4.0])
 def test_relpos_edges_of_tiles_and_growing_scores(b200, orc, T, spread):
     """Sizes around the kernel's 64-column blocks and 128-key tiles; keys scaled by 4 make scores outgrow the reference of the
-    running softmax in later tiles (the bias, whose F16 rounding is the kernel's own, stays as it is)."""
+    running softmax in later tiles."""
     rng = np.random.default_rng(461)
     q_u, q_v, k, v, r = _relpos_case(orc, rng, T, H=2, d_model=256)
     k *= np.float32(spread)
@@ -723,7 +723,7 @@ def test_relpos_mask_rows_of_every_alignment(b200, orc, T):
 
 @pytest.mark.parametrize("scale", [2.0 ** -16, 0.04, 0.125, 1.0, 2.0 ** 14])
 def test_relpos_scales(b200, orc, scale):
-    """Scales whose inverse is an F16 number, is not one, or is none within F16's range (the general kernel takes those)."""
+    """Scales that are powers of two, are not, or lie outside the range of the tensor-core kernel (the general kernel takes those)."""
     rng = np.random.default_rng(463)
     q_u, q_v, k, v, r = _relpos_case(orc, rng, 150, H=2, d_model=256)
     f = np.float32(min(1.0, 128 ** -0.5 / scale))   # scores of ordinary size also under a large scale
